@@ -35,8 +35,9 @@ struct fgpu_engine {
     double *field[FGPU_FIELD_COUNT] = {};
     double *sigma_alt = nullptr, *vr_alt = nullptr, *vaz_alt = nullptr, *energy_alt = nullptr;
     double *mom[4] = {};
+    double *mom_t[4] = {};  // pair form: the azimuthal pass's momenta (mom: the radial pass's)
     double *ring_ws = nullptr;
-    int *ring_shift = nullptr;  // the pair azimuthal pass's shift per ring
+    RingPhase *ring_phase = nullptr;  // pair form: the azimuthal pass's constants per ring
     size_t az_smem = 0;
     int az_block = 256;
     bool pair_arith = true;  // the kernels' arithmetic in float pairs (else FP64)
@@ -1013,27 +1014,31 @@ static int create_engine(const fgpu_params *params, const double *radii, cudaStr
     // resident blocks (2048x6144 in float pairs: 0.707 ms with 32 rings, six
     // waves; 0.694 with 33 and 0.683 with 34, five)
     eng->radial_chunk = radial_chunk_for(eng->pair_arith, eng->ph.adiabatic, eng->nr, eng->nz);
-    // azimuthal transport: whole ring in shared memory when it fits
-    {
-        const int per = azimuthal_cells_per_thread(eng->nz);
-        eng->az_block = std::max(128, std::min(512, ((eng->nz + per - 1) / per + 31) / 32 * 32));
-    }
-    if (cudaMalloc(&eng->ring_shift, sizeof(int) * (size_t)eng->nr) != cudaSuccess ||
-        cudaMemsetAsync(eng->ring_shift, 0, sizeof(int) * (size_t)eng->nr, eng->stream) !=
-            cudaSuccess) {
-        eng->err = "out of device memory (ring shifts)";
-        return fail(FGPU_ERR_OOM);
-    }
-    eng->az_smem = azimuthal_smem_bytes(eng->nz);
-    if (eng->az_smem > 220 * 1024) {
-        if (cudaMalloc(&eng->ring_ws, eng->az_smem * (size_t)eng->nr) != cudaSuccess) {
-            eng->err = "out of device memory (ring workspace)";
+    if (eng->pair_arith) {
+        // the float-pair azimuthal pass works out of place
+        for (int k = 0; k < 4; ++k) {
+            if (cudaMalloc(&eng->mom_t[k], eng->cells * sizeof(double)) != cudaSuccess) {
+                eng->err = "out of device memory (momenta)";
+                return fail(FGPU_ERR_OOM);
+            }
+        }
+        if (cudaMalloc(&eng->ring_phase, sizeof(RingPhase) * (size_t)eng->nr) != cudaSuccess) {
+            eng->err = "out of device memory (ring phases)";
             return fail(FGPU_ERR_OOM);
         }
     } else {
-        // the kernel also has static shared memory: opt in for the dynamic size
-        // whatever it is
-        if (prepare_azimuthal(eng->az_smem) != cudaSuccess) {
+        // FP64 azimuthal transport: whole ring in shared memory when it fits
+        const int per = azimuthal_cells_per_thread(eng->nz);
+        eng->az_block = std::max(128, std::min(512, ((eng->nz + per - 1) / per + 31) / 32 * 32));
+        eng->az_smem = azimuthal_smem_bytes(eng->nz);
+        if (eng->az_smem > 220 * 1024) {
+            if (cudaMalloc(&eng->ring_ws, eng->az_smem * (size_t)eng->nr) != cudaSuccess) {
+                eng->err = "out of device memory (ring workspace)";
+                return fail(FGPU_ERR_OOM);
+            }
+        } else if (prepare_azimuthal(eng->az_smem) != cudaSuccess) {
+            // the kernel also has static shared memory: opt in for the
+            // dynamic size whatever it is
             eng->err = "cannot reserve shared memory for the azimuthal kernel";
             return fail(FGPU_ERR_CUDA);
         }
@@ -1059,8 +1064,11 @@ extern "C" int fgpu_destroy(fgpu_engine *eng)
     for (auto ev : eng->ev_free) cudaEventDestroy(ev);
     for (int f = 0; f < FGPU_FIELD_COUNT; ++f) cudaFree(eng->field[f]);
     cudaFree(eng->sigma_alt); cudaFree(eng->vr_alt); cudaFree(eng->vaz_alt); cudaFree(eng->energy_alt);
-    for (int k = 0; k < 4; ++k) cudaFree(eng->mom[k]);
-    cudaFree(eng->ring_ws); cudaFree(eng->ring_shift); cudaFree(eng->tables_mem);
+    for (int k = 0; k < 4; ++k) {
+        cudaFree(eng->mom[k]);
+        cudaFree(eng->mom_t[k]);
+    }
+    cudaFree(eng->ring_ws); cudaFree(eng->ring_phase); cudaFree(eng->tables_mem);
     cudaFree(eng->damp_mem);
     cudaFree(eng->damp_rings); cudaFree(eng->partial); cudaFree(eng->red_out);
     cudaFree(eng->pair_mem);
@@ -1647,13 +1655,26 @@ static void transport(fgpu_engine *eng, double dt)
     double **f = eng->field;
     State s = state_of(eng);
     launch_transport_radial(L, dt, omf, eng->radial_chunk, s.sigma, s.vr, s.vaz, s.energy,
-                            eng->mom, eng->energy_alt, eng->sigma_alt);
+                            eng->mom, eng->energy_alt, eng->sigma_alt, eng->ring_phase);
     mark(eng, 7);
-    launch_transport_azimuthal(L, dt, eng->az_block, eng->mom, eng->energy_alt, eng->sigma_alt,
-                               s.vaz, eng->ring_ws, eng->az_smem, eng->ring_shift);
-    mark(eng, 8);
-    launch_finish(L, omf, eng->mom, eng->sigma_alt, eng->energy_alt, s.vr, eng->vr_alt,
-                  eng->vaz_alt, s.sigma, s.energy, eng->ring_shift);
+    if (L.pair) {
+        // out of place: into the state's sigma and energy, which the radial
+        // pass was the last to read; the rebuild writes back to the others
+        launch_transport_azimuthal_pair(L, eng->mom, eng->energy_alt, eng->sigma_alt, s.vaz,
+                                        eng->mom_t, s.energy, s.sigma, eng->ring_phase);
+        mark(eng, 8);
+        launch_finish(L, omf, eng->mom_t, s.sigma, s.energy, s.vr, eng->vr_alt, eng->vaz_alt,
+                      eng->sigma_alt, eng->energy_alt, eng->ring_phase);
+        std::swap(f[FGPU_SIGMA], eng->sigma_alt);
+        // the isothermal step leaves the energy field alone
+        if (eng->ph.adiabatic) std::swap(f[FGPU_ENERGY], eng->energy_alt);
+    } else {
+        launch_transport_azimuthal(L, dt, eng->az_block, eng->mom, eng->energy_alt,
+                                   eng->sigma_alt, s.vaz, eng->ring_ws, eng->az_smem);
+        mark(eng, 8);
+        launch_finish(L, omf, eng->mom, eng->sigma_alt, eng->energy_alt, s.vr, eng->vr_alt,
+                      eng->vaz_alt, s.sigma, s.energy, nullptr);
+    }
     std::swap(f[FGPU_V_RADIAL], eng->vr_alt);
     std::swap(f[FGPU_V_AZIMUTHAL], eng->vaz_alt);
     mark(eng, 9);

@@ -199,9 +199,95 @@ __device__ __forceinline__ f2 f2_sdiv(f2 p, f2 s)
 {
     const float r = rcp_approx(s.h);
     const float q = __fmul_rn(p.h, r);
-    const f2 qs = two_prod(q, s.h);
-    const float d = __fmaf_rn(-q, s.l, __fadd_rn(__fsub_rn(__fsub_rn(p.h, qs.h), qs.l), p.l));
+    // p.h - q s.h in one rounding (q s.h is within a few ulps of p.h)
+    const float d = __fmaf_rn(-q, s.l, __fadd_rn(__fmaf_rn(-q, s.h, p.h), p.l));
     return fast_two_sum(q, __fmul_rn(d, r));
+}
+
+// ---------------------------------------------------------------------------
+// Two pairs at a time: every operation is the packed FP32 instruction of the
+// two values (add, mul, fma .rn.f32x2), which rounds each as the scalar one
+// does, so a packed operation gives the bits of the scalar functions above.
+// GB300's FP32 pipe takes a packed instruction for two cycles (measured: 120
+// results per clock per SM packed, 119 scalar), so packing does not speed the
+// arithmetic itself; it halves the issue slots it takes, which the loads,
+// selects and integer conversions around it need.
+// ---------------------------------------------------------------------------
+struct f2x2 {
+    float2 h, l;
+};
+
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 vneg(float2 a) { return make_float2(-a.x, -a.y); }
+// a - b (the product by -1 is exact)
+__device__ __forceinline__ float2 vsub(float2 a, float2 b)
+{
+    return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+}
+__device__ __forceinline__ float2 vrcp(float2 a)
+{
+    return make_float2(rcp_approx(a.x), rcp_approx(a.y));
+}
+
+__device__ __forceinline__ f2x2 pack(f2 a, f2 b)
+{
+    return f2x2{make_float2(a.h, b.h), make_float2(a.l, b.l)};
+}
+__device__ __forceinline__ f2x2 pack(f2 a) { return pack(a, a); }
+__device__ __forceinline__ f2 first(f2x2 a) { return f2{a.h.x, a.l.x}; }
+__device__ __forceinline__ f2 second(f2x2 a) { return f2{a.h.y, a.l.y}; }
+
+__device__ __forceinline__ f2x2 fast_two_sum(float2 a, float2 b)
+{
+    const float2 s = vadd(a, b);
+    return f2x2{s, vsub(b, vsub(s, a))};
+}
+__device__ __forceinline__ f2x2 two_sum(float2 a, float2 b)
+{
+    const float2 s = vadd(a, b);
+    const float2 bb = vsub(s, a);
+    return f2x2{s, vadd(vsub(a, vsub(s, bb)), vsub(b, bb))};
+}
+__device__ __forceinline__ f2x2 two_prod(float2 a, float2 b)
+{
+    const float2 p = vmul(a, b);
+    return f2x2{p, vfma(a, b, vneg(p))};
+}
+__device__ __forceinline__ f2x2 f2_neg(f2x2 x) { return f2x2{vneg(x.h), vneg(x.l)}; }
+__device__ __forceinline__ f2x2 f2_sadd(f2x2 x, f2x2 y)
+{
+    const f2x2 s = two_sum(x.h, y.h);
+    return fast_two_sum(s.h, vadd(s.l, vadd(x.l, y.l)));
+}
+__device__ __forceinline__ f2x2 f2_ssub(f2x2 x, f2x2 y)
+{
+    // two_sum of x.h and -y.h with the signs carried by the subtractions
+    const float2 s = vsub(x.h, y.h);
+    const float2 bb = vsub(s, x.h);
+    const float2 e = vsub(vsub(x.h, vsub(s, bb)), vadd(y.h, bb));
+    return fast_two_sum(s, vadd(e, vsub(x.l, y.l)));
+}
+__device__ __forceinline__ f2x2 f2_smul(f2x2 x, f2x2 y)
+{
+    const f2x2 c = two_prod(x.h, y.h);
+    return fast_two_sum(c.h, vadd(c.l, vfma(x.l, y.h, vmul(x.h, y.l))));
+}
+__device__ __forceinline__ f2x2 f2_sfma(f2x2 x, f2x2 a, f2x2 d)
+{
+    const f2x2 p = two_prod(a.h, d.h);
+    const float2 pl = vfma(a.l, d.h, vfma(a.h, d.l, p.l));
+    const f2x2 s = two_sum(x.h, p.h);
+    return fast_two_sum(s.h, vadd(s.l, vadd(x.l, pl)));
+}
+__device__ __forceinline__ f2x2 f2_sdiv(f2x2 p, f2x2 s)
+{
+    const float2 r = vrcp(s.h);
+    const float2 q = vmul(p.h, r);
+    const float2 nq = vneg(q);
+    const float2 d = vfma(nq, s.l, vadd(vfma(nq, s.h, p.h), p.l));
+    return fast_two_sum(q, vmul(d, r));
 }
 
 }  // namespace fgpu

@@ -21,6 +21,18 @@ struct Launch {
     bool pair = false;
 };
 
+// Constants of one ring's azimuthal passes (pair form), from its mean v_phi
+// (ComputeConstantResidual, TransportEuler.cpp:207-236): the velocity the
+// residual is about; as pairs k dt, the flux factor dxrad / (Surf k dt), the
+// uniform pass's interpolation distance and flux factor (k = 1 / dx for van
+// Leer, 1 / (2 dx) for MC: the slopes carry no constant factor); the integer
+// shift, in [0, nz); whether the uniform velocity is positive.
+struct RingPhase {
+    double about;
+    float2 kdt, face, au, fu;
+    int shift, upwind;
+};
+
 void launch_potential(const Launch &L, const Bodies &b, const double *H, double *pot);
 void launch_source(const Launch &L, double dt, double omf, const double *S, const double *P,
                    const double *pot, const double *vr_in, const double *vaz_in, double *vr_out,
@@ -41,22 +53,29 @@ void launch_cfl_cells(const Launch &L, const State &s, double *out);
 void launch_com_damping(const Launch &L, const ComSpec &c, double dt, const State &s);
 // rings per radial sweep chunk for this device and disk
 int radial_chunk_for(bool pair, bool adiabatic, int nr, int nz);
+// pair form: also the ring phases of the azimuthal pass, from vaz
 void launch_transport_radial(const Launch &L, double dt, double omf, int chunk, const double *S,
                              const double *vr, const double *vaz, const double *E,
-                             double *const mom[4], double *E_out, double *S_out);
+                             double *const mom[4], double *E_out, double *S_out,
+                             RingPhase *phase);
+// the FP64-arithmetic azimuthal pass, in place (AdvectSHIFT included)
 size_t azimuthal_smem_bytes(int nz);
 int azimuthal_cells_per_thread(int nz);
 cudaError_t prepare_azimuthal(size_t smem);
-// block: threads of the FP64 kernel (the pair kernel chooses its own)
-// ring_shift (nr ints): the pair kernel leaves AdvectSHIFT to the velocity
-// rebuild and writes each ring's shift there
 void launch_transport_azimuthal(const Launch &L, double dt, int block, double *const mom[4],
                                 double *E, double *S, const double *vaz, double *ring_ws,
-                                size_t smem, int *ring_shift);
-// ring_shift: the azimuthal shifts the pair rebuild applies (pair form)
+                                size_t smem);
+// the float-pair azimuthal pass (kernels_azimuthal.cu): momenta as float
+// pairs, into buffers other than its inputs; AdvectSHIFT is left to the
+// velocity rebuild
+void launch_transport_azimuthal_pair(const Launch &L, double *const mom[4], const double *E,
+                                     const double *S, const double *vaz,
+                                     double *const mom_out[4], double *E_out, double *S_out,
+                                     const RingPhase *phase);
+// phase: the azimuthal shifts the pair rebuild applies (pair form)
 void launch_finish(const Launch &L, double omf, double *const mom[4], const double *S_t,
                    const double *E_t, const double *vr_in, double *vr_out, double *vaz_out,
-                   double *S_out, double *E_out, const int *ring_shift);
+                   double *S_out, double *E_out, const RingPhase *phase);
 void launch_damping(const Launch &L, const Damping &dm, double dt, const int *rings, int nrings,
                     const State &s);
 void launch_derived_cfl(const Launch &L, int mode, const State &s, unsigned long long *dt_min);
@@ -84,7 +103,7 @@ inline bool stress_as_pairs(const Launch &L) { return L.pair && L.ph.stabilize !
 void launch_join_pairs(cudaStream_t stream, double *x, size_t n);
 void launch_finish_pair(const Launch &L, double omf, double *const mom[4], const double *S_t,
                         const double *E_t, const double *vr_in, double *vr_out, double *vaz_out,
-                        double *S_out, double *E_out, const int *ring_shift);
+                        double *S_out, double *E_out, const RingPhase *phase);
 // bodies one disk-force pass handles
 constexpr int kForceBodies = 4;
 

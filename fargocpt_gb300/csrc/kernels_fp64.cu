@@ -973,10 +973,10 @@ __device__ __forceinline__ void radial_sweep_f2(const Geo &g, const Tables &t, d
                                                 const double *__restrict__ vr,
                                                 const double *__restrict__ vaz,
                                                 const double *__restrict__ E,
-                                                double *__restrict__ mom0,
-                                                double *__restrict__ mom1,
-                                                double *__restrict__ mom2,
-                                                double *__restrict__ mom3,
+                                                f2 *__restrict__ mom0,
+                                                f2 *__restrict__ mom1,
+                                                f2 *__restrict__ mom2,
+                                                f2 *__restrict__ mom3,
                                                 double *__restrict__ E_out,
                                                 double *__restrict__ S_out)
 {
@@ -987,7 +987,7 @@ __device__ __forceinline__ void radial_sweep_f2(const Geo &g, const Tables &t, d
     const int i1 = min(i0 + chunk, nr);
     const double dtdphi = dt * g.dphi;
     const f2 zero{0.f, 0.f};
-    double *const outq[5] = {mom0, mom1, mom2, mom3, E_out};
+    f2 *const outq[4] = {mom0, mom1, mom2, mom3};
 
     // rolling state as in k_transport_radial: rings k-1 (wa, da), k (wb, db,
     // ub: its upward difference) and k+1 (wn)
@@ -1067,7 +1067,7 @@ __device__ __forceinline__ void radial_sweep_f2(const Geo &g, const Tables &t, d
             for (int s = 0; s < NW; ++s) {
                 const f2 dq = f2_smul(f2_ssub(flux_prev[s], flux[s]), invs);
                 if (s < 4 && s < NH)
-                    outq[s][c] = f2_to_double(f2_sadd(f2_smul(wa[NH], wa[s]), dq));
+                    outq[s][c] = f2_sadd(f2_smul(wa[NH], wa[s]), dq);
                 else if (s == 4 && NQ == 5) E_out[c] = E[c] + f2_to_double(dq);
                 else S_out[c] = S[c] + f2_to_double(dq);
             }
@@ -1096,17 +1096,74 @@ __device__ __forceinline__ void radial_sweep_f2(const Geo &g, const Tables &t, d
     }
 }
 
+// The azimuthal pass's constants of ring i from its mean v_phi, by the 64
+// threads of a block (compute_average_azimuthal_velocity :174-189,
+// ComputeConstantResidual :207-236; the shift phase in FP64)
+__device__ void ring_phase(const Geo &g, const Tables &t, double dt, double invdt, double inv_nz,
+                           int mc, int fast, const double *__restrict__ vaz, int i, RingPhase *out)
+{
+    __shared__ double half;
+    const int nz = g.nz;
+    const double *v = vaz + (size_t)i * nz;
+    // four sums per thread: four loads in flight
+    double p0 = 0.0, p1 = 0.0, p2 = 0.0, p3 = 0.0;
+    int j = threadIdx.x;
+    for (; j + 192 < nz; j += 256) {
+        p0 += v[j];
+        p1 += v[j + 64];
+        p2 += v[j + 128];
+        p3 += v[j + 192];
+    }
+    for (; j < nz; j += 64) p0 += v[j];
+    double s = (p0 + p1) + (p2 + p3);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 32) half = s;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const double vmean = (s + half) * inv_nz;
+    const double Ntilde = vmean * t.InvRmed[i] * dt * g.invdphi;
+    const double Nround = floor(Ntilde + 0.5);
+    const double phase = Ntilde - Nround;  // of the uniform velocity, in cells
+    const int n = (int)Nround;
+    const double h = mc ? 0.5 : 1.0, dx = g.dphi * t.Rmed[i];
+    const double face = (t.Rsup[i] - t.Rinf[i]) * t.InvSurf[i] * dx * (mc ? 2.0 : 1.0);
+    auto pr = [](double x) {
+        const f2 p = f2_split(x);
+        return make_float2(p.h, p.l);
+    };
+    RingPhase r;
+    // without FARGO the residual keeps the uniform velocity
+    r.about = fast ? vmean : vmean - phase * dx * invdt;
+    r.kdt = pr(h * t.InvDxTheta[i] * dt);
+    r.face = pr(face);
+    r.au = pr(phase > 0.0 ? h - h * phase : -(h + h * phase));
+    r.fu = pr(face * (h * phase));
+    r.shift = ((n % nz) + nz) % nz;
+    r.upwind = phase > 0.0;
+    out[i] = r;
+}
+
 // 64-thread blocks, 8 per SM: 128 registers (84 bytes of spills, to L1,
 // which this kernel leaves unshared).  Measured on the 2048 x 6144 disk,
 // ms per pass: 0.708 at 128 registers, 0.761 at 156 (no spills), 0.780 at 96.
 template <int NQ>
 __global__ void __launch_bounds__(64, 8) k_transport_radial_f2(Geo g, Tables t, double dt, double omf, int mc, int chunk,
+                                      int chunks, int fast, double invdt, double inv_nz,
+                                      RingPhase *__restrict__ phase,
                                       const double *__restrict__ S, const double *__restrict__ vr,
                                       const double *__restrict__ vaz, const double *__restrict__ E,
-                                      double *__restrict__ mom0, double *__restrict__ mom1,
-                                      double *__restrict__ mom2, double *__restrict__ mom3,
+                                      f2 *__restrict__ mom0, f2 *__restrict__ mom1,
+                                      f2 *__restrict__ mom2, f2 *__restrict__ mom3,
                                       double *__restrict__ E_out, double *__restrict__ S_out)
 {
+    // blocks past the chunks form the ring phases: latency-bound sums beside
+    // the arithmetic-bound sweep, instead of a launch or a block-wide
+    // reduction in the azimuthal pass
+    if ((int)blockIdx.y >= chunks) {
+        const int i = (blockIdx.y - chunks) * gridDim.x + blockIdx.x;
+        if (i < g.nr) ring_phase(g, t, dt, invdt, inv_nz, mc, fast, vaz, i, phase);
+        return;
+    }
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= g.nz) return;
     radial_sweep_f2<NQ>(g, t, dt, omf, mc, chunk, j, S, vr, vaz, E, mom0, mom1, mom2, mom3,
@@ -1386,308 +1443,6 @@ __global__ void __launch_bounds__(512) k_transport_azimuthal(Geo g, Tables t, do
         }
         __syncthreads();
     }
-}
-
-// ---------------------------------------------------------------------------
-// The same azimuthal transport with its arithmetic in float pairs
-// (fp64_pair.cuh).  The ring pass above is bound by GB300's FP64 pipe (about
-// 1.6 FP64 results per clock per SM against about 113 FP32); here every
-// slope, star value and flux is formed in pair arithmetic (48 significant
-// bits, errors within a few 2^-47 of the operands), the doubles are split and
-// joined on the integer pipe, and FP64 is kept for the state: each quantity's
-// update Q += F_j - F_j+1 adds the pair flux difference, joined into a
-// double, to the FP64 value, so what a step loses is the pair's rounding of
-// the fluxes, not of the state.  The upwind choice and the interpolation
-// distance come from the FP64 velocity as before; the ring mean and the FARGO
-// shift phase stay in FP64.
-//
-// Layout as in the FP64 pass (4 x naz x 8 bytes of shared memory, or the
-// per-ring global workspace): the sigma pair, the specific quantity, the
-// slopes and the fluxes, each a pair.  Sigma's FP64 values are updated in
-// place in its global row (the block owns the ring), the transported
-// quantities in theirs, and AdvectSHIFT stages each row through shared
-// memory.
-// ---------------------------------------------------------------------------
-// One QuantitiesAdvection pass (TransportEuler.cpp:292-304) in pairs.  SP
-// holds sigma's pair, Sg its FP64 row; both advance.  v[n] is the owned
-// cells' FP64 velocity (ignored when uniform).
-//
-// Each face forms the limited slope of its upwind cell itself, from that
-// cell and its two neighbours, instead of reading a slope array: every
-// cell's slope is still formed once per face that uses it (van Leer's
-// upwind cell of face j is j - 1 or j), the slope array and its barrier
-// go, and shared memory holds the face factors in their place, so that a
-// thread keeps only its faces' interpolation distances in registers.
-//
-// The four ring arrays carry the periodic neighbours as halo cells: index -2
-// and -1 hold cells nz - 2 and nz - 1, index nz holds cell 0, written by the
-// owners of those cells with the cell itself, so that no index wraps.
-// EXACT (nz == PER blockDim.x): every thread owns PER cells; otherwise the
-// loops compute with the index clamped into the ring and guard only their
-// stores.  Either way the loop bodies have no branch.
-// The quantity rows, chosen by a select chain: an indexed array of their
-// pointers would sit in local memory and put a load before every row access.
-struct QRows {
-    double *r0, *r1, *r2, *r3, *r4;
-    __device__ __forceinline__ double *operator[](int q) const
-    {
-        return q == 0 ? r0 : q == 1 ? r1 : q == 2 ? r2 : q == 3 ? r3 : r4;
-    }
-};
-
-// The face fluxes of an exact ring with whole warps (SHFL): each cell's
-// update F[j] - F[j + 1] takes the right neighbour's flux from the next lane
-// by a shuffle, so no flux array exists.  Its shared memory holds instead
-// the quantity's FP64 value of each cell, read from global memory once per
-// quantity and pass (the specific value and the update both use it).  Lane
-// 31's right neighbour is lane 0 of the next warp (of the next slot after
-// the last warp, cell 0 after the last cell): lane 0 publishes its flux, lane
-// 31 its flux and value, and after the quantity's closing barrier threads
-// 0 .. K - 1 (K = PER x warps, one per lane-31 cell) complete those updates.
-// The exchange buffers alternate with the quantity, so that the next
-// quantity's writes never meet this one's deferred reads.
-template <int K>
-struct PairEdges {
-    f2 first[2][K];   // lane 0's flux, slot-major: n x warps + warp
-    f2 last[2][K];    // lane 31's flux
-    double val[2][K]; // lane 31's quantity value
-};
-
-template <int PER, int NQ, bool EXACT, bool SHFL, int K>
-__device__ void ring_advection_pass_f2(double *Sg, f2 *SP, f2 *W, f2 *CF, f2 *F,
-                                       PairEdges<K> &xe, const QRows &qrow, const double *v,
-                                       double dt, double dxtheta, double half_invdx,
-                                       double dxrad_invsurf, int nz, int mc, bool uniform,
-                                       double vconst)
-{
-    static_assert(!SHFL || EXACT, "the shuffled fluxes need an exact ring");
-    const int tid = threadIdx.x, bs = blockDim.x;
-    // the slopes carry no constant factor; the distance does (as in
-    // ring_advection_pass): k (dx - v dt) or -k (dx + v dt), k = 1 / dx
-    // (van Leer) or 1 / (2 dx) (MC)
-    const double kfac = mc ? half_invdx : 2.0 * half_invdx;
-    const double kdt = kfac * dt;
-    const double dxk = dxtheta * kfac;
-    const f2 cvel = f2_split(dxrad_invsurf / kdt);
-    f2 am[PER];
-    unsigned pos = 0;  // bit n: the upwind cell of face tid + n bs is its left neighbour
-    auto cell = [&](int n) { return EXACT ? tid + n * bs : min(tid + n * bs, nz - 1); };
-    auto owned = [&](int n) { return EXACT || tid + n * bs < nz; };
-    // X[j] and its halo copy (cells nz - 2, nz - 1 at -2, -1; cell 0 at nz);
-    // n is the compile-time cell slot of j, so that in an exact ring only the
-    // first and last slots test for the halo
-    auto put = [&](f2 *X, int j, f2 x, int n) {
-        X[j] = x;
-        if (EXACT) {
-            if (n == 0 && tid == 0) X[nz] = x;
-            if (n == PER - 1 && tid >= bs - 2) X[j - nz] = x;
-        } else {
-            if (j >= nz - 2) X[j - nz] = x;
-            if (j == 0) X[nz] = x;
-        }
-    };
-    // the star value at a face of the quantity X from its upwind cell u
-    // (u in -1 .. nz - 1)
-    auto star = [&](const f2 *X, int u, f2 a) {
-        const f2 x = X[u];
-        const f2 d = lim_f2(f2_ssub(X[u + 1], x), f2_ssub(x, X[u - 1]), mc);
-        return f2_sfma(x, a, d);
-    };
-    // DensityStar and the face factor dxrad S* v / Surf every flux shares
-    const double vu = vconst * kdt;
-    const bool pu = positive(vu);
-    const f2 au = f2_split(pu ? dxk - vu : -(dxk + vu));
-#pragma unroll
-    for (int n = 0; n < PER; ++n) {
-        const int j = cell(n);
-        const double vk = uniform ? vu : v[n] * kdt;
-        const bool p = positive(vk);
-        am[n] = uniform ? au : f2_split(p ? dxk - vk : -(dxk + vk));
-        pos |= (unsigned)p << n;
-        const f2 c = f2_smul(f2_smul(cvel, star(SP, p ? j - 1 : j, am[n])), f2_split(vk));
-        if (owned(n)) put(CF, j, c, n);
-    }
-    if constexpr (SHFL) {
-        double *Qs = reinterpret_cast<double *>(F);
-        const int lane = tid & 31, w = tid >> 5, nw = bs >> 5, kk = PER * nw;
-        // the lane-31 cells' updates of quantity q (slot n, warp ww: cell
-        // n bs + 32 ww + 31; the next entry is its right neighbour's lane 0)
-        auto complete = [&](int q) {
-            if (tid < kk) {
-                const int b = q & 1, nx = tid + 1 == kk ? 0 : tid + 1;
-                const int n = tid / nw, ww = tid - n * nw;
-                qrow[q][n * bs + 32 * ww + 31] =
-                    xe.val[b][tid] + f2_to_double(f2_ssub(xe.last[b][tid], xe.first[b][nx]));
-            }
-        };
-#pragma unroll 1
-        for (int q = 0; q < NQ; ++q) {
-            if (q > 0) complete(q - 1);
-            double *Q = qrow[q];
-            const int b = q & 1;
-#pragma unroll
-            for (int n = 0; n < PER; ++n) {
-                const int j = tid + n * bs;
-                const double x = Q[j];
-                Qs[j] = x;
-                if (lane == 31) xe.val[b][n * nw + w] = x;
-                put(W, j, f2_sdiv(f2_split(x), SP[j]), n);
-            }
-            __syncthreads();
-#pragma unroll
-            for (int n = 0; n < PER; ++n) {
-                const int j = tid + n * bs;
-                const f2 f = f2_smul(star(W, (pos >> n) & 1u ? j - 1 : j, am[n]), CF[j]);
-                const f2 fr{__shfl_down_sync(0xffffffffu, f.h, 1),
-                            __shfl_down_sync(0xffffffffu, f.l, 1)};
-                if (lane == 0) xe.first[b][n * nw + w] = f;
-                if (lane == 31) xe.last[b][n * nw + w] = f;
-                const double qn = Qs[j] + f2_to_double(f2_ssub(f, fr));
-                if (lane != 31) Q[j] = qn;
-            }
-            __syncthreads();
-        }
-        if (NQ > 0) complete(NQ - 1);
-    } else {
-    // per quantity: specific values (with the previous quantity's update),
-    // then the fluxes
-#pragma unroll 1
-    for (int q = 0; q <= NQ; ++q) {
-#pragma unroll
-        for (int n = 0; n < PER; ++n) {
-            const int j = cell(n);
-            if (q > 0) {
-                double *Qp = qrow[q - 1];
-                const double qn = Qp[j] + f2_to_double(f2_ssub(F[j], F[j + 1]));
-                if (owned(n)) Qp[j] = qn;
-            }
-            if (q < NQ) {
-                const f2 w = f2_sdiv(f2_split(qrow[q][j]), SP[j]);
-                if (owned(n)) put(W, j, w, n);
-            }
-        }
-        if (q == NQ) break;
-        __syncthreads();
-#pragma unroll
-        for (int n = 0; n < PER; ++n) {
-            const int j = cell(n);
-            const f2 f = f2_smul(star(W, (pos >> n) & 1u ? j - 1 : j, am[n]), CF[j]);
-            if (owned(n)) put(F, j, f, n);
-        }
-        __syncthreads();
-    }
-    }
-    // sigma: QRStar == 1, the flux is the face factor itself (CF is
-    // complete: the barriers of the quantities, or this one when there are
-    // none, separate its writes from these reads)
-    if (NQ == 0) __syncthreads();
-#pragma unroll
-    for (int n = 0; n < PER; ++n) {
-        const int j = cell(n);
-        // nothing reads SP in this phase
-        const double s = Sg[j] + f2_to_double(f2_ssub(CF[j], CF[j + 1]));
-        const f2 sp = f2_split(s);
-        if (owned(n)) {
-            Sg[j] = s;
-            put(SP, j, sp, n);
-        }
-    }
-    __syncthreads();
-}
-
-// Shared memory of the pair kernel per ring: four arrays of nz + 4 pairs
-// (two halo cells on either side)
-__host__ __device__ constexpr size_t pair_ring_f2s(int nz) { return (size_t)4 * (nz + 4); }
-
-// WS: the ring's arrays in the per-ring global workspace (rings beyond the
-// shared memory), else in shared memory
-// The integer shift of AdvectSHIFT is not applied here: ring_shift[i]
-// receives it (in [0, nz)), and the velocity rebuild (k_finish_p) reads each
-// ring's transported cells at their shifted places.
-template <int PER, int MAXT, int NQ, bool WS, bool EXACT>
-__global__ void __launch_bounds__(MAXT) k_transport_azimuthal_f2(
-    Geo g, Tables t, double dt, int mc, int fast, const double *__restrict__ vaz, double *mom0,
-    double *mom1, double *mom2, double *mom3, double *E, double *S, double *ring_ws,
-    int *__restrict__ ring_shift)
-{
-    // the shuffled fluxes on exact rings of up to 6 cells per thread (their
-    // exchange buffers, 9 KB at 6 x 1024, fit beside the ring's arrays)
-    constexpr bool SHFL = EXACT && !WS && PER <= 6;
-    constexpr int K = SHFL ? PER * (MAXT / 32) : 1;
-    extern __shared__ double smem[];
-    __shared__ double red[33];
-    __shared__ PairEdges<K> xe;
-    const int nz = g.nz;
-    const int i = blockIdx.x;
-    const int tid = threadIdx.x, bs = blockDim.x;
-    const size_t row = (size_t)i * nz;
-    f2 *base = WS ? reinterpret_cast<f2 *>(ring_ws) + (size_t)i * pair_ring_f2s(nz)
-                  : reinterpret_cast<f2 *>(smem);
-    f2 *SP = base + 2, *W = SP + (nz + 4), *CF = W + (nz + 4), *F = CF + (nz + 4);
-    double *Sg = S + row;
-    auto owned = [&](int n) { return EXACT || tid + n * bs < nz; };
-    // the ring's transported rows come from DRAM (the radial pass wrote the
-    // whole disk since): ask L2 for all of them now, so that their reads in
-    // the first pass, one quantity after the other, find them there
-    {
-        const int lines = (nz + 15) >> 4;  // 128-byte lines of a row
-        const double *rows[6] = {Sg, mom0 + row, mom1 + row, mom2 + row, mom3 + row, E + row};
-#pragma unroll
-        for (int r = 0; r < 6; ++r) {
-            if (r == 5 && NQ < 5) break;
-            for (int l = tid; l < lines; l += bs)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(rows[r] + min(16 * l, nz - 1)));
-        }
-    }
-
-    // compute_average_azimuthal_velocity, :174-189
-    double vown[PER];
-    double part = 0.0;
-#pragma unroll
-    for (int n = 0; n < PER; ++n) {
-        const int j = tid + n * bs;
-        if (owned(n)) {
-            vown[n] = vaz[row + j];
-            part += vown[n];
-        }
-    }
-    const double vmean = block_sum(part, red) / (double)nz;
-    // ComputeConstantResidual, :207-236: FP64 shift phase of the ring
-    const double Ntilde = vmean * t.InvRmed[i] * dt * g.invdphi;
-    const double Nround = floor(Ntilde + 0.5);
-    const int nshift = (int)Nround;
-    const double invdt = 1.0 / dt;
-    const double vt = (Ntilde - Nround) * t.Rmed[i] * invdt * g.dphi;
-#pragma unroll
-    for (int n = 0; n < PER; ++n) {
-        const int j = tid + n * bs;
-        if (owned(n)) {
-            double vres = vown[n] - vmean;
-            if (!fast) vres = vt + vres;
-            vown[n] = vres;
-            const f2 sp = f2_split(Sg[j]);
-            SP[j] = sp;
-            if (j >= nz - 2) SP[j - nz] = sp;
-            if (j == 0) SP[nz] = sp;
-        }
-    }
-    __syncthreads();
-
-    const QRows qrow{mom0 + row, mom1 + row, mom2 + row, mom3 + row, E + row};
-    const double dxtheta = g.dphi * t.Rmed[i];
-    const double half_invdx = 0.5 * (1.0 / dxtheta);
-    const double dxrad = (t.Rsup[i] - t.Rinf[i]) * dt;
-    const double invsurf = t.InvSurf[i];
-    ring_advection_pass_f2<PER, NQ, EXACT, SHFL>(Sg, SP, W, CF, F, xe, qrow, vown, dt, dxtheta,
-                                                 half_invdx, dxrad * invsurf, nz, mc, false, 0.0);
-    if (fast) {
-        ring_advection_pass_f2<PER, NQ, EXACT, SHFL>(Sg, SP, W, CF, F, xe, qrow, vown, dt,
-                                                     dxtheta, half_invdx, dxrad * invsurf, nz,
-                                                     mc, true, vt);
-    }
-    // AdvectSHIFT (:238-268) is the rebuild's: it reads cell j of this ring
-    // from cell j - nshift
-    if (threadIdx.x == 0) ring_shift[i] = ((nshift % nz) + nz) % nz;
 }
 
 // ---------------------------------------------------------------------------
@@ -2546,21 +2301,28 @@ int radial_chunk_for(bool pair, bool adiabatic, int nr, int nz)
 
 void launch_transport_radial(const Launch &L, double dt, double omf, int chunk, const double *S,
                              const double *vr, const double *vaz, const double *E,
-                             double *const mom[4], double *E_out, double *S_out)
+                             double *const mom[4], double *E_out, double *S_out,
+                             RingPhase *phase)
 {
     const bool pair = L.pair;
     const int chunks = (L.g.nr + chunk - 1) / chunk;
     const int bx = 64;
     dim3 grid((L.g.nz + bx - 1) / bx, chunks);
     if (pair) {
+        // the momenta stay pairs up to the velocity rebuild
+        grid.y += (L.g.nr + grid.x - 1) / grid.x;
+        f2 *pm[4];
+        for (int q = 0; q < 4; ++q) pm[q] = reinterpret_cast<f2 *>(mom[q]);
         if (L.ph.adiabatic) {
             k_transport_radial_f2<5><<<grid, bx, 0, L.stream>>>(
-                L.g, L.t, dt, omf, L.ph.limiter_mc, chunk, S, vr, vaz, E, mom[0], mom[1], mom[2],
-                mom[3], E_out, S_out);
+                L.g, L.t, dt, omf, L.ph.limiter_mc, chunk, chunks, L.ph.fast_transport, 1.0 / dt,
+                1.0 / L.g.nz, phase, S, vr, vaz, E, pm[0], pm[1], pm[2],
+                pm[3], E_out, S_out);
         } else {
             k_transport_radial_f2<4><<<grid, bx, 0, L.stream>>>(
-                L.g, L.t, dt, omf, L.ph.limiter_mc, chunk, S, vr, vaz, E, mom[0], mom[1], mom[2],
-                mom[3], E_out, S_out);
+                L.g, L.t, dt, omf, L.ph.limiter_mc, chunk, chunks, L.ph.fast_transport, 1.0 / dt,
+                1.0 / L.g.nz, phase, S, vr, vaz, E, pm[0], pm[1], pm[2],
+                pm[3], E_out, S_out);
         }
         return;
     }
@@ -2575,8 +2337,8 @@ void launch_transport_radial(const Launch &L, double dt, double omf, int chunk, 
     }
 }
 
-// the larger of the two kernels' rings: the pair kernel's halo cells
-size_t azimuthal_smem_bytes(int nz) { return pair_ring_f2s(nz) * sizeof(f2); }
+// the FP64 kernel's ring arrays
+size_t azimuthal_smem_bytes(int nz) { return (size_t)4 * nz * sizeof(double); }
 
 // Cells per thread of the azimuthal kernel: blocks stay at <= 512 threads so
 // that the per-thread cell arrays fit 128 registers.
@@ -2587,61 +2349,15 @@ cudaError_t prepare_azimuthal(size_t smem)
     cudaError_t e = raise_smem_limit((const void *)k_transport_azimuthal<4>, smem);
     if (e == cudaSuccess) e = raise_smem_limit((const void *)k_transport_azimuthal<8>, smem);
     if (e == cudaSuccess) e = raise_smem_limit((const void *)k_transport_azimuthal<16>, smem);
-#define AZ2_FN(P, T, Q, X) (const void *)k_transport_azimuthal_f2<P, T, Q, false, X>
-    const void *pair_kernels[12] = {
-        AZ2_FN(2, 1024, 4, false), AZ2_FN(2, 1024, 5, false), AZ2_FN(2, 1024, 4, true),
-        AZ2_FN(2, 1024, 5, true), AZ2_FN(6, 1024, 4, false), AZ2_FN(6, 1024, 5, false),
-        AZ2_FN(6, 1024, 4, true), AZ2_FN(6, 1024, 5, true), AZ2_FN(16, 512, 4, false),
-        AZ2_FN(16, 512, 5, false), AZ2_FN(16, 512, 4, true), AZ2_FN(16, 512, 5, true)};
-#undef AZ2_FN
-    for (const void *fn : pair_kernels)
-        if (e == cudaSuccess) e = raise_smem_limit(fn, smem);
     return e;
 }
 
-// Cells per thread of the pair kernel: 2 up to 1024 cells (<= 512 threads),
-// 6 up to 6144 (<= 1024), 16 beyond (<= 512 threads for 8192 cells); the
-// thread count is the ring length over that, in whole warps.  Measured
-// (ms per azimuthal pass): 384-cell rings 0.021 with 2 cells per thread
-// (4: 0.029, 6: 0.039); 1536: 0.127 with 6 (4: 0.132, 8: 0.135, 2: 0.169);
-// 3072: 0.378 with 6 (8: 0.412); 6144: 1.87 with 6 (8: 2.01, 12: 2.55).
-int azimuthal_pair_cells_per_thread(int nz) { return nz <= 1024 ? 2 : (nz <= 6144 ? 6 : 16); }
-
 void launch_transport_azimuthal(const Launch &L, double dt, int block, double *const mom[4],
                                 double *E, double *S, const double *vaz, double *ring_ws,
-                                size_t smem, int *ring_shift)
+                                size_t smem)
 {
-    const bool pair = L.pair;
     const int nq = L.ph.adiabatic ? 5 : 4;
     const size_t dyn = ring_ws ? 0 : smem;
-    if (pair) {
-        const int per = azimuthal_pair_cells_per_thread(L.g.nz);
-        const int threads = ((L.g.nz + per - 1) / per + 31) / 32 * 32;
-        const bool exact = L.g.nz == per * threads;
-#define AZ2_LAUNCH1(P, T, Q, WS, X)                                                             \
-    k_transport_azimuthal_f2<P, T, Q, WS, X><<<L.g.nr, threads, dyn, L.stream>>>(                \
-        L.g, L.t, dt, L.ph.limiter_mc, L.ph.fast_transport, vaz, mom[0], mom[1], mom[2], mom[3], \
-        E, S, ring_ws, ring_shift)
-#define AZ2_LAUNCH2(P, T, Q)                                                                    \
-    if (exact) AZ2_LAUNCH1(P, T, Q, false, true); else AZ2_LAUNCH1(P, T, Q, false, false)
-#define AZ2_LAUNCH(P, T)                                                                        \
-    if (nq == 5) { AZ2_LAUNCH2(P, T, 5); } else { AZ2_LAUNCH2(P, T, 4); }
-        if (ring_ws) {
-            // rings beyond the shared memory: 16 cells per thread
-            if (nq == 5) AZ2_LAUNCH1(16, 512, 5, true, false);
-            else AZ2_LAUNCH1(16, 512, 4, true, false);
-        } else if (per == 2) {
-            AZ2_LAUNCH(2, 1024);
-        } else if (per == 6) {
-            AZ2_LAUNCH(6, 1024);
-        } else {
-            AZ2_LAUNCH(16, 512);
-        }
-#undef AZ2_LAUNCH
-#undef AZ2_LAUNCH1
-#undef AZ2_LAUNCH2
-        return;
-    }
     const int per = azimuthal_cells_per_thread(L.g.nz);
 #define AZ_LAUNCH(P)                                                                          \
     k_transport_azimuthal<P><<<L.g.nr, block, dyn, L.stream>>>(                               \
@@ -2659,11 +2375,11 @@ void launch_transport_azimuthal(const Launch &L, double dt, int block, double *c
 
 void launch_finish(const Launch &L, double omf, double *const mom[4], const double *S_t,
                    const double *E_t, const double *vr_in, double *vr_out, double *vaz_out,
-                   double *S_out, double *E_out, const int *ring_shift)
+                   double *S_out, double *E_out, const RingPhase *phase)
 {
     if (L.pair)
         return launch_finish_pair(L, omf, mom, S_t, E_t, vr_in, vr_out, vaz_out, S_out, E_out,
-                                  ring_shift);
+                                  phase);
     k_finish<<<grid2d(L.g.nz, L.g.nr + 1, L.bx), L.bx, 0, L.stream>>>(
         L.g, L.t, L.ph, omf, mom[0], mom[1], mom[2], mom[3], S_t, E_t, vr_in, vr_out, vaz_out,
         S_out, E_out);

@@ -429,14 +429,14 @@ __global__ void k_viscous_p(Geo g, Tables t, Phys ph, float2 dtp, float2 beta_in
 // compute_velocities_from_momenta (TransportEuler.cpp:498-535), the sigma
 // floor (SourceEuler.cpp:102-134) and the temperature floor, as k_finish,
 // with the azimuthal transport's AdvectSHIFT (:238-268): the transported
-// fields of ring i are read at j - shift[i]
-__global__ void k_finish_p(Geo g, Tables t, Phys ph, float2 omf, const double *__restrict__ mom0,
-                           const double *__restrict__ mom1, const double *__restrict__ mom2,
-                           const double *__restrict__ mom3, const double *__restrict__ S_t,
+// fields of ring i are read at j - its shift; the momenta are pairs
+__global__ void k_finish_p(Geo g, Tables t, Phys ph, float2 omf, const f2 *__restrict__ mom0,
+                           const f2 *__restrict__ mom1, const f2 *__restrict__ mom2,
+                           const f2 *__restrict__ mom3, const double *__restrict__ S_t,
                            const double *__restrict__ E_t, const double *__restrict__ vr_in,
                            double *__restrict__ vr_out, double *__restrict__ vaz_out,
                            double *__restrict__ S_out, double *__restrict__ E_out,
-                           const int *__restrict__ shift)
+                           const RingPhase *__restrict__ phase)
 {
     const int nz = g.nz, nr = g.nr;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -449,7 +449,7 @@ __global__ void k_finish_p(Geo g, Tables t, Phys ph, float2 omf, const double *_
     }
     // cell j of ring k before the shift
     auto at = [&](int k, int jj) {
-        int a = jj - __ldg(shift + k);
+        int a = jj - __ldg(&phase[k].shift);
         if (a < 0) a += nz;
         return CELL(k, a);
     };
@@ -460,10 +460,10 @@ __global__ void k_finish_p(Geo g, Tables t, Phys ph, float2 omf, const double *_
         vr_out[c] = 0.0;
     } else {
         const size_t cm = at(i - 1, j);
-        vr_out[c] = f2_to_double((P(mom0[cm]) + P(mom1[cs])) / (P(S_t[cm]) + sp));
+        vr_out[c] = f2_to_double((mom0[cm] + mom1[cs]) / (P(S_t[cm]) + sp));
     }
     const size_t cjm = at(i, prv(j, nz));
-    vaz_out[c] = f2_to_double((P(mom2[cjm]) + P(mom3[cs])) / (P(S_t[cjm]) + sp) *
+    vaz_out[c] = f2_to_double((mom2[cjm] + mom3[cs]) / (P(S_t[cjm]) + sp) *
                                   T(t, t.InvRmed, i) -
                               T(t, t.Rmed, i) * K(omf));
     // s < sigma_min on the bit patterns (sigma_min >= 0; a NaN stays)
@@ -533,12 +533,13 @@ void launch_viscous_pair(const Launch &L, double dt, double beta_inv, int mode, 
 
 void launch_finish_pair(const Launch &L, double omf, double *const mom[4], const double *S_t,
                         const double *E_t, const double *vr_in, double *vr_out, double *vaz_out,
-                        double *S_out, double *E_out, const int *ring_shift)
+                        double *S_out, double *E_out, const RingPhase *phase)
 {
+    auto m = [&](int q) { return reinterpret_cast<const f2 *>(mom[q]); };
     k_finish_p<<<grid2(L.g.nz, L.g.nr + 1, L.bx), L.bx, 0, L.stream>>>(
-        L.g, L.t, L.ph, split_pair_host(omf), mom[0], mom[1], mom[2], mom[3], S_t, E_t, vr_in,
+        L.g, L.t, L.ph, split_pair_host(omf), m(0), m(1), m(2), m(3), S_t, E_t, vr_in,
         vr_out, vaz_out,
-        S_out, E_out, ring_shift);
+        S_out, E_out, phase);
 }
 
 }  // namespace fgpu
