@@ -143,10 +143,9 @@ __global__ void b_finish(const DiskF *__restrict__ D, const StepF *__restrict__ 
                          const int *__restrict__ start, int nd, int rpb)
 {
     for_cells(D, S, start, nd, rpb, 1, [&](const DiskF &k, const StepF &, int i, int j) {
-        finish_cell(k.g, k.t, k.ph, k.mom[0], k.mom[1], k.mom[2], k.mom[3], k.sigma_t, k.energy_t,
-                    k.vr_b, k.s.vr, k.s.dv, k.s.sigma, k.s.energy, k.sigma_lo_t, k.s.sigma_lo,
-                    k.ring_shift, i,
-                    j);
+        finish_cell(k.g, k.t, k.ph, k.mom_w[0], k.mom_w[1], k.mom_w[2], k.mom_w[3], k.sigma_w,
+                    k.energy_w, k.vr_b, k.s.vr, k.s.dv, k.s.sigma, k.s.energy, k.sigma_lo_w,
+                    k.s.sigma_lo, k.ring_shift, i, j);
     });
 }
 
@@ -175,8 +174,24 @@ __global__ void b_ghost(const DiskF *__restrict__ D, const StepF *__restrict__ S
 // kind skipped
 template <int NQ>
 __global__ void b_transport_radial(const DiskF *__restrict__ D, const StepF *__restrict__ S,
-                                   const int *__restrict__ start, int nd, int chunk)
+                                   const int *__restrict__ start, int nd, int chunk,
+                                   const int *__restrict__ rings)
 {
+    // the ring phases of the window azimuthal pass first (rings: tile starts
+    // of one tile per ring, or null): latency-bound sums that the sweep's
+    // tiles overlap
+    if (rings) {
+        const int nrings = __ldg(rings + nd), warps = blockDim.x >> 5;
+        for (int item = blockIdx.x * warps + (threadIdx.x >> 5); item < nrings;
+             item += gridDim.x * warps) {
+            const int d = disk_of(rings, nd, item);
+            if (!S[d].run) continue;
+            const DiskF &k = D[d];
+            if (k.nq != NQ) continue;
+            ring_phase_f(k.g, k.t, S[d].dt, k.dv_b, item - __ldg(rings + d), k.ring_phase,
+                         k.ring_shift);
+        }
+    }
     const int total = __ldg(start + nd);
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
         const int d = disk_of(start, nd, tile);
@@ -225,43 +240,29 @@ __global__ void __launch_bounds__(PER <= 4 ? 384 : 512, PER <= 4 ? 2 : 1)
     }
 }
 
-// the register-blocked ring transport (azimuthal_ring_rb) over the rings of
-// one group of disks with the same ring length nz = PER x blockDim.x and
-// quantity count; start holds only the group's disks' rings
-template <int PER, int NQ>
-__global__ void __launch_bounds__(rb_max_threads(PER))
-    b_transport_azimuthal_rb(const DiskF *__restrict__ D, const StepF *__restrict__ S,
-                             const int *__restrict__ start, int nd)
+// the window azimuthal pass (azimuthal_window): one window per warp, windows
+// of all disks' rings in one grid-stride sequence
+template <int NQ>
+__global__ void __launch_bounds__(512)
+    b_transport_azimuthal_w(const DiskF *__restrict__ D, const StepF *__restrict__ S,
+                            const int *__restrict__ start, int nd)
 {
-    extern __shared__ __align__(16) float smf[];
-    __shared__ float redf[33];
-    __shared__ long long redl[33];
-    const int total = __ldg(start + nd);
-    for (int item = blockIdx.x; item < total; item += gridDim.x) {
-        const int d = disk_of(start, nd, item);
+    const int total = __ldg(start + nd), warps = blockDim.x >> 5;
+    for (int job = blockIdx.x * warps + (threadIdx.x >> 5); job < total;
+         job += gridDim.x * warps) {
+        const int d = disk_of(start, nd, job);
         if (!S[d].run) continue;
         const DiskF &k = D[d];
-        const int i = item - __ldg(start + d);
-        azimuthal_ring_rb<PER, NQ>(k.g, k.t, S[d].dt, k.ph.limiter_mc, k.ph.fast_transport,
-                                   k.dv_b, k.mom[0], k.mom[1], k.mom[2], k.mom[3], k.energy_t,
-                                   k.sigma_t, k.sigma_lo_t, i, smf, redf, redl,
-                                   k.ring_shift);
+        if (k.nq != NQ) continue;
+        const int local = job - __ldg(start + d), nwin = windows_of(k.g.nz);
+        const int i = local / nwin;
+        const WindowRows r{k.dv_b,     k.mom[0],   k.mom[1],    k.mom[2],  k.mom[3],
+                           k.energy_t, k.sigma_t,  k.sigma_lo_t, k.mom_w[0], k.mom_w[1],
+                           k.mom_w[2], k.mom_w[3], k.energy_w,  k.sigma_w, k.sigma_lo_w};
+        azimuthal_window<NQ>(k.g, k.t, S[d].dt, k.ph.limiter_mc, k.ph.fast_transport, r,
+                             k.ring_phase[i], i, local - i * nwin);
     }
 }
-
-typedef void (*AzRbFn)(const DiskF *, const StepF *, const int *, int);
-template <int NQ>
-static AzRbFn az_rb_fn_nq(int per)
-{
-    switch (per) {
-    case 4: return b_transport_azimuthal_rb<4, NQ>;
-    case 8: return b_transport_azimuthal_rb<8, NQ>;
-    case 12: return b_transport_azimuthal_rb<12, NQ>;
-    case 16: return b_transport_azimuthal_rb<16, NQ>;
-    default: return nullptr;
-    }
-}
-static AzRbFn az_rb_fn(int per, int nq) { return nq == 5 ? az_rb_fn_nq<5>(per) : az_rb_fn_nq<4>(per); }
 
 // damping rings: items = (disk, ring) of every disk with damping zones, each
 // taken four times, once per damped field (the fields are independent)
@@ -392,9 +393,9 @@ __global__ void b_close_sequence(const DiskF *__restrict__ D, const StepF *__res
     auto tab = [&](int k) { return tabs + (size_t)k * (nd + 1); };
     for_cells(D, S, tab(FGPU_BK_FINISH), nd, tl.k[FGPU_BK_FINISH].rings, 1,
               [&](const DiskF &k, const StepF &, int i, int j) {
-                  finish_cell(k.g, k.t, k.ph, k.mom[0], k.mom[1], k.mom[2], k.mom[3], k.sigma_t,
-                              k.energy_t, k.vr_b, k.s.vr, k.s.dv, k.s.sigma, k.s.energy,
-                              k.sigma_lo_t, k.s.sigma_lo, k.ring_shift, i, j);
+                  finish_cell(k.g, k.t, k.ph, k.mom_w[0], k.mom_w[1], k.mom_w[2], k.mom_w[3], k.sigma_w,
+                              k.energy_w, k.vr_b, k.s.vr, k.s.dv, k.s.sigma, k.s.energy,
+                              k.sigma_lo_w, k.s.sigma_lo, k.ring_shift, i, j);
               });
     grid.sync();
     // damping zones, as b_damping (its block reductions are block-wide)
@@ -578,7 +579,8 @@ static const void *kernel_fn(int k, int per)
     case FGPU_BK_VISCOUS: return (const void *)b_viscous;
     case FGPU_BK_GHOST: return (const void *)b_ghost;
     case FGPU_BK_TRANSPORT_RADIAL: return (const void *)b_transport_radial<5>;
-    case FGPU_BK_TRANSPORT_AZIMUTHAL: return (const void *)az_fn(per, 5);
+    case FGPU_BK_TRANSPORT_AZIMUTHAL:  // per 0: the window pass
+        return per ? (const void *)az_fn(per, 5) : (const void *)b_transport_azimuthal_w<5>;
     case FGPU_BK_FINISH: return (const void *)b_finish;
     case FGPU_BK_DAMPING: return (const void *)b_damping;
     case FGPU_BK_DERIVED_CFL: return (const void *)b_derived_cfl;
@@ -614,17 +616,9 @@ struct fgpu_batch {
     int grid[FGPU_BK_COUNT] = {};
     int az_per = 0;
     size_t az_smem = 0;
-    // disks whose rings take the register-blocked pass, grouped by ring
-    // length and quantity count (one launch per group); the strided pass
-    // takes the rest
-    struct RbGroup {
-        int nz, nq, per, grid;
-        size_t smem;
-    };
-    std::vector<RbGroup> rb;
-    std::vector<char> rb_disk;
-    int *d_rb_tables = nullptr;  // rb.size() tables of nd + 1 tile starts
-    long long az_strided_rings = 0;
+    // the window pass, or with FARGO_GB300_AZIMUTHAL=strided the strided ring
+    // pass
+    bool windows = true;
 
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
@@ -746,7 +740,7 @@ static int apply_tiles(fgpu_batch *b, const fgpu_tiles &t)
             } else if (k == FGPU_BK_TRANSPORT_RADIAL) {
                 n = ((b->nr[d] + r - 1) / r) * ncol;
             } else if (k == FGPU_BK_TRANSPORT_AZIMUTHAL) {
-                n = b->rb_disk[d] ? 0 : b->nr[d];
+                n = (long long)b->nr[d] * (b->windows ? windows_of(b->nz[d]) : 1);
             } else if (k == FGPU_BK_DERIVED_CFL) {
                 n = b->nr[d];
             }
@@ -758,15 +752,18 @@ static int apply_tiles(fgpu_batch *b, const fgpu_tiles &t)
         }
         s[nd] = (int)acc;
         totals[k] = k == FGPU_BK_DAMPING ? 4LL * b->n_damp_items : acc;
-        if (k == FGPU_BK_TRANSPORT_AZIMUTHAL) b->az_strided_rings = acc;
+        if (k == FGPU_BK_TRANSPORT_AZIMUTHAL && b->windows) {
+            const int warps = th / 32;  // windows per block
+            totals[k] = (acc + warps - 1) / warps;
+        }
     }
     CKB(cudaMemcpyAsync(b->d_tables, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice,
                         b->stream));
     CKB(cudaStreamSynchronize(b->stream));
     b->az_per = per_for(b->nz_max, t.k[FGPU_BK_TRANSPORT_AZIMUTHAL].threads);
     for (int k = 0; k < FGPU_BK_COUNT; ++k) {
-        const void *fn = kernel_fn(k, b->az_per);
-        const size_t smem = k == FGPU_BK_TRANSPORT_AZIMUTHAL ? b->az_smem : 0;
+        const void *fn = kernel_fn(k, b->windows ? 0 : b->az_per);
+        const size_t smem = k == FGPU_BK_TRANSPORT_AZIMUTHAL && !b->windows ? b->az_smem : 0;
         cudaFuncAttributes attr;
         CKB(cudaFuncGetAttributes(&attr, fn));
         if (t.k[k].threads > attr.maxThreadsPerBlock) {
@@ -819,19 +816,19 @@ static void launch_kernel(fgpu_batch *b, int k, int ghost_b = 0)
     case FGPU_BK_STRESS: b_stress<<<g, th, 0, s>>>(D, S, b->table(k), nd, r); break;
     case FGPU_BK_VISCOUS: b_viscous<<<g, th, 0, s>>>(D, S, b->table(k), nd, r); break;
     case FGPU_BK_GHOST: b_ghost<<<g, th, 0, s>>>(D, S, b->table(k), nd, ghost_b); break;
-    case FGPU_BK_TRANSPORT_RADIAL:
-        if (b->any_iso) b_transport_radial<4><<<g, th, 0, s>>>(D, S, b->table(k), nd, r);
-        if (b->any_adi) b_transport_radial<5><<<g, th, 0, s>>>(D, S, b->table(k), nd, r);
+    case FGPU_BK_TRANSPORT_RADIAL: {
+        const int *rings = b->windows ? b->table(FGPU_BK_DERIVED_CFL) : nullptr;
+        if (b->any_iso) b_transport_radial<4><<<g, th, 0, s>>>(D, S, b->table(k), nd, r, rings);
+        if (b->any_adi) b_transport_radial<5><<<g, th, 0, s>>>(D, S, b->table(k), nd, r, rings);
         break;
+    }
     case FGPU_BK_TRANSPORT_AZIMUTHAL:
-        if (b->az_strided_rings > 0) {
+        if (b->windows) {
+            if (b->any_iso) b_transport_azimuthal_w<4><<<g, th, 0, s>>>(D, S, b->table(k), nd);
+            if (b->any_adi) b_transport_azimuthal_w<5><<<g, th, 0, s>>>(D, S, b->table(k), nd);
+        } else {
             if (b->any_iso) az_fn(b->az_per, 4)<<<g, th, b->az_smem, s>>>(D, S, b->table(k), nd);
             if (b->any_adi) az_fn(b->az_per, 5)<<<g, th, b->az_smem, s>>>(D, S, b->table(k), nd);
-        }
-        for (size_t q = 0; q < b->rb.size(); ++q) {
-            const fgpu_batch::RbGroup &grp = b->rb[q];
-            az_rb_fn(grp.per, grp.nq)<<<grp.grid, grp.nz / grp.per, grp.smem, s>>>(
-                D, S, b->d_rb_tables + q * (size_t)(nd + 1), nd);
         }
         break;
     case FGPU_BK_FINISH: b_finish<<<g, th, 0, s>>>(D, S, b->table(k), nd, r); break;
@@ -917,7 +914,6 @@ static void release(fgpu_batch *b)
     cudaFree(b->d_tables);
     cudaFree(b->d_seq_tables);
     cudaFree(b->d_seq_err);
-    cudaFree(b->d_rb_tables);
     cudaFree(b->d_damp_items);
     if (b->h_steps) cudaFreeHost(b->h_steps);
     if (b->h_clocks) cudaFreeHost(b->h_clocks);
@@ -985,6 +981,7 @@ extern "C" int fgpu_batch_create(int n, const fgpu_params *params, const double 
         b->nr.push_back(e->rings());
         b->nz.push_back(e->azimuthal());
         b->nz_max = std::max(b->nz_max, e->azimuthal());
+        b->windows = b->windows && e->window_pass();
         desc[k] = e->describe();
         b->any_art = b->any_art || desc[k].ph.adiabatic || desc[k].ph.art_visc_sn ||
                      desc[k].ph.art_visc_tw;
@@ -1034,53 +1031,6 @@ extern "C" int fgpu_batch_create(int n, const fgpu_params *params, const double 
     CKC(cudaMalloc(&b->d_seq_tables, sizeof(int) * FGPU_BK_COUNT * (n + 1)));
     CKC(cudaMalloc(&b->d_seq_err, sizeof(int)));
     CKC(cudaMemsetAsync(b->d_seq_err, 0, sizeof(int), b->stream));
-    {
-        // register-blocked groups: disks with the same ring length and
-        // quantity count whose rings split into whole segments
-        // (rb_default_per); FARGO_GB300_AZIMUTHAL=strided keeps them all on
-        // the strided pass
-        const char *env = getenv("FARGO_GB300_AZIMUTHAL");
-        const bool strided_only = env && std::string(env) == "strided";
-        b->rb_disk.assign(n, 0);
-        for (int d = 0; d < n && !strided_only; ++d) {
-            const int nq = params[d].eos == FGPU_EOS_IDEAL ? 5 : 4;
-            const int per = rb_default_per(b->nz[d], nq, kMaxRingSmem);
-            if (!per) continue;
-            b->rb_disk[d] = 1;
-            bool found = false;
-            for (auto &g : b->rb) found = found || (g.nz == b->nz[d] && g.nq == nq);
-            if (!found)
-                b->rb.push_back({b->nz[d], nq, per, 1,
-                                 rb_smem_floats(b->nz[d], nq, b->nz[d] / per) * sizeof(float)});
-        }
-        if (!b->rb.empty()) {
-            std::vector<int> h((size_t)b->rb.size() * (n + 1), 0);
-            for (size_t q = 0; q < b->rb.size(); ++q) {
-                fgpu_batch::RbGroup &g = b->rb[q];
-                int *st = h.data() + q * (size_t)(n + 1);
-                long long acc = 0;
-                for (int d = 0; d < n; ++d) {
-                    st[d] = (int)acc;
-                    const int nq = params[d].eos == FGPU_EOS_IDEAL ? 5 : 4;
-                    if (b->rb_disk[d] && b->nz[d] == g.nz && nq == g.nq) acc += b->nr[d];
-                }
-                st[n] = (int)acc;
-                const void *fn = (const void *)az_rb_fn(g.per, g.nq);
-                CKC(raise_smem_limit(fn, g.smem));
-                int per_sm = 0;
-                CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, g.nz / g.per,
-                                                                  g.smem));
-                if (per_sm < 1) {
-                    b->err = "the register-blocked ring pass cannot run on this device";
-                    return fail(FGPU_ERR_UNSUPPORTED);
-                }
-                g.grid = (int)std::max(1LL, std::min((long long)per_sm * b->nsm, acc));
-            }
-            CKC(cudaMalloc(&b->d_rb_tables, sizeof(int) * h.size()));
-            CKC(cudaMemcpy(b->d_rb_tables, h.data(), sizeof(int) * h.size(),
-                           cudaMemcpyHostToDevice));
-        }
-    }
     if (!damp.empty()) {
         CKC(cudaMalloc(&b->d_damp_items, sizeof(int2) * damp.size()));
         CKC(cudaMemcpy(b->d_damp_items, damp.data(), sizeof(int2) * damp.size(),

@@ -1407,6 +1407,243 @@ __device__ __forceinline__ void azimuthal_ring_rb(const GeoF &g, const TablesF &
     __syncthreads();
 }
 
+// ---------------------------------------------------------------------------
+// The same ring transport without barriers: a warp owns a window of 128
+// consecutive cells of a ring, four per lane in registers, and writes the 120
+// inner ones; the four cells at either end, which both passes of the inner
+// cells need, are computed along with them, so that no warp waits for
+// another and a ring needs no shared memory.  Neighbours beyond a lane's
+// four cells come by shuffles.  The ring means and the shift phase are the
+// radial launch's (ring_phase_f), and the output goes to other buffers than the
+// input, since neighbouring windows overlap.  Every cell's arithmetic is the
+// ring kernels' above, expression for expression: the same bits.
+//
+// The ring kernels are bound by latency (two or three block barriers per
+// quantity and pass, a block of at most 512 threads per SM: issue 29% of the
+// cycles, DRAM 10%); this one keeps 24 warps per SM resident and has no
+// barrier.  Measured, ms per azimuthal pass (register-blocked or strided
+// ring kernel -> this): 2048 x 6144 0.547 -> 0.236, 512 x 1536 0.049 -> 0.021,
+// 128 x 384 0.014 -> 0.010, the 64-disk sweep's step 3.84 -> 3.15.  Issue is
+// 71% busy, DRAM 29%.
+// ---------------------------------------------------------------------------
+constexpr int kWinCells = 4;                            // cells per lane
+constexpr int kWinInner = 30 * kWinCells;               // cells a warp writes
+__host__ __device__ constexpr int windows_of(int nz) { return (nz + kWinInner - 1) / kWinInner; }
+
+// A ring's mean residual velocity and uniform velocity (ComputeConstantResidual,
+// TransportEuler.cpp:174-236), and its integer shift, by one warp (the exact
+// integer sum of exact_sum_scale / exact_sum_result: the ring kernels' bits).
+__device__ __forceinline__ void ring_phase_f(const GeoF &g, const TablesF &t, double dt,
+                                             const float *__restrict__ dv, int i, float2 *phase,
+                                             int *ring_shift)
+{
+    const int nz = g.nz, lane = threadIdx.x & 31;
+    const float *v = dv + (size_t)i * nz;
+    float m = 0.f;
+#pragma unroll 8
+    for (int j = lane; j < nz; j += 32) m = fmaxf(m, fabsf(v[j]));
+    m = __shfl_sync(0xffffffffu, warp_max_f(m), 0);
+    int e = 0;
+    frexpf(m, &e);
+    const int ks = 62 - e - (32 - __clz(nz));
+    long long part = 0;
+#pragma unroll 8
+    for (int j = lane; j < nz; j += 32) part += to_fixed(v[j], ks);
+    part = warp_sum_ll(part);
+    if (lane == 0) {
+        const double mean_dv = ldexp((double)part, -ks) / (double)nz;
+        const double vmean = (t.Vref_d[i] - t.Rmed_d[i] * g.omega_frame) + mean_dv;
+        const double Ntilde = vmean * t.InvRmed_d[i] * dt * g.invdphi_d;
+        const double Nround = floor(Ntilde + 0.5);
+        const int nshift = (int)Nround;
+        const float vt = (float)((Ntilde - Nround) * t.Rmed_d[i] * (1.0 / dt) * g.dphi_d);
+        phase[i] = make_float2((float)mean_dv, vt);
+        ring_shift[i] = ((nshift % nz) + nz) % nz;
+    }
+}
+
+// the rows a window reads and writes (m: momenta, e: energy, s, slo: sigma)
+struct WindowRows {
+    const float *dv, *m0, *m1, *m2, *m3, *e, *s, *slo;
+    float *om0, *om1, *om2, *om3, *oe, *os, *oslo;
+    __device__ __forceinline__ const float *in(int q) const
+    {
+        return q == 0 ? m0 : q == 1 ? m1 : q == 2 ? m2 : q == 3 ? m3 : e;
+    }
+    __device__ __forceinline__ float *out(int q) const
+    {
+        return q == 0 ? om0 : q == 1 ? om1 : q == 2 ? om2 : q == 3 ? om3 : oe;
+    }
+};
+
+template <int NQ>
+__device__ __forceinline__ void azimuthal_window(const GeoF &g, const TablesF &t, double dt,
+                                                 int mc, int fast, const WindowRows &rows,
+                                                 float2 phase, int i, int window)
+{
+    constexpr unsigned all = 0xffffffffu;
+    constexpr int N = kWinCells;
+    const int nz = g.nz, lane = threadIdx.x & 31;
+    const size_t row = (size_t)i * nz;
+    const int base = window * kWinInner + (lane - 1) * N;
+    const int valid = lane == 0 || lane == 31 ? 0 : min(N, nz - base);
+    const bool aligned = (nz & 3) == 0;  // a lane's cells are one 128-bit word
+    int j[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        int b = base + k;
+        if (b < 0) b += nz;
+        if (b >= nz) b = b - nz < nz ? b - nz : b % nz;
+        j[k] = b;
+    }
+    auto load = [&](const float *p, float *x) {
+        if (aligned) {
+            const float4 w = *reinterpret_cast<const float4 *>(p + row + j[0]);
+            x[0] = w.x; x[1] = w.y; x[2] = w.z; x[3] = w.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; ++k) x[k] = p[row + j[k]];
+        }
+    };
+    auto store = [&](float *p, const float *x) {
+        if (aligned) {
+            if (valid > 0)
+                *reinterpret_cast<float4 *>(p + row + base) = make_float4(x[0], x[1], x[2], x[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                if (k < valid) p[row + base + k] = x[k];
+        }
+    };
+    auto left = [&](float x) { return __shfl_up_sync(all, x, 1); };
+    auto right = [&](float x) { return __shfl_down_sync(all, x, 1); };
+
+    float v[N], s[N], slo[N], next[N];
+    load(rows.dv, v);
+    load(rows.s, s);
+    load(rows.slo, slo);
+    load(rows.m0, next);
+    // the other rows come from DRAM: ask L2 for them now
+#pragma unroll
+    for (int q = 1; q < NQ; ++q)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(rows.in(q) + row + j[0]));
+    const float mdv = phase.x, vt = phase.y;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        float vres = v[n] - mdv;
+        if (!fast) vres = vt + vres;
+        v[n] = vres;
+    }
+    const float dxtheta = g.dphi * t.Rmed[i];
+    const float half_invdx = 0.5f / dxtheta;
+    const float dxrad = t.DRsup[i] * (float)dt;
+    const float invsurf = t.InvSurf[i];
+    const float fdt = (float)dt;
+    const float dxrad_invsurf = dxrad * invsurf;
+
+    // cells -1 .. 3 of X and of its slopes at index + 1
+    auto slopes = [&](float *X, float *D) {
+        X[0] = left(X[N]);
+        float d[N + 1];
+#pragma unroll
+        for (int k = 0; k < N; ++k) d[k] = __fsub_rn(X[k + 1], X[k]);
+        d[N] = right(d[0]);
+#pragma unroll
+        for (int k = 0; k < N; ++k) D[k + 1] = __fmul_rn(lim_f(d[k + 1], d[k], mc), half_invdx);
+        D[0] = left(D[N]);
+    };
+    float cf[N + 1], invs[N];
+    // the uniform pass: face factors in difference form (ring_pass_uniform_f)
+    const float ksi_u = vt * fdt;
+    const bool pos = ksi_u > 0.f;
+    const float a = pos ? dxtheta - ksi_u : -(dxtheta + ksi_u);
+    const float c = dxrad * vt * invsurf;
+    float dss[N], Fs[N], invs2[N];
+    // X_u, X_u1, D_u, D_u1 of face n, upwind cell u and its right neighbour u1
+    auto uniform_sides = [&](float *X, float *D) {
+        if (pos) return;
+        // cells 0 .. 4 instead of -1 .. 3
+        const float xr = right(X[1]), dr = right(D[1]);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            X[k] = X[k + 1];
+            D[k] = D[k + 1];
+        }
+        X[N] = xr;
+        D[N] = dr;
+    };
+    {
+        float X[N + 1], D[N + 1];
+#pragma unroll
+        for (int n = 0; n < N; ++n) X[n + 1] = s[n];
+        slopes(X, D);
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            invs[n] = __frcp_rn(s[n]);
+            const float vv = v[n];
+            const float ksi = __fmul_rn(vv, fdt);
+            const float ss = ksi > 0.f ? star_pos(X[n], D[n], dxtheta, ksi)
+                                       : star_neg(X[n + 1], D[n + 1], dxtheta, ksi);
+            cf[n] = __fmul_rn(__fmul_rn(dxrad_invsurf, ss), vv);
+        }
+        cf[N] = right(cf[0]);
+#pragma unroll
+        for (int n = 0; n < N; ++n) comp_add(s[n], slo[n], cf[n] - cf[n + 1]);
+    }
+    if (fast) {
+        float X[N + 1], D[N + 1];
+#pragma unroll
+        for (int n = 0; n < N; ++n) X[n + 1] = s[n];
+        slopes(X, D);
+        uniform_sides(X, D);
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            invs2[n] = __frcp_rn(s[n]);
+            dss[n] = star_diff(X[n], X[n + 1], D[n], D[n + 1], a);
+            Fs[n] = star_at(X[n + 1], D[n + 1], a);
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n) comp_add(s[n], slo[n], __fmul_rn(c, dss[n]));
+    }
+    store(rows.os, s);
+    store(rows.oslo, slo);
+#pragma unroll 1
+    for (int q = 0; q < NQ; ++q) {
+        float qv[N], X[N + 1], D[N + 1];
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            qv[n] = next[n];
+            X[n + 1] = __fmul_rn(qv[n], invs[n]);
+        }
+        if (q + 1 < NQ) load(rows.in(q + 1), next);
+        slopes(X, D);
+        float F[N + 1];
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const float ksi = __fmul_rn(v[n], fdt);
+            const float qs = ksi > 0.f ? star_pos(X[n], D[n], dxtheta, ksi)
+                                       : star_neg(X[n + 1], D[n + 1], dxtheta, ksi);
+            F[n] = __fmul_rn(qs, cf[n]);
+        }
+        F[N] = right(F[0]);
+#pragma unroll
+        for (int n = 0; n < N; ++n) qv[n] = __fadd_rn(qv[n], __fsub_rn(F[n], F[n + 1]));
+        if (fast) {
+#pragma unroll
+            for (int n = 0; n < N; ++n) X[n + 1] = __fmul_rn(qv[n], invs2[n]);
+            slopes(X, D);
+            uniform_sides(X, D);
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                const float qs = star_at(X[n], D[n], a);
+                const float dqs = star_diff(X[n], X[n + 1], D[n], D[n + 1], a);
+                qv[n] = uniform_update(qv[n], c, qs, dss[n], Fs[n], dqs);
+            }
+        }
+        store(rows.out(q), qv);
+    }
+}
+
 // compute_pressure (SourceEuler.cpp:1345-1376): P alone
 __device__ __forceinline__ void pressure_cell(const GeoF &g, const TablesF &t, const PhysF &ph,
                                               const float *__restrict__ S,

@@ -146,7 +146,11 @@ struct DiskF {
     float *vr_b, *dv_b;
     float *sigma_t, *energy_t, *sigma_lo_t;  // after radial transport
     int *ring_shift;  // the azimuthal pass's integer shift per ring (AdvectSHIFT)
+    float2 *ring_phase;  // mean residual and uniform velocity per ring (window pass)
     float *mom[4];
+    // after the azimuthal transport, for the velocity rebuild: the buffers
+    // above where the pass works in place, others after the window pass
+    float *mom_w[4], *sigma_w, *energy_w, *sigma_lo_w;
     float *pot, *P, *cs, *H, *nu, *T, *Qr, *Qp, *divv, *trr, *tpp, *trp, *qplus, *qminus;
     unsigned int *dtmin;
     int damping, nq;
@@ -221,6 +225,7 @@ class Engine32 {
     double beta_inv_at(double t) const { return beta_inv(t); }
     int rings() const { return nr; }
     int azimuthal() const { return nz; }
+    bool window_pass() const { return windows; }
     const int *damping_rings(int *n) const
     {
         *n = (p.damping && n_rings) ? n_rings : 0;
@@ -263,6 +268,11 @@ class Engine32 {
     float *vr_a = nullptr, *dv_a = nullptr;  // v_r, v_phi buffers at creation
     float *sigma_lo = nullptr, *alt_sigma_lo = nullptr;
     int *ring_shift = nullptr;  // AdvectSHIFT per ring, applied by the velocity rebuild
+    // the window azimuthal pass (out of place), unless FARGO_GB300_AZIMUTHAL
+    // selects a ring kernel (in place)
+    bool windows = true;
+    float2 *ring_phase = nullptr;
+    float *mom_w[4] = {}, *sigma_w = nullptr, *energy_w = nullptr, *sigma_lo_w = nullptr;
     float *mom[4] = {};
     float *tab_f = nullptr;
     double *tab_d = nullptr;
@@ -278,7 +288,7 @@ class Engine32 {
     double *h_pinned = nullptr;
     int per = 4, az_block = 128;
     size_t az_smem = 0;
-    int rb_per = 0;      // register-blocked azimuthal kernel: cells per thread (0: strided)
+    int rb_per = 0;      // register-blocked ring kernel: cells per thread (0: strided)
     size_t rb_smem = 0;
     bool az_stage = false;
     bool visc_recompute = false;  // c_s, H, nu before the final hooks (adiabatic)

@@ -134,12 +134,38 @@ __global__ void __launch_bounds__(64, 16) f_transport_radial(GeoF g, TablesF t, 
                                    float *__restrict__ m0, float *__restrict__ m1,
                                    float *__restrict__ m2, float *__restrict__ m3,
                                    float *__restrict__ E_out, float *__restrict__ S_out,
-                                   const float *__restrict__ S_lo, float *__restrict__ S_lo_out)
+                                   const float *__restrict__ S_lo, float *__restrict__ S_lo_out,
+                                   double dt_d, int phase_rows, float2 *__restrict__ phase,
+                                   int *__restrict__ ring_shift)
 {
+    // the first rows of blocks form the ring phases of the window azimuthal
+    // pass, a warp per ring: latency-bound sums that the sweep's blocks behind
+    // them overlap (2048 x 6144: 0.300 ms, the sweep alone 0.295; as a launch
+    // of their own 0.335; with block reductions, whose shared memory comes off
+    // the sweep's L1, 0.345)
+    if ((int)blockIdx.y < phase_rows) {
+        const int i = (blockIdx.y * gridDim.x + blockIdx.x) * 2 + (threadIdx.x >> 5);
+        if (i < g.nr) ring_phase_f(g, t, dt_d, dv, i, phase, ring_shift);
+        return;
+    }
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= g.nz) return;
     radial_col<NQ>(g, t, dt, mc, chunk, S, vr, dv, E, m0, m1, m2, m3, E_out, S_out, S_lo,
-                   S_lo_out, blockIdx.y * chunk, j);
+                   S_lo_out, (blockIdx.y - phase_rows) * chunk, j);
+}
+
+// the window azimuthal pass (azimuthal_window), one window per warp
+constexpr int kWinThreads = 128;
+template <int NQ>
+__global__ void __launch_bounds__(kWinThreads) f_transport_azimuthal_w(GeoF g, TablesF t, double dt,
+                                                                       int mc, int fast,
+                                                                       int nwin, WindowRows rows,
+                                                                       const float2 *__restrict__ phase)
+{
+    const int job = blockIdx.x * (kWinThreads / 32) + (threadIdx.x >> 5);
+    const int i = job / nwin;
+    if (i >= g.nr) return;
+    azimuthal_window<NQ>(g, t, dt, mc, fast, rows, phase[i], i, job - i * nwin);
 }
 
 template <int PER, int NQ, bool STAGE>
@@ -813,11 +839,11 @@ int Engine32::create(const fgpu_params &prm, const double *radii, cudaStream_t s
             return FGPU_ERR_CUDA;
         }
     }
-    // the register-blocked kernel where the ring splits into whole 128-bit
-    // segments (rb_default_per), unless FARGO_GB300_AZIMUTHAL asks for
+    // the window pass, unless FARGO_GB300_AZIMUTHAL asks for a ring kernel:
     // "strided" or "blocked<PER>" (an explicit request is honoured or
     // refused, never replaced)
     rb_per = 0;
+    windows = true;
     {
         const char *env = getenv("FARGO_GB300_AZIMUTHAL");
         const std::string want = env ? env : "";
@@ -826,13 +852,22 @@ int Engine32::create(const fgpu_params &prm, const double *radii, cudaStream_t s
             if ((pc == 4 || pc == 8 || pc == 12 || pc == 16) &&
                 rb_fits(nz, nq, pc, 1, kMaxRingSmem)) {
                 rb_per = pc;
+                windows = false;
             } else {
                 err = "FARGO_GB300_AZIMUTHAL=" + want + " does not fit this ring";
                 return FGPU_ERR_UNSUPPORTED;
             }
-        } else if (want != "strided") {
-            rb_per = rb_default_per(nz, nq, kMaxRingSmem);
+        } else if (want == "strided") {
+            windows = false;
         }
+    }
+    if (windows) {
+        CKF(cudaMalloc(&ring_phase, sizeof(float2) * (size_t)nr));
+        for (int k = 0; k < 4; ++k) CKF(cudaMalloc(&mom_w[k], cells * sizeof(float)));
+        CKF(cudaMalloc(&sigma_w, cells * sizeof(float)));
+        CKF(cudaMalloc(&sigma_lo_w, cells * sizeof(float)));
+        CKF(cudaMalloc(&energy_w, cells * sizeof(float)));
+        CKF(cudaMemset(energy_w, 0, cells * sizeof(float)));
     }
     if (rb_per) {
         rb_smem = rb_smem_floats(nz, nq, nz / rb_per) * sizeof(float);
@@ -858,7 +893,11 @@ void Engine32::destroy()
     for (int f = 0; f < FGPU_FIELD_COUNT; ++f) cudaFree(fld[f]);
     cudaFree(alt_sigma); cudaFree(alt_vr); cudaFree(alt_dv); cudaFree(alt_e);
     cudaFree(sigma_lo); cudaFree(alt_sigma_lo); cudaFree(ring_shift);
-    for (int k = 0; k < 4; ++k) cudaFree(mom[k]);
+    for (int k = 0; k < 4; ++k) {
+        cudaFree(mom[k]);
+        cudaFree(mom_w[k]);
+    }
+    cudaFree(ring_phase); cudaFree(sigma_w); cudaFree(sigma_lo_w); cudaFree(energy_w);
     cudaFree(partial); cudaFree(red_out); cudaFree(d_dtmin); cudaFree(d_bad); cudaFree(stage);
     cudaFree(corr_phi); cudaFree(corr_r);
     cudaFree(tab_f); cudaFree(tab_d); cudaFree(tab_c); cudaFree(vaz_offset); cudaFree(damp_mem); cudaFree(damp_aux); cudaFree(damp_rings);
@@ -890,7 +929,14 @@ DiskF Engine32::describe()
     d.energy_t = alt_e;
     d.sigma_lo_t = alt_sigma_lo;
     d.ring_shift = ring_shift;
-    for (int k = 0; k < 4; ++k) d.mom[k] = mom[k];
+    d.ring_phase = ring_phase;
+    for (int k = 0; k < 4; ++k) {
+        d.mom[k] = mom[k];
+        d.mom_w[k] = windows ? mom_w[k] : mom[k];
+    }
+    d.sigma_w = windows ? sigma_w : alt_sigma;
+    d.energy_w = windows ? energy_w : alt_e;
+    d.sigma_lo_w = windows ? sigma_lo_w : alt_sigma_lo;
     d.pot = fld[FGPU_POTENTIAL];
     d.P = fld[FGPU_PRESSURE];
     d.cs = fld[FGPU_SOUNDSPEED];
@@ -1210,21 +1256,32 @@ int Engine32::transport(double dt)
         const int cols = (nz + 63) / 64;
         int chunk = 16;
         while (chunk > 4 && (long long)cols * ((nr + chunk - 1) / chunk) < 16LL * nsm) chunk /= 2;
-        dim3 grid(cols, (nr + chunk - 1) / chunk);
+        const int phase_rows = windows ? (nr + 2 * cols - 1) / (2 * cols) : 0;
+        dim3 grid(cols, phase_rows + (nr + chunk - 1) / chunk);
         if (adi)
             f_transport_radial<5><<<grid, 64, 0, stream>>>(geo, tabs, fdt, phys.limiter_mc, chunk,
                                                            s.sigma, s.vr, s.dv, s.energy, mom[0],
                                                            mom[1], mom[2], mom[3], alt_e, alt_sigma,
-                                                           sigma_lo, alt_sigma_lo);
+                                                           sigma_lo, alt_sigma_lo, dt, phase_rows,
+                                                           ring_phase, ring_shift);
         else
             f_transport_radial<4><<<grid, 64, 0, stream>>>(geo, tabs, fdt, phys.limiter_mc, chunk,
                                                            s.sigma, s.vr, s.dv, s.energy, mom[0],
                                                            mom[1], mom[2], mom[3], alt_e, alt_sigma,
-                                                           sigma_lo, alt_sigma_lo);
+                                                           sigma_lo, alt_sigma_lo, dt, phase_rows,
+                                                           ring_phase, ring_shift);
     }
     CKL("transport_radial");
     mark(7);
-    {
+    if (windows) {
+        const WindowRows r{s.dv,     mom[0],   mom[1],   mom[2],   mom[3],   alt_e,   alt_sigma, alt_sigma_lo,
+                           mom_w[0], mom_w[1], mom_w[2], mom_w[3], energy_w, sigma_w, sigma_lo_w};
+        const int nwin = windows_of(nz), per_block = kWinThreads / 32;
+        const int blocks = (nr * nwin + per_block - 1) / per_block;
+        auto k = adi ? f_transport_azimuthal_w<5> : f_transport_azimuthal_w<4>;
+        k<<<blocks, kWinThreads, 0, stream>>>(geo, tabs, dt, phys.limiter_mc, phys.fast_transport,
+                                              nwin, r, ring_phase);
+    } else {
 #define AZ32(P, NQ, ST)                                                                          \
     f_transport_azimuthal<P, NQ, ST><<<nr, az_block, az_smem, stream>>>(                         \
         geo, tabs, dt, phys.limiter_mc, phys.fast_transport, s.dv, mom[0], mom[1], mom[2],      \
@@ -1268,10 +1325,11 @@ int Engine32::transport(double dt)
     }
     CKL("transport_azimuthal");
     mark(8);
-    f_finish<<<grid2(nz, nr + 1), 128, 0, stream>>>(geo, tabs, phys, mom[0], mom[1], mom[2],
-                                                    mom[3], alt_sigma, alt_e, s.vr, alt_vr,
-                                                    alt_dv, s.sigma, s.energy, alt_sigma_lo,
-                                                    sigma_lo, ring_shift);
+    float *const *m = windows ? mom_w : mom;
+    f_finish<<<grid2(nz, nr + 1), 128, 0, stream>>>(
+        geo, tabs, phys, m[0], m[1], m[2], m[3], windows ? sigma_w : alt_sigma,
+        windows ? energy_w : alt_e, s.vr, alt_vr, alt_dv, s.sigma, s.energy,
+        windows ? sigma_lo_w : alt_sigma_lo, sigma_lo, ring_shift);
     CKL("finish");
     std::swap(fld[FGPU_V_RADIAL], alt_vr);
     std::swap(fld[FGPU_V_AZIMUTHAL], alt_dv);

@@ -481,9 +481,10 @@ typedef struct fgpu_batch fgpu_batch;
 
 /* Tile shape of one batched kernel: threads per block and, for the per-cell
  * kernels, rings per block (cells per thread along the radius); for the
- * radial transport, rings one thread walks.  Ring kernels (azimuthal
- * transport, damping, CFL) use one block per ring; their cells per thread
- * follow from threads and the longest ring. */
+ * radial transport, rings one thread walks.  Ring kernels (damping, CFL) use
+ * one block per ring; the azimuthal transport takes threads / 32 windows of 120
+ * cells per block (its threads must still cover the longest ring at 16 cells
+ * each, as the strided ring kernel of FARGO_GB300_AZIMUTHAL=strided needs). */
 typedef struct {
 	int threads;
 	int rings;
