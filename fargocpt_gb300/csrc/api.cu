@@ -584,7 +584,7 @@ static int setup_tables(fgpu_engine *eng, const double *radii)
     enum { RINF, RSUP, RMED, SURF, INVRMED, INVSURF, INVDIFFRMED, INVDIFFRSUP, INVDIFFRSUPRB,
            INVRINF, RINFSQ, TWOOVER, OMEGAK, INVOMEGAK, CSISO, INVDXSRC, INVDXTHETA, EMODEL,
            HFACADI, INVCELL, INVCELL2, TWOOVERRMEDSUM, LSQTW, TWOOVERDRMED2, DIFFRMED,
-           RA3IDRMED, F43, CRPP1, CRPP2, CRRR1, CRRR2, CRRP, CRSCALE, NTAB };
+           RA3IDRMED, F43, CRPP1, CRPP2, CRRR1, CRRR2, CRRP, CRSCALE, DINVRMED, NTAB };
     std::vector<double> h((size_t)NTAB * R, 0.0);
     auto T = [&](int k) { return h.data() + (size_t)k * R; };
     for (int n = 0; n <= nr; ++n) {
@@ -618,6 +618,9 @@ static int setup_tables(fgpu_engine *eng, const double *radii)
         T(INVCELL2)[n] = 1.0 / (cell * cell);
     }
     for (int n = 1; n <= nr; ++n) T(TWOOVERRMEDSUM)[n] = 2.0 / (T(RMED)[n] + T(RMED)[n - 1]);
+    // 1 / Rmed[n] - 1 / Rmed[n - 1] without its cancellation
+    for (int n = 1; n <= nr; ++n)
+        T(DINVRMED)[n] = (T(RMED)[n - 1] - T(RMED)[n]) / (T(RMED)[n] * T(RMED)[n - 1]);
     for (int n = 1; n <= nr; ++n) T(INVDIFFRMED)[n] = 1.0 / (T(RMED)[n] - T(RMED)[n - 1]);
     for (int n = 0; n < nr; ++n) {
         T(TWOOVER)[n] = 2.0 / (std::pow(T(RINF)[n + 1], 2) - std::pow(T(RINF)[n], 2));
@@ -669,6 +672,7 @@ static int setup_tables(fgpu_engine *eng, const double *radii)
     t.LSqTW = D(LSQTW); t.TwoOverDRmed2 = D(TWOOVERDRMED2); t.DiffRmed = D(DIFFRMED);
     t.Ra3IDRmed = D(RA3IDRMED); t.F43 = D(F43); t.CrPp1 = D(CRPP1); t.CrPp2 = D(CRPP2);
     t.CrRr1 = D(CRRR1); t.CrRr2 = D(CRRR2); t.CrRp = D(CRRP); t.CrScale = D(CRSCALE);
+    t.DInvRmed = D(DINVRMED);
     t.cosj = tc; t.sinj = tc + nz;
     {
         // Rmed, cos and sin, InvDiffRmed and InvSurf as float pairs hi + lo
@@ -1354,10 +1358,14 @@ extern "C" int fgpu_init_euler(fgpu_engine *eng, double t)
     launch_derived_cfl(L, 1 | 2, s, nullptr);
     if (eng->ph.adiabatic) {
         // compute_heating_cooling_for_CFL, SourceEuler.cpp:1410-1450
-        launch_stress(L, s.sigma, s.vr, s.vaz, s.nu, s.divv, s.trr, s.tpp, s.trp);
         eng->stress_pairs = stress_as_pairs(L);
         if (eng->ph.stabilize) launch_visc_corr(L, s);
-        launch_viscous(L, 0.0, beta_inv_at(eng->p, t), 2, s);
+        if (eng->stress_pairs) {
+            launch_viscous_pair(L, 0.0, beta_inv_at(eng->p, t), 2, s, nullptr, nullptr);
+        } else {
+            launch_stress(L, s.sigma, s.vr, s.vaz, s.nu, s.divv, s.trr, s.tpp, s.trp);
+            launch_viscous(L, 0.0, beta_inv_at(eng->p, t), 2, s);
+        }
     }
     eng->cfl_valid = false;
     return check_launch(eng);
@@ -1617,33 +1625,58 @@ static void gas_kick(fgpu_engine *eng, double dt, double t)
     const double omf = eng->bodies.omega_frame;
     double **f = eng->field;
     const bool adi = eng->ph.adiabatic;
-    // CalculateNbodyPotential (simulation.cpp:170-174)
-    launch_potential(L, eng->bodies, f[FGPU_SCALE_HEIGHT], f[FGPU_POTENTIAL]);
-    mark(eng, 0);
-    // update_with_sourceterms (simulation.cpp:190): momentum updates
-    launch_source(L, dt, omf, f[FGPU_SIGMA], f[FGPU_PRESSURE], f[FGPU_POTENTIAL],
-                  f[FGPU_V_RADIAL], f[FGPU_V_AZIMUTHAL], eng->vr_alt, eng->vaz_alt);
+    // CalculateNbodyPotential (simulation.cpp:170-174) and
+    // update_with_sourceterms (:190), momentum updates
+    if (L.pair && eng->bodies.star_plain) {
+        // one kernel for both, timed as the source phase
+        mark(eng, 0);
+        launch_source_window(L, dt, omf, eng->bodies, state_of(eng), eng->vr_alt, eng->vaz_alt);
+    } else {
+        launch_potential(L, eng->bodies, f[FGPU_SCALE_HEIGHT], f[FGPU_POTENTIAL]);
+        mark(eng, 0);
+        launch_source(L, dt, omf, f[FGPU_SIGMA], f[FGPU_PRESSURE], f[FGPU_POTENTIAL],
+                      f[FGPU_V_RADIAL], f[FGPU_V_AZIMUTHAL], eng->vr_alt, eng->vaz_alt);
+    }
     std::swap(f[FGPU_V_RADIAL], eng->vr_alt);
     std::swap(f[FGPU_V_AZIMUTHAL], eng->vaz_alt);
     mark(eng, 1);
     State s = state_of(eng);
     // compression heating + artificial viscosity (simulation.cpp:190-194)
     if (adi || eng->ph.art_visc_sn || eng->ph.art_visc_tw) {
-        launch_artvisc_q(L, dt, s.sigma, s.vr, s.vaz, s.energy, s.qr, s.qphi);
-        if (L.pair && (eng->ph.art_visc_sn || eng->ph.art_visc_tw)) eng->q_pairs = true;
-        mark(eng, 2);
-        launch_artvisc_v(L, dt, s.sigma, s.energy, s.qr, s.qphi, s.vr, s.vaz, s.cs, s.H, s.nu);
+        if (L.pair) {
+            // one kernel for both, timed as the second
+            if (eng->ph.art_visc_sn || eng->ph.art_visc_tw) eng->q_pairs = true;
+            mark(eng, 2);
+            launch_artvisc_pair(L, dt, s, eng->vr_alt, eng->vaz_alt);
+            std::swap(f[FGPU_V_RADIAL], eng->vr_alt);
+            std::swap(f[FGPU_V_AZIMUTHAL], eng->vaz_alt);
+            s = state_of(eng);
+        } else {
+            launch_artvisc_q(L, dt, s.sigma, s.vr, s.vaz, s.energy, s.qr, s.qphi);
+            mark(eng, 2);
+            launch_artvisc_v(L, dt, s.sigma, s.energy, s.qr, s.qphi, s.vr, s.vaz, s.cs, s.H,
+                             s.nu);
+        }
         mark(eng, 3);
     } else {
         mark(eng, 2);
         mark(eng, 3);
     }
     // viscous stress and velocity update, SubStep3 (simulation.cpp:196-203)
-    launch_stress(L, s.sigma, s.vr, s.vaz, s.nu, s.divv, s.trr, s.tpp, s.trp);
     eng->stress_pairs = stress_as_pairs(L);
     if (eng->ph.stabilize) launch_visc_corr(L, s);
-    mark(eng, 4);
-    launch_viscous(L, dt, beta_inv_at(eng->p, t), adi ? 7 : 1, s);
+    if (eng->stress_pairs) {
+        // one kernel for both, timed as the viscous phase
+        mark(eng, 4);
+        launch_viscous_pair(L, dt, beta_inv_at(eng->p, t), adi ? 7 : 1, s, eng->vr_alt,
+                            eng->vaz_alt);
+        std::swap(f[FGPU_V_RADIAL], eng->vr_alt);
+        std::swap(f[FGPU_V_AZIMUTHAL], eng->vaz_alt);
+    } else {
+        launch_stress(L, s.sigma, s.vr, s.vaz, s.nu, s.divv, s.trr, s.tpp, s.trp);
+        mark(eng, 4);
+        launch_viscous(L, dt, beta_inv_at(eng->p, t), adi ? 7 : 1, s);
+    }
     mark(eng, 5);
 }
 

@@ -281,6 +281,18 @@ __device__ __forceinline__ f2x2 f2_sfma(f2x2 x, f2x2 a, f2x2 d)
     const f2x2 s = two_sum(x.h, p.h);
     return fast_two_sum(s.h, vadd(s.l, vadd(x.l, pl)));
 }
+// 1 / sqrt(d) for d > 0: the hardware estimate, one FP32 Newton step, then
+// one whose residual 1 - d r^2 is formed from the error-free square of r
+__device__ __forceinline__ f2x2 f2_rsqrt(f2x2 d)
+{
+    float2 r = make_float2(rsqrtf(d.h.x), rsqrtf(d.h.y));
+    const float2 half = make_float2(0.5f, 0.5f), one = make_float2(1.f, 1.f);
+    const float2 mh = vneg(d.h);
+    r = vmul(r, vfma(vmul(half, mh), vmul(r, r), make_float2(1.5f, 1.5f)));
+    const f2x2 r2 = two_prod(r, r);
+    const float2 e = vfma(vneg(d.l), r2.h, vfma(mh, r2.l, vfma(mh, r2.h, one)));
+    return fast_two_sum(r, vmul(vmul(half, r), e));
+}
 __device__ __forceinline__ f2x2 f2_sdiv(f2x2 p, f2x2 s)
 {
     const float2 r = vrcp(s.h);

@@ -37,6 +37,7 @@ struct Tables {
     const double *LSqTW;       // pow(C, 2) * pow(max(Ra[i+1] - Ra[i], Rmed dphi), 2)
     const double *TwoOverDRmed2; // 2 / (pow(Rmed[i], 2) - pow(Rmed[i-1], 2))
     const double *DiffRmed;    // Rmed[i] - Rmed[i-1]
+    const double *DInvRmed;    // 1 / Rmed[i] - 1 / Rmed[i-1]
     // StabilizeViscosity correction factors (viscosity.cpp:256-348)
     const double *Ra3IDRmed;   // pow(Ra[i], 3) * InvDiffRmed[i]
     const double *F43;         // FourThirdInvRbInvdphiSq (init.cpp:213-214)

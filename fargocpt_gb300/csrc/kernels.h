@@ -85,14 +85,20 @@ void launch_pressure(const Launch &L, const double *S, const double *E, double *
 void launch_source_pair(const Launch &L, double dt, double omf, const double *S, const double *Pr,
                         const double *pot, const double *vr_in, const double *vaz_in,
                         double *vr_out, double *vaz_out);
-void launch_artvisc_q_pair(const Launch &L, double dt, const double *S, const double *vr,
-                           const double *vaz, double *E, double *Qr, double *Qp);
-void launch_artvisc_v_pair(const Launch &L, double dt, const double *S, const double *E,
-                           const double *Qr, const double *Qp, double *vr, double *vaz, double *cs,
-                           double *H, double *nu);
 void launch_stress_pair(const Launch &L, const double *S, const double *vr, const double *vaz,
                         const double *nu, double *divv, double *trr, double *tpp, double *trp);
-void launch_viscous_pair(const Launch &L, double dt, double beta_inv, int mode, const State &s);
+// kernels that march windows of cells through the rings (kernels_kick.cu), the
+// velocities into vr_out, vaz_out:
+// the potential and the momentum source terms, for bodies.star_plain
+void launch_source_window(const Launch &L, double dt, double omf, const Bodies &b,
+                          const State &s, double *vr_out, double *vaz_out);
+// compression heating and artificial viscosity
+void launch_artvisc_pair(const Launch &L, double dt, const State &s, double *vr_out,
+                         double *vaz_out);
+// the stress tensor, the viscous velocity update into vr_out, vaz_out (mode
+// bit 1) and SubStep3 (kernels_kick.cu), where stress_as_pairs
+void launch_viscous_pair(const Launch &L, double dt, double beta_inv, int mode, const State &s,
+                         double *vr_out, double *vaz_out);
 // Whether the stress kernel leaves div v and the stress tensor as float pairs
 // (hi, lo in the 8 bytes of each double) for the float-pair viscous kernel,
 // which reads them so, instead of joined doubles; StabilizeViscosity 1's

@@ -2190,7 +2190,6 @@ void launch_source(const Launch &L, double dt, double omf, const double *S, cons
 void launch_artvisc_q(const Launch &L, double dt, const double *S, const double *vr,
                       const double *vaz, double *E, double *Qr, double *Qp)
 {
-    if (L.pair) return launch_artvisc_q_pair(L, dt, S, vr, vaz, E, Qr, Qp);
     k_artvisc_q<<<grid2d(L.g.nz, L.g.nr, L.bx), L.bx, 0, L.stream>>>(L.g, L.t, L.ph, dt, S, vr,
                                                                       vaz, E, Qr, Qp);
 }
@@ -2199,7 +2198,6 @@ void launch_artvisc_v(const Launch &L, double dt, const double *S, const double 
                       const double *Qr, const double *Qp, double *vr, double *vaz, double *cs,
                       double *H, double *nu)
 {
-    if (L.pair) return launch_artvisc_v_pair(L, dt, S, E, Qr, Qp, vr, vaz, cs, H, nu);
     k_artvisc_v<<<grid2d(L.g.nz, L.g.nr, L.bx), L.bx, 0, L.stream>>>(L.g, L.t, L.ph, dt, S, E, Qr,
                                                                       Qp, vr, vaz, cs, H, nu);
 }
@@ -2214,8 +2212,6 @@ void launch_stress(const Launch &L, const double *S, const double *vr, const dou
 
 void launch_viscous(const Launch &L, double dt, double beta_inv, int mode, const State &s)
 {
-    // StabilizeViscosity's corrected update is the FP64 kernel's
-    if (L.pair && L.ph.stabilize != 1) return launch_viscous_pair(L, dt, beta_inv, mode, s);
     k_viscous<<<grid2d(L.g.nz, L.g.nr, L.bx), L.bx, 0, L.stream>>>(
         L.g, L.t, L.ph, dt, beta_inv, mode, s.sigma, s.trr, s.tpp, s.trp, s.divv, s.nu, s.H,
         s.sigma0, s.energy0, s.vr, s.vaz, s.energy, s.qplus, s.qminus, s.corr_phi, s.corr_r);
