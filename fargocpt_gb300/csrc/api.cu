@@ -1414,9 +1414,9 @@ static void viscous_recompute(fgpu_engine *eng, const Launch &L)
     }
 }
 
-static void ghost(fgpu_engine *eng, const Launch &L)
+static void ghost(fgpu_engine *eng, const Launch &L, unsigned long long *dt_min = nullptr)
 {
-    launch_ghost(L, eng->bc, eng->bodies.omega_frame, state_of(eng));
+    launch_ghost(L, eng->bc, eng->bodies.omega_frame, state_of(eng), dt_min);
 }
 
 // The centre-of-mass composite: its damping runs after the regular damping
@@ -1736,12 +1736,11 @@ extern "C" int fgpu_step_euler(fgpu_engine *eng, double dt, double t)
         com_damping(eng, L, dt, eng->com_after);
     }
     mark(eng, 10);
-    ghost(eng, L);
+    ghost(eng, L, eng->d_dtmin);  // resets the CFL minimum formed below
     com_boundary(eng, L, eng->com_after);
     keep_mass(eng, L);
     mark(eng, 11);
     // recalculate_derived_disk_quantities (simulation.cpp:265) + the next CFL
-    CK(cudaMemsetAsync(eng->d_dtmin, 0x7f, sizeof(unsigned long long), eng->stream));
     launch_derived_cfl(L, 1 | 4, s, eng->d_dtmin);
     mark(eng, 12);
     eng->cfl_valid = true;

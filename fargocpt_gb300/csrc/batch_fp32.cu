@@ -22,6 +22,7 @@
 // Tile shapes (threads per block, rings per block or per thread) are
 // per-kernel and chosen by an autotuner that times candidates on the batch's
 // own state with CUDA events and restores the state afterwards.
+#include "launch.cuh"
 #include "../../include/fargocpt_gb300.h"
 #include "fp32_device.cuh"
 #include "fp32_engine.h"
@@ -88,6 +89,7 @@ __device__ __forceinline__ void for_cells(const DiskF *__restrict__ D, const Ste
 __global__ void b_potential(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                             const int *__restrict__ start, int nd, int rpb)
 {
+    fgpu::follow_predecessor();
     for_cells(D, S, start, nd, rpb, 0, [&](const DiskF &k, const StepF &st, int i, int j) {
         potential_cell(k.g, k.t, k.ph, st.b, k.H, k.pot, i, j);
     });
@@ -96,6 +98,7 @@ __global__ void b_potential(const DiskF *__restrict__ D, const StepF *__restrict
 __global__ void b_source(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                          const int *__restrict__ start, int nd, int rpb)
 {
+    fgpu::follow_predecessor();
     for_cells(D, S, start, nd, rpb, 1, [&](const DiskF &k, const StepF &st, int i, int j) {
         source_cell(k.g, k.t, st.fdt, k.s.sigma, k.P, k.pot, k.s.vr, k.s.dv, k.vr_b, k.dv_b, i, j);
     });
@@ -104,6 +107,7 @@ __global__ void b_source(const DiskF *__restrict__ D, const StepF *__restrict__ 
 __global__ void b_artvisc_q(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                             const int *__restrict__ start, int nd, int rpb)
 {
+    fgpu::follow_predecessor();
     for_cells(D, S, start, nd, rpb, 0, [&](const DiskF &k, const StepF &st, int i, int j) {
         if (!(k.ph.adiabatic || k.ph.art_visc_sn || k.ph.art_visc_tw)) return;
         artvisc_q_cell(k.g, k.t, k.ph, st.fdt, k.s.sigma, k.vr_b, k.dv_b, k.s.energy, k.Qr, k.Qp,
@@ -114,6 +118,7 @@ __global__ void b_artvisc_q(const DiskF *__restrict__ D, const StepF *__restrict
 __global__ void b_artvisc_v(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                             const int *__restrict__ start, int nd, int rpb)
 {
+    fgpu::follow_predecessor();
     for_cells(D, S, start, nd, rpb, 0, [&](const DiskF &k, const StepF &st, int i, int j) {
         if (!(k.ph.adiabatic || k.ph.art_visc_sn || k.ph.art_visc_tw)) return;
         artvisc_v_cell(k.g, k.t, k.ph, st.fdt, k.s.sigma, k.s.energy, k.Qr, k.Qp, k.vr_b, k.dv_b,
@@ -124,6 +129,7 @@ __global__ void b_artvisc_v(const DiskF *__restrict__ D, const StepF *__restrict
 __global__ void b_stress(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                          const int *__restrict__ start, int nd, int rpb)
 {
+    fgpu::follow_predecessor();
     for_cells(D, S, start, nd, rpb, 0, [&](const DiskF &k, const StepF &, int i, int j) {
         stress_cell(k.g, k.t, k.s.sigma, k.vr_b, k.dv_b, k.nu, k.divv, k.trr, k.tpp, k.trp, i, j);
     });
@@ -132,6 +138,7 @@ __global__ void b_stress(const DiskF *__restrict__ D, const StepF *__restrict__ 
 __global__ void b_viscous(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                           const int *__restrict__ start, int nd, int rpb)
 {
+    fgpu::follow_predecessor();
     for_cells(D, S, start, nd, rpb, 0, [&](const DiskF &k, const StepF &st, int i, int j) {
         viscous_cell(k.g, k.t, k.ph, st.fdt, st.beta_inv, k.ph.adiabatic ? 7 : 1, k.s.sigma, k.trr,
                      k.tpp, k.trp, k.divv, k.nu, k.H, k.s.sigma0, k.s.energy0, k.vr_b, k.dv_b,
@@ -142,6 +149,7 @@ __global__ void b_viscous(const DiskF *__restrict__ D, const StepF *__restrict__
 __global__ void b_finish(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                          const int *__restrict__ start, int nd, int rpb)
 {
+    fgpu::follow_predecessor();
     for_cells(D, S, start, nd, rpb, 1, [&](const DiskF &k, const StepF &, int i, int j) {
         finish_cell(k.g, k.t, k.ph, k.mom_w[0], k.mom_w[1], k.mom_w[2], k.mom_w[3], k.sigma_w,
                     k.energy_w, k.vr_b, k.s.vr, k.s.dv, k.s.sigma, k.s.energy, k.sigma_lo_w,
@@ -153,8 +161,10 @@ __global__ void b_finish(const DiskF *__restrict__ D, const StepF *__restrict__ 
 __global__ void b_ghost(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                         const int *__restrict__ start, int nd, int use_b)
 {
-    const int total = __ldg(start + nd);
-    for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
+    fgpu::follow_predecessor();
+    const int total = __ldg(start + nd) * kGhostParts;
+    for (int item = blockIdx.x; item < total; item += gridDim.x) {
+        const int tile = item / kGhostParts;
         const int d = disk_of(start, nd, tile);
         if (!S[d].run) continue;
         const DiskF &k = D[d];
@@ -165,7 +175,7 @@ __global__ void b_ghost(const DiskF *__restrict__ D, const StepF *__restrict__ S
             st.vr = k.vr_b;
             st.dv = k.dv_b;
         }
-        ghost_col(k.g, k.bc, st, j);
+        ghost_col(k.g, k.bc, st, j, item % kGhostParts);
     }
 }
 
@@ -177,6 +187,7 @@ __global__ void b_transport_radial(const DiskF *__restrict__ D, const StepF *__r
                                    const int *__restrict__ start, int nd, int chunk,
                                    const int *__restrict__ rings)
 {
+    fgpu::follow_predecessor();
     // the ring phases of the window azimuthal pass first (rings: tile starts
     // of one tile per ring, or null): latency-bound sums that the sweep's
     // tiles overlap
@@ -247,6 +258,7 @@ __global__ void __launch_bounds__(512)
     b_transport_azimuthal_w(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                             const int *__restrict__ start, int nd)
 {
+    fgpu::follow_predecessor();
     const int total = __ldg(start + nd), warps = blockDim.x >> 5;
     for (int job = blockIdx.x * warps + (threadIdx.x >> 5); job < total;
          job += gridDim.x * warps) {
@@ -269,6 +281,7 @@ __global__ void __launch_bounds__(512)
 __global__ void b_damping(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                           const int2 *__restrict__ items, int n)
 {
+    fgpu::follow_predecessor();
     __shared__ float red[33];
     __shared__ long long redl[33];
     for (int it = blockIdx.x; it < 4 * n; it += gridDim.x) {
@@ -284,6 +297,7 @@ __global__ void b_damping(const DiskF *__restrict__ D, const StepF *__restrict__
 __global__ void b_derived_cfl(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                               const int *__restrict__ start, int nd, int mode, int all)
 {
+    fgpu::follow_predecessor();
     __shared__ float red[33];
     __shared__ longlong2 red2[33];
     const int total = __ldg(start + nd);
@@ -364,8 +378,9 @@ __global__ void b_kick_sequence(const DiskF *__restrict__ D, const StepF *__rest
     grid.sync();
     // the mid-step ghost rings (B buffers), as b_ghost
     const int *gt = tab(FGPU_BK_GHOST);
-    const int total = __ldg(gt + nd);
-    for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
+    const int total = __ldg(gt + nd) * kGhostParts;
+    for (int item = blockIdx.x; item < total; item += gridDim.x) {
+        const int tile = item / kGhostParts;
         const int d = disk_of(gt, nd, tile);
         if (!S[d].run) continue;
         const DiskF &k = D[d];
@@ -374,7 +389,7 @@ __global__ void b_kick_sequence(const DiskF *__restrict__ D, const StepF *__rest
         StateF st = k.s;
         st.vr = k.vr_b;
         st.dv = k.dv_b;
-        ghost_col(k.g, k.bc, st, j);
+        ghost_col(k.g, k.bc, st, j, item % kGhostParts);
     }
 }
 
@@ -409,14 +424,15 @@ __global__ void b_close_sequence(const DiskF *__restrict__ D, const StepF *__res
     grid.sync();
     // the end-of-step ghost rings (A buffers), as b_ghost
     const int *gt = tab(FGPU_BK_GHOST);
-    const int total = __ldg(gt + nd);
-    for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
+    const int total = __ldg(gt + nd) * kGhostParts;
+    for (int item = blockIdx.x; item < total; item += gridDim.x) {
+        const int tile = item / kGhostParts;
         const int d = disk_of(gt, nd, tile);
         if (!S[d].run) continue;
         const DiskF &k = D[d];
         const int j = (tile - __ldg(gt + d)) * blockDim.x + threadIdx.x;
         if (j >= k.g.nz) continue;
-        ghost_col(k.g, k.bc, k.s, j);
+        ghost_col(k.g, k.bc, k.s, j, item % kGhostParts);
     }
     grid.sync();
     // derived quantities and the CFL minimum, as b_derived_cfl
@@ -435,6 +451,7 @@ __global__ void b_close_sequence(const DiskF *__restrict__ D, const StepF *__res
 
 __global__ void b_reset_dtmin(const DiskF *__restrict__ D, const StepF *__restrict__ S, int nd)
 {
+    fgpu::follow_predecessor();
     const int d = blockIdx.x * blockDim.x + threadIdx.x;
     if (d < nd && S[d].run) *D[d].dtmin = 0x7f7f7f7fu;
 }
@@ -485,6 +502,7 @@ struct ClockAux {
 __global__ void b_clock(const DiskF *__restrict__ D, const ClockAux *__restrict__ aux,
                         ClockF *__restrict__ C, StepF *__restrict__ S, int nd, int *n_active)
 {
+    fgpu::follow_predecessor();
     const int d = threadIdx.x;
     int act = 0;
     if (d < nd) {
@@ -751,7 +769,9 @@ static int apply_tiles(fgpu_batch *b, const fgpu_tiles &t)
             return FGPU_ERR_UNSUPPORTED;
         }
         s[nd] = (int)acc;
-        totals[k] = k == FGPU_BK_DAMPING ? 4LL * b->n_damp_items : acc;
+        totals[k] = k == FGPU_BK_DAMPING ? 4LL * b->n_damp_items
+                    : k == FGPU_BK_GHOST ? kGhostParts * acc
+                                         : acc;
         if (k == FGPU_BK_TRANSPORT_AZIMUTHAL && b->windows) {
             const int warps = th / 32;  // windows per block
             totals[k] = (acc + warps - 1) / warps;
@@ -809,35 +829,35 @@ static void launch_kernel(fgpu_batch *b, int k, int ghost_b = 0)
     const StepF *S = b->d_steps;
     cudaStream_t s = b->stream;
     switch (k) {
-    case FGPU_BK_POTENTIAL: b_potential<<<g, th, 0, s>>>(D, S, b->table(k), nd, r); break;
-    case FGPU_BK_SOURCE: b_source<<<g, th, 0, s>>>(D, S, b->table(k), nd, r); break;
-    case FGPU_BK_ARTVISC_Q: b_artvisc_q<<<g, th, 0, s>>>(D, S, b->table(k), nd, r); break;
-    case FGPU_BK_ARTVISC_V: b_artvisc_v<<<g, th, 0, s>>>(D, S, b->table(k), nd, r); break;
-    case FGPU_BK_STRESS: b_stress<<<g, th, 0, s>>>(D, S, b->table(k), nd, r); break;
-    case FGPU_BK_VISCOUS: b_viscous<<<g, th, 0, s>>>(D, S, b->table(k), nd, r); break;
-    case FGPU_BK_GHOST: b_ghost<<<g, th, 0, s>>>(D, S, b->table(k), nd, ghost_b); break;
+    case FGPU_BK_POTENTIAL: fgpu::launch(b_potential, g, th, 0, s, D, S, b->table(k), nd, r); break;
+    case FGPU_BK_SOURCE: fgpu::launch(b_source, g, th, 0, s, D, S, b->table(k), nd, r); break;
+    case FGPU_BK_ARTVISC_Q: fgpu::launch(b_artvisc_q, g, th, 0, s, D, S, b->table(k), nd, r); break;
+    case FGPU_BK_ARTVISC_V: fgpu::launch(b_artvisc_v, g, th, 0, s, D, S, b->table(k), nd, r); break;
+    case FGPU_BK_STRESS: fgpu::launch(b_stress, g, th, 0, s, D, S, b->table(k), nd, r); break;
+    case FGPU_BK_VISCOUS: fgpu::launch(b_viscous, g, th, 0, s, D, S, b->table(k), nd, r); break;
+    case FGPU_BK_GHOST: fgpu::launch(b_ghost, g, th, 0, s, D, S, b->table(k), nd, ghost_b); break;
     case FGPU_BK_TRANSPORT_RADIAL: {
         const int *rings = b->windows ? b->table(FGPU_BK_DERIVED_CFL) : nullptr;
-        if (b->any_iso) b_transport_radial<4><<<g, th, 0, s>>>(D, S, b->table(k), nd, r, rings);
-        if (b->any_adi) b_transport_radial<5><<<g, th, 0, s>>>(D, S, b->table(k), nd, r, rings);
+        if (b->any_iso) fgpu::launch(b_transport_radial<4>, g, th, 0, s, D, S, b->table(k), nd, r, rings);
+        if (b->any_adi) fgpu::launch(b_transport_radial<5>, g, th, 0, s, D, S, b->table(k), nd, r, rings);
         break;
     }
     case FGPU_BK_TRANSPORT_AZIMUTHAL:
         if (b->windows) {
-            if (b->any_iso) b_transport_azimuthal_w<4><<<g, th, 0, s>>>(D, S, b->table(k), nd);
-            if (b->any_adi) b_transport_azimuthal_w<5><<<g, th, 0, s>>>(D, S, b->table(k), nd);
+            if (b->any_iso) fgpu::launch(b_transport_azimuthal_w<4>, g, th, 0, s, D, S, b->table(k), nd);
+            if (b->any_adi) fgpu::launch(b_transport_azimuthal_w<5>, g, th, 0, s, D, S, b->table(k), nd);
         } else {
             if (b->any_iso) az_fn(b->az_per, 4)<<<g, th, b->az_smem, s>>>(D, S, b->table(k), nd);
             if (b->any_adi) az_fn(b->az_per, 5)<<<g, th, b->az_smem, s>>>(D, S, b->table(k), nd);
         }
         break;
-    case FGPU_BK_FINISH: b_finish<<<g, th, 0, s>>>(D, S, b->table(k), nd, r); break;
+    case FGPU_BK_FINISH: fgpu::launch(b_finish, g, th, 0, s, D, S, b->table(k), nd, r); break;
     case FGPU_BK_DAMPING:
         if (b->n_damp_items)
-            b_damping<<<g, th, 0, s>>>(D, S, b->d_damp_items, b->n_damp_items);
+            fgpu::launch(b_damping, g, th, 0, s, D, S, b->d_damp_items, b->n_damp_items);
         break;
     case FGPU_BK_DERIVED_CFL:
-        b_derived_cfl<<<g, th, 0, s>>>(D, S, b->table(k), nd, 1 | 4, 0);
+        fgpu::launch(b_derived_cfl, g, th, 0, s, D, S, b->table(k), nd, 1 | 4, 0);
         break;
     default: break;
     }
@@ -872,10 +892,10 @@ static void launch_sequence(fgpu_batch *b, int q)
 static void enqueue_step(fgpu_batch *b, bool device_clock)
 {
     if (device_clock)
-        b_clock<<<1, (b->nd + 31) / 32 * 32, 0, b->stream>>>(b->d_disks, b->d_aux, b->d_clocks,
+        fgpu::launch(b_clock, 1, (b->nd + 31) / 32 * 32, 0, b->stream, b->d_disks, b->d_aux, b->d_clocks,
                                                              b->d_steps, b->nd, b->d_active);
     else
-        b_reset_dtmin<<<(b->nd + 127) / 128, 128, 0, b->stream>>>(b->d_disks, b->d_steps, b->nd);
+        fgpu::launch(b_reset_dtmin, (b->nd + 127) / 128, 128, 0, b->stream, b->d_disks, b->d_steps, b->nd);
     if (b->mode == FGPU_BATCH_PERSISTENT) {
         launch_sequence(b, 0);
         launch_kernel(b, FGPU_BK_TRANSPORT_RADIAL);

@@ -675,26 +675,40 @@ __device__ __forceinline__ void ghost_f(float *x, const float *x0, int kind, int
     }
 }
 
-__device__ __forceinline__ void ghost_col(const GeoF &g, const BcF &bc, const StateF &s, int j)
+// hook part (0 .. 7: field, then edge) of column j; the hooks are independent
+// (each writes the ghost rings of its field and edge)
+constexpr int kGhostParts = 8;
+__device__ __forceinline__ void ghost_col(const GeoF &g, const BcF &bc, const StateF &s, int j,
+                                          int part)
 {
-    const int nz = g.nz, nr = g.nr;
-    ghost_f(s.sigma, s.sigma0, bc.sigma_in, 0, 0, nr, nz, j, 0.f, 0.f, bc.val_in[0], bc.nu);
-    ghost_f(s.sigma, s.sigma0, bc.sigma_out, 1, 0, nr, nz, j, 0.f, 0.f, bc.val_out[0], bc.nu);
-    // low part of sigma: copied by zero-gradient, cleared by reference hooks,
-    // the disk model's own low part
-    if (bc.sigma_in == 1) s.sigma_lo[CELL(0, j)] = s.sigma_lo[CELL(1, j)];
-    else if (bc.sigma_in == 3) s.sigma_lo[CELL(0, j)] = 0.f;
-    else if (bc.sigma_in == 5) s.sigma_lo[CELL(0, j)] = bc.val_in[0][1];
-    if (bc.sigma_out == 1) s.sigma_lo[CELL(nr - 1, j)] = s.sigma_lo[CELL(nr - 2, j)];
-    else if (bc.sigma_out == 3) s.sigma_lo[CELL(nr - 1, j)] = 0.f;
-    else if (bc.sigma_out == 5) s.sigma_lo[CELL(nr - 1, j)] = bc.val_out[0][1];
-    ghost_f(s.energy, s.energy0, bc.energy_in, 0, 0, nr, nz, j, 0.f, 0.f, bc.val_in[1], bc.nu);
-    ghost_f(s.energy, s.energy0, bc.energy_out, 1, 0, nr, nz, j, 0.f, 0.f, bc.val_out[1], bc.nu);
-    ghost_f(s.vr, s.vr0, bc.vr_in, 0, 1, nr, nz, j, 0.f, 0.f, bc.val_in[2], bc.nu);
-    ghost_f(s.vr, s.vr0, bc.vr_out, 1, 1, nr, nz, j, 0.f, 0.f, bc.val_out[2], bc.nu);
-    ghost_f(s.dv, s.dv0, bc.vaz_in, 0, 0, nr, nz, j, bc.kep_in, bc.zg_in, bc.val_in[3], bc.nu);
-    ghost_f(s.dv, s.dv0, bc.vaz_out, 1, 0, nr, nz, j, bc.kep_out, bc.zg_out, bc.val_out[3],
-            bc.nu);
+    const int nz = g.nz, nr = g.nr, outer = part & 1;
+    switch (part >> 1) {
+    case 0: {
+        const int kind = outer ? bc.sigma_out : bc.sigma_in;
+        const float *val = outer ? bc.val_out[0] : bc.val_in[0];
+        ghost_f(s.sigma, s.sigma0, kind, outer, 0, nr, nz, j, 0.f, 0.f, val, bc.nu);
+        // low part of sigma: copied by zero-gradient, cleared by reference hooks,
+        // the disk model's own low part
+        const int e = outer ? nr - 1 : 0, n = outer ? nr - 2 : 1;
+        if (kind == 1) s.sigma_lo[CELL(e, j)] = s.sigma_lo[CELL(n, j)];
+        else if (kind == 3) s.sigma_lo[CELL(e, j)] = 0.f;
+        else if (kind == 5) s.sigma_lo[CELL(e, j)] = val[1];
+        break;
+    }
+    case 1:
+        ghost_f(s.energy, s.energy0, outer ? bc.energy_out : bc.energy_in, outer, 0, nr, nz, j,
+                0.f, 0.f, outer ? bc.val_out[1] : bc.val_in[1], bc.nu);
+        break;
+    case 2:
+        ghost_f(s.vr, s.vr0, outer ? bc.vr_out : bc.vr_in, outer, 1, nr, nz, j, 0.f, 0.f,
+                outer ? bc.val_out[2] : bc.val_in[2], bc.nu);
+        break;
+    default:
+        ghost_f(s.dv, s.dv0, outer ? bc.vaz_out : bc.vaz_in, outer, 0, nr, nz, j,
+                outer ? bc.kep_out : bc.kep_in, outer ? bc.zg_out : bc.zg_in,
+                outer ? bc.val_out[3] : bc.val_in[3], bc.nu);
+        break;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1708,9 +1722,10 @@ __device__ __forceinline__ void finish_cell(
 // red: 33 floats, redl: 33 long longs (shared memory)
 __device__ __forceinline__ void damp_ring_f(float *X, float *X0, const DampQF &d, int i, int nz,
                                             int outer, float dt, float *red, float *Xlo,
-                                            long long *redl)
+                                            long long *redl, int part, int parts)
 {
     const int kind = outer ? d.kind_out : d.kind_in;
+    if (kind == 3 && part > 0) return;  // the whole block
     const size_t row = (size_t)i * nz;
     float x0c = 0.f;
     if (kind == 3) {
@@ -1723,10 +1738,25 @@ __device__ __forceinline__ void damp_ring_f(float *X, float *X0, const DampQF &d
     const float factor = outer ? d.fac_out[i] : d.fac_in[i];
     const float tau = outer ? d.tau_out : d.tau_in;
     const float ef = __expf(-dt * factor / tau);
-    for (int j = threadIdx.x; j < nz; j += blockDim.x) {
-        const float x0 = kind == 1 ? X0[row + j] : x0c;
-        X[row + j] = (X[row + j] - x0) * ef + x0;
-        if (Xlo) Xlo[row + j] *= ef;
+    // a ring's blocks share its columns (the mean kind's one block takes them
+    // all), four loads of each thread in flight
+    const int step = kind == 3 ? blockDim.x : blockDim.x * parts;
+    const int first = kind == 3 ? threadIdx.x : part * blockDim.x + threadIdx.x;
+    for (int j = first; j < nz; j += 4 * step) {
+        float x[4], x0[4], lo[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int jj = min(j + k * step, nz - 1);
+            x[k] = X[row + jj];
+            x0[k] = kind == 1 ? X0[row + jj] : x0c;
+            lo[k] = Xlo ? Xlo[row + jj] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (j + k * step >= nz) break;
+            X[row + j + k * step] = (x[k] - x0[k]) * ef + x0[k];
+            if (Xlo) Xlo[row + j + k * step] = lo[k] * ef;
+        }
     }
     __syncthreads();
 }
@@ -1735,7 +1765,8 @@ __device__ __forceinline__ void damp_ring_f(float *X, float *X0, const DampQF &d
 // independent of one another)
 __device__ __forceinline__ void damping_ring(const GeoF &g, const DampingF &dm, float dt,
                                              const StateF &s, int i, float *red, long long *redl,
-                                             int q0 = 0, int q1 = 4)
+                                             int q0 = 0, int q1 = 4, int part = 0,
+                                             int parts = 1)
 {
     const int nz = g.nz, nr = g.nr;
     float *X[4] = {s.vr, s.dv, s.sigma, s.energy};
@@ -1745,9 +1776,9 @@ __device__ __forceinline__ void damping_ring(const GeoF &g, const DampingF &dm, 
         const int size = d.vector ? nr + 1 : nr;
         float *lo = q == 2 ? s.sigma_lo : nullptr;
         if (d.kind_in != 0 && d.active_in && i <= d.limit_in)
-            damp_ring_f(X[q], X0[q], d, i, nz, 0, dt, red, lo, redl);
+            damp_ring_f(X[q], X0[q], d, i, nz, 0, dt, red, lo, redl, part, parts);
         if (d.kind_out != 0 && d.active_out && i >= d.limit_out && i < size)
-            damp_ring_f(X[q], X0[q], d, i, nz, 1, dt, red, lo, redl);
+            damp_ring_f(X[q], X0[q], d, i, nz, 1, dt, red, lo, redl, part, parts);
     }
 }
 

@@ -192,7 +192,8 @@ class Engine32 {
     // correct_v_azimuthal: the frame velocities less dOmega * Rmed
     void correct_v_azimuthal(double domega) { pend_dv -= domega; }
     int init_euler(double t);
-    int derived_cfl(int mode);
+    // reset: clear the CFL minimum first (mode bit 4)
+    int derived_cfl(int mode, bool reset = true);
     int cfl(double *dt_out);
     int boundary(double dt, bool final);
     int step(double dt, double t);

@@ -46,7 +46,9 @@ void launch_stress(const Launch &L, const double *S, const double *vr, const dou
                    const double *nu, double *divv, double *trr, double *tpp, double *trp);
 void launch_viscous(const Launch &L, double dt, double beta_inv, int mode, const State &s);
 void launch_visc_corr(const Launch &L, const State &s);
-void launch_ghost(const Launch &L, const BcSpec &bc, double omf, const State &s);
+// dt_min: reset to a huge step, for the CFL kernel that follows (or null)
+void launch_ghost(const Launch &L, const BcSpec &bc, double omf, const State &s,
+                  unsigned long long *dt_min);
 void launch_com_boundary(const Launch &L, const ComSpec &c, const State &s);
 void launch_correct_vaz(const Launch &L, double domega, double *vaz);
 void launch_cfl_cells(const Launch &L, const State &s, double *out);

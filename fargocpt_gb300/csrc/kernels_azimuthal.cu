@@ -35,6 +35,7 @@
 // Measured, ms per pass (ring kernel in shared memory -> this): 2048 x 6144
 // 1.377 -> 0.543, 512 x 1536 0.127 -> 0.041, 128 x 384 isothermal 0.020 ->
 // 0.010.  At 96 registers (5 blocks per SM, 92 bytes of spills) 0.551.
+#include "launch.cuh"
 #include "fp64_pair.cuh"
 #include "hydro.cuh"
 #include "kernels.h"
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(kThreads, 4)
                             const double *__restrict__ vaz, Rows rows,
                             const RingPhase *__restrict__ phase)
 {
+    follow_predecessor();
     const int lane = threadIdx.x & 31;
     const int job = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const int i = job / windows;
@@ -336,7 +338,7 @@ void launch_transport_azimuthal_pair(const Launch &L, double *const mom[4], cons
     using F = std::false_type;
     auto k = L.ph.adiabatic ? (aligned ? pick(T{}, T{}) : pick(T{}, F{}))
                             : (aligned ? pick(F{}, T{}) : pick(F{}, F{}));
-    k<<<(L.g.nr * windows + per - 1) / per, kThreads, 0, L.stream>>>(
+    launch(k, (L.g.nr * windows + per - 1) / per, kThreads, 0, L.stream,
         L.g.nz, L.g.nr, windows, L.ph.fast_transport, vaz, r, phase);
 }
 

@@ -22,6 +22,7 @@
 // and per-ring bodies live in fp32_device.cuh, shared with the batched
 // many-disk kernels (batch_fp32.cu); this file holds the single-disk kernels
 // around them and the host engine.
+#include "launch.cuh"
 #include "../../include/fargocpt_gb300.h"
 #include "fp32_engine.h"
 #include "fp32_device.cuh"
@@ -45,6 +46,7 @@ namespace fgpu32 {
 __global__ void f_potential(GeoF g, TablesF t, PhysF ph, BodiesF b, const float *__restrict__ H,
                             float *__restrict__ pot)
 {
+    fgpu::follow_predecessor();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= g.nz) return;
     potential_cell(g, t, ph, b, H, pot, blockIdx.y, j);
@@ -55,6 +57,7 @@ __global__ void f_source(GeoF g, TablesF t, float dt, const float *__restrict__ 
                          const float *__restrict__ vr_in, const float *__restrict__ dv_in,
                          float *__restrict__ vr_out, float *__restrict__ dv_out)
 {
+    fgpu::follow_predecessor();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= g.nz) return;
     source_cell(g, t, dt, S, P, pot, vr_in, dv_in, vr_out, dv_out, blockIdx.y, j);
@@ -64,6 +67,7 @@ __global__ void f_artvisc_q(GeoF g, TablesF t, PhysF ph, float dt, const float *
                             const float *__restrict__ vr, const float *__restrict__ dv,
                             float *__restrict__ E, float *__restrict__ Qr, float *__restrict__ Qp)
 {
+    fgpu::follow_predecessor();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= g.nz) return;
     artvisc_q_cell(g, t, ph, dt, S, vr, dv, E, Qr, Qp, blockIdx.y, j);
@@ -75,6 +79,7 @@ __global__ void f_artvisc_v(GeoF g, TablesF t, PhysF ph, float dt, const float *
                             float *__restrict__ dv, float *__restrict__ cs, float *__restrict__ H,
                             float *__restrict__ nu)
 {
+    fgpu::follow_predecessor();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= g.nz) return;
     artvisc_v_cell(g, t, ph, dt, S, E, Qr, Qp, vr, dv, cs, H, nu, blockIdx.y, j);
@@ -85,6 +90,7 @@ __global__ void f_stress(GeoF g, TablesF t, const float *__restrict__ S, const f
                          float *__restrict__ divv, float *__restrict__ trr, float *__restrict__ tpp,
                          float *__restrict__ trp)
 {
+    fgpu::follow_predecessor();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= g.nz) return;
     stress_cell(g, t, S, vr, dv, nu, divv, trr, tpp, trp, blockIdx.y, j);
@@ -100,6 +106,7 @@ __global__ void f_viscous(GeoF g, TablesF t, PhysF ph, float dt, float beta_inv,
                           float *__restrict__ qminus, const float *__restrict__ corr_phi,
                           const float *__restrict__ corr_r)
 {
+    fgpu::follow_predecessor();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= g.nz) return;
     viscous_cell(g, t, ph, dt, beta_inv, mode, S, trr, tpp, trp, divv, nu, H, S0, E0, vr, dv, E,
@@ -117,11 +124,14 @@ __global__ void f_visc_corr(GeoF g, TablesF t, const float *__restrict__ S,
     visc_corr_cell(g, t, S, nu, corr_phi, corr_r, i, j);
 }
 
-__global__ void f_ghost(GeoF g, BcF bc, StateF s)
+__global__ void f_ghost(GeoF g, BcF bc, StateF s, unsigned int *dt_min)
 {
+    fgpu::follow_predecessor();
+    // the CFL minimum the next kernel forms (its start, as a memset of 0x7f)
+    if (dt_min && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *dt_min = 0x7f7f7f7fu;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= g.nz) return;
-    ghost_col(g, bc, s, j);
+    ghost_col(g, bc, s, j, blockIdx.y);
 }
 
 // 64-thread blocks, 16 per SM (64 registers, about 100 bytes of spills to
@@ -138,6 +148,7 @@ __global__ void __launch_bounds__(64, 16) f_transport_radial(GeoF g, TablesF t, 
                                    double dt_d, int phase_rows, float2 *__restrict__ phase,
                                    int *__restrict__ ring_shift)
 {
+    fgpu::follow_predecessor();
     // the first rows of blocks form the ring phases of the window azimuthal
     // pass, a warp per ring: latency-bound sums that the sweep's blocks behind
     // them overlap (2048 x 6144: 0.300 ms, the sweep alone 0.295; as a launch
@@ -162,6 +173,7 @@ __global__ void __launch_bounds__(kWinThreads) f_transport_azimuthal_w(GeoF g, T
                                                                        int nwin, WindowRows rows,
                                                                        const float2 *__restrict__ phase)
 {
+    fgpu::follow_predecessor();
     const int job = blockIdx.x * (kWinThreads / 32) + (threadIdx.x >> 5);
     const int i = job / nwin;
     if (i >= g.nr) return;
@@ -216,6 +228,7 @@ __global__ void f_finish(GeoF g, TablesF t, PhysF ph, const float *__restrict__ 
                          const float *__restrict__ Slo_t, float *__restrict__ Slo_out,
                          const int *__restrict__ shift)
 {
+    fgpu::follow_predecessor();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= g.nz) return;
     finish_cell(g, t, ph, m0, m1, m2, m3, S_t, E_t, vr_in, vr_out, dv_out, S_out, E_out, Slo_t,
@@ -224,10 +237,12 @@ __global__ void f_finish(GeoF g, TablesF t, PhysF ph, const float *__restrict__ 
 
 __global__ void f_damping(GeoF g, DampingF dm, float dt, const int *__restrict__ rings, StateF s)
 {
+    fgpu::follow_predecessor();
     __shared__ float red[33];
     __shared__ long long redl[33];
     // one block per (ring, damped field)
-    damping_ring(g, dm, dt, s, rings[blockIdx.x], red, redl, blockIdx.y, blockIdx.y + 1);
+    damping_ring(g, dm, dt, s, rings[blockIdx.x], red, redl, blockIdx.y, blockIdx.y + 1,
+                 blockIdx.z, gridDim.z);
 }
 
 __global__ void f_derived_cfl(GeoF g, TablesF t, PhysF ph, int mode, const float *__restrict__ S,
@@ -239,6 +254,7 @@ __global__ void f_derived_cfl(GeoF g, TablesF t, PhysF ph, int mode, const float
                               const float *__restrict__ corr_phi,
                               const float *__restrict__ corr_r)
 {
+    fgpu::follow_predecessor();
     __shared__ float red[33];
     __shared__ longlong2 red2[33];
     derived_cfl_ring(g, t, ph, mode, S, E, vr, dv, qplus, qminus, cs, H, P, T, nu, dt_min,
@@ -262,6 +278,7 @@ __global__ void f_disk_force_bodies(GeoF g, TablesF t, PhysF ph, ForceBodies32 f
                                     const float *__restrict__ S_lo, const float *__restrict__ H,
                                     double *__restrict__ partial, int width)
 {
+    fgpu::follow_predecessor();
     __shared__ double red[33];
     const int nz = g.nz;
     const int i = blockIdx.x + 1;
@@ -348,7 +365,8 @@ __global__ void f_disk_force_bodies(GeoF g, TablesF t, PhysF ph, ForceBodies32 f
 __global__ void f_reduce_cols(const double *__restrict__ partial, int rows, int width,
                               double *__restrict__ out)
 {
-    warp_compensated_rows(partial, rows, width, blockIdx.x, out);
+    fgpu::follow_predecessor();
+    block_compensated_rows(partial, rows, width, blockIdx.x, out);
 }
 
 // one warp per component
@@ -1069,12 +1087,12 @@ void Engine32::set_bodies(int n, const fgpu_body *b, double ix, double iy, doubl
 
 static dim3 grid2(int nz, int rows) { return dim3((nz + 127) / 128, rows); }
 
-int Engine32::derived_cfl(int mode)
+int Engine32::derived_cfl(int mode, bool reset)
 {
     if (int rc_ = sync_frame()) return rc_;
     StateF s = state();
-    if (mode & 4) CKF(cudaMemsetAsync(d_dtmin, 0x7f, sizeof(unsigned int), stream));
-    f_derived_cfl<<<nr, 256, 0, stream>>>(geo, tabs, phys, mode, s.sigma, s.energy, s.vr, s.dv,
+    if ((mode & 4) && reset) CKF(cudaMemsetAsync(d_dtmin, 0x7f, sizeof(unsigned int), stream));
+    fgpu::launch(f_derived_cfl, nr, 256, 0, stream, geo, tabs, phys, mode, s.sigma, s.energy, s.vr, s.dv,
                                           fld[FGPU_QPLUS], fld[FGPU_QMINUS], fld[FGPU_SOUNDSPEED],
                                           fld[FGPU_SCALE_HEIGHT], fld[FGPU_PRESSURE],
                                           fld[FGPU_TEMPERATURE], fld[FGPU_VISCOSITY], d_dtmin,
@@ -1098,12 +1116,12 @@ int Engine32::init_euler(double t)
     if (rc) return rc;
     if (phys.adiabatic) {
         StateF s = state();
-        f_stress<<<grid2(nz, nr), 128, 0, stream>>>(geo, tabs, s.sigma, s.vr, s.dv,
+        fgpu::launch(f_stress, grid2(nz, nr), 128, 0, stream, geo, tabs, s.sigma, s.vr, s.dv,
                                                     fld[FGPU_VISCOSITY], fld[FGPU_DIV_V],
                                                     fld[FGPU_TAU_R_R], fld[FGPU_TAU_PHI_PHI],
                                                     fld[FGPU_TAU_R_PHI]);
         if (phys.stabilize) visc_corr(s);
-        f_viscous<<<grid2(nz, nr), 128, 0, stream>>>(
+        fgpu::launch(f_viscous, grid2(nz, nr), 128, 0, stream, 
             geo, tabs, phys, 0.f, (float)beta_inv(t), 2, s.sigma, fld[FGPU_TAU_R_R],
             fld[FGPU_TAU_PHI_PHI], fld[FGPU_TAU_R_PHI], fld[FGPU_DIV_V], fld[FGPU_VISCOSITY],
             fld[FGPU_SCALE_HEIGHT], s.sigma0, s.energy0, s.vr, s.dv, s.energy, fld[FGPU_QPLUS],
@@ -1171,9 +1189,9 @@ int Engine32::boundary(double dt, bool final)
         if (rc) return rc;
     }
     if (final && p.damping && n_rings)
-        f_damping<<<dim3(n_rings, 4), 256, 0, stream>>>(geo, dm, (float)dt, damp_rings, state());
+        fgpu::launch(f_damping, dim3(n_rings, 4, (nz + 1023) / 1024), 256, 0, stream, geo, dm, (float)dt, damp_rings, state());
     if (final) com_damping(dt, com_now);
-    f_ghost<<<(nz + 127) / 128, 128, 0, stream>>>(geo, bc, state());
+    fgpu::launch(f_ghost, dim3((nz + 127) / 128, kGhostParts), 128, 0, stream, geo, bc, state(), nullptr);
     com_boundary(com_now);
     CKF(cudaGetLastError());
     if (final)
@@ -1193,11 +1211,11 @@ int Engine32::kick(double dt, double t)
     auto mark = [&](int k) {
         if (mark_fn) mark_fn(mark_ctx, k);
     };
-    f_potential<<<grid2(nz, nr), 128, 0, stream>>>(geo, tabs, phys, bodies, fld[FGPU_SCALE_HEIGHT],
+    fgpu::launch(f_potential, grid2(nz, nr), 128, 0, stream, geo, tabs, phys, bodies, fld[FGPU_SCALE_HEIGHT],
                                                    fld[FGPU_POTENTIAL]);
     CKL("potential");
     mark(0);
-    f_source<<<grid2(nz, nr + 1), 128, 0, stream>>>(geo, tabs, fdt, fld[FGPU_SIGMA],
+    fgpu::launch(f_source, grid2(nz, nr + 1), 128, 0, stream, geo, tabs, fdt, fld[FGPU_SIGMA],
                                                     fld[FGPU_PRESSURE], fld[FGPU_POTENTIAL],
                                                     fld[FGPU_V_RADIAL], fld[FGPU_V_AZIMUTHAL],
                                                     alt_vr, alt_dv);
@@ -1207,11 +1225,11 @@ int Engine32::kick(double dt, double t)
     mark(1);
     StateF s = state();
     if (adi || phys.art_visc_sn || phys.art_visc_tw) {
-        f_artvisc_q<<<grid2(nz, nr), 128, 0, stream>>>(geo, tabs, phys, fdt, s.sigma, s.vr, s.dv,
+        fgpu::launch(f_artvisc_q, grid2(nz, nr), 128, 0, stream, geo, tabs, phys, fdt, s.sigma, s.vr, s.dv,
                                                        s.energy, fld[FGPU_Q_R], fld[FGPU_Q_PHI]);
         CKL("artvisc_q");
         mark(2);
-        f_artvisc_v<<<grid2(nz, nr), 128, 0, stream>>>(
+        fgpu::launch(f_artvisc_v, grid2(nz, nr), 128, 0, stream, 
             geo, tabs, phys, fdt, s.sigma, s.energy, fld[FGPU_Q_R], fld[FGPU_Q_PHI], s.vr, s.dv,
             fld[FGPU_SOUNDSPEED], fld[FGPU_SCALE_HEIGHT], fld[FGPU_VISCOSITY]);
         CKL("artvisc_v");
@@ -1220,14 +1238,14 @@ int Engine32::kick(double dt, double t)
         mark(2);
         mark(3);
     }
-    f_stress<<<grid2(nz, nr), 128, 0, stream>>>(geo, tabs, s.sigma, s.vr, s.dv,
+    fgpu::launch(f_stress, grid2(nz, nr), 128, 0, stream, geo, tabs, s.sigma, s.vr, s.dv,
                                                 fld[FGPU_VISCOSITY], fld[FGPU_DIV_V],
                                                 fld[FGPU_TAU_R_R], fld[FGPU_TAU_PHI_PHI],
                                                 fld[FGPU_TAU_R_PHI]);
     CKL("stress");
     if (phys.stabilize) visc_corr(s);
     mark(4);
-    f_viscous<<<grid2(nz, nr), 128, 0, stream>>>(
+    fgpu::launch(f_viscous, grid2(nz, nr), 128, 0, stream, 
         geo, tabs, phys, fdt, (float)beta_inv(t), adi ? 7 : 1, s.sigma, fld[FGPU_TAU_R_R],
         fld[FGPU_TAU_PHI_PHI], fld[FGPU_TAU_R_PHI], fld[FGPU_DIV_V], fld[FGPU_VISCOSITY],
         fld[FGPU_SCALE_HEIGHT], s.sigma0, s.energy0, s.vr, s.dv, s.energy, fld[FGPU_QPLUS],
@@ -1252,20 +1270,21 @@ int Engine32::transport(double dt)
     {
         // rings per thread: the longest walk that still gives every SM
         // sixteen blocks of columns (each thread's rings are a dependent
-        // chain of loads, so short grids need short walks to hide latency)
+        // chain of loads, so short grids need short walks to hide latency:
+        // 128 x 384 0.0140 ms with 4 rings, 0.0114 with 2, 0.0098 with 1)
         const int cols = (nz + 63) / 64;
         int chunk = 16;
-        while (chunk > 4 && (long long)cols * ((nr + chunk - 1) / chunk) < 16LL * nsm) chunk /= 2;
+        while (chunk > 1 && (long long)cols * ((nr + chunk - 1) / chunk) < 16LL * nsm) chunk /= 2;
         const int phase_rows = windows ? (nr + 2 * cols - 1) / (2 * cols) : 0;
         dim3 grid(cols, phase_rows + (nr + chunk - 1) / chunk);
         if (adi)
-            f_transport_radial<5><<<grid, 64, 0, stream>>>(geo, tabs, fdt, phys.limiter_mc, chunk,
+            fgpu::launch(f_transport_radial<5>, grid, 64, 0, stream, geo, tabs, fdt, phys.limiter_mc, chunk,
                                                            s.sigma, s.vr, s.dv, s.energy, mom[0],
                                                            mom[1], mom[2], mom[3], alt_e, alt_sigma,
                                                            sigma_lo, alt_sigma_lo, dt, phase_rows,
                                                            ring_phase, ring_shift);
         else
-            f_transport_radial<4><<<grid, 64, 0, stream>>>(geo, tabs, fdt, phys.limiter_mc, chunk,
+            fgpu::launch(f_transport_radial<4>, grid, 64, 0, stream, geo, tabs, fdt, phys.limiter_mc, chunk,
                                                            s.sigma, s.vr, s.dv, s.energy, mom[0],
                                                            mom[1], mom[2], mom[3], alt_e, alt_sigma,
                                                            sigma_lo, alt_sigma_lo, dt, phase_rows,
@@ -1279,8 +1298,8 @@ int Engine32::transport(double dt)
         const int nwin = windows_of(nz), per_block = kWinThreads / 32;
         const int blocks = (nr * nwin + per_block - 1) / per_block;
         auto k = adi ? f_transport_azimuthal_w<5> : f_transport_azimuthal_w<4>;
-        k<<<blocks, kWinThreads, 0, stream>>>(geo, tabs, dt, phys.limiter_mc, phys.fast_transport,
-                                              nwin, r, ring_phase);
+        fgpu::launch(k, blocks, kWinThreads, 0, stream, geo, tabs, dt, phys.limiter_mc,
+                     phys.fast_transport, nwin, r, ring_phase);
     } else {
 #define AZ32(P, NQ, ST)                                                                          \
     f_transport_azimuthal<P, NQ, ST><<<nr, az_block, az_smem, stream>>>(                         \
@@ -1326,7 +1345,7 @@ int Engine32::transport(double dt)
     CKL("transport_azimuthal");
     mark(8);
     float *const *m = windows ? mom_w : mom;
-    f_finish<<<grid2(nz, nr + 1), 128, 0, stream>>>(
+    fgpu::launch(f_finish, grid2(nz, nr + 1), 128, 0, stream, 
         geo, tabs, phys, m[0], m[1], m[2], m[3], windows ? sigma_w : alt_sigma,
         windows ? energy_w : alt_e, s.vr, alt_vr, alt_dv, s.sigma, s.energy,
         windows ? sigma_lo_w : alt_sigma_lo, sigma_lo, ring_shift);
@@ -1354,7 +1373,7 @@ int Engine32::step(double dt, double t)
     mark(-1);
     int rc = kick(dt, t);
     if (rc) return rc;
-    f_ghost<<<(nz + 127) / 128, 128, 0, stream>>>(geo, bc, state());
+    fgpu::launch(f_ghost, dim3((nz + 127) / 128, kGhostParts), 128, 0, stream, geo, bc, state(), nullptr);
     CKL("ghost");
     com_boundary(com_now);
     CKL("com_boundary");
@@ -1367,19 +1386,19 @@ int Engine32::step(double dt, double t)
     }
     StateF s = state();
     if (p.damping && n_rings)
-        f_damping<<<dim3(n_rings, 4), 256, 0, stream>>>(geo, dm, (float)dt, damp_rings, s);
+        fgpu::launch(f_damping, dim3(n_rings, 4, (nz + 1023) / 1024), 256, 0, stream, geo, dm, (float)dt, damp_rings, s);
     CKL("damping");
     com_damping(dt, com_after);
     CKL("com_damping");
     mark(10);
-    f_ghost<<<(nz + 127) / 128, 128, 0, stream>>>(geo, bc, s);
+    fgpu::launch(f_ghost, dim3((nz + 127) / 128, kGhostParts), 128, 0, stream, geo, bc, s, d_dtmin);
     CKL("ghost");
     com_boundary(com_after);
     CKL("com_boundary");
     rc = keep_mass();
     if (rc) return rc;
     mark(11);
-    rc = derived_cfl(1 | 4);
+    rc = derived_cfl(1 | 4, false);  // the ghost kernel has reset the minimum
     if (rc) return rc;
     mark(12);
     CKF(cudaGetLastError());
@@ -1404,10 +1423,10 @@ int Engine32::disk_forces(int n, const double *x, const double *y, const double 
             fb.rsm[b] = rsm[b0 + b];
         }
         const int width = 5 * fb.n;
-        f_disk_force_bodies<<<rows, 256, 0, stream>>>(geo, tabs, phys, fb, fld[FGPU_SIGMA],
+        fgpu::launch(f_disk_force_bodies, rows, 256, 0, stream, geo, tabs, phys, fb, fld[FGPU_SIGMA],
                                                       sigma_lo, fld[FGPU_SCALE_HEIGHT], partial,
                                                       width);
-        f_reduce_cols<<<width, 32, 0, stream>>>(partial, rows, width, dev + 5 * b0);
+        fgpu::launch(f_reduce_cols, width, kReduceThreads, 0, stream, partial, rows, width, dev + 5 * b0);
     }
     CKF(cudaGetLastError());
     CKF(cudaMemcpyAsync(h_pinned + 16, dev, sizeof(double) * 5 * n, cudaMemcpyDeviceToHost,

@@ -6,6 +6,7 @@
 // round-off.  Work is fused where the fusion recomputes nothing: GB300's FP64
 // rate is low, so every FP64 operation is done once and intermediates that
 // several neighbours reuse go through HBM/L2 instead of being recomputed.
+#include "launch.cuh"
 #include "hydro.cuh"
 #include "fp64_pair.cuh"
 #include "kernels.h"
@@ -179,6 +180,7 @@ template <bool PAIR>
 __global__ void k_potential(Geo g, Tables t, Phys ph, Bodies b, const double *__restrict__ H,
                             double *__restrict__ pot)
 {
+    follow_predecessor();
     const int nz = g.nz;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;
@@ -705,20 +707,38 @@ __device__ void ghost_hook(double *x, const double *x0, int kind, int outer, int
     }
 }
 
-__global__ void k_ghost(Geo g, Tables t, BcSpec bc, double omf, State s)
+// one hook per row of blocks (they are independent: each writes the ghost
+// rings of its field and edge): eight serial chains of loads and stores in one
+// thread took 8 us
+__global__ void k_ghost(Geo g, Tables t, BcSpec bc, double omf, State s,
+                        unsigned long long *dt_min)
 {
+    follow_predecessor();
+    // the CFL minimum the next kernel forms (its start, as a memset of 0x7f)
+    if (dt_min && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+        *dt_min = 0x7f7f7f7f7f7f7f7full;
     const int nz = g.nz, nr = g.nr;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nz) return;
-    ghost_hook(s.sigma, s.sigma0, bc.sigma_in, 0, 0, nr, nz, j, bc.val_in[0], s.nu, 0, 0);
-    ghost_hook(s.sigma, s.sigma0, bc.sigma_out, 1, 0, nr, nz, j, bc.val_out[0], s.nu, 0, 0);
-    ghost_hook(s.energy, s.energy0, bc.energy_in, 0, 0, nr, nz, j, bc.val_in[1], s.nu, 0, 0);
-    ghost_hook(s.energy, s.energy0, bc.energy_out, 1, 0, nr, nz, j, bc.val_out[1], s.nu, 0, 0);
-    ghost_hook(s.vr, s.vr0, bc.vr_in, 0, 1, nr, nz, j, bc.val_in[2], s.nu, 0, 0);
-    ghost_hook(s.vr, s.vr0, bc.vr_out, 1, 1, nr, nz, j, bc.val_out[2], s.nu, 0, 0);
-    ghost_hook(s.vaz, s.vaz0, bc.vaz_in, 0, 0, nr, nz, j, bc.val_in[3], s.nu, t.Rmed[0], omf);
-    ghost_hook(s.vaz, s.vaz0, bc.vaz_out, 1, 0, nr, nz, j, bc.val_out[3], s.nu, t.Rmed[nr - 1],
-               omf);
+    const int outer = blockIdx.y & 1;
+    switch (blockIdx.y >> 1) {
+    case 0:
+        ghost_hook(s.sigma, s.sigma0, outer ? bc.sigma_out : bc.sigma_in, outer, 0, nr, nz, j,
+                   outer ? bc.val_out[0] : bc.val_in[0], s.nu, 0, 0);
+        break;
+    case 1:
+        ghost_hook(s.energy, s.energy0, outer ? bc.energy_out : bc.energy_in, outer, 0, nr, nz, j,
+                   outer ? bc.val_out[1] : bc.val_in[1], s.nu, 0, 0);
+        break;
+    case 2:
+        ghost_hook(s.vr, s.vr0, outer ? bc.vr_out : bc.vr_in, outer, 1, nr, nz, j,
+                   outer ? bc.val_out[2] : bc.val_in[2], s.nu, 0, 0);
+        break;
+    default:
+        ghost_hook(s.vaz, s.vaz0, outer ? bc.vaz_out : bc.vaz_in, outer, 0, nr, nz, j,
+                   outer ? bc.val_out[3] : bc.val_in[3], s.nu, t.Rmed[outer ? nr - 1 : 0], omf);
+        break;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1156,6 +1176,7 @@ __global__ void __launch_bounds__(64, 8) k_transport_radial_f2(Geo g, Tables t, 
                                       f2 *__restrict__ mom2, f2 *__restrict__ mom3,
                                       double *__restrict__ E_out, double *__restrict__ S_out)
 {
+    follow_predecessor();
     // blocks past the chunks form the ring phases: latency-bound sums beside
     // the arithmetic-bound sweep, instead of a launch or a block-wide
     // reduction in the azimuthal pass
@@ -1491,6 +1512,7 @@ __device__ void damp_ring(double *X, double *X0, const DampQ &d, int i, int nz, 
                           double dt, double *red)
 {
     const int kind = outer ? d.kind_out : d.kind_in;
+    if (kind == 3 && blockIdx.z > 0) return;  // the whole block
     const size_t row = (size_t)i * nz;
     double x0c = 0.0;
     if (kind == 3) {
@@ -1504,10 +1526,26 @@ __device__ void damp_ring(double *X, double *X0, const DampQ &d, int i, int nz, 
     }
     const double factor = outer ? d.fac_out[i] : d.fac_in[i];
     const double tau = outer ? d.tau_out : d.tau_in;
-    const double ef = exp(-dt * factor / tau);
-    for (int j = threadIdx.x; j < nz; j += blockDim.x) {
-        const double x0 = kind == 1 ? X0[row + j] : x0c;
-        X[row + j] = (X[row + j] - x0) * ef + x0;
+    // one exponential per block: FP64, about 30 operations
+    __syncthreads();
+    if (threadIdx.x == 0) red[0] = exp(-dt * factor / tau);
+    __syncthreads();
+    const double ef = red[0];
+    // the blocks of a ring share its columns (the mean kind's one block takes
+    // them all), four loads of each thread in flight
+    const int step = kind == 3 ? blockDim.x : blockDim.x * gridDim.z;
+    const int first = kind == 3 ? threadIdx.x : blockIdx.z * blockDim.x + threadIdx.x;
+    for (int j = first; j < nz; j += 4 * step) {
+        double x[4], x0[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int jj = min(j + k * step, nz - 1);
+            x[k] = X[row + jj];
+            x0[k] = kind == 1 ? X0[row + jj] : x0c;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (j + k * step < nz) X[row + j + k * step] = (x[k] - x0[k]) * ef + x0[k];
     }
     __syncthreads();
 }
@@ -1515,6 +1553,7 @@ __device__ void damp_ring(double *X, double *X0, const DampQ &d, int i, int nz, 
 __global__ void k_damping(Geo g, Damping dm, double dt, const int *__restrict__ rings,
                           State s)
 {
+    follow_predecessor();
     __shared__ double red[33];
     const int nz = g.nz, nr = g.nr;
     const int i = rings[blockIdx.x];
@@ -1798,6 +1837,7 @@ __global__ void __launch_bounds__(256, PAIR ? 4 : 3) k_derived_cfl(Geo g, Tables
                               const double *__restrict__ corr_r,
                               unsigned long long *__restrict__ dt_min)
 {
+    follow_predecessor();
     __shared__ double red[33];
     __shared__ float redf[66];
     extern __shared__ float d32s[];  // the ring's FP32 cell steps (nz floats)
@@ -2034,6 +2074,7 @@ __global__ void __launch_bounds__(256, 4) k_disk_force_bodies(Geo g, Tables t, P
                                     const double *__restrict__ S, const double *__restrict__ H,
                                     double *__restrict__ partial, int width)
 {
+    follow_predecessor();
     __shared__ double red[33];
     const int nz = g.nz;
     const int i = blockIdx.x + 1;  // radial_first_active .. radial_active_size - 1
@@ -2153,11 +2194,12 @@ __global__ void k_reduce_rows(const double *__restrict__ partial, int rows, int 
     const int w = threadIdx.x >> 5;
     if (w < width) warp_compensated_rows(partial, rows, width, w, out);
 }
-// the same with one block (one warp) per component, for wide records
+// the same with one block per component, for wide records
 __global__ void k_reduce_cols(const double *__restrict__ partial, int rows, int width,
                               double *__restrict__ out)
 {
-    warp_compensated_rows(partial, rows, width, blockIdx.x, out);
+    follow_predecessor();
+    block_compensated_rows(partial, rows, width, blockIdx.x, out);
 }
 
 // NaN/Inf scan of one field: records the first bad flat index (atomicMin).
@@ -2175,7 +2217,7 @@ static inline dim3 grid2d(int nz, int rows, int bx) { return dim3((nz + bx - 1) 
 void launch_potential(const Launch &L, const Bodies &b, const double *H, double *pot)
 {
     auto k = L.pair ? k_potential<true> : k_potential<false>;
-    k<<<grid2d(L.g.nz, L.g.nr, L.bx), L.bx, 0, L.stream>>>(L.g, L.t, L.ph, b, H, pot);
+    launch(k, grid2d(L.g.nz, L.g.nr, L.bx), L.bx, 0, L.stream, L.g, L.t, L.ph, b, H, pot);
 }
 
 void launch_source(const Launch &L, double dt, double omf, const double *S, const double *P,
@@ -2257,9 +2299,11 @@ void launch_com_damping(const Launch &L, const ComSpec &c, double dt, const Stat
     launch_com_damping_sides(c, L.g.nz, dt, f, L.stream);
 }
 
-void launch_ghost(const Launch &L, const BcSpec &bc, double omf, const State &s)
+void launch_ghost(const Launch &L, const BcSpec &bc, double omf, const State &s,
+                  unsigned long long *dt_min)
 {
-    k_ghost<<<(L.g.nz + 127) / 128, 128, 0, L.stream>>>(L.g, L.t, bc, omf, s);
+    launch(k_ghost, dim3((L.g.nz + 127) / 128, 8), 128, 0, L.stream, L.g, L.t, bc, omf, s,
+           dt_min);
 }
 
 int radial_chunk_for(bool pair, bool adiabatic, int nr, int nz)
@@ -2277,14 +2321,15 @@ int radial_chunk_for(bool pair, bool adiabatic, int nr, int nz)
         cudaGetLastError();
         return (size_t)nr * nz >= ((size_t)8 << 20) ? 32 : 16;
     }
-    if ((size_t)nr * nz < ((size_t)8 << 20)) return 16;
-    // large disks: the chunk of 28 .. 40 rings whose grid fills the fewest
-    // waves of resident blocks for the rings walked (each chunk also primes
-    // about three rings)
+    // the chunk whose grid takes the least time: its waves of resident blocks
+    // times the rings a block walks (each chunk also primes about three).
+    // Measured, ms per pass: 128 x 384 with 1 (the rule's), 4, 16 rings 0.0138,
+    // 0.0180, 0.0385; 512 x 1536 with 4, 8, 11 (the rule's), 16 0.0645, 0.0653,
+    // 0.0538, 0.0618.
     const long long cols = (nz + 63) / 64, slots = (long long)per_sm * nsm;
-    int best = 32;
+    int best = 16;
     long long best_cost = -1;
-    for (int c = 28; c <= 40; ++c) {
+    for (int c = 1; c <= 40; ++c) {
         const long long blocks = cols * ((nr + c - 1) / c);
         const long long cost = (blocks + slots - 1) / slots * (c + 3);
         if (best_cost < 0 || cost < best_cost) {
@@ -2310,12 +2355,12 @@ void launch_transport_radial(const Launch &L, double dt, double omf, int chunk, 
         f2 *pm[4];
         for (int q = 0; q < 4; ++q) pm[q] = reinterpret_cast<f2 *>(mom[q]);
         if (L.ph.adiabatic) {
-            k_transport_radial_f2<5><<<grid, bx, 0, L.stream>>>(
+            launch(k_transport_radial_f2<5>, grid, bx, 0, L.stream,
                 L.g, L.t, dt, omf, L.ph.limiter_mc, chunk, chunks, L.ph.fast_transport, 1.0 / dt,
                 1.0 / L.g.nz, phase, S, vr, vaz, E, pm[0], pm[1], pm[2],
                 pm[3], E_out, S_out);
         } else {
-            k_transport_radial_f2<4><<<grid, bx, 0, L.stream>>>(
+            launch(k_transport_radial_f2<4>, grid, bx, 0, L.stream,
                 L.g, L.t, dt, omf, L.ph.limiter_mc, chunk, chunks, L.ph.fast_transport, 1.0 / dt,
                 1.0 / L.g.nz, phase, S, vr, vaz, E, pm[0], pm[1], pm[2],
                 pm[3], E_out, S_out);
@@ -2385,7 +2430,8 @@ void launch_damping(const Launch &L, const Damping &dm, double dt, const int *ri
                     const State &s)
 {
     if (nrings <= 0) return;
-    k_damping<<<dim3(nrings, 4), 256, 0, L.stream>>>(L.g, dm, dt, rings, s);
+    launch(k_damping, dim3(nrings, 4, (L.g.nz + 1023) / 1024), 256, 0, L.stream, L.g, dm, dt,
+           rings, s);
 }
 
 // compute_pressure (SourceEuler.cpp:1345-1376): P alone, from sigma and c_s
@@ -2491,8 +2537,8 @@ void launch_derived_cfl(const Launch &L, int mode, const State &s, unsigned long
     // StabilizeViscosity 2 use them (the pair kernel keeps the shared memory
     // for L1)
     const bool screen = !L.pair || L.ph.stabilize == 2;
-    k<<<L.g.nr, 256, screen ? (size_t)L.g.nz * sizeof(float) : 0, L.stream>>>(
-        L.g, L.t, L.ph, mode, L.ph.art_visc_sn, s.sigma, s.energy, s.vr, s.vaz, s.qplus,
+    launch(
+        k, L.g.nr, 256, screen ? (size_t)L.g.nz * sizeof(float) : 0, L.stream, L.g, L.t, L.ph, mode, L.ph.art_visc_sn, s.sigma, s.energy, s.vr, s.vaz, s.qplus,
         s.qminus, s.cs, s.H, s.P, s.T, s.nu, s.corr_phi, s.corr_r, dt_min);
 }
 
@@ -2529,8 +2575,10 @@ void launch_disk_force(const Launch &L, int n, const double *px, const double *p
             if (fb.rsm[b] > 0.0) fb.klahr |= 1u << b;
         }
         const int width = 5 * fb.n;
-        k_disk_force_bodies<<<rows, 256, 0, L.stream>>>(L.g, L.t, L.ph, fb, S, H, partial, width);
-        k_reduce_cols<<<width, 32, 0, L.stream>>>(partial, rows, width, out + 5 * b0);
+        launch(k_disk_force_bodies, rows, 256, 0, L.stream, L.g, L.t, L.ph, fb, S, H, partial,
+               width);
+        launch(k_reduce_cols, width, kReduceThreads, 0, L.stream, partial, rows, width,
+               out + 5 * b0);
     }
 }
 

@@ -3,6 +3,7 @@
 // (pair_window.cuh).  FP64 is kept for the state updates x += dx and for the
 // differences of neighbouring stored values that cancel (v_phi along the ring,
 // the pressure), as the pair format carries 2^-48 of each value.
+#include "launch.cuh"
 #include "kernels.h"
 #include "pair_window.cuh"
 
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(kThreads, 5)
                const double *__restrict__ vaz, double *__restrict__ pot,
                double *__restrict__ vr_out, double *__restrict__ vaz_out)
 {
+    follow_predecessor();
     const int nz = g.nz, nr = g.nr;
     Job job;
     if (!job_of(nwin, nr, chunk, job)) return;
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(kThreads, 5)
                 double *__restrict__ Qp, double *__restrict__ vr_out, double *__restrict__ vaz_out,
                 double *__restrict__ cs, double *__restrict__ H, double *__restrict__ nu)
 {
+    follow_predecessor();
     const int nz = g.nz, nr = g.nr;
     Job job;
     if (!job_of(nwin, nr, chunk, job)) return;
@@ -345,6 +348,7 @@ __global__ void __launch_bounds__(kThreads, 4)
                 double *__restrict__ vr_out, double *__restrict__ vaz_out,
                 double *__restrict__ qplus, double *__restrict__ qminus)
 {
+    follow_predecessor();
     const int nz = g.nz, nr = g.nr;
     Job job;
     if (!job_of(nwin, nr, chunk, job)) return;
@@ -562,7 +566,7 @@ void launch_source_window(const Launch &L, double dt, double omf, const Bodies &
     const int nwin = windows(L.g.nz), chunk = chunk_for(L.g.nr, nwin);
     const int jobs = nwin * ((L.g.nr + chunk - 1) / chunk), per = kThreads / 32;
     auto k = L.g.nz % 2 == 0 ? k_source_w<true> : k_source_w<false>;
-    k<<<(jobs + per - 1) / per, kThreads, 0, L.stream>>>(
+    launch(k, (jobs + per - 1) / per, kThreads, 0, L.stream,
         L.g, L.t, L.ph, b, split_pair_host(b.gm0), split_pair_host(dt), split_pair_host(omf), nwin,
         chunk, s.H, s.sigma, s.P, s.vr, s.vaz, s.pot, vr_out, vaz_out);
 }
@@ -576,7 +580,7 @@ void launch_artvisc_pair(const Launch &L, double dt, const State &s, double *vr_
         return L.ph.adiabatic ? k_artvisc_w<even.value, true> : k_artvisc_w<even.value, false>;
     };
     auto k = L.g.nz % 2 == 0 ? pick(std::true_type{}) : pick(std::false_type{});
-    k<<<(jobs + per - 1) / per, kThreads, 0, L.stream>>>(
+    launch(k, (jobs + per - 1) / per, kThreads, 0, L.stream,
         L.g, L.t, L.ph, split_pair_host(dt), nwin, chunk, s.sigma, s.vr, s.vaz, s.energy, s.qr,
         s.qphi, vr_out, vaz_out, s.cs, s.H, s.nu);
 }
@@ -590,7 +594,7 @@ void launch_viscous_pair(const Launch &L, double dt, double beta_inv, int mode, 
         return L.ph.adiabatic ? k_viscous_w<even.value, true> : k_viscous_w<even.value, false>;
     };
     auto k = L.g.nz % 2 == 0 ? pick(std::true_type{}) : pick(std::false_type{});
-    k<<<(jobs + per - 1) / per, kThreads, 0, L.stream>>>(
+    launch(k, (jobs + per - 1) / per, kThreads, 0, L.stream,
         L.g, L.t, L.ph, split_pair_host(dt), split_pair_host(beta_inv), mode, nwin, chunk, s.sigma,
         s.nu, s.H, s.sigma0, s.energy0, s.vr, s.vaz, s.energy, s.divv, s.trr, s.tpp, s.trp, vr_out,
         vaz_out, s.qplus, s.qminus);

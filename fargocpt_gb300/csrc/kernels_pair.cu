@@ -17,6 +17,7 @@
 //    gives the reference's clamped value exactly.
 // Each kernel cites the reference function it follows and has the grid and
 // the ring ranges of its FP64 counterpart.
+#include "launch.cuh"
 #include "fp64_pair.cuh"
 #include "hydro.cuh"
 #include "kernels.h"
@@ -65,6 +66,7 @@ __global__ void k_source_p(Geo g, Tables t, float2 dtp, float2 omega_frame,
                            const double *__restrict__ vaz_in, double *__restrict__ vr_out,
                            double *__restrict__ vaz_out)
 {
+    follow_predecessor();
     const int nz = g.nz, nr = g.nr;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;  // 0 .. nr
@@ -105,6 +107,7 @@ __global__ void k_stress_p(Geo g, Tables t, const double *__restrict__ S,
                            double *__restrict__ trr, double *__restrict__ tpp,
                            double *__restrict__ trp)
 {
+    follow_predecessor();
     const int nz = g.nz;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;  // 0 .. nr - 1
@@ -153,6 +156,7 @@ __global__ void k_finish_p(Geo g, Tables t, Phys ph, float2 omf, const f2 *__res
                            double *__restrict__ S_out, double *__restrict__ E_out,
                            const RingPhase *__restrict__ phase)
 {
+    follow_predecessor();
     const int nz = g.nz, nr = g.nr;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;  // 0 .. nr
@@ -204,7 +208,7 @@ void launch_source_pair(const Launch &L, double dt, double omf, const double *S,
                         const double *pot, const double *vr_in, const double *vaz_in,
                         double *vr_out, double *vaz_out)
 {
-    k_source_p<<<grid2(L.g.nz, L.g.nr + 1, L.bx), L.bx, 0, L.stream>>>(
+    launch(k_source_p, grid2(L.g.nz, L.g.nr + 1, L.bx), L.bx, 0, L.stream,
         L.g, L.t, split_pair_host(dt), split_pair_host(omf), S, Pr, pot, vr_in, vaz_in, vr_out,
         vaz_out);
 }
@@ -212,7 +216,7 @@ void launch_source_pair(const Launch &L, double dt, double omf, const double *S,
 void launch_stress_pair(const Launch &L, const double *S, const double *vr, const double *vaz,
                         const double *nu, double *divv, double *trr, double *tpp, double *trp)
 {
-    k_stress_p<<<grid2(L.g.nz, L.g.nr, L.bx), L.bx, 0, L.stream>>>(L.g, L.t, S, vr, vaz, nu, divv,
+    launch(k_stress_p, grid2(L.g.nz, L.g.nr, L.bx), L.bx, 0, L.stream, L.g, L.t, S, vr, vaz, nu, divv,
                                                                    trr, tpp, trp);
 }
 
@@ -227,7 +231,7 @@ void launch_finish_pair(const Launch &L, double omf, double *const mom[4], const
                         double *S_out, double *E_out, const RingPhase *phase)
 {
     auto m = [&](int q) { return reinterpret_cast<const f2 *>(mom[q]); };
-    k_finish_p<<<grid2(L.g.nz, L.g.nr + 1, L.bx), L.bx, 0, L.stream>>>(
+    launch(k_finish_p, grid2(L.g.nz, L.g.nr + 1, L.bx), L.bx, 0, L.stream,
         L.g, L.t, L.ph, split_pair_host(omf), m(0), m(1), m(2), m(3), S_t, E_t, vr_in,
         vr_out, vaz_out,
         S_out, E_out, phase);
