@@ -274,6 +274,7 @@ class Engine32 {
     bool windows = true;
     float2 *ring_phase = nullptr;
     float *mom_w[4] = {}, *sigma_w = nullptr, *energy_w = nullptr, *sigma_lo_w = nullptr;
+    char *mom_mem = nullptr;  // the momenta, the window pass's rows and ring phases
     float *mom[4] = {};
     float *tab_f = nullptr;
     double *tab_d = nullptr;

@@ -695,7 +695,6 @@ int Engine32::create(const fgpu_params &prm, const double *radii, cudaStream_t s
     CKF(cudaMemset(alt_sigma_lo, 0, cells * sizeof(float)));
     CKF(cudaMalloc(&ring_shift, sizeof(int) * (size_t)nr));
     CKF(cudaMemset(ring_shift, 0, sizeof(int) * (size_t)nr));
-    for (int k = 0; k < 4; ++k) CKF(cudaMalloc(&mom[k], cells * sizeof(float)));
     CKF(cudaMalloc(&partial, sizeof(double) * 5 * kForceBodies32 * (size_t)nr));
     CKF(cudaMalloc(&red_out, sizeof(double) * (8 + 5 * kMaxBodies)));
     CKF(cudaMalloc(&d_dtmin, sizeof(unsigned int)));
@@ -879,13 +878,21 @@ int Engine32::create(const fgpu_params &prm, const double *radii, cudaStream_t s
             windows = false;
         }
     }
-    if (windows) {
-        CKF(cudaMalloc(&ring_phase, sizeof(float2) * (size_t)nr));
-        for (int k = 0; k < 4; ++k) CKF(cudaMalloc(&mom_w[k], cells * sizeof(float)));
-        CKF(cudaMalloc(&sigma_w, cells * sizeof(float)));
-        CKF(cudaMalloc(&sigma_lo_w, cells * sizeof(float)));
-        CKF(cudaMalloc(&energy_w, cells * sizeof(float)));
-        CKF(cudaMemset(energy_w, 0, cells * sizeof(float)));
+    {
+        // the transported momenta, and for the window pass its output rows and
+        // ring phases, as parts of one allocation, each from a 256-byte
+        // boundary
+        const size_t part = (cells * sizeof(float) + 255) / 256 * 256;
+        CKF(cudaMalloc(&mom_mem, (windows ? 11 : 4) * part + sizeof(float2) * (size_t)nr));
+        auto at = [&](int k) { return reinterpret_cast<float *>(mom_mem + k * part); };
+        for (int k = 0; k < 4; ++k) mom[k] = at(k);
+        if (windows) {
+            for (int k = 0; k < 4; ++k) mom_w[k] = at(4 + k);
+            sigma_w = at(8);
+            sigma_lo_w = at(9);
+            energy_w = at(10);
+            ring_phase = reinterpret_cast<float2 *>(mom_mem + 11 * part);
+        }
     }
     if (rb_per) {
         rb_smem = rb_smem_floats(nz, nq, nz / rb_per) * sizeof(float);
@@ -911,11 +918,7 @@ void Engine32::destroy()
     for (int f = 0; f < FGPU_FIELD_COUNT; ++f) cudaFree(fld[f]);
     cudaFree(alt_sigma); cudaFree(alt_vr); cudaFree(alt_dv); cudaFree(alt_e);
     cudaFree(sigma_lo); cudaFree(alt_sigma_lo); cudaFree(ring_shift);
-    for (int k = 0; k < 4; ++k) {
-        cudaFree(mom[k]);
-        cudaFree(mom_w[k]);
-    }
-    cudaFree(ring_phase); cudaFree(sigma_w); cudaFree(sigma_lo_w); cudaFree(energy_w);
+    cudaFree(mom_mem);
     cudaFree(partial); cudaFree(red_out); cudaFree(d_dtmin); cudaFree(d_bad); cudaFree(stage);
     cudaFree(corr_phi); cudaFree(corr_r);
     cudaFree(tab_f); cudaFree(tab_d); cudaFree(tab_c); cudaFree(vaz_offset); cudaFree(damp_mem); cudaFree(damp_aux); cudaFree(damp_rings);
