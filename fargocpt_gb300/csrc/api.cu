@@ -25,6 +25,9 @@
 
 using namespace fgpu;
 
+// slot of h_pinned the CFL step arrives in
+constexpr int kHostDt = 15;
+
 struct fgpu_engine {
     fgpu_params p;
     int nr = 0, nz = 0;
@@ -34,12 +37,16 @@ struct fgpu_engine {
 
     double *field[FGPU_FIELD_COUNT] = {};
     double *sigma_alt = nullptr, *vr_alt = nullptr, *vaz_alt = nullptr, *energy_alt = nullptr;
+    char *mom_mem = nullptr;  // the momenta and ring phases below
     double *mom[4] = {};
     double *mom_t[4] = {};  // pair form: the azimuthal pass's momenta (mom: the radial pass's)
     double *ring_ws = nullptr;
     RingPhase *ring_phase = nullptr;  // pair form: the azimuthal pass's constants per ring
     size_t az_smem = 0;
     int az_block = 256;
+    double *ring_mean = nullptr;    // pair form: mean v_phi per ring, for the CFL kernel
+    unsigned *cfl_done = nullptr;   // blocks of the CFL kernel that have finished
+    bool dt_arrived = false;        // the last CFL step has reached h_pinned[kHostDt]
     bool pair_arith = true;  // the kernels' arithmetic in float pairs (else FP64)
     // div v and the stress tensor hold the stress kernel's float pairs
     // (stress_as_pairs), the artificial pressures those of the float-pair
@@ -981,21 +988,17 @@ static int create_engine(const fgpu_params *params, const double *radii, cudaStr
         cudaMemset(eng->corr_phi, 0, eng->cells * sizeof(double));
         cudaMemset(eng->corr_r, 0, eng->cells * sizeof(double));
     }
-    for (int k = 0; k < 4; ++k) {
-        if (cudaMalloc(&eng->mom[k], eng->cells * sizeof(double)) != cudaSuccess) {
-            eng->err = "out of device memory (momenta)";
-            return fail(FGPU_ERR_OOM);
-        }
-    }
     if (cudaMalloc(&eng->partial, sizeof(double) * 5 * kForceBodies * (size_t)eng->nr) !=
             cudaSuccess ||
         cudaMalloc(&eng->red_out, sizeof(double) * (8 + 5 * kMaxBodies)) != cudaSuccess ||
-        cudaMalloc(&eng->d_dtmin, sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMalloc(&eng->d_dtmin, 2 * sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMemset(eng->d_dtmin, 0, 2 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMalloc(&eng->d_bad, sizeof(unsigned long long)) != cudaSuccess ||
         cudaMallocHost(&eng->h_pinned, sizeof(double) * (16 + 5 * kMaxBodies)) != cudaSuccess) {
         eng->err = "out of memory (reductions)";
         return fail(FGPU_ERR_OOM);
     }
+    eng->cfl_done = reinterpret_cast<unsigned *>(eng->d_dtmin + 1);
     rc = setup_tables(eng, radii);
     if (rc != FGPU_OK) return fail(rc);
 
@@ -1012,25 +1015,28 @@ static int create_engine(const fgpu_params *params, const double *radii, cudaStr
         }
     }
     // rings per radial sweep chunk (radial_chunk_for): longer chunks prime
-    // fewer rings, shorter ones give more blocks; 16 below 8M cells
-    // (measured, ms per radial pass on 512x1536: 0.064 with 16, 0.068 with
-    // 8, 0.098 with 32), else the chunk whose grid fills the fewest waves of
-    // resident blocks (2048x6144 in float pairs: 0.707 ms with 32 rings, six
-    // waves; 0.694 with 33 and 0.683 with 34, five)
+    // fewer rings, shorter ones give more blocks
     eng->radial_chunk = radial_chunk_for(eng->pair_arith, eng->ph.adiabatic, eng->nr, eng->nz);
-    if (eng->pair_arith) {
-        // the float-pair azimuthal pass works out of place
-        for (int k = 0; k < 4; ++k) {
-            if (cudaMalloc(&eng->mom_t[k], eng->cells * sizeof(double)) != cudaSuccess) {
-                eng->err = "out of device memory (momenta)";
-                return fail(FGPU_ERR_OOM);
-            }
-        }
-        if (cudaMalloc(&eng->ring_phase, sizeof(RingPhase) * (size_t)eng->nr) != cudaSuccess) {
-            eng->err = "out of device memory (ring phases)";
+    {
+        // the transported momenta (a second set in the pair form, whose
+        // azimuthal pass works out of place) and the ring phases, as parts of
+        // one allocation, each from a 256-byte boundary
+        const int sets = eng->pair_arith ? 2 : 1;
+        const size_t part = (eng->cells * sizeof(double) + 255) / 256 * 256;
+        const size_t per_ring = sizeof(RingPhase) + sizeof(double);
+        if (cudaMalloc(&eng->mom_mem, 4 * sets * part + per_ring * (size_t)eng->nr) !=
+            cudaSuccess) {
+            eng->err = "out of device memory (momenta)";
             return fail(FGPU_ERR_OOM);
         }
-    } else {
+        for (int k = 0; k < 4; ++k) {
+            eng->mom[k] = reinterpret_cast<double *>(eng->mom_mem + k * part);
+            if (sets == 2) eng->mom_t[k] = reinterpret_cast<double *>(eng->mom_mem + (4 + k) * part);
+        }
+        eng->ring_phase = reinterpret_cast<RingPhase *>(eng->mom_mem + 4 * sets * part);
+        eng->ring_mean = reinterpret_cast<double *>(eng->ring_phase + eng->nr);
+    }
+    if (!eng->pair_arith) {
         // FP64 azimuthal transport: whole ring in shared memory when it fits
         const int per = azimuthal_cells_per_thread(eng->nz);
         eng->az_block = std::max(128, std::min(512, ((eng->nz + per - 1) / per + 31) / 32 * 32));
@@ -1068,11 +1074,8 @@ extern "C" int fgpu_destroy(fgpu_engine *eng)
     for (auto ev : eng->ev_free) cudaEventDestroy(ev);
     for (int f = 0; f < FGPU_FIELD_COUNT; ++f) cudaFree(eng->field[f]);
     cudaFree(eng->sigma_alt); cudaFree(eng->vr_alt); cudaFree(eng->vaz_alt); cudaFree(eng->energy_alt);
-    for (int k = 0; k < 4; ++k) {
-        cudaFree(eng->mom[k]);
-        cudaFree(eng->mom_t[k]);
-    }
-    cudaFree(eng->ring_ws); cudaFree(eng->ring_phase); cudaFree(eng->tables_mem);
+    cudaFree(eng->mom_mem);
+    cudaFree(eng->ring_ws); cudaFree(eng->tables_mem);
     cudaFree(eng->damp_mem);
     cudaFree(eng->damp_rings); cudaFree(eng->partial); cudaFree(eng->red_out);
     cudaFree(eng->pair_mem);
@@ -1348,6 +1351,8 @@ static double beta_inv_at(const fgpu_params &p, double t)
         return rc_;                             \
     }
 
+static void derived_cfl(fgpu_engine *eng, const Launch &L, int mode);
+
 extern "C" int fgpu_init_euler(fgpu_engine *eng, double t)
 {
     NvtxCall nvtx_("fgpu_init_euler");
@@ -1355,7 +1360,7 @@ extern "C" int fgpu_init_euler(fgpu_engine *eng, double t)
     ROUTE32(eng->e32->init_euler(t));
     Launch L = launch_of(eng);
     State s = state_of(eng);
-    launch_derived_cfl(L, 1 | 2, s, nullptr);
+    derived_cfl(eng, L, 1 | 2);
     if (eng->ph.adiabatic) {
         // compute_heating_cooling_for_CFL, SourceEuler.cpp:1410-1450
         eng->stress_pairs = stress_as_pairs(L);
@@ -1378,7 +1383,7 @@ extern "C" int fgpu_recalculate_derived(fgpu_engine *eng, double t)
     if (!eng) return FGPU_ERR_BAD_ARG;
     ROUTE32(eng->e32->derived_cfl(1));
     Launch L = launch_of(eng);
-    launch_derived_cfl(L, 1, state_of(eng), nullptr);
+    derived_cfl(eng, L, 1);
     eng->cfl_valid = false;
     return check_launch(eng);
 }
@@ -1390,15 +1395,20 @@ extern "C" int fgpu_condition_cfl(fgpu_engine *eng, double *dt_out)
     ROUTE32(eng->e32->cfl(dt_out));
     if (!eng->cfl_valid) {
         CK(cudaMemsetAsync(eng->d_dtmin, 0x7f, sizeof(unsigned long long), eng->stream));
-        launch_derived_cfl(launch_of(eng), 4, state_of(eng), eng->d_dtmin);
+        const Launch L = launch_of(eng);
+        if (cfl_as_pairs(L)) launch_ring_means(L, eng->field[FGPU_V_AZIMUTHAL], eng->ring_mean);
+        derived_cfl(eng, L, 4);
         int rc = check_launch(eng);
         if (rc) return rc;
         eng->cfl_valid = true;
     }
-    CK(cudaMemcpyAsync(eng->h_pinned, eng->d_dtmin, sizeof(double), cudaMemcpyDeviceToHost,
-                       eng->stream));
-    CK(cudaStreamSynchronize(eng->stream));
-    *dt_out = eng->h_pinned[0];
+    // the step is written to the host by the kernel that formed it; a call that
+    // waited for the stream since then has already brought it
+    if (!eng->dt_arrived) {
+        CK(cudaStreamSynchronize(eng->stream));
+        eng->dt_arrived = true;
+    }
+    *dt_out = eng->h_pinned[kHostDt];
     return FGPU_OK;
 }
 
@@ -1410,13 +1420,33 @@ static void viscous_recompute(fgpu_engine *eng, const Launch &L)
 {
     const fgpu_params &p = eng->p;
     if (eng->ph.adiabatic && (p.viscous_accretion || p.bc_vrad_inner == FGPU_BC_VISCOUS)) {
-        launch_derived_cfl(L, 1, state_of(eng), nullptr);
+        derived_cfl(eng, L, 1);
     }
 }
 
-static void ghost(fgpu_engine *eng, const Launch &L, unsigned long long *dt_min = nullptr)
+// cfl: prepares the CFL kernel that follows (its minimum, the ring means)
+static void ghost(fgpu_engine *eng, const Launch &L, bool cfl = false)
 {
-    launch_ghost(L, eng->bc, eng->bodies.omega_frame, state_of(eng), dt_min);
+    const bool means = cfl && cfl_as_pairs(L);
+    launch_ghost(L, eng->bc, eng->bodies.omega_frame, state_of(eng), cfl ? eng->d_dtmin : nullptr,
+                 means ? eng->ring_mean : nullptr);
+}
+
+// derived quantities (mode 1, 2) and the CFL minimum (4; reset and, in the pair
+// form, the ring means are the caller's)
+static void derived_cfl(fgpu_engine *eng, const Launch &L, int mode)
+{
+    const bool cfl = (mode & 4) != 0;
+    if (cfl_as_pairs(L)) {
+        launch_derived_cfl_pair(L, mode, state_of(eng), eng->ring_mean, eng->d_dtmin, eng->cfl_done,
+                                cfl ? eng->h_pinned + kHostDt : nullptr);
+    } else {
+        launch_derived_cfl(L, mode, state_of(eng), eng->d_dtmin);
+        if (cfl)
+            cudaMemcpyAsync(eng->h_pinned + kHostDt, eng->d_dtmin, sizeof(double),
+                            cudaMemcpyDeviceToHost, eng->stream);
+    }
+    if (cfl) eng->dt_arrived = false;
 }
 
 // The centre-of-mass composite: its damping runs after the regular damping
@@ -1736,12 +1766,12 @@ extern "C" int fgpu_step_euler(fgpu_engine *eng, double dt, double t)
         com_damping(eng, L, dt, eng->com_after);
     }
     mark(eng, 10);
-    ghost(eng, L, eng->d_dtmin);  // resets the CFL minimum formed below
+    ghost(eng, L, true);
     com_boundary(eng, L, eng->com_after);
     keep_mass(eng, L);
     mark(eng, 11);
     // recalculate_derived_disk_quantities (simulation.cpp:265) + the next CFL
-    launch_derived_cfl(L, 1 | 4, s, eng->d_dtmin);
+    derived_cfl(eng, L, 1 | 4);
     mark(eng, 12);
     eng->cfl_valid = true;
     return check_launch(eng);
@@ -1797,12 +1827,11 @@ extern "C" int fgpu_disk_on_planet_accel(fgpu_engine *eng, int k, double accel[2
     // the cubic smoothing radius is the same r_sm the gas feels
     launch_disk_force(launch_of(eng), 1, &b.x[k], &b.y[k], &b.a[k], &b.rsm[k],
                       eng->field[FGPU_SIGMA], eng->field[FGPU_SCALE_HEIGHT], eng->partial,
-                      eng->red_out);
+                      eng->h_pinned);
     int rc = check_launch(eng);
     if (rc) return rc;
-    CK(cudaMemcpyAsync(eng->h_pinned, eng->red_out, sizeof(double) * 5, cudaMemcpyDeviceToHost,
-                       eng->stream));
     CK(cudaStreamSynchronize(eng->stream));
+    eng->dt_arrived = true;
     accel[0] = eng->h_pinned[0] + eng->h_pinned[2];
     accel[1] = eng->h_pinned[1] + eng->h_pinned[3];
     return FGPU_OK;
@@ -1825,14 +1854,14 @@ extern "C" int fgpu_disk_on_nbody_accel(fgpu_engine *eng, double *accel)
             return rc;
         }
     } else {
-        double *out = eng->red_out + 8;
+        // the sums go straight to page-locked host memory
+        double *out = eng->h_pinned + 16;
         launch_disk_force(launch_of(eng), n, b.x, b.y, b.a, b.rsm, eng->field[FGPU_SIGMA],
                           eng->field[FGPU_SCALE_HEIGHT], eng->partial, out);
         int rc = check_launch(eng);
         if (rc) return rc;
-        CK(cudaMemcpyAsync(eng->h_pinned + 16, out, sizeof(double) * 5 * n,
-                           cudaMemcpyDeviceToHost, eng->stream));
         CK(cudaStreamSynchronize(eng->stream));
+        eng->dt_arrived = true;
         std::copy(eng->h_pinned + 16, eng->h_pinned + 16 + 5 * n, sums);
     }
     for (int k = 0; k < n; ++k) {

@@ -46,9 +46,10 @@ void launch_stress(const Launch &L, const double *S, const double *vr, const dou
                    const double *nu, double *divv, double *trr, double *tpp, double *trp);
 void launch_viscous(const Launch &L, double dt, double beta_inv, int mode, const State &s);
 void launch_visc_corr(const Launch &L, const State &s);
-// dt_min: reset to a huge step, for the CFL kernel that follows (or null)
+// for the CFL kernel that follows (or null): dt_min, reset to a huge step;
+// mean, the ring means of v_phi of rings 1 .. nr - 2
 void launch_ghost(const Launch &L, const BcSpec &bc, double omf, const State &s,
-                  unsigned long long *dt_min);
+                  unsigned long long *dt_min, double *mean);
 void launch_com_boundary(const Launch &L, const ComSpec &c, const State &s);
 void launch_correct_vaz(const Launch &L, double domega, double *vaz);
 void launch_cfl_cells(const Launch &L, const State &s, double *out);
@@ -89,6 +90,21 @@ void launch_source_pair(const Launch &L, double dt, double omf, const double *S,
                         double *vr_out, double *vaz_out);
 void launch_stress_pair(const Launch &L, const double *S, const double *vr, const double *vaz,
                         const double *nu, double *divv, double *trr, double *tpp, double *trp);
+// ring means of v_phi, and the derived quantities and CFL step
+// (kernels_cfl.cu; not for StabilizeViscosity 2).  mode: 1 derived quantities, 2
+// also the isothermal disk's constant ones, 4 CFL, from the ring means, into
+// *dt_min and, if host_dt is given, by the last block to finish (*done counts
+// them, zero between launches) into page-locked host memory.
+// the CFL kernel of the pair form (StabilizeViscosity 2's limit is the FP64
+// kernel's)
+inline bool cfl_as_pairs(const Launch &L) { return L.pair && L.ph.stabilize != 2; }
+struct CflPairs {
+    float2 four_C2, inv_hc, leapfrog, c_v_inv, constant_viscosity;
+    float cfl_f;
+};
+void launch_ring_means(const Launch &L, const double *vaz, double *mean);
+void launch_derived_cfl_pair(const Launch &L, int mode, const State &s, const double *mean,
+                             unsigned long long *dt_min, unsigned *done, double *host_dt);
 // kernels that march windows of cells through the rings (kernels_kick.cu), the
 // velocities into vr_out, vaz_out:
 // the potential and the momentum source terms, for bodies.star_plain

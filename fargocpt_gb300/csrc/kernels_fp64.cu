@@ -710,10 +710,22 @@ __device__ void ghost_hook(double *x, const double *x0, int kind, int outer, int
 // one hook per row of blocks (they are independent: each writes the ghost
 // rings of its field and edge): eight serial chains of loads and stores in one
 // thread took 8 us
-__global__ void k_ghost(Geo g, Tables t, BcSpec bc, double omf, State s,
-                        unsigned long long *dt_min)
+__global__ void __launch_bounds__(128)
+    k_ghost(Geo g, Tables t, BcSpec bc, double omf, State s, unsigned long long *dt_min,
+            double *mean)
 {
     follow_predecessor();
+    // rows of blocks past the hooks: the ring means of v_phi that the CFL kernel
+    // takes, a block per ring (rings 1 .. nr - 2, which no hook writes)
+    if (blockIdx.y >= 8) {
+        const int blocks = gridDim.x * (gridDim.y - 8);
+        for (int k = (blockIdx.y - 8) * gridDim.x + blockIdx.x; k < g.nr - 2; k += blocks) {
+            const int i = g.nr - 2 - k;
+            const double m = block_row_mean(s.vaz + (size_t)i * g.nz, g.nz);
+            if (threadIdx.x == 0) mean[i] = m;
+        }
+        return;
+    }
     // the CFL minimum the next kernel forms (its start, as a memset of 0x7f)
     if (dt_min && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
         *dt_min = 0x7f7f7f7f7f7f7f7full;
@@ -1722,110 +1734,10 @@ __device__ __forceinline__ double cfl_cell64(const Geo &g, const Tables &t, cons
     return dt_cell;
 }
 
-// The sum of the squares of cell (i, j)'s six inverse times in float pairs
-// (cfl_cell64's; LeapFrog's 0.6 on the last three): the cell's step is CFL
-// over its square root, so the ring's smallest step is CFL / sqrt of the
-// ring's largest sum, formed once per ring; within a few 2^-46 of the FP64
-// value, far inside the CFL step's bar.  The
-// differences of stored velocities and Q+ - Q- are FP64 subtractions (they
-// cancel); StabilizeViscosity 2 is served by the FP64 path.
-__device__ __forceinline__ f2 cfl_cell_f2(const Geo &g, const Tables &t, const Phys &ph, int sn,
-                                          int i, int j, f2 c_s, f2 n,
-                                          const double *__restrict__ vr,
-                                          const double *__restrict__ vaz, double vm0,
-                                          const double *__restrict__ qplus,
-                                          const double *__restrict__ qminus,
-                                          const double *__restrict__ E)
-{
-    const int nz = g.nz;
-    const size_t row = (size_t)i * nz;
-    const size_t c = row + j;
-    auto tp = [&](const double *tab) {
-        const float2 v = t.ptab[(tab - t.tbase) + i];
-        return f2{v.x, v.y};
-    };
-    auto fmax2 = [](f2 a, f2 b) {  // a, b >= 0
-        return (a.h > b.h || (a.h == b.h && a.l > b.l)) ? a : b;
-    };
-    const double va = vaz[c], vr0 = vr[c], vr1 = vr[c + nz];
-    const double va1 = vaz[row + (j == nz - 1 ? 0 : j + 1)];
-    const f2 inv_drsup = tp(t.InvDiffRsup), inv_dxt = tp(t.InvDxTheta);
-    const f2 i1 = f2_smul(c_s, tp(t.InvCell));
-    const f2 i2 = f2_smul(f2_split(vr0), inv_drsup);
-    const f2 i3 = f2_smul(f2_split(ph.fast_transport ? va - vm0 : va), inv_dxt);
-    f2 i4;
-    if (sn) {
-        const double dvR = vr1 - vr0, dvA = va1 - va;
-        const f2 a = f2_smul(f2_split(positive(dvR) ? 0.0 : -dvR), inv_drsup);
-        const f2 b = f2_smul(f2_split(positive(dvA) ? 0.0 : -dvA), inv_dxt);
-        i4 = f2_smul(f2_split(ph.four_C2), fmax2(a, b));
-    } else {
-        const f2 eps_rr = f2_smul(f2_split(vr1 - vr0), inv_drsup);
-        const f2 h = f2_split(0.5 * (vr1 + vr0));
-        const f2 eps_pp = f2_smul(tp(t.InvRmed),
-                                  f2_sadd(f2_smul(f2_split(va1 - va), f2_split(g.invdphi)), h));
-        const f2 d = f2_sadd(eps_rr, eps_pp);
-        i4 = f2_smul(f2_split(ph.four_C2), d.h < 0.f ? f2_neg(d) : f2{0.f, 0.f});
-    }
-    f2 i5 = f2_smul(n, tp(t.InvCell2));
-    i5 = f2{__fmul_rn(4.0f, i5.h), __fmul_rn(4.0f, i5.l)};
-    f2 i6{0.f, 0.f};
-    if (ph.adiabatic) {
-        const f2 q = f2_sdiv(f2_split(qplus[c] - qminus[c]), f2_split(E[c]));
-        i6 = f2_smul(f2_split(ph.inv_hc_limit), q.h < 0.f ? f2_neg(q) : q);
-    }
-    if (ph.leapfrog) {
-        const f2 k = f2_split(0.6);
-        i4 = f2_smul(i4, k);
-        i5 = f2_smul(i5, k);
-        i6 = f2_smul(i6, k);
-    }
-    f2 sum = f2_smul(i1, i1);
-    sum = f2_sadd(sum, f2_smul(i2, i2));
-    sum = f2_sadd(sum, f2_smul(i3, i3));
-    sum = f2_sadd(sum, f2_smul(i4, i4));
-    sum = f2_sadd(sum, f2_smul(i5, i5));
-    sum = f2_sadd(sum, f2_smul(i6, i6));
-    return sum;
-}
-
-// the larger of two non-negative pairs
-__device__ __forceinline__ f2 pair_max(f2 a, f2 b)
-{
-    return (b.h > a.h || (b.h == a.h && b.l > a.l)) ? b : a;
-}
-__device__ f2 block_max_f2(f2 v, float *red)
-{
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
-    for (int o = 16; o > 0; o >>= 1)
-        v = pair_max(v, f2{__shfl_down_sync(0xffffffffu, v.h, o), __shfl_down_sync(0xffffffffu, v.l, o)});
-    __syncthreads();
-    if (lane == 0) {
-        red[2 * wid] = v.h;
-        red[2 * wid + 1] = v.l;
-    }
-    __syncthreads();
-    if (wid == 0) {
-        f2 x = lane < nw ? f2{red[2 * lane], red[2 * lane + 1]} : f2{0.f, 0.f};
-        for (int o = 16; o > 0; o >>= 1)
-            x = pair_max(x, f2{__shfl_down_sync(0xffffffffu, x.h, o), __shfl_down_sync(0xffffffffu, x.l, o)});
-        if (lane == 0) {
-            red[64] = x.h;
-            red[65] = x.l;
-        }
-    }
-    __syncthreads();
-    return f2{red[64], red[65]};
-}
-
-
-// PAIR: the ideal-EOS derived quantities (T, c_s, H, nu) in float-pair
-// arithmetic (P = (gamma - 1) e stays one FP64 product: the source terms
-// difference it)
-// 256-thread blocks; the pair form held to 64 registers, 4 blocks per SM (at
-// its free choice of 121 registers, 2 blocks: 0.67 ms on the 2048 x 6144
-// disk, at 80: 0.557, at 64: 0.502)
+// The engine in FP64 arithmetic, and StabilizeViscosity 2 (the others of the
+// pair form: kernels_cfl.cu).  PAIR: the ideal-EOS derived quantities (T, c_s, H,
+// nu) in float-pair arithmetic (P = (gamma - 1) e stays one FP64 product: the
+// source terms difference it).
 template <bool PAIR>
 __global__ void __launch_bounds__(256, PAIR ? 4 : 3) k_derived_cfl(Geo g, Tables t, Phys ph, int mode, int sn, const double *__restrict__ S,
                               const double *__restrict__ E, const double *__restrict__ vr,
@@ -1841,12 +1753,6 @@ __global__ void __launch_bounds__(256, PAIR ? 4 : 3) k_derived_cfl(Geo g, Tables
     __shared__ double red[33];
     __shared__ float redf[66];
     extern __shared__ float d32s[];  // the ring's FP32 cell steps (nz floats)
-    // PAIR: every cell's squared inverse step in float pairs, the ring's
-    // largest kept as a pair and turned into the ring's step once (no FP32
-    // screen: in a nearly axisymmetric ring most cells fall inside any
-    // screen's margin, and each would then take FP64)
-    const bool pair_cfl = PAIR && ph.stabilize != 2;
-    f2 local2{0.f, 0.f};
     const int nz = g.nz, nr = g.nr;
     const int i = blockIdx.x;
     float local32 = 3.0e38f;
@@ -1888,8 +1794,6 @@ __global__ void __launch_bounds__(256, PAIR ? 4 : 3) k_derived_cfl(Geo g, Tables
     for (int j = threadIdx.x; j < nz; j += blockDim.x) {
         const size_t c = row + j;
         double c_s, n;
-        f2 cp2{0.f, 0.f};  // c_s as a pair where the pair path formed it
-        bool have_cp2 = false;
         if (mode & 1) {
             const double sg = S[c];
             if (ph.adiabatic && PAIR) {
@@ -1899,8 +1803,6 @@ __global__ void __launch_bounds__(256, PAIR ? 4 : 3) k_derived_cfl(Geo g, Tables
                 const f2 cp = f2_sqrt(f2_smul(f2_split(ph.g_gm1), es));
                 const float2 hf = t.ptab[(t.HFacAdi - t.tbase) + i];
                 const f2 hp = f2_smul(cp, f2{hf.x, hf.y});
-                cp2 = cp;
-                have_cp2 = true;
                 c_s = f2_to_double(cp);
                 cs[c] = c_s;
                 H[c] = f2_to_double(hp);
@@ -1933,11 +1835,7 @@ __global__ void __launch_bounds__(256, PAIR ? 4 : 3) k_derived_cfl(Geo g, Tables
             c_s = cs[c];
             n = nu[c];
         }
-        if (cfl_ring && pair_cfl) {
-            const f2 cpair = have_cp2 ? cp2 : f2_split(c_s);
-            local2 = pair_max(local2, cfl_cell_f2(g, t, ph, sn, i, j, cpair, f2_split(n), vr, vaz,
-                                                  vm0, qplus, qminus, E));
-        } else if (cfl_ring) {
+        if (cfl_ring) {
             const float d32 = cfl_cell32(t32, ph, sn, c_s, n, vr[c], vr[c + nz], vaz[c],
                                          vaz[row + (j == nz - 1 ? 0 : j + 1)], vm0,
                                          ph.adiabatic ? qplus[c] : 0.0,
@@ -1949,11 +1847,7 @@ __global__ void __launch_bounds__(256, PAIR ? 4 : 3) k_derived_cfl(Geo g, Tables
             local32 = fminf(local32, d32);
         }
     }
-    if (cfl_ring && pair_cfl) {
-        const f2 m = block_max_f2(local2, redf);
-        const double d = f2_to_double(f2_sdiv(f2_split(ph.cfl), f2_sqrt(m)));
-        if (dbits(d) < dbits(local)) local = d;
-    } else if (cfl_ring) {
+    if (cfl_ring) {
         // the FP64 dt of the cells the FP32 screen puts within 2^-15 of the
         // ring's FP32 minimum; that set holds the FP64 minimum, since the
         // screen's error is below 2^-19 (each thread reads back the screen
@@ -2300,10 +2194,12 @@ void launch_com_damping(const Launch &L, const ComSpec &c, double dt, const Stat
 }
 
 void launch_ghost(const Launch &L, const BcSpec &bc, double omf, const State &s,
-                  unsigned long long *dt_min)
+                  unsigned long long *dt_min, double *mean)
 {
-    launch(k_ghost, dim3((L.g.nz + 127) / 128, 8), 128, 0, L.stream, L.g, L.t, bc, omf, s,
-           dt_min);
+    const int cols = (L.g.nz + 127) / 128;
+    const int mean_rows = mean ? std::min((L.g.nr - 2 + cols - 1) / cols, 4096) : 0;
+    launch(k_ghost, dim3(cols, 8 + mean_rows), 128, 0, L.stream, L.g, L.t, bc, omf, s, dt_min,
+           mean);
 }
 
 int radial_chunk_for(bool pair, bool adiabatic, int nr, int nz)
@@ -2533,13 +2429,9 @@ void launch_cfl_cells(const Launch &L, const State &s, double *out)
 void launch_derived_cfl(const Launch &L, int mode, const State &s, unsigned long long *dt_min)
 {
     auto k = L.pair ? k_derived_cfl<true> : k_derived_cfl<false>;
-    // the FP32 screen's per-cell steps: only the FP64-arithmetic kernel and
-    // StabilizeViscosity 2 use them (the pair kernel keeps the shared memory
-    // for L1)
-    const bool screen = !L.pair || L.ph.stabilize == 2;
-    launch(
-        k, L.g.nr, 256, screen ? (size_t)L.g.nz * sizeof(float) : 0, L.stream, L.g, L.t, L.ph, mode, L.ph.art_visc_sn, s.sigma, s.energy, s.vr, s.vaz, s.qplus,
-        s.qminus, s.cs, s.H, s.P, s.T, s.nu, s.corr_phi, s.corr_r, dt_min);
+    launch(k, L.g.nr, 256, (size_t)L.g.nz * sizeof(float), L.stream, L.g, L.t, L.ph, mode,
+           L.ph.art_visc_sn, s.sigma, s.energy, s.vr, s.vaz, s.qplus, s.qminus, s.cs, s.H, s.P, s.T,
+           s.nu, s.corr_phi, s.corr_r, dt_min);
 }
 
 void launch_gas_quantities(const Launch &L, double radius, double omf, const double *S,

@@ -540,12 +540,14 @@ __global__ void __launch_bounds__(kThreads, 4)
     }
 }
 
+}  // namespace
+
 // Rings per march: as many as leave the device two rounds of resident warps
 // (a march forms a ring or less twice, but a short grid needs its warps), at
 // most 16.  Measured, ms of the three kernels per step: 2048 x 6144 with 2, 8 and
 // 16 rings 1.551, 1.327, 1.308; 512 x 1536 with 1, 2, 4, 8 rings 0.129, 0.115,
 // 0.119, 0.126; 128 x 384 with 1, 2, 4 rings 0.029, 0.032, 0.043.
-int chunk_for(int nr, int nwin)
+int win::march_rings(int nr, int nwin)
 {
     static const int nsm = [] {
         int dev = 0, n = 0;
@@ -558,12 +560,10 @@ int chunk_for(int nr, int nwin)
     return (int)std::max(1LL, std::min(16LL, (long long)nr * nwin / two_rounds));
 }
 
-}  // namespace
-
 void launch_source_window(const Launch &L, double dt, double omf, const Bodies &b,
                           const State &s, double *vr_out, double *vaz_out)
 {
-    const int nwin = windows(L.g.nz), chunk = chunk_for(L.g.nr, nwin);
+    const int nwin = windows(L.g.nz), chunk = march_rings(L.g.nr, nwin);
     const int jobs = nwin * ((L.g.nr + chunk - 1) / chunk), per = kThreads / 32;
     auto k = L.g.nz % 2 == 0 ? k_source_w<true> : k_source_w<false>;
     launch(k, (jobs + per - 1) / per, kThreads, 0, L.stream,
@@ -574,7 +574,7 @@ void launch_source_window(const Launch &L, double dt, double omf, const Bodies &
 void launch_artvisc_pair(const Launch &L, double dt, const State &s, double *vr_out,
                          double *vaz_out)
 {
-    const int nwin = windows(L.g.nz), chunk = chunk_for(L.g.nr, nwin);
+    const int nwin = windows(L.g.nz), chunk = march_rings(L.g.nr, nwin);
     const int jobs = nwin * ((L.g.nr + chunk - 1) / chunk), per = kThreads / 32;
     auto pick = [&](auto even) {
         return L.ph.adiabatic ? k_artvisc_w<even.value, true> : k_artvisc_w<even.value, false>;
@@ -588,7 +588,7 @@ void launch_artvisc_pair(const Launch &L, double dt, const State &s, double *vr_
 void launch_viscous_pair(const Launch &L, double dt, double beta_inv, int mode, const State &s,
                          double *vr_out, double *vaz_out)
 {
-    const int nwin = windows(L.g.nz), chunk = chunk_for(L.g.nr, nwin);
+    const int nwin = windows(L.g.nz), chunk = march_rings(L.g.nr, nwin);
     const int jobs = nwin * ((L.g.nr + chunk - 1) / chunk), per = kThreads / 32;
     auto pick = [&](auto even) {
         return L.ph.adiabatic ? k_viscous_w<even.value, true> : k_viscous_w<even.value, false>;

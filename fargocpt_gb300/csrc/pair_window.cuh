@@ -18,6 +18,8 @@ constexpr int kInner = 60;      // cells a warp writes per ring
 constexpr int kThreads = 128;   // threads per block
 
 inline int windows(int nz) { return (nz + kInner - 1) / kInner; }
+// rings per march of a grid of nwin windows (kernels_kick.cu)
+int march_rings(int nr, int nwin);
 
 __device__ __forceinline__ f2x2 operator+(f2x2 a, f2x2 b) { return f2_sadd(a, b); }
 __device__ __forceinline__ f2x2 operator-(f2x2 a, f2x2 b) { return f2_ssub(a, b); }
