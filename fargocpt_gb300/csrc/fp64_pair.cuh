@@ -182,6 +182,13 @@ __device__ __forceinline__ float rcp_approx(float x)
     return r;
 }
 
+__device__ __forceinline__ float rsqrt_approx(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // 1 / d for a normal d: r = rcp(d.h), then r + r (1 - d r)
 __device__ __forceinline__ f2 f2_rcp(f2 d)
 {

@@ -262,102 +262,135 @@ __global__ void f_derived_cfl(GeoF g, TablesF t, PhysF ph, int mode, const float
 }
 
 // disk force on up to kForceBodies32 bodies in one pass over the ring, and the
-// gas mass: separations as float pairs, sums as compensated float pairs per
-// thread and in FP64 across the block.  partial[5 b .. 5 b + 4] of the ring's
+// gas mass: separations as float pairs, sums as compensated float pairs within
+// the warps and in FP64 across them.  partial[5 b .. 5 b + 4] of the ring's
 // row: inner x, inner y, outer x, outer y, mass (ComputeDiskOnPlanetAccel,
 // Force.cpp:23-122; the ring mean removed with CorrectDiskSelfgravity,
 // Force.cpp:64-66; gas_total_mass, quantities.cpp:51-74).
 constexpr int kForceBodies32 = 4;
 struct ForceBodies32 {
     int n;
-    double x[kForceBodies32], y[kForceBodies32], a[kForceBodies32], rsm[kForceBodies32];
+    double a[kForceBodies32];
+    float xh[kForceBodies32], xl[kForceBodies32], yh[kForceBodies32], yl[kForceBodies32];
+    float frsm[kForceBodies32];
 };
 
-__global__ void f_disk_force_bodies(GeoF g, TablesF t, PhysF ph, ForceBodies32 fb,
-                                    const float *__restrict__ S,
-                                    const float *__restrict__ S_lo, const float *__restrict__ H,
-                                    double *__restrict__ partial, int width)
+//
+// A lane takes two adjacent cells in packed FP32 instructions; the block's sums
+// as block_pair_sum and block_eight_sums form them: with scalar instructions and
+// every sum in FP64 across the block (9 sums of 256 threads: 38% of the FP64 pipe)
+// 4 bodies on 2048 x 6144 cells took 0.239 ms, this 0.083.
+constexpr int kForceThreads32 = 128;
+template <bool EVEN>
+__global__ void __launch_bounds__(kForceThreads32, 8)
+    f_disk_force_bodies(GeoF g, TablesF t, PhysF ph, ForceBodies32 fb, const float *__restrict__ S,
+                        const float *__restrict__ S_lo, const float *__restrict__ H,
+                        double *__restrict__ partial, int width)
 {
+    using fgpu::vadd;
+    using fgpu::vfma;
+    using fgpu::vmul;
+    using fgpu::vsub;
     fgpu::follow_predecessor();
-    __shared__ double red[33];
+    __shared__ double part[kForceThreads32 / 4], total[8], ring;
+    __shared__ float2 mean;
     const int nz = g.nz;
     const int i = blockIdx.x + 1;
     const size_t row = (size_t)i * nz;
+    auto both = [](float a) { return make_float2(a, a); };
+    // cells j and j + 1 (past the ring's end: rest)
+    auto load = [&](const float *p, int j, float rest) {
+        if (EVEN) return *reinterpret_cast<const float2 *>(p + j);
+        return make_float2(p[j], j + 1 < nz ? p[j + 1] : rest);
+    };
+    // sum += x, compensated (TwoSum, Knuth 1969)
+    auto add = [](fgpu::f2x2 &sum, float2 x) {
+        const fgpu::f2x2 s = fgpu::two_sum(sum.h, x);
+        sum = fgpu::f2x2{s.h, vadd(sum.l, s.l)};
+    };
     // sigma as its compensated pair; the ring sum gives the ring mean and,
-    // times the cell area, the ring's mass.  Each thread sums its cells as a
-    // compensated float pair (TwoSum, Knuth 1969), the block in FP64.
-    float sh_ = 0.f, sl_ = 0.f;
-    for (int j = threadIdx.x; j < nz; j += blockDim.x) {
-        two_sum_add(sh_, sl_, S[row + j]);
-        sl_ += S_lo[row + j];
+    // times the cell area, the ring's mass
+    const fgpu::f2x2 zero{both(0.f), both(0.f)};
+    fgpu::f2x2 sum = zero;
+#pragma unroll 4
+    for (int j = 2 * threadIdx.x; j < nz; j += 2 * kForceThreads32) {
+        add(sum, load(S + row, j, 0.f));
+        sum.l = vadd(sum.l, load(S_lo + row, j, 0.f));
     }
-    const double ring_sum = bsum_d((double)sh_ + (double)sl_, red);
-    const double sigma1d = ph.correct_sg ? ring_sum / nz : 0.0;
-    const float mh = (float)sigma1d, ml = (float)(sigma1d - (double)mh);
+    const double ring_sum = block_pair_sum(fgpu::pair_halves(sum), part);
+    if (threadIdx.x == 0) {
+        const double sigma1d = ph.correct_sg ? ring_sum / nz : 0.0;
+        const float h = (float)sigma1d;
+        ring = ring_sum;
+        mean = make_float2(h, (float)(sigma1d - (double)h));
+    }
+    __syncthreads();
+    const float2 m = mean;
     // cell centres and the bodies as float pairs (see potential_cell): the
     // distance loses nothing to cancellation near a body
     float pxh[kForceBodies32], pxl[kForceBodies32], pyh[kForceBodies32], pyl[kForceBodies32];
     float frsm[kForceBodies32];
+    fgpu::f2x2 ax[kForceBodies32], ay[kForceBodies32];
 #pragma unroll
     for (int b = 0; b < kForceBodies32; ++b) {
-        const double px = b < fb.n ? fb.x[b] : 0.0, py = b < fb.n ? fb.y[b] : 0.0;
-        pxh[b] = (float)px;
-        pxl[b] = (float)(px - (double)pxh[b]);
-        pyh[b] = (float)py;
-        pyl[b] = (float)(py - (double)pyh[b]);
-        frsm[b] = b < fb.n ? (float)fb.rsm[b] : 0.f;
+        pxh[b] = fb.xh[b];
+        pxl[b] = fb.xl[b];
+        pyh[b] = fb.yh[b];
+        pyl[b] = fb.yl[b];
+        frsm[b] = fb.frsm[b];
+        ax[b] = ay[b] = zero;
     }
-    const float rh = t.Rmed[i], rl = t.RmedLo[i];
-    float axh[kForceBodies32], axl[kForceBodies32], ayh[kForceBodies32], ayl[kForceBodies32];
-#pragma unroll
-    for (int b = 0; b < kForceBodies32; ++b) axh[b] = axl[b] = ayh[b] = ayl[b] = 0.f;
-    for (int j = threadIdx.x; j < nz; j += blockDim.x) {
-        const float ch = t.cosHi[j], cl = t.cosLo[j], sh = t.sinHi[j], sl = t.sinLo[j];
-        const float xh = rh * ch, yh = rh * sh;
-        const float xl = fmaf(rh, ch, -xh) + fmaf(rh, cl, rl * ch);
-        const float yl = fmaf(rh, sh, -yh) + fmaf(rh, sl, rl * sh);
-        const float sm = ph.eps_smooth * H[row + j];
-        const float sm2 = sm * sm;
+    const float2 rh = both(t.Rmed[i]), rl = both(t.RmedLo[i]);
+    const float2 eps = both(ph.eps_smooth);
+#pragma unroll 2
+    for (int j = 2 * threadIdx.x; j < nz; j += 2 * kForceThreads32) {
+        const float2 ch = load(t.cosHi, j, 0.f), cl = load(t.cosLo, j, 0.f);
+        const float2 sh = load(t.sinHi, j, 0.f), sl = load(t.sinLo, j, 0.f);
+        // (the cell past the ring's end: sigma at the mean, its terms zero)
+        const float2 sg = load(S + row, j, m.x), sg_lo = load(S_lo + row, j, m.y);
+        const float2 sm = vmul(eps, load(H + row, j, 1.f));
+        const float2 sm2 = vmul(sm, sm);
+        const float2 xh = vmul(rh, ch), yh = vmul(rh, sh);
+        const float2 xl = vadd(vfma(rh, ch, fgpu::vneg(xh)), vfma(rh, cl, vmul(rl, ch)));
+        const float2 yl = vadd(vfma(rh, sh, fgpu::vneg(yh)), vfma(rh, sl, vmul(rl, sh)));
         // the ring mean removed (CorrectDiskSelfgravity) from the pair
-        const float dsig = ph.correct_sg ? (S[row + j] - mh) + (S_lo[row + j] - ml)
-                                         : S[row + j] + S_lo[row + j];
+        const float2 dsig = vadd(vsub(sg, both(m.x)), vsub(sg_lo, both(m.y)));
 #pragma unroll
         for (int b = 0; b < kForceBodies32; ++b) {
             if (b < fb.n) {
-                const float dx = (xh - pxh[b]) + (xl - pxl[b]);
-                const float dy = (yh - pyh[b]) + (yl - pyl[b]);
-                const float d2 = fmaf(dx, dx, fmaf(dy, dy, sm2));
-                const float rinv = rsqrtf(d2);
-                float fk = 1.f;
+                const float2 dx = vadd(vsub(xh, both(pxh[b])), vsub(xl, both(pxl[b])));
+                const float2 dy = vadd(vsub(yh, both(pyh[b])), vsub(yl, both(pyl[b])));
+                const float2 d2 = vfma(dx, dx, vfma(dy, dy, sm2));
+                const float2 r = make_float2(fgpu::rsqrt_approx(d2.x), fgpu::rsqrt_approx(d2.y));
+                float2 r3 = vmul(vmul(r, r), r);
                 if (frsm[b] > 0.f) {
-                    const float dsm = d2 * rinv;
-                    if (dsm < frsm[b]) {
+                    auto klahr = [&](float dsm) {
                         const float q = dsm / frsm[b];
-                        fk = -(3.f * q * q * q * q - 4.f * q * q * q);
-                    }
+                        return dsm < frsm[b] ? -(3.f * q * q * q * q - 4.f * q * q * q) : 1.f;
+                    };
+                    r3 = vmul(r3, make_float2(klahr(d2.x * r.x), klahr(d2.y * r.y)));
                 }
-                const float w = dsig * (rinv * rinv * rinv * fk);
-                two_sum_add(axh[b], axl[b], w * dx);
-                two_sum_add(ayh[b], ayl[b], w * dy);
+                const float2 w = vmul(dsig, r3);
+                add(ax[b], vmul(w, dx));
+                add(ay[b], vmul(w, dy));
             }
         }
     }
-    const double f = t.Surf_d[i] * ph.G_d;
-    double *p = partial + (size_t)blockIdx.x * width;
+    fgpu::f2 v[2 * kForceBodies32];
 #pragma unroll
     for (int b = 0; b < kForceBodies32; ++b) {
-        if (b < fb.n) {
-            const double ax = bsum_d((double)axh[b] + (double)axl[b], red);
-            const double ay = bsum_d((double)ayh[b] + (double)ayl[b], red);
-            if (threadIdx.x == 0) {
-                const bool inner = t.Rmed_d[i] < fb.a[b];
-                p[5 * b + 0] = inner ? f * ax : 0.0;
-                p[5 * b + 1] = inner ? f * ay : 0.0;
-                p[5 * b + 2] = inner ? 0.0 : f * ax;
-                p[5 * b + 3] = inner ? 0.0 : f * ay;
-                p[5 * b + 4] = t.Surf_d[i] * ring_sum;
-            }
-        }
+        v[2 * b] = fgpu::pair_halves(ax[b]);
+        v[2 * b + 1] = fgpu::pair_halves(ay[b]);
+    }
+    block_eight_sums(v, part, total);
+    if (threadIdx.x < 2 * fb.n) {
+        const int b = threadIdx.x >> 1, c = threadIdx.x & 1;
+        const double s = t.Surf_d[i] * ph.G_d * total[threadIdx.x];
+        const bool inner = t.Rmed_d[i] < fb.a[b];
+        double *p = partial + (size_t)blockIdx.x * width + 5 * b;
+        p[c] = inner ? s : 0.0;
+        p[2 + c] = inner ? 0.0 : s;
+        if (c == 0) p[4] = t.Surf_d[i] * ring;
     }
 }
 
@@ -1420,15 +1453,19 @@ int Engine32::disk_forces(int n, const double *x, const double *y, const double 
         ForceBodies32 fb{};
         fb.n = std::min(kForceBodies32, n - b0);
         for (int b = 0; b < fb.n; ++b) {
-            fb.x[b] = x[b0 + b];
-            fb.y[b] = y[b0 + b];
+            auto split = [](double v, float &h, float &l) {
+                h = (float)v;
+                l = (float)(v - (double)h);
+            };
+            split(x[b0 + b], fb.xh[b], fb.xl[b]);
+            split(y[b0 + b], fb.yh[b], fb.yl[b]);
             fb.a[b] = a[b0 + b];
-            fb.rsm[b] = rsm[b0 + b];
+            fb.frsm[b] = (float)rsm[b0 + b];
         }
         const int width = 5 * fb.n;
-        fgpu::launch(f_disk_force_bodies, rows, 256, 0, stream, geo, tabs, phys, fb, fld[FGPU_SIGMA],
-                                                      sigma_lo, fld[FGPU_SCALE_HEIGHT], partial,
-                                                      width);
+        fgpu::launch(nz % 2 == 0 ? f_disk_force_bodies<true> : f_disk_force_bodies<false>, rows,
+                     kForceThreads32, 0, stream, geo, tabs, phys, fb, fld[FGPU_SIGMA], sigma_lo,
+                     fld[FGPU_SCALE_HEIGHT], partial, width);
         fgpu::launch(f_reduce_cols, width, kReduceThreads, 0, stream, partial, rows, width, dev + 5 * b0);
     }
     CKF(cudaGetLastError());

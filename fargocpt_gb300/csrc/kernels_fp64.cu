@@ -1943,101 +1943,6 @@ __global__ void k_accrete(Geo g, Tables t, Phys ph, AccretionSpec a, double *__r
     }
 }
 
-// ---------------------------------------------------------------------------
-// ComputeDiskOnPlanetAccel (src/Force.cpp:23-122) for up to kForceBodies
-// bodies in one pass over the ring: with CorrectDiskSelfgravity the ring mean
-// of sigma is subtracted (Force.cpp:64-66), and the gas mass of the ring
-// (gas_total_mass, quantities.cpp:51-74) comes along.  One CTA per active
-// ring writes, for body b, partial[5 b .. 5 b + 4] = (inner x, inner y,
-// outer x, outer y, mass) of its ring (split at Rmed < a, the body's distance
-// from the origin); k_reduce_cols adds the rings with compensation in a
-// fixed order.  Per body and cell: the separation, its smoothed inverse cube
-// (one rsqrt), Klahr's cubic factor inside r_sm, and the two products into
-// the sums, all in float-pair arithmetic (fp64_pair.cuh, about 2^-46
-// relative; sums of pairs per thread, FP64 across the block); G and the
-// ring's Surf multiply the ring's sums once.
-// ---------------------------------------------------------------------------
-struct ForceBodies {
-    int n;  // bodies in this pass (1 .. kForceBodies)
-    unsigned klahr;  // bit b: body b has Klahr smoothing (rsm > 0)
-    double a[kForceBodies], rsm[kForceBodies];
-    float xh[kForceBodies], xl[kForceBodies], yh[kForceBodies], yl[kForceBodies];
-};
-
-__global__ void __launch_bounds__(256, 4) k_disk_force_bodies(Geo g, Tables t, Phys ph, ForceBodies fb,
-                                    const double *__restrict__ S, const double *__restrict__ H,
-                                    double *__restrict__ partial, int width)
-{
-    follow_predecessor();
-    __shared__ double red[33];
-    const int nz = g.nz;
-    const int i = blockIdx.x + 1;  // radial_first_active .. radial_active_size - 1
-    const size_t row = (size_t)i * nz;
-    double ps = 0.0;
-    for (int j = threadIdx.x; j < nz; j += blockDim.x) ps += S[row + j];
-    const double ring_sum = block_sum(ps, red);
-    const double sigma1d = ph.correct_sg ? ring_sum / nz : 0.0;
-    const double rmed = t.Rmed[i];
-    const f2 rm{t.RmedHi[i], t.RmedLo[i]};
-    // per body and thread, the sums of the x and y terms as float pairs
-    float axh[kForceBodies], axl[kForceBodies], ayh[kForceBodies], ayl[kForceBodies];
-#pragma unroll
-    for (int b = 0; b < kForceBodies; ++b) axh[b] = axl[b] = ayh[b] = ayl[b] = 0.f;
-    const f2 eps = f2_split(ph.eps_smooth);
-    float rsm_f[kForceBodies];
-#pragma unroll
-    for (int b = 0; b < kForceBodies; ++b) rsm_f[b] = b < fb.n ? f2_split(fb.rsm[b]).h : 0.f;
-    for (int j = threadIdx.x; j < nz; j += blockDim.x) {
-        const f2 smooth = f2_smul(eps, f2_split(H[row + j]));
-        const f2 s2 = f2_smul(smooth, smooth);
-        const f2 xc = f2_smul(rm, f2{t.cosHi[j], t.cosLo[j]});
-        const f2 yc = f2_smul(rm, f2{t.sinHi[j], t.sinLo[j]});
-        // sigma less the ring mean: the FP64 difference (they agree closely)
-        const f2 dsig = f2_split(S[row + j] - sigma1d);
-#pragma unroll
-        for (int b = 0; b < kForceBodies; ++b) {
-            if (b < fb.n) {
-                const f2 dx = f2_ssub(xc, f2{fb.xh[b], fb.xl[b]});
-                const f2 dy = f2_ssub(yc, f2{fb.yh[b], fb.yl[b]});
-                const f2 dsm2 = f2_sadd(f2_sadd(f2_smul(dx, dx), f2_smul(dy, dy)), s2);
-                const f2 rinv = f2_rsqrt(dsm2);
-                f2 w = f2_smul(dsig, f2_smul(f2_smul(rinv, rinv), rinv));
-                if ((fb.klahr >> b) & 1u) {
-                    // Klahr's factor inside r_sm (Force.cpp:88-100): rare, in FP64
-                    const f2 dsm_p = f2_mul(dsm2, rinv);
-                    if (maybe_inside(dsm_p, rsm_f[b])) {
-                        const double dsm = f2_to_double(dsm_p);
-                        if (dsm < fb.rsm[b]) {
-                            const double q = dsm / fb.rsm[b];
-                            w = f2_split(f2_to_double(w) *
-                                         -(3.0 * (q * q * q * q) - 4.0 * (q * q * q)));
-                        }
-                    }
-                }
-                f2_accumulate(axh[b], axl[b], f2_smul(w, dx));
-                f2_accumulate(ayh[b], ayl[b], f2_smul(w, dy));
-            }
-        }
-    }
-    const double gs = ph.G * t.Surf[i];
-    double *p = partial + (size_t)blockIdx.x * width;
-#pragma unroll
-    for (int b = 0; b < kForceBodies; ++b) {
-        if (b < fb.n) {
-            const double sx = block_sum((double)axh[b] + (double)axl[b], red) * gs;
-            const double sy = block_sum((double)ayh[b] + (double)ayl[b], red) * gs;
-            if (threadIdx.x == 0) {
-                const bool inner = rmed < fb.a[b];
-                p[5 * b + 0] = inner ? sx : 0.0;
-                p[5 * b + 1] = inner ? sy : 0.0;
-                p[5 * b + 2] = inner ? 0.0 : sx;
-                p[5 * b + 3] = inner ? 0.0 : sy;
-                p[5 * b + 4] = t.Surf[i] * ring_sum;
-            }
-        }
-    }
-}
-
 // gas_total_mass (quantities.cpp:51-74) and gas_angular_momentum
 // (quantities.cpp:242-276) of each active ring with Rmed <= radius (zero
 // otherwise): one CTA per ring writes (mass, angular momentum).  The ring's
@@ -2088,14 +1993,6 @@ __global__ void k_reduce_rows(const double *__restrict__ partial, int rows, int 
     const int w = threadIdx.x >> 5;
     if (w < width) warp_compensated_rows(partial, rows, width, w, out);
 }
-// the same with one block per component, for wide records
-__global__ void k_reduce_cols(const double *__restrict__ partial, int rows, int width,
-                              double *__restrict__ out)
-{
-    follow_predecessor();
-    block_compensated_rows(partial, rows, width, blockIdx.x, out);
-}
-
 // NaN/Inf scan of one field: records the first bad flat index (atomicMin).
 __global__ void k_check_finite(const double *__restrict__ x, size_t n, unsigned long long *bad)
 {
@@ -2447,31 +2344,6 @@ void launch_scale_sigma(const Launch &L, double *S, double target, const double 
     const size_t n = (size_t)L.g.nr * L.g.nz;
     const int blocks = (int)std::min<size_t>((n + 255) / 256, 4096);
     k_scale_sigma<<<blocks, 256, 0, L.stream>>>(S, n, target, mass);
-}
-
-void launch_disk_force(const Launch &L, int n, const double *px, const double *py,
-                       const double *pa, const double *rsm, const double *S, const double *H,
-                       double *partial, double *out)
-{
-    const int rows = L.g.nr - 2;
-    for (int b0 = 0; b0 < n; b0 += kForceBodies) {
-        ForceBodies fb{};
-        fb.n = std::min(kForceBodies, n - b0);
-        for (int b = 0; b < fb.n; ++b) {
-            fb.xh[b] = (float)px[b0 + b];
-            fb.xl[b] = (float)(px[b0 + b] - (double)fb.xh[b]);
-            fb.yh[b] = (float)py[b0 + b];
-            fb.yl[b] = (float)(py[b0 + b] - (double)fb.yh[b]);
-            fb.a[b] = pa[b0 + b];
-            fb.rsm[b] = rsm[b0 + b];
-            if (fb.rsm[b] > 0.0) fb.klahr |= 1u << b;
-        }
-        const int width = 5 * fb.n;
-        launch(k_disk_force_bodies, rows, 256, 0, L.stream, L.g, L.t, L.ph, fb, S, H, partial,
-               width);
-        launch(k_reduce_cols, width, kReduceThreads, 0, L.stream, partial, rows, width,
-               out + 5 * b0);
-    }
 }
 
 void launch_check_finite(const Launch &L, const double *x, size_t n, unsigned long long *bad)

@@ -1,30 +1,35 @@
-// Reproducible compensated sum of per-ring partial sums (disk force, mass).
+// Sums over a block: ring means, the disk force's terms, and the reproducible
+// compensated sum of per-ring partial sums.
 #pragma once
+
+#include "fp64_pair.cuh"
 
 #include <cuda_runtime.h>
 
-// The mean of a ring's n values by a block of 128 threads, eight loads of a
-// thread in flight; complete in every thread's return value.  A value of the
-// first one's sign and exponent differs from it by a whole number of units in
-// its last place, the difference of the two bit patterns: those are summed as
-// integers, exactly; only blocks of eight with another take FP64 additions (1.6 per
-// clock and SM, also where a predicate is off: 2048 x 6144 cells in 55 us with a
-// choice per value, in 22 with one per block).
+// The mean of a ring's n values by the block (at least 128 threads), complete in
+// every thread's return value.  A value of the first one's sign and exponent
+// differs from it by a whole number of units in its last place, the difference of
+// the two bit patterns: those are summed as integers, exactly; only blocks of
+// eight with another take FP64 additions (1.6 per clock and SM, also where a
+// predicate is off: 2048 x 6144 cells in 55 us with a choice per value, in 22 with
+// one per block).  n <= 2^18, or all take them (the integers' range).
 __device__ __forceinline__ double block_row_mean(const double *__restrict__ v, int n)
 {
-    __shared__ double part[4];
+    __shared__ double part[33], part_other[32];
+    const int tid = threadIdx.x, bs = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const double v0 = v[0];
     const long long b0 = __double_as_longlong(v0);
     const int top = (int)(b0 >> 52), e = top & 0x7ff;
-    const bool finite = e != 0x7ff;
+    const bool exact = e != 0x7ff && n <= 1 << 18;
     long long ulps = 0;
+    int others = 0;
     double other = 0.0;
-    for (int j = threadIdx.x; j < n; j += 8 * 128) {
+    for (int j = tid; j < n; j += 8 * bs) {
         long long u[8];
-        bool same = finite;
+        bool same = exact;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            const int c = j + k * 128;
+            const int c = j + k * bs;
             const long long b = c < n ? __double_as_longlong(v[c]) : b0;
             same = same && (int)(b >> 52) == top;
             u[k] = b - b0;
@@ -34,16 +39,92 @@ __device__ __forceinline__ double block_row_mean(const double *__restrict__ v, i
             for (int k = 0; k < 8; ++k) ulps += u[k];
         } else {
 #pragma unroll 1
-            for (int c = j; c < n && c < j + 8 * 128; c += 128) other += v[c] - v0;
+            for (int c = j; c < n && c < j + 8 * bs; c += bs) {
+                other += v[c];
+                ++others;
+            }
         }
     }
-    const double ulp = ldexp(top < 0 ? -1.0 : 1.0, (e > 1 ? e : 1) - 1075);
-    double s = other + (double)ulps * ulp;
+    double s = (double)ulps;
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    __syncthreads();  // part of a call before this one has been read
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    const bool any = __syncthreads_or(others);  // (part of a call before this has been read)
+    if (any) {
+        other = fma(-(double)others, v0, other);
+        for (int o = 16; o > 0; o >>= 1) other += __shfl_down_sync(0xffffffffu, other, o);
+        if (lane == 0) part_other[warp] = other;
+    }
+    if (lane == 0) part[warp] = s;
     __syncthreads();
-    return v0 + ((part[0] + part[1]) + (part[2] + part[3])) / (double)n;
+    if (tid == 0) {
+        double t = 0.0, to = 0.0;
+        for (int w = 0; w < bs >> 5; ++w) {
+            t += part[w];
+            if (any) to += part_other[w];
+        }
+        const double ulp = ldexp(top < 0 ? -1.0 : 1.0, (e > 1 ? e : 1) - 1075);
+        part[32] = v0 + (t * ulp + to) / (double)n;
+    }
+    __syncthreads();
+    return part[32];
+}
+
+namespace fgpu {
+__device__ __forceinline__ f2 pair_plus(f2 a, f2 b)
+{
+    const f2 s = two_sum(a.h, b.h);
+    return f2{s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l))};
+}
+__device__ __forceinline__ f2 pair_from(f2 a, int o)
+{
+    return f2{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)};
+}
+// the sum of a lane's two cells
+__device__ __forceinline__ f2 pair_halves(f2x2 s) { return pair_plus(first(s), second(s)); }
+}  // namespace fgpu
+
+// One sum over the block, a float pair of every thread: pairs within the warps,
+// the warps' sums in FP64; the value is thread 0's (part: a double per warp)
+__device__ __forceinline__ double block_pair_sum(fgpu::f2 v, double *part)
+{
+    for (int o = 16; o > 0; o >>= 1) v = fgpu::pair_plus(v, fgpu::pair_from(v, o));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = (double)v.h + (double)v.l;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < blockDim.x >> 5; ++w) t += part[w];
+    return t;
+}
+
+// Eight sums of every thread of the block, float pairs (hi, lo) each: the halves
+// of a warp exchange four of the eight, then two, then one, so a warp adds nine
+// pairs where eight separate sums would add forty (in FP64, 20 cycles an SM each,
+// these took longer than a 128-cell ring's terms); the warps' sums in FP64.
+// Complete in total[0 .. 7] after the call; every sum is formed along the same
+// tree.
+__device__ __forceinline__ void block_eight_sums(const fgpu::f2 (&v)[8], double *part, double *total)
+{
+    using fgpu::f2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    f2 a[4], b[2];
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a[k] = fgpu::pair_plus(b4 ? v[k + 4] : v[k],
+                               fgpu::pair_from(b4 ? v[k] : v[k + 4], 16));
+#pragma unroll
+    for (int k = 0; k < 2; ++k) b[k] = fgpu::pair_plus(b3 ? a[k + 2] : a[k],
+                               fgpu::pair_from(b3 ? a[k] : a[k + 2], 8));
+    f2 s = fgpu::pair_plus(b2 ? b[1] : b[0], fgpu::pair_from(b2 ? b[0] : b[1], 4));
+    s = fgpu::pair_plus(s, fgpu::pair_from(s, 2));
+    s = fgpu::pair_plus(s, fgpu::pair_from(s, 1));
+    // lane 4 q holds sum q (bits 4, 3, 2 of the lane: 4, 2, 1)
+    if ((lane & 3) == 0) part[8 * warp + (lane >> 2)] = (double)s.h + (double)s.l;
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        double t = 0.0;
+        for (int w = 0; w < blockDim.x >> 5; ++w) t += part[8 * w + threadIdx.x];
+        total[threadIdx.x] = t;
+    }
+    __syncthreads();
 }
 
 // hi + lo with lo the compensation still to be subtracted: s + s2 exactly
