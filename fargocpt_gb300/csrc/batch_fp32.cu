@@ -64,7 +64,11 @@ __device__ __forceinline__ int disk_of(const int *__restrict__ start, int nd, in
     return lo;
 }
 
-// Per-cell tiles: blockDim.x columns x rpb rings of one disk; rows nr + extra.
+// a tile of more threads is walked by this many
+constexpr int kCellThreads = 512;
+
+// Per-cell tiles: 4 blockDim.x columns (a Quad per thread) x rpb rings of one
+// disk; rows nr + extra.
 template <class F>
 __device__ __forceinline__ void for_cells(const DiskF *__restrict__ D, const StepF *__restrict__ S,
                                           const int *__restrict__ start, int nd, int rpb,
@@ -75,86 +79,138 @@ __device__ __forceinline__ void for_cells(const DiskF *__restrict__ D, const Ste
         const int d = disk_of(start, nd, tile);
         if (!S[d].run) continue;
         const DiskF &k = D[d];
-        const int nz = k.g.nz;
-        const int ncol = (nz + blockDim.x - 1) / blockDim.x;
+        const int nz = k.g.nz, wide = 4 * blockDim.x;
+        const int ncol = (nz + wide - 1) / wide;
         const int local = tile - __ldg(start + d);
-        const int j = (local % ncol) * blockDim.x + threadIdx.x;
-        if (j >= nz) continue;
+        const int j0 = (local % ncol) * wide;
         const int i0 = (local / ncol) * rpb;
         const int i1 = min(i0 + rpb, k.g.nr + extra);
-        for (int i = i0; i < i1; ++i) f(k, S[d], i, j);
+        if (nz % 4 == 0) {
+            const Quad<true> q{nz, j0 + 4 * (int)threadIdx.x, 1};
+            if (q.first < nz)
+                for (int i = i0; i < i1; ++i) f(k, S[d], q, i);
+        } else {
+            const Quad<false> q{nz, j0 + (int)threadIdx.x, (int)blockDim.x};
+            if (q.first < nz)
+                for (int i = i0; i < i1; ++i) f(k, S[d], q, i);
+        }
     }
 }
 
-__global__ void b_potential(const DiskF *__restrict__ D, const StepF *__restrict__ S,
-                            const int *__restrict__ start, int nd, int rpb)
-{
-    fgpu::follow_predecessor();
-    for_cells(D, S, start, nd, rpb, 0, [&](const DiskF &k, const StepF &st, int i, int j) {
-        potential_cell(k.g, k.t, k.ph, st.b, k.H, k.pot, i, j);
-    });
-}
-
-__global__ void b_source(const DiskF *__restrict__ D, const StepF *__restrict__ S,
-                         const int *__restrict__ start, int nd, int rpb)
-{
-    fgpu::follow_predecessor();
-    for_cells(D, S, start, nd, rpb, 1, [&](const DiskF &k, const StepF &st, int i, int j) {
-        source_cell(k.g, k.t, st.fdt, k.s.sigma, k.P, k.pot, k.s.vr, k.s.dv, k.vr_b, k.dv_b, i, j);
-    });
-}
-
-__global__ void b_artvisc_q(const DiskF *__restrict__ D, const StepF *__restrict__ S,
-                            const int *__restrict__ start, int nd, int rpb)
-{
-    fgpu::follow_predecessor();
-    for_cells(D, S, start, nd, rpb, 0, [&](const DiskF &k, const StepF &st, int i, int j) {
+// the substeps for_cells takes
+struct CellsPotential {
+    template <class Q>
+    __device__ void operator()(const DiskF &k, const StepF &st, const Q &q, int i) const
+    {
+        potential_cells(q, k.g, k.t, k.ph, st.b, k.H, k.pot, i);
+    }
+};
+struct CellsSource {
+    template <class Q>
+    __device__ void operator()(const DiskF &k, const StepF &st, const Q &q, int i) const
+    {
+        source_cells(q, k.g, k.t, st.fdt, k.s.sigma, k.P, k.pot, k.s.vr, k.s.dv, k.vr_b, k.dv_b,
+                     i);
+    }
+};
+struct CellsArtviscQ {
+    template <class Q>
+    __device__ void operator()(const DiskF &k, const StepF &st, const Q &q, int i) const
+    {
         if (!(k.ph.adiabatic || k.ph.art_visc_sn || k.ph.art_visc_tw)) return;
-        artvisc_q_cell(k.g, k.t, k.ph, st.fdt, k.s.sigma, k.vr_b, k.dv_b, k.s.energy, k.Qr, k.Qp,
-                       i, j);
-    });
-}
-
-__global__ void b_artvisc_v(const DiskF *__restrict__ D, const StepF *__restrict__ S,
-                            const int *__restrict__ start, int nd, int rpb)
-{
-    fgpu::follow_predecessor();
-    for_cells(D, S, start, nd, rpb, 0, [&](const DiskF &k, const StepF &st, int i, int j) {
+        artvisc_q_cells(q, k.g, k.t, k.ph, st.fdt, k.s.sigma, k.vr_b, k.dv_b, k.s.energy, k.Qr,
+                        k.Qp, i);
+    }
+};
+struct CellsArtviscV {
+    template <class Q>
+    __device__ void operator()(const DiskF &k, const StepF &st, const Q &q, int i) const
+    {
         if (!(k.ph.adiabatic || k.ph.art_visc_sn || k.ph.art_visc_tw)) return;
-        artvisc_v_cell(k.g, k.t, k.ph, st.fdt, k.s.sigma, k.s.energy, k.Qr, k.Qp, k.vr_b, k.dv_b,
-                       k.cs, k.H, k.nu, i, j);
-    });
-}
+        artvisc_v_cells(q, k.g, k.t, k.ph, st.fdt, k.s.sigma, k.s.energy, k.Qr, k.Qp, k.vr_b,
+                        k.dv_b, k.cs, k.H, k.nu, i);
+    }
+};
+struct CellsStress {
+    template <class Q>
+    __device__ void operator()(const DiskF &k, const StepF &, const Q &q, int i) const
+    {
+        stress_cells(q, k.g, k.t, k.s.sigma, k.vr_b, k.dv_b, k.nu, k.divv, k.trr, k.tpp, k.trp, i);
+    }
+};
+struct CellsViscous {
+    template <class Q>
+    __device__ void operator()(const DiskF &k, const StepF &st, const Q &q, int i) const
+    {
+        viscous_cells(q, k.g, k.t, k.ph, st.fdt, st.beta_inv, k.ph.adiabatic ? 7 : 1, k.s.sigma,
+                      k.trr, k.tpp, k.trp, k.divv, k.nu, k.H, k.s.sigma0, k.s.energy0, k.vr_b,
+                      k.dv_b, k.s.energy, k.qplus, k.qminus, nullptr, nullptr, i);
+    }
+};
+struct CellsFinish {
+    template <class Q>
+    __device__ void operator()(const DiskF &k, const StepF &, const Q &q, int i) const
+    {
+        finish_cells(q, k.g, k.t, k.ph, k.mom_w[0], k.mom_w[1], k.mom_w[2], k.mom_w[3], k.sigma_w,
+                     k.energy_w, k.vr_b, k.s.vr, k.s.dv, k.s.sigma, k.s.energy, k.sigma_lo_w,
+                     k.s.sigma_lo, k.ring_shift, i);
+    }
+};
 
-__global__ void b_stress(const DiskF *__restrict__ D, const StepF *__restrict__ S,
-                         const int *__restrict__ start, int nd, int rpb)
+__global__ void __launch_bounds__(kCellThreads)
+    b_potential(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
+                int nd, int rpb)
 {
     fgpu::follow_predecessor();
-    for_cells(D, S, start, nd, rpb, 0, [&](const DiskF &k, const StepF &, int i, int j) {
-        stress_cell(k.g, k.t, k.s.sigma, k.vr_b, k.dv_b, k.nu, k.divv, k.trr, k.tpp, k.trp, i, j);
-    });
+    for_cells(D, S, start, nd, rpb, 0, CellsPotential{});
 }
 
-__global__ void b_viscous(const DiskF *__restrict__ D, const StepF *__restrict__ S,
-                          const int *__restrict__ start, int nd, int rpb)
+__global__ void __launch_bounds__(kCellThreads)
+    b_source(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
+             int nd, int rpb)
 {
     fgpu::follow_predecessor();
-    for_cells(D, S, start, nd, rpb, 0, [&](const DiskF &k, const StepF &st, int i, int j) {
-        viscous_cell(k.g, k.t, k.ph, st.fdt, st.beta_inv, k.ph.adiabatic ? 7 : 1, k.s.sigma, k.trr,
-                     k.tpp, k.trp, k.divv, k.nu, k.H, k.s.sigma0, k.s.energy0, k.vr_b, k.dv_b,
-                     k.s.energy, k.qplus, k.qminus, nullptr, nullptr, i, j);
-    });
+    for_cells(D, S, start, nd, rpb, 1, CellsSource{});
 }
 
-__global__ void b_finish(const DiskF *__restrict__ D, const StepF *__restrict__ S,
-                         const int *__restrict__ start, int nd, int rpb)
+__global__ void __launch_bounds__(kCellThreads)
+    b_artvisc_q(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
+                int nd, int rpb)
 {
     fgpu::follow_predecessor();
-    for_cells(D, S, start, nd, rpb, 1, [&](const DiskF &k, const StepF &, int i, int j) {
-        finish_cell(k.g, k.t, k.ph, k.mom_w[0], k.mom_w[1], k.mom_w[2], k.mom_w[3], k.sigma_w,
-                    k.energy_w, k.vr_b, k.s.vr, k.s.dv, k.s.sigma, k.s.energy, k.sigma_lo_w,
-                    k.s.sigma_lo, k.ring_shift, i, j);
-    });
+    for_cells(D, S, start, nd, rpb, 0, CellsArtviscQ{});
+}
+
+__global__ void __launch_bounds__(kCellThreads)
+    b_artvisc_v(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
+                int nd, int rpb)
+{
+    fgpu::follow_predecessor();
+    for_cells(D, S, start, nd, rpb, 0, CellsArtviscV{});
+}
+
+__global__ void __launch_bounds__(kCellThreads)
+    b_stress(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
+             int nd, int rpb)
+{
+    fgpu::follow_predecessor();
+    for_cells(D, S, start, nd, rpb, 0, CellsStress{});
+}
+
+__global__ void __launch_bounds__(kCellThreads)
+    b_viscous(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
+              int nd, int rpb)
+{
+    fgpu::follow_predecessor();
+    for_cells(D, S, start, nd, rpb, 0, CellsViscous{});
+}
+
+__global__ void __launch_bounds__(kCellThreads)
+    b_finish(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
+             int nd, int rpb)
+{
+    fgpu::follow_predecessor();
+    for_cells(D, S, start, nd, rpb, 1, CellsFinish{});
 }
 
 // ghost rings of the mid-step (B buffers) or end-of-step (A buffers) state
@@ -336,45 +392,24 @@ __global__ void b_kick_sequence(const DiskF *__restrict__ D, const StepF *__rest
     }
     auto tab = [&](int k) { return tabs + (size_t)k * (nd + 1); };
     for_cells(D, S, tab(FGPU_BK_POTENTIAL), nd, tl.k[FGPU_BK_POTENTIAL].rings, 0,
-              [&](const DiskF &k, const StepF &st, int i, int j) {
-                  potential_cell(k.g, k.t, k.ph, st.b, k.H, k.pot, i, j);
-              });
+              CellsPotential{});
     grid.sync();
     for_cells(D, S, tab(FGPU_BK_SOURCE), nd, tl.k[FGPU_BK_SOURCE].rings, 1,
-              [&](const DiskF &k, const StepF &st, int i, int j) {
-                  source_cell(k.g, k.t, st.fdt, k.s.sigma, k.P, k.pot, k.s.vr, k.s.dv, k.vr_b,
-                              k.dv_b, i, j);
-              });
+              CellsSource{});
     grid.sync();
     if (any_art) {
         for_cells(D, S, tab(FGPU_BK_ARTVISC_Q), nd, tl.k[FGPU_BK_ARTVISC_Q].rings, 0,
-                  [&](const DiskF &k, const StepF &st, int i, int j) {
-                      if (!(k.ph.adiabatic || k.ph.art_visc_sn || k.ph.art_visc_tw)) return;
-                      artvisc_q_cell(k.g, k.t, k.ph, st.fdt, k.s.sigma, k.vr_b, k.dv_b,
-                                     k.s.energy, k.Qr, k.Qp, i, j);
-                  });
+                  CellsArtviscQ{});
         grid.sync();
         for_cells(D, S, tab(FGPU_BK_ARTVISC_V), nd, tl.k[FGPU_BK_ARTVISC_V].rings, 0,
-                  [&](const DiskF &k, const StepF &st, int i, int j) {
-                      if (!(k.ph.adiabatic || k.ph.art_visc_sn || k.ph.art_visc_tw)) return;
-                      artvisc_v_cell(k.g, k.t, k.ph, st.fdt, k.s.sigma, k.s.energy, k.Qr, k.Qp,
-                                     k.vr_b, k.dv_b, k.cs, k.H, k.nu, i, j);
-                  });
+                  CellsArtviscV{});
         grid.sync();
     }
     for_cells(D, S, tab(FGPU_BK_STRESS), nd, tl.k[FGPU_BK_STRESS].rings, 0,
-              [&](const DiskF &k, const StepF &, int i, int j) {
-                  stress_cell(k.g, k.t, k.s.sigma, k.vr_b, k.dv_b, k.nu, k.divv, k.trr, k.tpp,
-                              k.trp, i, j);
-              });
+              CellsStress{});
     grid.sync();
     for_cells(D, S, tab(FGPU_BK_VISCOUS), nd, tl.k[FGPU_BK_VISCOUS].rings, 0,
-              [&](const DiskF &k, const StepF &st, int i, int j) {
-                  viscous_cell(k.g, k.t, k.ph, st.fdt, st.beta_inv, k.ph.adiabatic ? 7 : 1,
-                               k.s.sigma, k.trr, k.tpp, k.trp, k.divv, k.nu, k.H, k.s.sigma0,
-                               k.s.energy0, k.vr_b, k.dv_b, k.s.energy, k.qplus, k.qminus,
-                               nullptr, nullptr, i, j);
-              });
+              CellsViscous{});
     grid.sync();
     // the mid-step ghost rings (B buffers), as b_ghost
     const int *gt = tab(FGPU_BK_GHOST);
@@ -407,11 +442,7 @@ __global__ void b_close_sequence(const DiskF *__restrict__ D, const StepF *__res
     }
     auto tab = [&](int k) { return tabs + (size_t)k * (nd + 1); };
     for_cells(D, S, tab(FGPU_BK_FINISH), nd, tl.k[FGPU_BK_FINISH].rings, 1,
-              [&](const DiskF &k, const StepF &, int i, int j) {
-                  finish_cell(k.g, k.t, k.ph, k.mom_w[0], k.mom_w[1], k.mom_w[2], k.mom_w[3], k.sigma_w,
-                              k.energy_w, k.vr_b, k.s.vr, k.s.dv, k.s.sigma, k.s.energy,
-                              k.sigma_lo_w, k.s.sigma_lo, k.ring_shift, i, j);
-              });
+              CellsFinish{});
     grid.sync();
     // damping zones, as b_damping (its block reductions are block-wide)
     for (int it = blockIdx.x; it < 4 * n_damp; it += gridDim.x) {
@@ -690,6 +721,12 @@ static int check_tiles(const fgpu_batch *b, const fgpu_tiles &t, std::string &wh
     return FGPU_OK;
 }
 
+// threads per block of kernel k
+static int launch_threads(const fgpu_tiles &t, int k)
+{
+    return is_cell_kernel(k) ? std::min(t.k[k].threads, kCellThreads) : t.k[k].threads;
+}
+
 // tile tables and grid sizes of the current tile shapes
 static int apply_tiles(fgpu_batch *b, const fgpu_tiles &t)
 {
@@ -711,7 +748,8 @@ static int apply_tiles(fgpu_batch *b, const fgpu_tiles &t)
             long long acc = 0;
             for (int d = 0; d < nd; ++d) {
                 s[d] = (int)acc;
-                const long long ncol = (b->nz[d] + th - 1) / th;
+                const int wide = is_cell_kernel(k) ? 4 * th : th;
+                const long long ncol = (b->nz[d] + wide - 1) / wide;
                 long long n = 0;
                 if (is_cell_kernel(k)) {
                     const int extra = (k == FGPU_BK_SOURCE || k == FGPU_BK_FINISH) ? 1 : 0;
@@ -744,11 +782,12 @@ static int apply_tiles(fgpu_batch *b, const fgpu_tiles &t)
     std::vector<long long> totals(FGPU_BK_COUNT, 0);
     for (int k = 0; k < FGPU_BK_COUNT; ++k) {
         int *s = h.data() + (size_t)k * (nd + 1);
-        const int th = t.k[k].threads, r = t.k[k].rings;
+        const int th = launch_threads(t, k), r = t.k[k].rings;
         long long acc = 0;
         for (int d = 0; d < nd; ++d) {
             s[d] = (int)acc;
-            const long long ncol = (b->nz[d] + th - 1) / th;
+            const int wide = is_cell_kernel(k) ? 4 * th : th;
+            const long long ncol = (b->nz[d] + wide - 1) / wide;
             long long n = 0;
             if (is_cell_kernel(k)) {
                 const int extra = (k == FGPU_BK_SOURCE || k == FGPU_BK_FINISH) ? 1 : 0;
@@ -786,13 +825,13 @@ static int apply_tiles(fgpu_batch *b, const fgpu_tiles &t)
         const size_t smem = k == FGPU_BK_TRANSPORT_AZIMUTHAL && !b->windows ? b->az_smem : 0;
         cudaFuncAttributes attr;
         CKB(cudaFuncGetAttributes(&attr, fn));
-        if (t.k[k].threads > attr.maxThreadsPerBlock) {
+        if (launch_threads(t, k) > attr.maxThreadsPerBlock) {
             b->err = "kernel " + std::to_string(k) + " takes at most " +
                      std::to_string(attr.maxThreadsPerBlock) + " threads per block";
             return FGPU_ERR_UNSUPPORTED;
         }
         int per_sm = 0;
-        CKB(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, t.k[k].threads, smem));
+        CKB(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, launch_threads(t, k), smem));
         if (per_sm < 1) {
             b->err = "kernel " + std::to_string(k) + " cannot run with " +
                      std::to_string(t.k[k].threads) + " threads";
@@ -824,7 +863,7 @@ static void default_tiles(const fgpu_batch *b, fgpu_tiles &t)
 // one batched kernel on the batch stream
 static void launch_kernel(fgpu_batch *b, int k, int ghost_b = 0)
 {
-    const int nd = b->nd, th = b->tiles.k[k].threads, r = b->tiles.k[k].rings, g = b->grid[k];
+    const int nd = b->nd, th = launch_threads(b->tiles, k), r = b->tiles.k[k].rings, g = b->grid[k];
     const DiskF *D = b->d_disks;
     const StepF *S = b->d_steps;
     cudaStream_t s = b->stream;

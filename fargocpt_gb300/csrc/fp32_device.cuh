@@ -229,247 +229,432 @@ __device__ __forceinline__ float exact_row_mean(const float *row, int n, float *
 }
 
 // ---------------------------------------------------------------------------
+// Four cells of a ring per thread, for the kernels that form cells one by one.
+// Such a cell is 20 to 60 operations on some ten loaded values; with one cell per
+// thread the index arithmetic, the ring's table values, the ring search of the
+// batch and the launch's prologue were most of the 240 to 330 instructions it
+// took (issue bound them, at a third of the memory's rate).  2048 x 6144 cells,
+// one cell -> four: potential 0.102 -> 0.047 ms, source terms 0.102 -> 0.059,
+// artificial pressures 0.102 -> 0.047, their update 0.110 -> 0.079, stress 0.102
+// -> 0.061, viscous update 0.215 -> 0.122, finish 0.134 -> 0.087 (now near the
+// memory's rate: 7 to 14 rows of 4 bytes each); a batch of 16 disks, 4.8M
+// cells: 0.53 -> 0.30 ms together.
+// VEC (nz a multiple of 4): adjacent cells in 16-byte accesses, whose neighbours
+// within the four come from registers.  Otherwise rows do not start on 16-byte
+// boundaries: cells `stride` apart in scalar accesses (adjacent ones would spread
+// each access over four times the cache lines); those past the ring's end repeat
+// its last cell and are not stored.
+// ---------------------------------------------------------------------------
+template <bool VEC>
+struct Quad {
+    int nz, first, stride;
+
+    __device__ __forceinline__ int col(int k) const
+    {
+        return VEC ? first + k : min(first + k * stride, nz - 1);
+    }
+    __device__ __forceinline__ void load(const float *p, size_t row, float (&x)[4]) const
+    {
+        if (VEC) {
+            const float4 v = *reinterpret_cast<const float4 *>(p + row + first);
+            x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) x[k] = p[row + col(k)];
+        }
+    }
+    // the left (right) neighbours of the cells x
+    __device__ __forceinline__ void left(const float *p, size_t row, const float (&x)[4],
+                                         float (&l)[4]) const
+    {
+        if (VEC) {
+            l[0] = p[row + jprev(first, nz)];
+            l[1] = x[0], l[2] = x[1], l[3] = x[2];
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) l[k] = p[row + jprev(col(k), nz)];
+        }
+    }
+    __device__ __forceinline__ void right(const float *p, size_t row, const float (&x)[4],
+                                          float (&r)[4]) const
+    {
+        if (VEC) {
+            r[0] = x[1], r[1] = x[2], r[2] = x[3];
+            r[3] = p[row + jnext(first + 3, nz)];
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) r[k] = p[row + jnext(col(k), nz)];
+        }
+    }
+    __device__ __forceinline__ void store(float *p, size_t row, const float (&x)[4]) const
+    {
+        if (VEC) {
+            *reinterpret_cast<float4 *>(p + row + first) = make_float4(x[0], x[1], x[2], x[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (first + k * stride < nz) p[row + first + k * stride] = x[k];
+        }
+    }
+};
+#define QUAD for (int k = 0; k < 4; ++k)
+
+// ---------------------------------------------------------------------------
 // Potential residual Phi - Phi_K (CalculateNbodyPotential, Pframeforce.cpp:21-86)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void potential_cell(const GeoF &g, const TablesF &t, const PhysF &ph,
-                                               const BodiesF &b, const float *__restrict__ H,
-                                               float *__restrict__ pot, int i, int j)
+// Klahr's u^4 - 2 u^3 + 2 u inside r_sm (u the distance in it)
+__device__ __forceinline__ float klahr_factor(float u)
 {
-    const int nz = g.nz;
-    // the cell centre as float pairs (x = xh + xl): the product's rounding
+    return fmaf(__fmul_rn(__fmul_rn(u, u), u), u, -__fmul_rn(__fmul_rn(2.f * u, u), u)) + 2.f * u;
+}
+
+// (fused multiply-adds of these substeps are spelled out where the compiler
+// would have a choice, so that every kernel built from them rounds alike)
+template <class Q>
+__device__ __forceinline__ void potential_cells(
+    const Q &q, const GeoF &g, const TablesF &t, const PhysF &ph, const BodiesF &b,
+    const float *__restrict__ H, float *__restrict__ pot, int i)
+{
+    const size_t row = (size_t)i * g.nz;
+    // the cell centres as float pairs (x = xh + xl): the product's rounding
     // error by FMA plus the cross terms of the split factors; the distance to
     // a body then loses nothing to cancellation however close the body is
     const float rh = t.Rmed[i], rl = t.RmedLo[i];
-    const float ch = t.cosHi[j], cl = t.cosLo[j], sh = t.sinHi[j], sl = t.sinLo[j];
-    const float xh = rh * ch, yh = rh * sh;
-    const float xl = fmaf(rh, ch, -xh) + fmaf(rh, cl, rl * ch);
-    const float yl = fmaf(rh, sh, -yh) + fmaf(rh, sl, rl * sh);
-    const float eps = ph.eps_smooth * H[CELL(i, j)];
-    const float s2 = eps * eps;
-    float acc = 0.f;
-    for (int k = 0; k < b.n; ++k) {
-        float term;
-        if (k == 0 && b.star_at_origin) {
+    float h[4], ch[4], cl[4], sh[4], sl[4], xh[4], yh[4], xl[4], yl[4], s2[4], acc[4];
+    q.load(H, row, h);
+    q.load(t.cosHi, 0, ch);
+    q.load(t.cosLo, 0, cl);
+    q.load(t.sinHi, 0, sh);
+    q.load(t.sinLo, 0, sl);
+#pragma unroll
+    QUAD {
+        xh[k] = rh * ch[k], yh[k] = rh * sh[k];
+        xl[k] = fmaf(rh, ch[k], -xh[k]) + fmaf(rh, cl[k], rl * ch[k]);
+        yl[k] = fmaf(rh, sh[k], -yh[k]) + fmaf(rh, sl[k], rl * sh[k]);
+        const float eps = ph.eps_smooth * h[k];
+        s2[k] = eps * eps;
+        acc[k] = 0.f;
+    }
+    for (int n = 0; n < b.n; ++n) {
+        if (n == 0 && b.star_at_origin) {
             // -G M / sqrt(r^2 + eps^2) + G M / r without cancellation:
             // 1/r - 1/d = (d - r) / (r d) = eps^2 / ((d + r) r d)
-            const float r = t.Rmed[i];
-            const float d = sqrtf(r * r + s2);
-            term = b.gm[0] * s2 / ((d + r) * r * d);
-        } else if (k == 0) {
+            const float gm = b.gm[0];
+#pragma unroll
+            QUAD {
+                const float d = sqrtf(rh * rh + s2[k]);
+                acc[k] += gm * s2[k] / ((d + rh) * rh * d);
+            }
+        } else if (n == 0) {
             // central object off the origin: residual against -G M / r in FP64
-            const double xd = t.Rmed_d[i] * t.cos_d[j], yd = t.Rmed_d[i] * t.sin_d[j];
-            const double dx = xd - b.x[0], dy = yd - b.y[0];
-            const float d2 = (float)(dx * dx + dy * dy) + s2;
-            const float inv_d = rsqrtf(d2);
-            float fk = 1.f;
-            if (b.rsm[0] > 0.f) {
-                const float dsm = d2 * inv_d;
-                if (dsm < b.rsm[0]) {
-                    const float q = dsm / b.rsm[0];
-                    fk = q * q * q * q - 2.f * q * q * q + 2.f * q;
+            const double rmed = t.Rmed_d[i], inv = t.InvRmed_d[i];
+#pragma unroll
+            QUAD {
+                const double xd = rmed * t.cos_d[q.col(k)], yd = rmed * t.sin_d[q.col(k)];
+                const double dx = xd - b.x[0], dy = yd - b.y[0];
+                const float d2 = (float)(dx * dx + dy * dy) + s2[k];
+                const float inv_d = rsqrtf(d2);
+                float fk = 1.f;
+                if (b.rsm[0] > 0.f) {
+                    const float dsm = d2 * inv_d;
+                    if (dsm < b.rsm[0]) fk = klahr_factor(dsm / b.rsm[0]);
                 }
+                acc[k] += (float)(-(double)b.gm[0] * fk / sqrt(dx * dx + dy * dy + (double)s2[k]) +
+                                  (double)b.gm_ref * inv);
             }
-            term = (float)(-(double)b.gm[0] * fk / sqrt(dx * dx + dy * dy + (double)s2) +
-                           (double)b.gm_ref * t.InvRmed_d[i]);
         } else {
-            const float dx = (xh - b.xh[k]) + (xl - b.xl[k]);
-            const float dy = (yh - b.yh[k]) + (yl - b.yl[k]);
-            const float d2 = fmaf(dx, dx, fmaf(dy, dy, s2));
-            const float inv_d = rsqrtf(d2);
-            float fk = 1.f;
-            if (b.rsm[k] > 0.f) {
-                const float dsm = d2 * inv_d;
-                if (dsm < b.rsm[k]) {
-                    const float q = dsm / b.rsm[k];
-                    fk = q * q * q * q - 2.f * q * q * q + 2.f * q;
+            const float bxh = b.xh[n], bxl = b.xl[n], byh = b.yh[n], byl = b.yl[n];
+            const float mgm = -b.gm[n], rsm = b.rsm[n];
+#pragma unroll
+            QUAD {
+                const float dx = (xh[k] - bxh) + (xl[k] - bxl);
+                const float dy = (yh[k] - byh) + (yl[k] - byl);
+                const float d2 = fmaf(dx, dx, fmaf(dy, dy, s2[k]));
+                const float inv_d = rsqrtf(d2);
+                float fk = 1.f;
+                if (rsm > 0.f) {
+                    const float dsm = d2 * inv_d;
+                    if (dsm < rsm) fk = klahr_factor(dsm / rsm);
                 }
+                acc[k] = fmaf(__fmul_rn(mgm, inv_d), fk, acc[k]);
             }
-            term = -b.gm[k] * inv_d * fk;
         }
-        acc += term;
     }
-    acc = fmaf(-b.iy, yh + yl, fmaf(-b.ix, xh + xl, acc));
-    pot[CELL(i, j)] = acc;
+#pragma unroll
+    QUAD acc[k] = fmaf(-b.iy, yh[k] + yl[k], fmaf(-b.ix, xh[k] + xl[k], acc[k]));
+    q.store(pot, row, acc);
 }
 
 // ---------------------------------------------------------------------------
 // momentum sources (SourceEuler.cpp:325-428) in residual form; rows 0..nr
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void source_cell(const GeoF &g, const TablesF &t, float dt,
-                                            const float *__restrict__ S,
-                                            const float *__restrict__ P,
-                                            const float *__restrict__ pot,
-                                            const float *__restrict__ vr_in,
-                                            const float *__restrict__ dv_in,
-                                            float *__restrict__ vr_out,
-                                            float *__restrict__ dv_out, int i, int j)
+template <class Q>
+__device__ __forceinline__ void source_cells(
+    const Q &q, const GeoF &g, const TablesF &t, float dt, const float *__restrict__ S,
+    const float *__restrict__ P, const float *__restrict__ pot,
+    const float *__restrict__ vr_in, const float *__restrict__ dv_in,
+    float *__restrict__ vr_out, float *__restrict__ dv_out, int i)
 {
     const int nz = g.nz, nr = g.nr;
-    float vr = vr_in[CELL(i, j)];
-    if (i >= 2 && i < nr - 1) {
-        const float gradp = 2.f * __fdividef(P[CELL(i, j)] - P[CELL(i - 1, j)],
-                                             S[CELL(i, j)] + S[CELL(i - 1, j)]) *
-                            t.InvDiffRmed[i];
-        const float gradphi = (pot[CELL(i, j)] - pot[CELL(i - 1, j)]) * t.InvDiffRmed[i];
-        const int jn = jnext(j, nz);
-        float d = 0.25f * (dv_in[CELL(i, j)] + dv_in[CELL(i, jn)] + dv_in[CELL(i - 1, j)] +
-                           dv_in[CELL(i - 1, jn)]);
-        // in a rotating frame the reference's vt (frame velocities averaged,
-        // plus Rinf OmegaFrame; SourceEuler.cpp:355-364) is the inertial mean
-        // plus OmegaFrame (Rinf - the mean of the two Rmed)
-        if (g.omega_f != 0.f) d += g.omega_f * t.RinfOff[i];
-        // vt^2 / r - dPhi_K/dr = Kbal + (2 A d + d^2) / Rinf
-        const float centri = t.Kbal[i] + (2.f * t.Aface[i] + d) * d * t.InvRinf[i];
-        vr += dt * (-gradp - gradphi + centri);
+    const size_t row = (size_t)i * nz, below = row - nz;
+    float vr[4], v[4], p[4], s[4], ph[4];
+    q.load(vr_in, row, vr);
+    const bool active = i >= 1 && i < nr - 1;
+    if (i < nr) q.load(dv_in, row, v);
+    if (active) {
+        q.load(P, row, p);
+        q.load(S, row, s);
+        q.load(pot, row, ph);
     }
-    vr_out[CELL(i, j)] = vr;
-    if (i < nr) {
-        float v = dv_in[CELL(i, j)];
-        if (i >= 1 && i < nr - 1) {
-            const int jp = jprev(j, nz);
-            const float invdx = t.InvDxSrc[i];
-            const float gradp = 2.f * __fdividef(P[CELL(i, j)] - P[CELL(i, jp)],
-                                                 S[CELL(i, j)] + S[CELL(i, jp)]) * invdx;
-            const float gradphi = (pot[CELL(i, j)] - pot[CELL(i, jp)]) * invdx;
-            v = v + dt * (-gradp - gradphi);
+    if (i >= 2 && active) {
+        const float invdr = t.InvDiffRmed[i], kbal = t.Kbal[i], aface = t.Aface[i],
+                    invr = t.InvRinf[i], off = t.RinfOff[i];
+        float pm[4], sm[4], phm[4], vn[4], vb[4], vbn[4];
+        q.load(P, below, pm);
+        q.load(S, below, sm);
+        q.load(pot, below, phm);
+        q.load(dv_in, below, vb);
+        q.right(dv_in, row, v, vn);
+        q.right(dv_in, below, vb, vbn);
+#pragma unroll
+        QUAD {
+            const float gradp = 2.f * __fdividef(p[k] - pm[k], s[k] + sm[k]) * invdr;
+            const float gradphi = (ph[k] - phm[k]) * invdr;
+            float d = 0.25f * (v[k] + vn[k] + vb[k] + vbn[k]);
+            // in a rotating frame the reference's vt (frame velocities averaged,
+            // plus Rinf OmegaFrame; SourceEuler.cpp:355-364) is the inertial mean
+            // plus OmegaFrame (Rinf - the mean of the two Rmed)
+            if (g.omega_f != 0.f) d += g.omega_f * off;
+            // vt^2 / r - dPhi_K/dr = Kbal + (2 A d + d^2) / Rinf
+            const float centri = kbal + (2.f * aface + d) * d * invr;
+            vr[k] += dt * (-gradp - gradphi + centri);
         }
-        dv_out[CELL(i, j)] = v;
+    }
+    q.store(vr_out, row, vr);
+    if (i < nr) {
+        if (active) {
+            const float invdx = t.InvDxSrc[i];
+            float pl[4], sl[4], phl[4];
+            q.left(P, row, p, pl);
+            q.left(S, row, s, sl);
+            q.left(pot, row, ph, phl);
+#pragma unroll
+            QUAD {
+                const float gradp = 2.f * __fdividef(p[k] - pl[k], s[k] + sl[k]) * invdx;
+                const float gradphi = (ph[k] - phl[k]) * invdx;
+                v[k] = v[k] + dt * (-gradp - gradphi);
+            }
+        }
+        q.store(dv_out, row, v);
     }
 }
 
+// div v, (vr1 Rinf[i+1] - vr0 Rinf[i]) / ((Rsup - Rinf) Rmed) + dv_phi / (dphi
+// Rmed), regrouped exactly (Rinf[i+1] = Rsup[i]) so that no product cancels; the
+// fused form is spelled out so that every kernel rounds it the same way
+__device__ __forceinline__ float div_v_of(float vr0, float vr1, float dvp, float invdphi,
+                                          float rsupidrr, float invrmed)
+{
+    return fmaf(__fmul_rn(dvp, invdphi), invrmed,
+                fmaf(vr1 - vr0, rsupidrr, __fmul_rn(vr0, invrmed)));
+}
+
 // compression heating + SN q and energy update + T floor
-__device__ __forceinline__ void artvisc_q_cell(const GeoF &g, const TablesF &t, const PhysF &ph,
-                                               float dt, const float *__restrict__ S,
-                                               const float *__restrict__ vr,
-                                               const float *__restrict__ dv, float *__restrict__ E,
-                                               float *__restrict__ Qr, float *__restrict__ Qp,
-                                               int i, int j)
+template <class Q>
+__device__ __forceinline__ void artvisc_q_cells(
+    const Q &q, const GeoF &g, const TablesF &t, const PhysF &ph, float dt,
+    const float *__restrict__ S, const float *__restrict__ vr, const float *__restrict__ dv,
+    float *__restrict__ E, float *__restrict__ Qr, float *__restrict__ Qp, int i)
 {
     const int nz = g.nz, nr = g.nr;
-    const size_t c = CELL(i, j);
-    const int jn = jnext(j, nz);
-    const float vr0 = vr[c], vr1 = vr[CELL(i + 1, j)];
-    const float dvp = dv[CELL(i, jn)] - dv[c];
-    float e = 0.f;
-    if (ph.adiabatic) {
-        e = E[c];
-        if (i < nr - 1) {
-            // (vr1 Rinf[i+1] - vr0 Rinf[i]) / ((Rsup - Rinf) Rmed), regrouped
-            // exactly (Rinf[i+1] = Rsup[i]) so that no product cancels
-            const float div_v = (vr1 - vr0) * t.RsupIDRR[i] + vr0 * t.InvRmed[i] +
-                                dvp * g.invdphi * t.InvRmed[i];
-            e = e * __expf(-ph.gm1 * dt * div_v);
+    const size_t row = (size_t)i * nz;
+    float vr0[4], vr1[4], d0[4], dvp[4], sig[4], e[4] = {};
+    q.load(vr, row, vr0);
+    q.load(vr, row + nz, vr1);
+    q.load(dv, row, d0);
+    q.right(dv, row, d0, dvp);
+    q.load(S, row, sig);
+    if (ph.adiabatic) q.load(E, row, e);
+    const float rsupidrr = t.RsupIDRR[i], invrmed = t.InvRmed[i], invdrsup = t.InvDiffRsup[i],
+                invdxt = t.InvDxTheta[i], lsq = t.LSqTW[i];
+    const bool active = i >= 1 && i < nr - 1;
+#pragma unroll
+    QUAD dvp[k] = dvp[k] - d0[k];
+    if (ph.adiabatic && i < nr - 1) {
+#pragma unroll
+        QUAD {
+            const float div_v = div_v_of(vr0[k], vr1[k], dvp[k], g.invdphi, rsupidrr, invrmed);
+            e[k] = e[k] * __expf(-ph.gm1 * dt * div_v);
         }
     }
     if (ph.art_visc_sn) {
-        const float sig = S[c];
-        const float dv_r = vr1 - vr0;
-        const float qr = dv_r < 0.f ? ph.C2 * sig * (dv_r * dv_r) : 0.f;
-        const float qp = dvp < 0.f ? ph.C2 * sig * (dvp * dvp) : 0.f;
-        Qr[c] = qr;
-        Qp[c] = qp;
-        if (ph.adiabatic && ph.dissipation && i >= 1 && i < nr - 1) {
-            e = e - dt * qr * dv_r * t.InvDiffRsup[i] - dt * qp * dvp * t.InvDxTheta[i];
+        float qr[4], qp[4];
+#pragma unroll
+        QUAD {
+            const float dv_r = vr1[k] - vr0[k];
+            qr[k] = dv_r < 0.f ? ph.C2 * sig[k] * (dv_r * dv_r) : 0.f;
+            qp[k] = dvp[k] < 0.f ? ph.C2 * sig[k] * (dvp[k] * dvp[k]) : 0.f;
+            if (ph.adiabatic && ph.dissipation && active)
+                e[k] = e[k] - dt * qr[k] * dv_r * invdrsup - dt * qp[k] * dvp[k] * invdxt;
         }
+        q.store(Qr, row, qr);
+        q.store(Qp, row, qp);
     }
     if (ph.art_visc_tw) {
         // update_with_artificial_viscosity_TW, artificial_viscosity.cpp:52-91
         // (velocity differences within a ring are the same for the residual)
-        const float sig = S[c];
-        const float eps_rr = (vr1 - vr0) * t.InvDiffRsup[i];
-        const float eps_pp = t.InvRmed[i] * (dvp * g.invdphi + 0.5f * (vr1 + vr0));
-        const float div_V = fminf(eps_rr + eps_pp, 0.f);
-        const float lsig = t.LSqTW[i] * sig;
-        Qr[c] = lsig * -div_V * (eps_rr - (1.f / 3.f) * div_V);
-        Qp[c] = lsig * -div_V * (eps_pp - (1.f / 3.f) * div_V);
-        if (ph.adiabatic && ph.dissipation && i >= 1 && i < nr - 1) {
-            const float d = eps_rr - eps_pp;
-            e += -lsig * div_V * (1.f / 3.f) * (eps_rr * eps_rr + eps_pp * eps_pp + d * d) * dt;
+        float qr[4], qp[4];
+#pragma unroll
+        QUAD {
+            const float eps_rr = __fmul_rn(vr1[k] - vr0[k], invdrsup);
+            const float eps_pp = __fmul_rn(
+                invrmed, __fadd_rn(__fmul_rn(dvp[k], g.invdphi), 0.5f * (vr1[k] + vr0[k])));
+            const float div_V = fminf(__fadd_rn(eps_rr, eps_pp), 0.f);
+            const float lsig = lsq * sig[k];
+            qr[k] = lsig * -div_V * fmaf(-(1.f / 3.f), div_V, eps_rr);
+            qp[k] = lsig * -div_V * fmaf(-(1.f / 3.f), div_V, eps_pp);
+            if (ph.adiabatic && ph.dissipation && active) {
+                const float d = __fsub_rn(eps_rr, eps_pp);
+                const float squares = fmaf(d, d, fmaf(eps_rr, eps_rr, __fmul_rn(eps_pp, eps_pp)));
+                e[k] = fmaf(-lsig * div_V * (1.f / 3.f) * squares, dt, e[k]);
+            }
         }
+        q.store(Qr, row, qr);
+        q.store(Qp, row, qp);
     }
     if (ph.adiabatic) {
-        if (ph.dissipation) e = tfloor(e, S[c], ph);
-        E[c] = e;
+        if (ph.dissipation) {
+#pragma unroll
+            QUAD e[k] = tfloor(e[k], sig[k], ph);
+        }
+        q.store(E, row, e);
     }
 }
 
-__device__ __forceinline__ void artvisc_v_cell(const GeoF &g, const TablesF &t, const PhysF &ph,
-                                               float dt, const float *__restrict__ S,
-                                               const float *__restrict__ E,
-                                               const float *__restrict__ Qr,
-                                               const float *__restrict__ Qp, float *__restrict__ vr,
-                                               float *__restrict__ dv, float *__restrict__ cs,
-                                               float *__restrict__ H, float *__restrict__ nu, int i,
-                                               int j)
+template <class Q>
+__device__ __forceinline__ void artvisc_v_cells(
+    const Q &q, const GeoF &g, const TablesF &t, const PhysF &ph, float dt,
+    const float *__restrict__ S, const float *__restrict__ E, const float *__restrict__ Qr,
+    const float *__restrict__ Qp, float *__restrict__ vr, float *__restrict__ dv,
+    float *__restrict__ cs, float *__restrict__ H, float *__restrict__ nu, int i)
 {
     const int nz = g.nz, nr = g.nr;
-    const size_t c = CELL(i, j);
-    if (ph.art_visc_sn) {
-        if (i >= 2 && i < nr - 1) {
-            vr[c] -= dt * 2.f * __fdividef(Qr[c] - Qr[CELL(i - 1, j)], S[c] + S[CELL(i - 1, j)]) *
-                     t.InvDiffRmed[i];
+    const size_t row = (size_t)i * nz, below = row - nz;
+    float s[4];
+    q.load(S, row, s);
+    const bool radial = i >= 2 && i < nr - 1, azimuthal = i >= 1 && i < nr - 1;
+    if (azimuthal && (ph.art_visc_sn || ph.art_visc_tw)) {
+        float sl[4], sb[4], qr[4], qrb[4], qp[4], qpl[4], qpb[4], v[4], d[4];
+        q.load(Qp, row, qp);
+        q.left(Qp, row, qp, qpl);
+        q.left(S, row, s, sl);
+        q.load(dv, row, d);
+        if (radial) {
+            q.load(S, below, sb);
+            q.load(Qr, row, qr);
+            q.load(Qr, below, qrb);
+            q.load(vr, row, v);
+            if (ph.art_visc_tw) q.load(Qp, below, qpb);
         }
-        if (i >= 1 && i < nr - 1) {
-            const int jp = jprev(j, nz);
-            dv[c] -= dt * 2.f * __fdividef(Qp[c] - Qp[CELL(i, jp)], S[c] + S[CELL(i, jp)]) *
-                     t.InvDxTheta[i];
+        if (ph.art_visc_sn) {
+            const float invdr = t.InvDiffRmed[i], invdxt = t.InvDxTheta[i];
+            if (radial) {
+#pragma unroll
+                QUAD v[k] -= dt * 2.f * __fdividef(qr[k] - qrb[k], s[k] + sb[k]) * invdr;
+            }
+#pragma unroll
+            QUAD d[k] -= dt * 2.f * __fdividef(qp[k] - qpl[k], s[k] + sl[k]) * invdxt;
         }
-    }
-    if (ph.art_visc_tw) {
-        // artificial_viscosity.cpp:93-139
-        if (i >= 1 && i < nr - 1) {
-            const int jp = jprev(j, nz);
-            dv[c] += __fdividef(dt, 0.5f * (S[c] + S[CELL(i, jp)])) * t.InvDxSrc[i] *
-                     (Qp[c] - Qp[CELL(i, jp)]);
+        if (ph.art_visc_tw) {
+            // artificial_viscosity.cpp:93-139
+            const float invdx = t.InvDxSrc[i];
+#pragma unroll
+            QUAD d[k] += __fdividef(dt, 0.5f * (s[k] + sl[k])) * invdx * (qp[k] - qpl[k]);
+            if (radial) {
+                const float two = t.TwoOverDRmed2[i], r0 = t.Rmed[i], rb = t.Rmed[i - 1],
+                            dr = t.DRmed[i];
+#pragma unroll
+                QUAD {
+                    const float fac = ph.rvf * __fdividef(dt, 0.5f * (s[k] + sb[k])) * two;
+                    const float rhs = fmaf(-(0.5f * (qp[k] + qpb[k])), dr,
+                                           fmaf(qr[k], r0, -__fmul_rn(qrb[k], rb)));
+                    v[k] = fmaf(fac, rhs, v[k]);
+                }
+            }
         }
-        if (i >= 2 && i < nr - 1) {
-            const size_t cm = CELL(i - 1, j);
-            vr[c] += ph.rvf * __fdividef(dt, 0.5f * (S[c] + S[cm])) * t.TwoOverDRmed2[i] *
-                     ((Qr[c] * t.Rmed[i] - Qr[cm] * t.Rmed[i - 1]) -
-                      0.5f * (Qp[c] + Qp[cm]) * t.DRmed[i]);
-        }
+        if (radial) q.store(vr, row, v);
+        q.store(dv, row, d);
     }
     if (ph.adiabatic) {
-        const float c_s = sqrtf(ph.g_gm1 * __fdividef(E[c], S[c]));
-        const float h = c_s * t.HFacAdi[i];
-        cs[c] = c_s;
-        H[c] = h;
-        nu[c] = ph.alpha > 0.f ? ph.alpha * h * c_s : ph.constant_viscosity;
+        float e[4], c[4], h[4], n[4];
+        q.load(E, row, e);
+        const float hfac = t.HFacAdi[i];
+#pragma unroll
+        QUAD {
+            c[k] = sqrtf(ph.g_gm1 * __fdividef(e[k], s[k]));
+            h[k] = c[k] * hfac;
+            n[k] = ph.alpha > 0.f ? ph.alpha * h[k] * c[k] : ph.constant_viscosity;
+        }
+        q.store(cs, row, c);
+        q.store(H, row, h);
+        q.store(nu, row, n);
     }
 }
 
 // stress tensor (viscosity.cpp:139-254); tau_r_phi adds the Keplerian shear
-__device__ __forceinline__ void stress_cell(const GeoF &g, const TablesF &t,
-                                            const float *__restrict__ S,
-                                            const float *__restrict__ vr,
-                                            const float *__restrict__ dv,
-                                            const float *__restrict__ nu, float *__restrict__ divv,
-                                            float *__restrict__ trr, float *__restrict__ tpp,
-                                            float *__restrict__ trp, int i, int j)
+template <class Q>
+__device__ __forceinline__ void stress_cells(
+    const Q &q, const GeoF &g, const TablesF &t, const float *__restrict__ S,
+    const float *__restrict__ vr, const float *__restrict__ dv, const float *__restrict__ nu,
+    float *__restrict__ divv, float *__restrict__ trr, float *__restrict__ tpp,
+    float *__restrict__ trp, int i)
 {
     const int nz = g.nz;
-    const size_t c = CELL(i, j);
-    const int jn = jnext(j, nz);
-    const float vr0 = vr[c], vr1 = vr[CELL(i + 1, j)];
-    const float dvp = dv[CELL(i, jn)] - dv[c];
-    const float n = nu[c], sg = S[c];
-    const float d = (vr1 - vr0) * t.RsupIDRR[i] + vr0 * t.InvRmed[i] +
-                    dvp * g.invdphi * t.InvRmed[i];
-    divv[c] = d;
-    const float drr = (vr1 - vr0) * t.InvDiffRsup[i];
-    trr[c] = 2.f * n * sg * (drr - (1.f / 3.f) * d);
-    const float dpp = dvp * g.invdphi * t.InvRmed[i] + 0.5f * (vr1 + vr0) * t.InvRmed[i];
-    tpp[c] = 2.f * n * sg * (dpp - (1.f / 3.f) * d);
+    const size_t row = (size_t)i * nz, below = row - nz;
+    float vr0[4], vr1[4], d0[4], dvp[4], n[4], sg[4], x[4], y[4], z[4];
+    q.load(vr, row, vr0);
+    q.load(vr, row + nz, vr1);
+    q.load(dv, row, d0);
+    q.right(dv, row, d0, dvp);
+    q.load(nu, row, n);
+    q.load(S, row, sg);
+    const float rsupidrr = t.RsupIDRR[i], invrmed = t.InvRmed[i], invdrsup = t.InvDiffRsup[i];
+#pragma unroll
+    QUAD {
+        dvp[k] = dvp[k] - d0[k];
+        const float d = div_v_of(vr0[k], vr1[k], dvp[k], g.invdphi, rsupidrr, invrmed);
+        x[k] = d;
+        const float drr = (vr1[k] - vr0[k]) * invdrsup;
+        y[k] = 2.f * n[k] * sg[k] * (drr - (1.f / 3.f) * d);
+        const float dpp = fmaf(__fmul_rn(dvp[k], g.invdphi), invrmed,
+                               __fmul_rn(0.5f * (vr1[k] + vr0[k]), invrmed));
+        z[k] = 2.f * n[k] * sg[k] * (dpp - (1.f / 3.f) * d);
+    }
+    q.store(divv, row, x);
+    q.store(trr, row, y);
+    q.store(tpp, row, z);
     if (i >= 1) {
-        const int jp = jprev(j, nz);
-        const float dvazirdr =
-            t.Shear[i] + (dv[c] * t.InvRmed[i] - dv[CELL(i - 1, j)] * t.InvRmed[i - 1]) *
-                             t.InvDiffRmed[i];
-        const float dvrdphi = (vr0 - vr[CELL(i, jp)]) * g.invdphi;
-        const float drp = t.Rinf[i] * dvazirdr + dvrdphi * t.InvRinf[i];
-        const float n4 = 0.25f * (n + nu[CELL(i - 1, j)] + nu[CELL(i, jp)] + nu[CELL(i - 1, jp)]);
-        const float s4 = 0.25f * (sg + S[CELL(i - 1, j)] + S[CELL(i, jp)] + S[CELL(i - 1, jp)]);
-        trp[c] = n4 * s4 * drp;
+        float db[4], vl[4], nb[4], nl[4], nbl[4], sb[4], sl[4], sbl[4];
+        q.load(dv, below, db);
+        q.left(vr, row, vr0, vl);
+        q.load(nu, below, nb);
+        q.left(nu, row, n, nl);
+        q.left(nu, below, nb, nbl);
+        q.load(S, below, sb);
+        q.left(S, row, sg, sl);
+        q.left(S, below, sb, sbl);
+        const float shear = t.Shear[i], invrb = t.InvRmed[i - 1], invdr = t.InvDiffRmed[i],
+                    rinf = t.Rinf[i], invrinf = t.InvRinf[i];
+#pragma unroll
+        QUAD {
+            const float dvazirdr = shear + (d0[k] * invrmed - db[k] * invrb) * invdr;
+            const float dvrdphi = (vr0[k] - vl[k]) * g.invdphi;
+            const float drp = rinf * dvazirdr + dvrdphi * invrinf;
+            const float n4 = 0.25f * (n[k] + nb[k] + nl[k] + nbl[k]);
+            const float s4 = 0.25f * (sg[k] + sb[k] + sl[k] + sbl[k]);
+            x[k] = n4 * s4 * drp;
+        }
+        q.store(trp, row, x);
     }
 }
 
@@ -514,94 +699,146 @@ __device__ __forceinline__ void visc_corr_cell(const GeoF &g, const TablesF &t,
 // viscous velocity update + SubStep3.  mode bits: 1 velocities
 // (viscosity.cpp:355-421), 2 heating/cooling rates, 4 energy update
 // (SourceEuler.cpp:859-954)
-__device__ __forceinline__ void viscous_cell(
-    const GeoF &g, const TablesF &t, const PhysF &ph, float dt, float beta_inv, int mode,
-    const float *__restrict__ S, const float *__restrict__ trr, const float *__restrict__ tpp,
-    const float *__restrict__ trp, const float *__restrict__ divv, const float *__restrict__ nu,
-    const float *__restrict__ H, const float *__restrict__ S0, const float *__restrict__ E0,
-    float *__restrict__ vr, float *__restrict__ dv, float *__restrict__ E,
-    float *__restrict__ qplus, float *__restrict__ qminus, const float *__restrict__ corr_phi,
-    const float *__restrict__ corr_r, int i, int j)
+template <class Q>
+__device__ __forceinline__ void viscous_cells(
+     const Q &q, const GeoF &g, const TablesF &t, const PhysF &ph, float dt, float beta_inv,
+    int mode, const float *__restrict__ S, const float *__restrict__ trr,
+    const float *__restrict__ tpp, const float *__restrict__ trp,
+    const float *__restrict__ divv, const float *__restrict__ nu, const float *__restrict__ H,
+    const float *__restrict__ S0, const float *__restrict__ E0, float *__restrict__ vr,
+    float *__restrict__ dv, float *__restrict__ E, float *__restrict__ qplus,
+    float *__restrict__ qminus, const float *__restrict__ corr_phi,
+    const float *__restrict__ corr_r, int i)
 {
     const int nz = g.nz, nr = g.nr;
-    const size_t c = CELL(i, j);
-    const int jp = jprev(j, nz), jn = jnext(j, nz);
+    const size_t row = (size_t)i * nz, below = row - nz, above = row + nz;
+    const bool active = i >= 1 && i < nr - 1;
     // pseudo-implicit limiter of StabilizeViscosity 1, viscosity.cpp:395-399
     auto stabilized = [&](float d, float cc) {
         const float a = 1.f + dt * cc;
         return d * (1.f / (fmaxf(a, 0.f) - dt * cc));
     };
-    if (mode & 1) {
-        if (i >= 1 && i < nr - 1) {
-            const float sa = 0.5f * (S[c] + S[CELL(i, jp)]);
-            const float fac = __fdividef(dt * t.InvRmed[i], sa);
-            const float rhs = t.TwoOverDRa2[i] * (t.RinfSq[i + 1] * trp[CELL(i + 1, j)] -
-                                                  t.RinfSq[i] * trp[c]) +
-                              (tpp[c] - tpp[CELL(i, jp)]) * g.invdphi;
+    float sg[4], rp[4], rpr[4], rpa[4], rr[4], pp[4];
+    q.load(S, row, sg);
+    if (active) {
+        q.load(trp, row, rp);
+        q.right(trp, row, rp, rpr);
+        q.load(trp, above, rpa);
+        q.load(trr, row, rr);
+        q.load(tpp, row, pp);
+    }
+    if ((mode & 1) && active) {
+        float sl[4], ppl[4], d[4], cc[4];
+        q.left(S, row, sg, sl);
+        q.left(tpp, row, pp, ppl);
+        q.load(dv, row, d);
+        if (ph.stabilize == 1) q.load(corr_phi, row, cc);
+        const float invrmed = t.InvRmed[i], two = t.TwoOverDRa2[i], r1 = t.RinfSq[i + 1],
+                    r0 = t.RinfSq[i];
+#pragma unroll
+        QUAD {
+            const float sa = 0.5f * (sg[k] + sl[k]);
+            const float fac = __fdividef(dt * invrmed, sa);
+            const float rhs = two * (r1 * rpa[k] - r0 * rp[k]) + (pp[k] - ppl[k]) * g.invdphi;
             // the fused form is spelled out so that every kernel built from
             // this body rounds the update the same way
             if (ph.stabilize == 1)
-                dv[c] += stabilized(fac * rhs, corr_phi[c]);
+                d[k] += stabilized(fac * rhs, cc[k]);
             else
-                dv[c] = fmaf(fac, rhs, dv[c]);
+                d[k] = fmaf(fac, rhs, d[k]);
         }
-        if (i >= 2 && i < nr - 1) {
-            const float sa = 0.5f * (S[c] + S[CELL(i - 1, j)]);
-            const float fac = __fdividef(dt, sa) * ph.rvf * t.TwoOverRmedSum[i];
-            const float rhs =
-                (t.Rmed[i] * trr[c] - t.Rmed[i - 1] * trr[CELL(i - 1, j)]) * t.InvDiffRmed[i] +
-                (trp[CELL(i, jn)] - trp[c]) * g.invdphi - 0.5f * (tpp[c] + tpp[CELL(i - 1, j)]);
-            if (ph.stabilize == 1)
-                vr[c] += stabilized(fac * rhs, corr_r[c]);
-            else
-                vr[c] = fmaf(fac, rhs, vr[c]);
+        q.store(dv, row, d);
+        if (i >= 2) {
+            float sb[4], rrb[4], ppb[4], v[4];
+            q.load(S, below, sb);
+            q.load(trr, below, rrb);
+            q.load(tpp, below, ppb);
+            q.load(vr, row, v);
+            if (ph.stabilize == 1) q.load(corr_r, row, cc);
+            const float twos = t.TwoOverRmedSum[i], rm = t.Rmed[i], rmb = t.Rmed[i - 1],
+                        invdr = t.InvDiffRmed[i];
+#pragma unroll
+            QUAD {
+                const float sa = 0.5f * (sg[k] + sb[k]);
+                const float fac = __fdividef(dt, sa) * ph.rvf * twos;
+                const float rhs = (rm * rr[k] - rmb * rrb[k]) * invdr +
+                                  (rpr[k] - rp[k]) * g.invdphi - 0.5f * (pp[k] + ppb[k]);
+                if (ph.stabilize == 1)
+                    v[k] += stabilized(fac * rhs, cc[k]);
+                else
+                    v[k] = fmaf(fac, rhs, v[k]);
+            }
+            q.store(vr, row, v);
         }
     }
     if (!(mode & 6) || !ph.adiabatic) return;
-    float qp = 0.f, qm = 0.f;
-    const float e = E[c], sig = S[c];
-    const bool active = i >= 1 && i < nr - 1;
+    float qp[4] = {}, qm[4] = {}, e[4];
+    q.load(E, row, e);
     if (active) {
         if (ph.cooling_beta) {
-            float dE = e;
-            if (ph.beta_ref == 1) dE -= __fdividef(E0[c], S0[c]) * sig;
-            else if (ph.beta_ref == 2) dE -= t.EModel[i] * sig;
-            else if (ph.beta_ref == 3) dE -= sig * ph.emin_fac;
-            qm = dE * t.OmegaK[i] * beta_inv;
+            float s0[4], e0[4];
+            if (ph.beta_ref == 1) {
+                q.load(S0, row, s0);
+                q.load(E0, row, e0);
+            }
+            const float emodel = t.EModel[i], omega = t.OmegaK[i];
+#pragma unroll
+            QUAD {
+                float dE = e[k];
+                if (ph.beta_ref == 1) dE -= __fdividef(e0[k], s0[k]) * sg[k];
+                else if (ph.beta_ref == 2) dE -= emodel * sg[k];
+                else if (ph.beta_ref == 3) dE -= sg[k] * ph.emin_fac;
+                qm[k] = dE * omega * beta_inv;
+            }
         }
         if (ph.heating_viscous) {
-            const float n = nu[c];
-            if (n != 0.f) {
-                const float trpa = 0.25f * (trp[c] + trp[CELL(i + 1, j)] + trp[CELL(i, jn)] +
-                                            trp[CELL(i + 1, jn)]);
-                const float a = trr[c], b2 = tpp[c], dd = divv[c];
-                float q = __fdividef(a * a + 2.f * trpa * trpa + b2 * b2, 2.f * n * sig);
-                q += (2.f / 9.f) * n * sig * dd * dd;
-                qp = q * ph.hvf;
+            float n[4], dd[4], rpar[4];
+            q.load(nu, row, n);
+            q.load(divv, row, dd);
+            q.right(trp, above, rpa, rpar);
+#pragma unroll
+            QUAD {
+                if (n[k] != 0.f) {
+                    const float trpa = 0.25f * (rp[k] + rpa[k] + rpr[k] + rpar[k]);
+                    const float a = rr[k], b2 = pp[k];
+                    float u = __fdividef(a * a + 2.f * trpa * trpa + b2 * b2, 2.f * n[k] * sg[k]);
+                    u += (2.f / 9.f) * n[k] * sg[k] * dd[k] * dd[k];
+                    qp[k] = u * ph.hvf;
+                }
             }
         }
-        // radiative alpha: 1 + 8 sigma_SB / c * H * x^4 e^3 with
-        // x = mu (gamma-1) / (R sigma), evaluated as x * (x e)^3
-        const float x = __fdividef(ph.mu_gm1_over_R, sig);
-        const float xe = x * e;
-        const float alpha = 1.f + H[c] * ph.cool_const * x * (xe * xe * xe);
-        const float ia = __frcp_rn(alpha);
-        qp *= ia;
-        qm *= ia;
+        float h[4];
+        q.load(H, row, h);
+#pragma unroll
+        QUAD {
+            // radiative alpha: 1 + 8 sigma_SB / c * H * x^4 e^3 with
+            // x = mu (gamma-1) / (R sigma), evaluated as x * (x e)^3
+            const float x = __fdividef(ph.mu_gm1_over_R, sg[k]);
+            const float xe = x * e[k];
+            const float alpha = 1.f + h[k] * ph.cool_const * x * (xe * xe * xe);
+            const float ia = __frcp_rn(alpha);
+            qp[k] *= ia;
+            qm[k] *= ia;
+        }
     }
     if (mode & 4) {
-        float en = e;
-        if (active) {
-            en = e + dt * (qp - qm);
-            if (sig < ph.sigma_floor10) {
-                qm = qp;
-                en = 0.f;
+        float en[4];
+#pragma unroll
+        QUAD {
+            en[k] = e[k];
+            if (active) {
+                en[k] = e[k] + dt * (qp[k] - qm[k]);
+                if (sg[k] < ph.sigma_floor10) {
+                    qm[k] = qp[k];
+                    en[k] = 0.f;
+                }
             }
+            en[k] = tfloor(en[k], sg[k], ph);
         }
-        E[c] = tfloor(en, sig, ph);
+        q.store(E, row, en);
     }
-    qplus[c] = qp;
-    qminus[c] = qm;
+    q.store(qplus, row, qp);
+    q.store(qminus, row, qm);
 }
 
 // ghost rings (boundary_conditions.cpp:65-114); v_phi hooks work on the
@@ -1675,47 +1912,79 @@ __device__ __forceinline__ void pressure_cell(const GeoF &g, const TablesF &t, c
 }
 
 // velocities from momenta (:498-535), floors; rows 0..nr
-__device__ __forceinline__ void finish_cell(
-    const GeoF &g, const TablesF &t, const PhysF &ph, const float *__restrict__ m0,
+template <class Q>
+__device__ __forceinline__ void finish_cells(
+    const Q &q, const GeoF &g, const TablesF &t, const PhysF &ph, const float *__restrict__ m0,
     const float *__restrict__ m1, const float *__restrict__ m2, const float *__restrict__ m3,
-    const float *__restrict__ S_t, const float *__restrict__ E_t, const float *__restrict__ vr_in,
-    float *__restrict__ vr_out, float *__restrict__ dv_out, float *__restrict__ S_out,
-    float *__restrict__ E_out, const float *__restrict__ Slo_t, float *__restrict__ Slo_out,
-    const int *__restrict__ shift, int i, int j)
+    const float *__restrict__ S_t, const float *__restrict__ E_t,
+    const float *__restrict__ vr_in, float *__restrict__ vr_out, float *__restrict__ dv_out,
+    float *__restrict__ S_out, float *__restrict__ E_out, const float *__restrict__ Slo_t,
+    float *__restrict__ Slo_out, const int *__restrict__ shift, int i)
 {
     const int nz = g.nz, nr = g.nr;
-    const size_t c = CELL(i, j);
+    const size_t row = (size_t)i * nz;
+    float v[4];
     if (i == nr) {
-        vr_out[c] = vr_in[c];
+        q.load(vr_in, row, v);
+        q.store(vr_out, row, v);
         return;
     }
     // AdvectSHIFT: the transported cell j of ring k sits at j - shift[k]
-    auto at = [&](int k, int jj) {
-        int a = jj - __ldg(shift + k);
+    auto at = [&](int ring, int sh, int j) {
+        int a = j - sh;
         if (a < 0) a += nz;
-        return CELL(k, a);
+        return (size_t)ring * nz + a;
     };
-    const size_t cs = at(i, j);
-    const float s = S_t[cs];
-    if (i == 0) {
-        vr_out[c] = 0.f;
-    } else {
-        const size_t cm = at(i - 1, j);
-        vr_out[c] = __fdiv_rn(m0[cm] + m1[cs], S_t[cm] + s);
+    const int sh = __ldg(shift + i);
+    float s[4], sl[4], lo[4], e[4], m2l[4], m3c[4];
+#pragma unroll
+    QUAD {
+        const int j = q.col(k);
+        const size_t c = at(i, sh, j), l = at(i, sh, jprev(j, nz));
+        s[k] = S_t[c];
+        sl[k] = S_t[l];
+        m2l[k] = m2[l];
+        m3c[k] = m3[c];
+        lo[k] = Slo_t[c];
+        if (ph.adiabatic) e[k] = E_t[c];
     }
-    const size_t cjm = at(i, jprev(j, nz));
+    if (i == 0) {
+#pragma unroll
+        QUAD v[k] = 0.f;
+    } else {
+        const int shb = __ldg(shift + i - 1);
+        float m0b[4], m1c[4], sb[4];
+#pragma unroll
+        QUAD {
+            const size_t c = at(i, sh, q.col(k)), b = at(i - 1, shb, q.col(k));
+            m0b[k] = m0[b];
+            m1c[k] = m1[c];
+            sb[k] = S_t[b];
+        }
+#pragma unroll
+        QUAD v[k] = __fdiv_rn(m0b[k] + m1c[k], sb[k] + s[k]);
+    }
+    q.store(vr_out, row, v);
     // the residual angular momenta were formed as sigma (dv Rmed) with the
     // FP32 Rmed of the ring: dividing by that same Rmed returns dv without
     // bias, where multiplying by the FP32 1/Rmed would scale every ring's
     // residual by Rmed 1/Rmed - 1 (up to ~6e-8) in every step, a drift that
     // accumulates over tens of thousands of steps; the divisions are
     // correctly rounded for the same reason
-    dv_out[c] = __fdiv_rn(m2[cjm] + m3[cs], __fmul_rn(S_t[cjm] + s, t.Rmed[i]));
-    const bool floored = s < ph.sigma_min;
-    const float sf = floored ? ph.sigma_min : s;
-    S_out[c] = sf;
-    Slo_out[c] = floored ? 0.f : Slo_t[cs];
-    if (ph.adiabatic) E_out[c] = tfloor(E_t[cs], sf, ph);
+    const float rmed = t.Rmed[i];
+#pragma unroll
+    QUAD v[k] = __fdiv_rn(m2l[k] + m3c[k], __fmul_rn(sl[k] + s[k], rmed));
+    q.store(dv_out, row, v);
+#pragma unroll
+    QUAD {
+        const bool floored = s[k] < ph.sigma_min;
+        s[k] = floored ? ph.sigma_min : s[k];
+        lo[k] = floored ? 0.f : lo[k];
+        if (ph.adiabatic) e[k] = tfloor(e[k], s[k], ph);
+    }
+    q.store(S_out, row, s);
+    q.store(Slo_out, row, lo);
+    if (ph.adiabatic) q.store(E_out, row, e);
 }
 
 // damping zones (damping.cpp:311-776); block-wide over ring i

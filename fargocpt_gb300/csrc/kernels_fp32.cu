@@ -35,44 +35,56 @@
 #include <cstring>
 #include <cstdlib>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace fgpu32 {
 
 // ---------------------------------------------------------------------------
-// single-disk kernels: one thread per cell (blockIdx.y = ring), one thread per
-// column and chunk of rings, or one block per ring
+// single-disk kernels: one thread per four cells of a ring (Quad; blockIdx.y =
+// ring), one thread per column and chunk of rings, or one block per ring
 // ---------------------------------------------------------------------------
+template <bool VEC>
+__device__ __forceinline__ Quad<VEC> quad_of(int nz)
+{
+    const int t = threadIdx.x, n = blockDim.x, b = blockIdx.x;
+    return VEC ? Quad<VEC>{nz, 4 * (b * n + t), 1} : Quad<VEC>{nz, 4 * b * n + t, n};
+}
+
+template <bool VEC>
 __global__ void f_potential(GeoF g, TablesF t, PhysF ph, BodiesF b, const float *__restrict__ H,
                             float *__restrict__ pot)
 {
     fgpu::follow_predecessor();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= g.nz) return;
-    potential_cell(g, t, ph, b, H, pot, blockIdx.y, j);
+    const Quad<VEC> q = quad_of<VEC>(g.nz);
+    if (q.first >= g.nz) return;
+    potential_cells(q, g, t, ph, b, H, pot, blockIdx.y);
 }
 
+template <bool VEC>
 __global__ void f_source(GeoF g, TablesF t, float dt, const float *__restrict__ S,
                          const float *__restrict__ P, const float *__restrict__ pot,
                          const float *__restrict__ vr_in, const float *__restrict__ dv_in,
                          float *__restrict__ vr_out, float *__restrict__ dv_out)
 {
     fgpu::follow_predecessor();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= g.nz) return;
-    source_cell(g, t, dt, S, P, pot, vr_in, dv_in, vr_out, dv_out, blockIdx.y, j);
+    const Quad<VEC> q = quad_of<VEC>(g.nz);
+    if (q.first >= g.nz) return;
+    source_cells(q, g, t, dt, S, P, pot, vr_in, dv_in, vr_out, dv_out, blockIdx.y);
 }
 
+template <bool VEC>
 __global__ void f_artvisc_q(GeoF g, TablesF t, PhysF ph, float dt, const float *__restrict__ S,
                             const float *__restrict__ vr, const float *__restrict__ dv,
                             float *__restrict__ E, float *__restrict__ Qr, float *__restrict__ Qp)
 {
     fgpu::follow_predecessor();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= g.nz) return;
-    artvisc_q_cell(g, t, ph, dt, S, vr, dv, E, Qr, Qp, blockIdx.y, j);
+    const Quad<VEC> q = quad_of<VEC>(g.nz);
+    if (q.first >= g.nz) return;
+    artvisc_q_cells(q, g, t, ph, dt, S, vr, dv, E, Qr, Qp, blockIdx.y);
 }
 
+template <bool VEC>
 __global__ void f_artvisc_v(GeoF g, TablesF t, PhysF ph, float dt, const float *__restrict__ S,
                             const float *__restrict__ E, const float *__restrict__ Qr,
                             const float *__restrict__ Qp, float *__restrict__ vr,
@@ -80,22 +92,24 @@ __global__ void f_artvisc_v(GeoF g, TablesF t, PhysF ph, float dt, const float *
                             float *__restrict__ nu)
 {
     fgpu::follow_predecessor();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= g.nz) return;
-    artvisc_v_cell(g, t, ph, dt, S, E, Qr, Qp, vr, dv, cs, H, nu, blockIdx.y, j);
+    const Quad<VEC> q = quad_of<VEC>(g.nz);
+    if (q.first >= g.nz) return;
+    artvisc_v_cells(q, g, t, ph, dt, S, E, Qr, Qp, vr, dv, cs, H, nu, blockIdx.y);
 }
 
+template <bool VEC>
 __global__ void f_stress(GeoF g, TablesF t, const float *__restrict__ S, const float *__restrict__ vr,
                          const float *__restrict__ dv, const float *__restrict__ nu,
                          float *__restrict__ divv, float *__restrict__ trr, float *__restrict__ tpp,
                          float *__restrict__ trp)
 {
     fgpu::follow_predecessor();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= g.nz) return;
-    stress_cell(g, t, S, vr, dv, nu, divv, trr, tpp, trp, blockIdx.y, j);
+    const Quad<VEC> q = quad_of<VEC>(g.nz);
+    if (q.first >= g.nz) return;
+    stress_cells(q, g, t, S, vr, dv, nu, divv, trr, tpp, trp, blockIdx.y);
 }
 
+template <bool VEC>
 __global__ void f_viscous(GeoF g, TablesF t, PhysF ph, float dt, float beta_inv, int mode,
                           const float *__restrict__ S, const float *__restrict__ trr,
                           const float *__restrict__ tpp, const float *__restrict__ trp,
@@ -107,10 +121,10 @@ __global__ void f_viscous(GeoF g, TablesF t, PhysF ph, float dt, float beta_inv,
                           const float *__restrict__ corr_r)
 {
     fgpu::follow_predecessor();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= g.nz) return;
-    viscous_cell(g, t, ph, dt, beta_inv, mode, S, trr, tpp, trp, divv, nu, H, S0, E0, vr, dv, E,
-                 qplus, qminus, corr_phi, corr_r, blockIdx.y, j);
+    const Quad<VEC> q = quad_of<VEC>(g.nz);
+    if (q.first >= g.nz) return;
+    viscous_cells(q, g, t, ph, dt, beta_inv, mode, S, trr, tpp, trp, divv, nu, H, S0, E0, vr, dv, E,
+                 qplus, qminus, corr_phi, corr_r, blockIdx.y);
 }
 
 // StabilizeViscosity's correction factors, rows 1 .. nr - 1
@@ -219,6 +233,7 @@ __global__ void f_pressure(GeoF g, TablesF t, PhysF ph, const float *__restrict_
     pressure_cell(g, t, ph, S, E, P, blockIdx.y, j);
 }
 
+template <bool VEC>
 __global__ void f_finish(GeoF g, TablesF t, PhysF ph, const float *__restrict__ m0,
                          const float *__restrict__ m1, const float *__restrict__ m2,
                          const float *__restrict__ m3, const float *__restrict__ S_t,
@@ -229,10 +244,10 @@ __global__ void f_finish(GeoF g, TablesF t, PhysF ph, const float *__restrict__ 
                          const int *__restrict__ shift)
 {
     fgpu::follow_predecessor();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= g.nz) return;
-    finish_cell(g, t, ph, m0, m1, m2, m3, S_t, E_t, vr_in, vr_out, dv_out, S_out, E_out, Slo_t,
-                Slo_out, shift, blockIdx.y, j);
+    const Quad<VEC> q = quad_of<VEC>(g.nz);
+    if (q.first >= g.nz) return;
+    finish_cells(q, g, t, ph, m0, m1, m2, m3, S_t, E_t, vr_in, vr_out, dv_out, S_out, E_out, Slo_t,
+                Slo_out, shift, blockIdx.y);
 }
 
 __global__ void f_damping(GeoF g, DampingF dm, float dt, const int *__restrict__ rings, StateF s)
@@ -1123,6 +1138,19 @@ void Engine32::set_bodies(int n, const fgpu_body *b, double ix, double iy, doubl
 
 static dim3 grid2(int nz, int rows) { return dim3((nz + 127) / 128, rows); }
 
+// a kernel of one Quad per thread over `rows` rings: blocks of up to 128 threads
+// that share a ring evenly (FP32 step of the 2048 x 6144 disk 1.413 ms, with 64
+// 1.435, with 256 1.439; 512 x 1536 0.160, 0.166, 0.162)
+template <class... P, class... A>
+static void launch_cells(void (*vec)(P...), void (*any)(P...), int nz, int rows,
+                         cudaStream_t stream, A &&...args)
+{
+    const int quads = (nz + 3) / 4, blocks = (quads + 127) / 128;
+    const int threads = ((quads + blocks - 1) / blocks + 31) / 32 * 32;
+    fgpu::launch(nz % 4 == 0 ? vec : any, dim3(blocks, rows), threads, 0, stream,
+                 std::forward<A>(args)...);
+}
+
 int Engine32::derived_cfl(int mode, bool reset)
 {
     if (int rc_ = sync_frame()) return rc_;
@@ -1152,13 +1180,12 @@ int Engine32::init_euler(double t)
     if (rc) return rc;
     if (phys.adiabatic) {
         StateF s = state();
-        fgpu::launch(f_stress, grid2(nz, nr), 128, 0, stream, geo, tabs, s.sigma, s.vr, s.dv,
+        launch_cells(f_stress<true>, f_stress<false>, nz, nr, stream, geo, tabs, s.sigma, s.vr, s.dv,
                                                     fld[FGPU_VISCOSITY], fld[FGPU_DIV_V],
                                                     fld[FGPU_TAU_R_R], fld[FGPU_TAU_PHI_PHI],
                                                     fld[FGPU_TAU_R_PHI]);
         if (phys.stabilize) visc_corr(s);
-        fgpu::launch(f_viscous, grid2(nz, nr), 128, 0, stream, 
-            geo, tabs, phys, 0.f, (float)beta_inv(t), 2, s.sigma, fld[FGPU_TAU_R_R],
+        launch_cells(f_viscous<true>, f_viscous<false>, nz, nr, stream, geo, tabs, phys, 0.f, (float)beta_inv(t), 2, s.sigma, fld[FGPU_TAU_R_R],
             fld[FGPU_TAU_PHI_PHI], fld[FGPU_TAU_R_PHI], fld[FGPU_DIV_V], fld[FGPU_VISCOSITY],
             fld[FGPU_SCALE_HEIGHT], s.sigma0, s.energy0, s.vr, s.dv, s.energy, fld[FGPU_QPLUS],
             fld[FGPU_QMINUS], corr_phi, corr_r);
@@ -1247,11 +1274,11 @@ int Engine32::kick(double dt, double t)
     auto mark = [&](int k) {
         if (mark_fn) mark_fn(mark_ctx, k);
     };
-    fgpu::launch(f_potential, grid2(nz, nr), 128, 0, stream, geo, tabs, phys, bodies, fld[FGPU_SCALE_HEIGHT],
+    launch_cells(f_potential<true>, f_potential<false>, nz, nr, stream, geo, tabs, phys, bodies, fld[FGPU_SCALE_HEIGHT],
                                                    fld[FGPU_POTENTIAL]);
     CKL("potential");
     mark(0);
-    fgpu::launch(f_source, grid2(nz, nr + 1), 128, 0, stream, geo, tabs, fdt, fld[FGPU_SIGMA],
+    launch_cells(f_source<true>, f_source<false>, nz, nr + 1, stream, geo, tabs, fdt, fld[FGPU_SIGMA],
                                                     fld[FGPU_PRESSURE], fld[FGPU_POTENTIAL],
                                                     fld[FGPU_V_RADIAL], fld[FGPU_V_AZIMUTHAL],
                                                     alt_vr, alt_dv);
@@ -1261,12 +1288,11 @@ int Engine32::kick(double dt, double t)
     mark(1);
     StateF s = state();
     if (adi || phys.art_visc_sn || phys.art_visc_tw) {
-        fgpu::launch(f_artvisc_q, grid2(nz, nr), 128, 0, stream, geo, tabs, phys, fdt, s.sigma, s.vr, s.dv,
+        launch_cells(f_artvisc_q<true>, f_artvisc_q<false>, nz, nr, stream, geo, tabs, phys, fdt, s.sigma, s.vr, s.dv,
                                                        s.energy, fld[FGPU_Q_R], fld[FGPU_Q_PHI]);
         CKL("artvisc_q");
         mark(2);
-        fgpu::launch(f_artvisc_v, grid2(nz, nr), 128, 0, stream, 
-            geo, tabs, phys, fdt, s.sigma, s.energy, fld[FGPU_Q_R], fld[FGPU_Q_PHI], s.vr, s.dv,
+        launch_cells(f_artvisc_v<true>, f_artvisc_v<false>, nz, nr, stream, geo, tabs, phys, fdt, s.sigma, s.energy, fld[FGPU_Q_R], fld[FGPU_Q_PHI], s.vr, s.dv,
             fld[FGPU_SOUNDSPEED], fld[FGPU_SCALE_HEIGHT], fld[FGPU_VISCOSITY]);
         CKL("artvisc_v");
         mark(3);
@@ -1274,15 +1300,14 @@ int Engine32::kick(double dt, double t)
         mark(2);
         mark(3);
     }
-    fgpu::launch(f_stress, grid2(nz, nr), 128, 0, stream, geo, tabs, s.sigma, s.vr, s.dv,
+    launch_cells(f_stress<true>, f_stress<false>, nz, nr, stream, geo, tabs, s.sigma, s.vr, s.dv,
                                                 fld[FGPU_VISCOSITY], fld[FGPU_DIV_V],
                                                 fld[FGPU_TAU_R_R], fld[FGPU_TAU_PHI_PHI],
                                                 fld[FGPU_TAU_R_PHI]);
     CKL("stress");
     if (phys.stabilize) visc_corr(s);
     mark(4);
-    fgpu::launch(f_viscous, grid2(nz, nr), 128, 0, stream, 
-        geo, tabs, phys, fdt, (float)beta_inv(t), adi ? 7 : 1, s.sigma, fld[FGPU_TAU_R_R],
+    launch_cells(f_viscous<true>, f_viscous<false>, nz, nr, stream, geo, tabs, phys, fdt, (float)beta_inv(t), adi ? 7 : 1, s.sigma, fld[FGPU_TAU_R_R],
         fld[FGPU_TAU_PHI_PHI], fld[FGPU_TAU_R_PHI], fld[FGPU_DIV_V], fld[FGPU_VISCOSITY],
         fld[FGPU_SCALE_HEIGHT], s.sigma0, s.energy0, s.vr, s.dv, s.energy, fld[FGPU_QPLUS],
         fld[FGPU_QMINUS], corr_phi, corr_r);
@@ -1381,8 +1406,7 @@ int Engine32::transport(double dt)
     CKL("transport_azimuthal");
     mark(8);
     float *const *m = windows ? mom_w : mom;
-    fgpu::launch(f_finish, grid2(nz, nr + 1), 128, 0, stream, 
-        geo, tabs, phys, m[0], m[1], m[2], m[3], windows ? sigma_w : alt_sigma,
+    launch_cells(f_finish<true>, f_finish<false>, nz, nr + 1, stream, geo, tabs, phys, m[0], m[1], m[2], m[3], windows ? sigma_w : alt_sigma,
         windows ? energy_w : alt_e, s.vr, alt_vr, alt_dv, s.sigma, s.energy,
         windows ? sigma_lo_w : alt_sigma_lo, sigma_lo, ring_shift);
     CKL("finish");
