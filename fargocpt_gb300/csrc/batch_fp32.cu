@@ -64,7 +64,9 @@ __device__ __forceinline__ int disk_of(const int *__restrict__ start, int nd, in
     return lo;
 }
 
-// a tile of more threads is walked by this many
+// a tile of more threads is walked by this many; two blocks of them per SM (64
+// registers: a batch of 16 disks, 4.8M cells, 0.254 ms in the seven kernels of a
+// Quad per thread, at 128 registers 0.296, at 40 0.377)
 constexpr int kCellThreads = 512;
 
 // Per-cell tiles: 4 blockDim.x columns (a Quad per thread) x rpb rings of one
@@ -157,7 +159,7 @@ struct CellsFinish {
     }
 };
 
-__global__ void __launch_bounds__(kCellThreads)
+__global__ void __launch_bounds__(kCellThreads, 2)
     b_potential(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
                 int nd, int rpb)
 {
@@ -165,7 +167,7 @@ __global__ void __launch_bounds__(kCellThreads)
     for_cells(D, S, start, nd, rpb, 0, CellsPotential{});
 }
 
-__global__ void __launch_bounds__(kCellThreads)
+__global__ void __launch_bounds__(kCellThreads, 2)
     b_source(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
              int nd, int rpb)
 {
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(kCellThreads)
     for_cells(D, S, start, nd, rpb, 1, CellsSource{});
 }
 
-__global__ void __launch_bounds__(kCellThreads)
+__global__ void __launch_bounds__(kCellThreads, 2)
     b_artvisc_q(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
                 int nd, int rpb)
 {
@@ -181,7 +183,7 @@ __global__ void __launch_bounds__(kCellThreads)
     for_cells(D, S, start, nd, rpb, 0, CellsArtviscQ{});
 }
 
-__global__ void __launch_bounds__(kCellThreads)
+__global__ void __launch_bounds__(kCellThreads, 2)
     b_artvisc_v(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
                 int nd, int rpb)
 {
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(kCellThreads)
     for_cells(D, S, start, nd, rpb, 0, CellsArtviscV{});
 }
 
-__global__ void __launch_bounds__(kCellThreads)
+__global__ void __launch_bounds__(kCellThreads, 2)
     b_stress(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
              int nd, int rpb)
 {
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(kCellThreads)
     for_cells(D, S, start, nd, rpb, 0, CellsStress{});
 }
 
-__global__ void __launch_bounds__(kCellThreads)
+__global__ void __launch_bounds__(kCellThreads, 2)
     b_viscous(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
               int nd, int rpb)
 {
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(kCellThreads)
     for_cells(D, S, start, nd, rpb, 0, CellsViscous{});
 }
 
-__global__ void __launch_bounds__(kCellThreads)
+__global__ void __launch_bounds__(kCellThreads, 2)
     b_finish(const DiskF *__restrict__ D, const StepF *__restrict__ S, const int *__restrict__ start,
              int nd, int rpb)
 {
@@ -350,12 +352,13 @@ __global__ void b_damping(const DiskF *__restrict__ D, const StepF *__restrict__
 }
 
 // derived quantities and CFL minimum: one ring per block iteration
-__global__ void b_derived_cfl(const DiskF *__restrict__ D, const StepF *__restrict__ S,
-                              const int *__restrict__ start, int nd, int mode, int all)
+__global__ void __launch_bounds__(kCellThreads, 2)
+    b_derived_cfl(const DiskF *__restrict__ D, const StepF *__restrict__ S,
+                  const int *__restrict__ start, int nd, int mode, int all)
 {
     fgpu::follow_predecessor();
     __shared__ float red[33];
-    __shared__ longlong2 red2[33];
+    __shared__ long long redl[33];
     const int total = __ldg(start + nd);
     for (int item = blockIdx.x; item < total; item += gridDim.x) {
         const int d = disk_of(start, nd, item);
@@ -363,7 +366,7 @@ __global__ void b_derived_cfl(const DiskF *__restrict__ D, const StepF *__restri
         const DiskF &k = D[d];
         const int i = item - __ldg(start + d);
         derived_cfl_ring(k.g, k.t, k.ph, mode, k.s.sigma, k.s.energy, k.s.vr, k.s.dv, k.qplus,
-                         k.qminus, k.cs, k.H, k.P, k.T, k.nu, k.dtmin, i, red, red2, nullptr,
+                         k.qminus, k.cs, k.H, k.P, k.T, k.nu, k.cfl, i, red, redl, nullptr,
                          nullptr);
     }
 }
@@ -434,7 +437,6 @@ __global__ void b_close_sequence(const DiskF *__restrict__ D, const StepF *__res
 {
     __shared__ float red[33];
     __shared__ long long redl[33];
-    __shared__ longlong2 red2[33];
     cg::grid_group grid = cg::this_grid();
     if (!grid.is_valid()) {
         if (blockIdx.x == 0 && threadIdx.x == 0) *err = 1;
@@ -475,7 +477,7 @@ __global__ void b_close_sequence(const DiskF *__restrict__ D, const StepF *__res
         const DiskF &k = D[d];
         const int i = item - __ldg(ct + d);
         derived_cfl_ring(k.g, k.t, k.ph, 1 | 4, k.s.sigma, k.s.energy, k.s.vr, k.s.dv, k.qplus,
-                         k.qminus, k.cs, k.H, k.P, k.T, k.nu, k.dtmin, i, red, red2, nullptr,
+                         k.qminus, k.cs, k.H, k.P, k.T, k.nu, k.cfl, i, red, redl, nullptr,
                          nullptr);
     }
 }
@@ -484,7 +486,7 @@ __global__ void b_reset_dtmin(const DiskF *__restrict__ D, const StepF *__restri
 {
     fgpu::follow_predecessor();
     const int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d < nd && S[d].run) *D[d].dtmin = 0x7f7f7f7fu;
+    if (d < nd && S[d].run) *D[d].cfl.dt_min = 0x7f7f7f7fu;
 }
 
 // Planets on circular orbits around the star at the origin and the indirect
@@ -541,7 +543,7 @@ __global__ void b_clock(const DiskF *__restrict__ D, const ClockAux *__restrict_
         StepF &s = S[d];
         const int run = c.active && c.t < c.t_end;
         if (run) {
-            unsigned int *dtmin = D[d].dtmin;
+            unsigned int *dtmin = D[d].cfl.dt_min;
             const double cfl = (double)__uint_as_float(*dtmin);
             *dtmin = 0x7f7f7f7fu;
             const double grown = __dmul_rn(c.cfl_max_var, c.last_dt);
@@ -724,7 +726,8 @@ static int check_tiles(const fgpu_batch *b, const fgpu_tiles &t, std::string &wh
 // threads per block of kernel k
 static int launch_threads(const fgpu_tiles &t, int k)
 {
-    return is_cell_kernel(k) ? std::min(t.k[k].threads, kCellThreads) : t.k[k].threads;
+    return is_cell_kernel(k) || k == FGPU_BK_DERIVED_CFL ? std::min(t.k[k].threads, kCellThreads)
+                                                         : t.k[k].threads;
 }
 
 // tile tables and grid sizes of the current tile shapes
@@ -853,7 +856,9 @@ static void default_tiles(const fgpu_batch *b, fgpu_tiles &t)
     for (int k = 0; k < FGPU_BK_COUNT; ++k) t.k[k] = {128, 1};
     t.k[FGPU_BK_TRANSPORT_RADIAL] = {64, 16};
     t.k[FGPU_BK_DAMPING] = {256, 1};
-    t.k[FGPU_BK_DERIVED_CFL] = {256, 1};
+    // a warp per ring (16 disks of 384 to 1536 cells per ring: 0.065 ms, 64 threads
+    // 0.072, 128 0.094; one cell per thread, 256 threads 0.124)
+    t.k[FGPU_BK_DERIVED_CFL] = {32, 1};
     const int per = b->nz_max <= 2048 ? 4 : (b->nz_max <= 4096 ? 8 : 16);
     int th = ((b->nz_max + per - 1) / per + 31) / 32 * 32;
     th = std::max(128, std::min(512, th));
@@ -1431,11 +1436,13 @@ static int take_snapshot(fgpu_batch *b, Snapshot &s, bool restore)
     }
     for (int d = 0; d < b->nd; ++d) {
         const DiskF k = b->disks[d]->describe();
-        if (restore)
-            CKB(cudaMemcpyAsync(k.dtmin, s.dtmin + d, sizeof(unsigned int),
+        if (restore) {
+            CKB(cudaMemcpyAsync(k.cfl.dt_min, s.dtmin + d, sizeof(unsigned int),
                                 cudaMemcpyDeviceToDevice, b->stream));
-        else
-            CKB(cudaMemcpyAsync(s.dtmin + d, k.dtmin, sizeof(unsigned int),
+            CKB(cudaMemcpyAsync(k.cfl.host_dt, s.dtmin + d, sizeof(unsigned int),
+                                cudaMemcpyDeviceToHost, b->stream));
+        } else
+            CKB(cudaMemcpyAsync(s.dtmin + d, k.cfl.dt_min, sizeof(unsigned int),
                                 cudaMemcpyDeviceToDevice, b->stream));
     }
     CKB(cudaStreamSynchronize(b->stream));
@@ -1456,6 +1463,8 @@ static void candidates(const fgpu_batch *b, int k, std::vector<fgpu_tile> &out)
     } else if (k == FGPU_BK_TRANSPORT_AZIMUTHAL) {
         for (int th : {96, 128, 192, 256, 384, 512})
             if (per_for(b->nz_max, th)) out.push_back({th, 1});
+    } else if (k == FGPU_BK_DERIVED_CFL) {
+        for (int th : {32, 64, 128, 256}) out.push_back({th, 1});
     } else {
         for (int th : {128, 256, 512}) out.push_back({th, 1});
     }

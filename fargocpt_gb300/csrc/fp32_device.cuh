@@ -165,7 +165,14 @@ __device__ __forceinline__ int exact_sum_scale(float local_absmax, int n, float 
     const int ln = 32 - __clz(n);  // n < 2^ln
     return 62 - e - ln;
 }
-__device__ __forceinline__ long long to_fixed(float x, int k) { return __float2ll_rn(ldexpf(x, k)); }
+// (x 2^k in two exact multiplications: |x 2^k| < 2^62, and what a first step
+// towards zero rounds in the subnormals is far below 1/2)
+__device__ __forceinline__ long long to_fixed(float x, int k)
+{
+    const int k1 = k >> 1;
+    const float a = __int_as_float((127 + k1) << 23), b = __int_as_float((127 + (k - k1)) << 23);
+    return __float2ll_rn(__fmul_rn(__fmul_rn(x, a), b));
+}
 // Step 2: the sum of the threads' integer partial sums.
 __device__ __forceinline__ double exact_sum_result(long long part, int k, long long *redl)
 {
@@ -173,59 +180,23 @@ __device__ __forceinline__ double exact_sum_result(long long part, int k, long l
     return ldexp((double)s, -k);
 }
 
-__device__ __forceinline__ float2 warp_max_f2(float2 v)
-{
-    for (int o = 16; o > 0; o >>= 1) {
-        v.x = fmaxf(v.x, __shfl_down_sync(0xffffffffu, v.x, o));
-        v.y = fmaxf(v.y, __shfl_down_sync(0xffffffffu, v.y, o));
-    }
-    return v;
-}
-__device__ __forceinline__ longlong2 warp_sum_ll2(longlong2 v)
-{
-    for (int o = 16; o > 0; o >>= 1) {
-        v.x += __shfl_down_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_down_sync(0xffffffffu, v.y, o);
-    }
-    return v;
-}
-
-// Means of two rows at once (the CFL's ring i and ring i + 1), each with its
-// own scale, in two block reductions.  red2: 33 float2, redl2: 33 longlong2.
-__device__ __forceinline__ float2 exact_row_means2(const float *a, const float *b, int n,
-                                                   float2 *red2, longlong2 *redl2)
-{
-    float2 m = make_float2(0.f, 0.f);
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        m.x = fmaxf(m.x, fabsf(a[j]));
-        m.y = fmaxf(m.y, fabsf(b[j]));
-    }
-    m = block_reduce<float2, warp_max_f2>(m, red2, make_float2(0.f, 0.f));
-    int ea = 0, eb = 0;
-    frexpf(m.x, &ea);
-    frexpf(m.y, &eb);
-    const int ln = 32 - __clz(n);
-    const int ka = 62 - ea - ln, kb = 62 - eb - ln;
-    longlong2 part = make_longlong2(0, 0);
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        part.x += to_fixed(a[j], ka);
-        part.y += to_fixed(b[j], kb);
-    }
-    part = block_reduce<longlong2, warp_sum_ll2>(part, redl2, make_longlong2(0, 0));
-    return make_float2((float)(ldexp((double)part.x, -ka) / (double)n),
-                       (float)(ldexp((double)part.y, -kb) / (double)n));
-}
-
-// Mean of row[0 .. n-1] (global memory, cells strided over the block).
+// Mean of row[0 .. n-1] (global memory, shared by the block; the last division
+// by one thread, red[32] to the others).
 __device__ __forceinline__ float exact_row_mean(const float *row, int n, float *redf,
                                                 long long *redl)
 {
+    const int bs = blockDim.x, tid = threadIdx.x;
     float m = 0.f;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) m = fmaxf(m, fabsf(row[j]));
+#pragma unroll 8
+    for (int j = tid; j < n; j += bs) m = fmaxf(m, fabsf(row[j]));
     const int k = exact_sum_scale(m, n, redf);
     long long part = 0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) part += to_fixed(row[j], k);
-    return (float)(exact_sum_result(part, k, redl) / (double)n);
+#pragma unroll 8
+    for (int j = tid; j < n; j += bs) part += to_fixed(row[j], k);
+    const long long s = block_reduce<long long, warp_sum_ll>(part, redl, 0LL);
+    if (tid == 0) redf[32] = (float)(ldexp((double)s, -k) / (double)n);
+    __syncthreads();
+    return redf[32];
 }
 
 // ---------------------------------------------------------------------------
@@ -2054,109 +2025,182 @@ __device__ __forceinline__ void damping_ring(const GeoF &g, const DampingF &dm, 
 // derived quantities + CFL (SourceEuler.cpp:225-249, cfl.cpp:185-382); block-
 // wide over ring i.  mode bits: 1 derived quantities, 2 also c_s, H, T of the
 // isothermal disk, 4 CFL minimum into dt_min (float bits, atomicMin)
+template <class Q>
+__device__ __forceinline__ float derived_cfl_cells(
+    const Q &q, const GeoF &g, const TablesF &t, const PhysF &ph, int mode, bool cfl_ring, float md0,
+    float vref_frame, const float *__restrict__ S, const float *__restrict__ E,
+    const float *__restrict__ vr, const float *__restrict__ dv, const float *__restrict__ qplus,
+    const float *__restrict__ qminus, float *__restrict__ cs, float *__restrict__ H,
+    float *__restrict__ P, float *__restrict__ T, float *__restrict__ nu,
+    const float *__restrict__ corr_phi, const float *__restrict__ corr_r, int i)
+{
+    const int nz = g.nz;
+    const size_t row = (size_t)i * nz;
+    float c[4], n[4], e[4], v0[4], v1[4], d0[4], dn[4], qp[4], qm[4];
+    if (ph.adiabatic) q.load(E, row, e);
+    if (cfl_ring) {
+        q.load(vr, row, v0);
+        q.load(vr, row + nz, v1);
+        q.load(dv, row, d0);
+        q.right(dv, row, d0, dn);
+        if (ph.adiabatic) {
+            q.load(qplus, row, qp);
+            q.load(qminus, row, qm);
+        }
+    }
+    if (mode & 1) {
+        float sg[4], x[4], h[4];
+        q.load(S, row, sg);
+        if (ph.adiabatic) {
+            const float hfac = t.HFacAdi[i];
+            float es[4];
+#pragma unroll
+            QUAD {
+                es[k] = __fdividef(e[k], sg[k]);
+                x[k] = ph.c_v_inv * es[k];
+                c[k] = sqrtf(ph.g_gm1 * es[k]);
+                h[k] = c[k] * hfac;
+                n[k] = ph.alpha > 0.f ? ph.alpha * h[k] * c[k] : ph.constant_viscosity;
+            }
+            q.store(T, row, x);
+            q.store(cs, row, c);
+            q.store(H, row, h);
+#pragma unroll
+            QUAD x[k] = ph.gm1 * e[k];
+            q.store(P, row, x);
+        } else {
+            const float c_s = t.CsIso[i], hi = c_s * t.InvOmegaK[i];
+            const float ni = ph.alpha > 0.f ? ph.alpha * hi * c_s : ph.constant_viscosity;
+#pragma unroll
+            QUAD {
+                c[k] = c_s;
+                h[k] = hi;
+                n[k] = ni;
+                x[k] = sg[k] * (c_s * c_s);
+            }
+            q.store(P, row, x);
+            if (mode & 2) {
+                q.store(cs, row, c);
+                q.store(H, row, h);
+#pragma unroll
+                QUAD x[k] = ph.mu_over_R * x[k] / sg[k];
+                q.store(T, row, x);
+            }
+        }
+        q.store(nu, row, n);
+    } else {
+        q.load(cs, row, c);
+        q.load(nu, row, n);
+    }
+    float local = 3.0e38f;
+    if (!cfl_ring) return local;
+    const float invcell = t.InvCell[i], invcell2 = t.InvCell2[i], invdrsup = t.InvDiffRsup[i],
+                invdxt = t.InvDxTheta[i], invrmed = t.InvRmed[i];
+    float cphi[4], cr[4];
+    if (ph.stabilize == 2) {
+        q.load(corr_phi, row, cphi);
+        q.load(corr_r, row, cr);
+    }
+#pragma unroll
+    QUAD {
+        const float vres = ph.fast_transport ? d0[k] - md0 : vref_frame + d0[k];
+        const float invdt1 = c[k] * invcell;
+        const float invdt2 = v0[k] * invdrsup;
+        const float invdt3 = vres * invdxt;
+        const float dvA = dn[k] - d0[k];
+        float invdt4;
+        if (ph.art_visc_sn) {
+            const float a = fmaxf(v0[k] - v1[k], 0.f) * invdrsup;
+            const float b = fmaxf(-dvA, 0.f) * invdxt;
+            invdt4 = ph.four_C2 * fmaxf(a, b);
+        } else {
+            const float eps_pp = __fmul_rn(invrmed, fmaf(dvA, g.invdphi, 0.5f * (v1[k] + v0[k])));
+            invdt4 = ph.four_C2 * fmaxf(-fmaf(v1[k] - v0[k], invdrsup, eps_pp), 0.f);
+        }
+        float invdt5 = 4.f * n[k] * invcell2;
+        float invdt6 = 0.f;
+        if (ph.adiabatic) invdt6 = ph.inv_hc_limit * fabsf(__fdividef(qp[k] - qm[k], e[k]));
+        if (ph.leapfrog) {
+            // LeapFrog applies the source terms twice with dt/2 (cfl.cpp:254-317)
+            invdt4 *= 0.6f;
+            invdt5 *= 0.6f;
+            invdt6 *= 0.6f;
+        }
+        const float s2 = fmaf(
+            invdt6, invdt6,
+            fmaf(invdt5, invdt5,
+                 fmaf(invdt4, invdt4,
+                      fmaf(invdt3, invdt3, fmaf(invdt1, invdt1, __fmul_rn(invdt2, invdt2))))));
+        float dt_cell = ph.cfl * rsqrtf(s2);
+        if (ph.stabilize == 2) {
+            // viscous stability limit, cfl.cpp:332-351
+            const float cc = fminf(cphi[k], cr[k]);
+            if (cc != 0.f) dt_cell = fminf(dt_cell, -ph.cfl / cc);
+        }
+        local = fminf(local, dt_cell);  // (a cell past the ring's end repeats its last)
+    }
+    return local;
+}
+
+// A ring's mean is formed by its block alone.  The first warp of the disk's ring
+// that finishes last takes the shear limits of all pairs of rings and writes the
+// disk's step to the host.
 __device__ __forceinline__ void derived_cfl_ring(
     const GeoF &g, const TablesF &t, const PhysF &ph, int mode, const float *__restrict__ S,
     const float *__restrict__ E, const float *__restrict__ vr, const float *__restrict__ dv,
     const float *__restrict__ qplus, const float *__restrict__ qminus, float *__restrict__ cs,
     float *__restrict__ H, float *__restrict__ P, float *__restrict__ T, float *__restrict__ nu,
-    unsigned int *__restrict__ dt_min, int i, float *red, longlong2 *red2,
-    const float *__restrict__ corr_phi, const float *__restrict__ corr_r)
+    const CflOut &out, int i, float *red, long long *redl, const float *__restrict__ corr_phi,
+    const float *__restrict__ corr_r)
 {
     const int nz = g.nz, nr = g.nr;
     const size_t row = (size_t)i * nz;
     const bool do_cfl = (mode & 4) != 0;
-    float md0 = 0.f, md1 = 0.f;
-    if (do_cfl && i < nr - 1) {
-        // ring means of dv, independent of the block's shape; red2 (33
-        // longlong2) serves both pair reductions one after the other
-        const float2 m = exact_row_means2(dv + row, dv + row + nz, nz,
-                                          reinterpret_cast<float2 *>(red2), red2);
-        md0 = m.x;
-        md1 = m.y;
-    }
-    float local = 3.0e38f;
-    if (do_cfl && i < nr - 1 && i >= 0 && (i == 0 || i < nr - 1)) {
-        // shear limit: |vm_i / R_i - vm_{i+1} / R_{i+1}| with vm = Vref + mean dv
-        const float denom = fabsf(t.OmRefDiff[i] + md0 * t.InvRmed[i] - md1 * t.InvRmed[i + 1]) +
-                            1.0e-30f;
-        local = ph.cfl * g.dphi / denom;
+    float md0 = 0.f, local = 3.0e38f;
+    if (do_cfl) {
+        // mean of dv, independent of the block's shape
+        md0 = exact_row_mean(dv + row, nz, red, redl);
+        if (threadIdx.x == 0) out.mean[i] = md0;
     }
     const bool cfl_ring = do_cfl && i >= 1 && i < nr - 1;
     // standard transport: the ring's frame speed of the Keplerian reference
     const float vref_frame =
         ph.fast_transport ? 0.f : (float)(t.Vref_d[i] - t.Rmed_d[i] * g.omega_frame);
-    for (int j = threadIdx.x; j < nz; j += blockDim.x) {
-        const size_t c = row + j;
-        float c_s, n;
-        if (mode & 1) {
-            const float sg = S[c];
-            if (ph.adiabatic) {
-                const float e = E[c];
-                const float es = __fdividef(e, sg);
-                T[c] = ph.c_v_inv * es;
-                c_s = sqrtf(ph.g_gm1 * es);
-                const float h = c_s * t.HFacAdi[i];
-                cs[c] = c_s;
-                H[c] = h;
-                P[c] = ph.gm1 * e;
-                n = ph.alpha > 0.f ? ph.alpha * h * c_s : ph.constant_viscosity;
-            } else {
-                c_s = t.CsIso[i];
-                const float h = c_s * t.InvOmegaK[i];
-                P[c] = sg * (c_s * c_s);
-                if (mode & 2) {
-                    cs[c] = c_s;
-                    H[c] = h;
-                    T[c] = ph.mu_over_R * P[c] / sg;
-                }
-                n = ph.alpha > 0.f ? ph.alpha * h * c_s : ph.constant_viscosity;
-            }
-            nu[c] = n;
-        } else {
-            c_s = cs[c];
-            n = nu[c];
-        }
-        if (cfl_ring) {
-            const float d0 = dv[c];
-            const float vres = ph.fast_transport ? d0 - md0 : vref_frame + d0;
-            const float invdt1 = c_s * t.InvCell[i];
-            const float invdt2 = vr[c] * t.InvDiffRsup[i];
-            const float invdt3 = vres * t.InvDxTheta[i];
-            const float vr1 = vr[c + nz];
-            const float dvA = dv[row + (j == nz - 1 ? 0 : j + 1)] - d0;
-            float invdt4;
-            if (ph.art_visc_sn) {
-                const float a = fmaxf(vr[c] - vr1, 0.f) * t.InvDiffRsup[i];
-                const float b = fmaxf(-dvA, 0.f) * t.InvDxTheta[i];
-                invdt4 = ph.four_C2 * fmaxf(a, b);
-            } else {
-                const float eps_rr = (vr1 - vr[c]) * t.InvDiffRsup[i];
-                const float eps_pp = t.InvRmed[i] * (dvA * g.invdphi + 0.5f * (vr1 + vr[c]));
-                invdt4 = ph.four_C2 * fmaxf(-(eps_rr + eps_pp), 0.f);
-            }
-            float invdt5 = 4.f * n * t.InvCell2[i];
-            float invdt6 = 0.f;
-            if (ph.adiabatic) invdt6 = ph.inv_hc_limit * fabsf(__fdividef(qplus[c] - qminus[c], E[c]));
-            if (ph.leapfrog) {
-                // LeapFrog applies the source terms twice with dt/2 (cfl.cpp:254-317)
-                invdt4 *= 0.6f;
-                invdt5 *= 0.6f;
-                invdt6 *= 0.6f;
-            }
-            const float s2 = invdt1 * invdt1 + invdt2 * invdt2 + invdt3 * invdt3 +
-                             invdt4 * invdt4 + invdt5 * invdt5 + invdt6 * invdt6;
-            float dt_cell = ph.cfl * rsqrtf(s2);
-            if (ph.stabilize == 2) {
-                // viscous stability limit, cfl.cpp:332-351
-                const float cc = fminf(corr_phi[c], corr_r[c]);
-                if (cc != 0.f) dt_cell = fminf(dt_cell, -ph.cfl / cc);
-            }
-            local = fminf(local, dt_cell);
-        }
+    auto cells = [&](const auto &q) {
+        local = fminf(local, derived_cfl_cells(q, g, t, ph, mode, cfl_ring, md0, vref_frame, S, E,
+                                               vr, dv, qplus, qminus, cs, H, P, T, nu, corr_phi,
+                                               corr_r, i));
+    };
+    const int bs = blockDim.x, tid = threadIdx.x;
+    if (nz % 4 == 0) {
+        for (int j = 4 * tid; j < nz; j += 4 * bs) cells(Quad<true>{nz, j, 1});
+    } else {
+        for (int j = tid; j < nz; j += 4 * bs) cells(Quad<false>{nz, j, bs});
     }
     if (do_cfl) {
         const float m = bmin_f(local, red);
-        if (threadIdx.x == 0 && m < 3.0e38f) atomicMin(dt_min, __float_as_uint(m));
+        if (tid >= 32) return;
+        unsigned int before = 0;
+        if (tid == 0) {
+            if (m < 3.0e38f) atomicMin(out.dt_min, __float_as_uint(m));
+            __threadfence();
+            before = atomicInc(out.done, nr - 1);
+        }
+        if (__shfl_sync(0xffffffffu, before, 0) != nr - 1u) return;
+        __threadfence();
+        // shear limit: |vm_i / R_i - vm_{i+1} / R_{i+1}| with vm = Vref + mean dv
+        const volatile float *mean = out.mean;
+        float shear = 3.0e38f;
+        for (int k = tid; k < nr - 1; k += 32) {
+            const float denom = fabsf(fmaf(-mean[k + 1], t.InvRmed[k + 1],
+                                           fmaf(mean[k], t.InvRmed[k], t.OmRefDiff[k]))) + 1.0e-30f;
+            shear = fminf(shear, ph.cfl * g.dphi / denom);
+        }
+        shear = warp_min_f(shear);
+        if (tid == 0) {
+            const unsigned int u = __float_as_uint(shear);
+            *out.host_dt = __uint_as_float(min(atomicMin(out.dt_min, u), u));
+        }
     }
 }
 

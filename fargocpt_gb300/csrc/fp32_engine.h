@@ -132,6 +132,14 @@ struct StateF {
     float *sigma_lo;  // low part of the compensated sigma (sigma = sigma + sigma_lo)
 };
 
+// what the derived-quantities kernel keeps and leaves beside the fields
+struct CflOut {
+    unsigned int *dt_min;  // the disk's smallest step (float bits)
+    float *mean;           // mean residual v_phi per ring
+    unsigned int *done;    // rings finished (0 between launches)
+    float *host_dt;        // page-locked host memory the step is written to
+};
+
 // Every buffer and constant one disk's step touches, as the batched kernels
 // read it from device memory.  s holds the step-start state (vr, dv buffers
 // A); the source terms write the B buffers, transport writes back to A, so
@@ -152,7 +160,7 @@ struct DiskF {
     // above where the pass works in place, others after the window pass
     float *mom_w[4], *sigma_w, *energy_w, *sigma_lo_w;
     float *pot, *P, *cs, *H, *nu, *T, *Qr, *Qp, *divv, *trr, *tpp, *trp, *qplus, *qminus;
-    unsigned int *dtmin;
+    CflOut cfl;
     int damping, nq;
 };
 
@@ -286,8 +294,9 @@ class Engine32 {
     std::vector<int> host_damp_rings;
     double *partial = nullptr, *red_out = nullptr, *stage = nullptr;
     unsigned int *d_dtmin = nullptr;
+    CflOut cfl_out{};
     unsigned long long *d_bad = nullptr;
-    double *h_pinned = nullptr;
+    double *h_pinned = nullptr;  // 16 (the last: the CFL step) + 5 per body
     int per = 4, az_block = 128;
     size_t az_smem = 0;
     int rb_per = 0;      // register-blocked ring kernel: cells per thread (0: strided)

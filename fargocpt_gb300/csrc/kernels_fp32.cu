@@ -260,20 +260,25 @@ __global__ void f_damping(GeoF g, DampingF dm, float dt, const int *__restrict__
                  blockIdx.z, gridDim.z);
 }
 
-__global__ void f_derived_cfl(GeoF g, TablesF t, PhysF ph, int mode, const float *__restrict__ S,
-                              const float *__restrict__ E, const float *__restrict__ vr,
-                              const float *__restrict__ dv, const float *__restrict__ qplus,
-                              const float *__restrict__ qminus, float *__restrict__ cs,
-                              float *__restrict__ H, float *__restrict__ P, float *__restrict__ T,
-                              float *__restrict__ nu, unsigned int *__restrict__ dt_min,
-                              const float *__restrict__ corr_phi,
-                              const float *__restrict__ corr_r)
+// a block of up to 128 threads per ring, 7 per SM (2048 x 6144 cells: 0.148 ms,
+// with 6 0.164, with 8 0.161, of 256 threads 0.161; one cell per thread and the
+// means of two rings per block 0.227)
+constexpr int kCflThreads = 128;
+__global__ void __launch_bounds__(kCflThreads, 7)
+    f_derived_cfl(GeoF g, TablesF t, PhysF ph, int mode, const float *__restrict__ S,
+                  const float *__restrict__ E, const float *__restrict__ vr,
+                  const float *__restrict__ dv, const float *__restrict__ qplus,
+                  const float *__restrict__ qminus, float *__restrict__ cs,
+                  float *__restrict__ H, float *__restrict__ P, float *__restrict__ T,
+                  float *__restrict__ nu, CflOut out,
+                  const float *__restrict__ corr_phi,
+                  const float *__restrict__ corr_r)
 {
     fgpu::follow_predecessor();
     __shared__ float red[33];
-    __shared__ longlong2 red2[33];
-    derived_cfl_ring(g, t, ph, mode, S, E, vr, dv, qplus, qminus, cs, H, P, T, nu, dt_min,
-                     blockIdx.x, red, red2, corr_phi, corr_r);
+    __shared__ long long redl[33];
+    derived_cfl_ring(g, t, ph, mode, S, E, vr, dv, qplus, qminus, cs, H, P, T, nu, out,
+                     blockIdx.x, red, redl, corr_phi, corr_r);
 }
 
 // disk force on up to kForceBodies32 bodies in one pass over the ring, and the
@@ -931,15 +936,24 @@ int Engine32::create(const fgpu_params &prm, const double *radii, cudaStream_t s
         // ring phases, as parts of one allocation, each from a 256-byte
         // boundary
         const size_t part = (cells * sizeof(float) + 255) / 256 * 256;
-        CKF(cudaMalloc(&mom_mem, (windows ? 11 : 4) * part + sizeof(float2) * (size_t)nr));
+        const size_t rings = ((size_t)(nr + 1) * sizeof(float2) + 255) / 256 * 256;
+        CKF(cudaMalloc(&mom_mem, (windows ? 11 : 4) * part + 2 * rings));
         auto at = [&](int k) { return reinterpret_cast<float *>(mom_mem + k * part); };
         for (int k = 0; k < 4; ++k) mom[k] = at(k);
+        // of the CFL kernel: the count of finished rings, ring means, the step in
+        // host memory
+        char *ring_mem = mom_mem + (windows ? 11 : 4) * part;
+        CKF(cudaMemset(ring_mem, 0, sizeof(unsigned int)));
+        cfl_out.dt_min = d_dtmin;
+        cfl_out.done = reinterpret_cast<unsigned int *>(ring_mem);
+        cfl_out.mean = reinterpret_cast<float *>(ring_mem) + 1;
+        cfl_out.host_dt = reinterpret_cast<float *>(h_pinned + 15);
         if (windows) {
             for (int k = 0; k < 4; ++k) mom_w[k] = at(4 + k);
             sigma_w = at(8);
             sigma_lo_w = at(9);
             energy_w = at(10);
-            ring_phase = reinterpret_cast<float2 *>(mom_mem + 11 * part);
+            ring_phase = reinterpret_cast<float2 *>(mom_mem + 11 * part + rings);
         }
     }
     if (rb_per) {
@@ -1020,7 +1034,7 @@ DiskF Engine32::describe()
     d.trp = fld[FGPU_TAU_R_PHI];
     d.qplus = fld[FGPU_QPLUS];
     d.qminus = fld[FGPU_QMINUS];
-    d.dtmin = d_dtmin;
+    d.cfl = cfl_out;
     d.damping = p.damping && n_rings;
     d.nq = phys.adiabatic ? 5 : 4;
     return d;
@@ -1156,10 +1170,12 @@ int Engine32::derived_cfl(int mode, bool reset)
     if (int rc_ = sync_frame()) return rc_;
     StateF s = state();
     if ((mode & 4) && reset) CKF(cudaMemsetAsync(d_dtmin, 0x7f, sizeof(unsigned int), stream));
-    fgpu::launch(f_derived_cfl, nr, 256, 0, stream, geo, tabs, phys, mode, s.sigma, s.energy, s.vr, s.dv,
+    // a block per ring, a Quad per thread and pass
+    const int threads = std::min(kCflThreads, ((nz + 3) / 4 + 31) / 32 * 32);
+    fgpu::launch(f_derived_cfl, nr, threads, 0, stream, geo, tabs, phys, mode, s.sigma, s.energy, s.vr, s.dv,
                                           fld[FGPU_QPLUS], fld[FGPU_QMINUS], fld[FGPU_SOUNDSPEED],
                                           fld[FGPU_SCALE_HEIGHT], fld[FGPU_PRESSURE],
-                                          fld[FGPU_TEMPERATURE], fld[FGPU_VISCOSITY], d_dtmin,
+                                          fld[FGPU_TEMPERATURE], fld[FGPU_VISCOSITY], cfl_out,
                                           corr_phi, corr_r);
     CKF(cudaGetLastError());
     if (mode & 4) cfl_valid = true;
@@ -1208,11 +1224,9 @@ int Engine32::cfl(double *dt_out)
         int rc = derived_cfl(4);
         if (rc) return rc;
     }
-    CKF(cudaMemcpyAsync(h_pinned, d_dtmin, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
+    // (written there by the kernel that formed it)
     CKF(cudaStreamSynchronize(stream));
-    float f;
-    std::memcpy(&f, h_pinned, sizeof(float));
-    *dt_out = (double)f;
+    *dt_out = (double)*cfl_out.host_dt;
     return FGPU_OK;
 }
 
@@ -1472,7 +1486,7 @@ int Engine32::disk_forces(int n, const double *x, const double *y, const double 
 {
     if (n < 0 || n > kMaxBodies) return FGPU_ERR_BAD_ARG;
     const int rows = nr - 2;
-    double *dev = red_out + 8;
+    double *sums = h_pinned + 16;  // the kernel writes them to page-locked host memory
     for (int b0 = 0; b0 < n; b0 += kForceBodies32) {
         ForceBodies32 fb{};
         fb.n = std::min(kForceBodies32, n - b0);
@@ -1490,13 +1504,11 @@ int Engine32::disk_forces(int n, const double *x, const double *y, const double 
         fgpu::launch(nz % 2 == 0 ? f_disk_force_bodies<true> : f_disk_force_bodies<false>, rows,
                      kForceThreads32, 0, stream, geo, tabs, phys, fb, fld[FGPU_SIGMA], sigma_lo,
                      fld[FGPU_SCALE_HEIGHT], partial, width);
-        fgpu::launch(f_reduce_cols, width, kReduceThreads, 0, stream, partial, rows, width, dev + 5 * b0);
+        fgpu::launch(f_reduce_cols, width, kReduceThreads, 0, stream, partial, rows, width, sums + 5 * b0);
     }
     CKF(cudaGetLastError());
-    CKF(cudaMemcpyAsync(h_pinned + 16, dev, sizeof(double) * 5 * n, cudaMemcpyDeviceToHost,
-                        stream));
     CKF(cudaStreamSynchronize(stream));
-    std::copy(h_pinned + 16, h_pinned + 16 + 5 * n, out);
+    std::copy(sums, sums + 5 * n, out);
     return FGPU_OK;
 }
 

@@ -74,3 +74,40 @@ def test_substeps_at_ring_lengths(naz, adiabatic, art):
     for f in fine + COARSE:
         assert np.array_equal(e.get_field(f), g.get_field(f)), f
     b.close()
+
+
+def sheared(st):
+    # alternating ring speeds: the shear of neighbouring rings limits
+    st["V_AZIMUTHAL"][:] *= 1.0 + 0.9 * (np.arange(len(st["V_AZIMUTHAL"])) % 2)[:, None]
+
+
+@pytest.mark.parametrize("nrad,naz", [(6, 8), (9, 59), (9, 128), (40, 511), (7, 516), (300, 64)])
+@pytest.mark.parametrize("change", [None, sheared])
+@pytest.mark.parametrize("adiabatic,art", [(True, 1), (False, 2)])
+def test_step_limit(nrad, naz, change, adiabatic, art):
+    """The CFL step of the FP32-mixed form (cells, and the shear limit that the last
+    ring to finish takes) against the oracle's to 1e-5, and in a batch bit for bit,
+    for any tile and after the autotuner has run other states through it."""
+    from fargocpt_gb300.abi import params_from_dict
+    from fargocpt_gb300.batch import Batch
+    from fargocpt_gb300.engine import Engine, grid_radii
+    from oracle.oracle_py import OracleState
+
+    params, d = make_params(nrad, naz, adiabatic=adiabatic, art_visc=art)
+    p32 = params_from_dict(dict(d, precision=1))
+    radii = grid_radii(d["radial_spacing"], d["rmin"], d["rmax"], d["nrad"])
+    st = initial_state(d, radii, seed=43, noise=2e-2)
+    if change:
+        change(st)
+    o, g, b = OracleState(params, radii), Engine(p32, radii), Batch([p32], [radii])
+    for x in (o, g, b.disks[0]):
+        load(x, st, BODIES)
+    dt = g.condition_cfl()
+    assert dt == pytest.approx(o.condition_cfl(), rel=1e-5)
+    assert b.disks[0].condition_cfl() == dt
+    b.autotune(reps=1)
+    assert b.disks[0].condition_cfl() == dt
+    g.step_euler(0.1 * dt, 0.0)
+    b.step(np.array([0.1 * dt]), np.zeros(1))
+    assert b.disks[0].condition_cfl() == g.condition_cfl()
+    b.close()
