@@ -47,22 +47,23 @@ KERNEL_BYTES_PER_CELL = {
     "transport_azimuthal": 104, "finish": 80, "damping": 0, "ghost_post": 0,
     "derived_cfl": 88,
 }
+# the float-pair FP64 form's fused kernels: the potential with the source terms,
+# the artificial pressures with their velocity update, the stress tensor with the
+# viscous update; the window azimuthal pass does not read v_phi
+KERNEL_BYTES_PER_CELL_FP64 = dict(KERNEL_BYTES_PER_CELL, potential=0, source=64, artvisc_q=0,
+                                  artvisc_v=96, stress=0, transport_azimuthal=96)
 STEP_BYTES_PER_CELL = {"adiabatic": 64, "isothermal": 48}   # one read + write of the state
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant
 # kernels from one-kernel ncu captures (profiles/ names the capture of each)
 NCU_DRAM_BYTES = {
     # 2048 x 6144 three-planet adiabatic disk (profiles/traffic_c5_transports.md;
     # the FP64 form's float-pair kernels)
-    ("c5", "fp64", "transport_azimuthal"): 713425664 + 602434048,
     ("c5", "fp64", "transport_radial"): 453888256 + 557087488,
-    ("c5", "fp32", "transport_azimuthal"): 402961408 + 288184320,
     ("c5", "fp32", "transport_radial"): 295241216 + 318492928,
-    # 512 x 1536 adiabatic disk (--set full captures)
-    ("c2", "fp64", "transport_azimuthal"): 44.127e6 + 0.422e6,
+    # 512 x 1536 adiabatic disk (--set full capture)
     ("c2", "fp64", "transport_radial"): 25.252e6 + 0.738e6,
-    ("c2", "fp32", "transport_azimuthal"): 25.286e6 + 0.0005e6,
 }
-STEP_KERNELS = 13   # the adiabatic step's kernels (the force adds two per 4 bodies)
+STEP_KERNELS = 10   # the float-pair step's kernels (the force adds two per 4 bodies)
 
 
 def parse():
@@ -410,7 +411,9 @@ def roofline(res, steps, bytes_scale, form, cfg_name):
     phases, nsteps, cells, d = res["phases"], res["nsteps"], res["cells"], res["d"]
     dom = max(phases, key=phases.get)
     dom_ms = phases[dom] / max(1, nsteps)
-    bpc = KERNEL_BYTES_PER_CELL.get(dom, 0) * bytes_scale
+    pairs = form == "fp64" and os.environ.get("FARGO_GB300_FP64_ARITH") != "fp64"
+    table = KERNEL_BYTES_PER_CELL_FP64 if pairs else KERNEL_BYTES_PER_CELL
+    bpc = table.get(dom, 0) * bytes_scale
     achieved = bpc * cells / (dom_ms * 1e-3) / 1e9
     kind = "adiabatic" if d["eos"] == 1 else "isothermal"
     sbpc = STEP_BYTES_PER_CELL[kind] * bytes_scale
@@ -420,7 +423,7 @@ def roofline(res, steps, bytes_scale, form, cfg_name):
     per_kernel = {}
     for k, tot in phases.items():
         ms = tot / max(1, nsteps)
-        b = KERNEL_BYTES_PER_CELL.get(k, 0) * bytes_scale
+        b = table.get(k, 0) * bytes_scale
         if ms > 0 and b > 0:
             gbs = b * cells / (ms * 1e-3) / 1e9
             per_kernel[k] = {"ms": ms, "bytes_per_cell": b, "achieved_gbs": gbs,
@@ -513,12 +516,11 @@ def main():
     value = world * cells * args.steps / (vals[0] * 1e-3)
     e2e = world * cells * args.steps / vals[1]
     rl, rls = roofline(r64, args.steps, 1.0, "fp64", args.config)
-    # what bounds the float-pair transports (ncu --set full on 512 rings of
-    # 6144 cells, profiles/transport_kernels_c5_fp64_pair.md): issue, the
-    # FP64 pipe and latency, not DRAM
+    # what bounds the float-pair transports (ncu on 512 rings of 6144 cells,
+    # profiles/step_kernels_c5s.md): issue, the FP32 pipe and latency, not DRAM
     rl["ncu_pipes_pct"] = {
-        "transport_azimuthal": {"issue_active": 53.4, "fp64_pipe": 54.5, "fma_pipe": 26.4},
-        "transport_radial": {"issue_active": 58.8, "fp64_pipe": 42.7, "fma_pipe": 31.6}}
+        "transport_azimuthal": {"issue_active": 60.1, "fp64_pipe": 12.0, "fma_pipe": 72.3},
+        "transport_radial": {"issue_active": 60.3, "fp64_pipe": 33.5, "fma_pipe": 33.7}}
     fp32 = None
     if r32 is not None:
         value32 = world * cells * args.steps / (vals[2] * 1e-3)

@@ -586,11 +586,6 @@ static bool is_cell_kernel(int k)
            k == FGPU_BK_ARTVISC_V || k == FGPU_BK_STRESS || k == FGPU_BK_VISCOUS ||
            k == FGPU_BK_FINISH;
 }
-static bool is_ring_kernel(int k)
-{
-    return k == FGPU_BK_TRANSPORT_AZIMUTHAL || k == FGPU_BK_DAMPING || k == FGPU_BK_DERIVED_CFL;
-}
-
 static const int kPerChoices[] = {1, 2, 3, 4, 6, 8, 12, 16};
 
 static int per_for(int nz_max, int threads)
@@ -675,9 +670,10 @@ struct fgpu_batch {
     int graph_steps = 0;
 
     // FGPU_BATCH_PERSISTENT: the two substep sequences as cooperative
-    // launches of seq_threads threads (measured on the 64-disk sweep: 5.86 ms
-    // per step with 128, 6.26 with 256, 8.79 with 512, against 3.80 with one
-    // launch per substep); their tile tables and grids
+    // launches of seq_threads threads (measured on the 64-disk sweep: 4.26 ms
+    // per step with 128, against 2.32 with one launch per substep; with one cell
+    // per thread 5.86, with 256 threads 6.26, with 512 8.79); their tile tables
+    // and grids
     int mode = FGPU_BATCH_LAUNCHES;
     static constexpr int seq_threads = 128;
     int *d_seq_tables = nullptr;  // FGPU_BK_COUNT tables of nd + 1 tile starts

@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kForceThreads32, 8)
     }
     __syncthreads();
     const float2 m = mean;
-    // cell centres and the bodies as float pairs (see potential_cell): the
+    // cell centres and the bodies as float pairs (see potential_cells): the
     // distance loses nothing to cancellation near a body
     float pxh[kForceBodies32], pxl[kForceBodies32], pyh[kForceBodies32], pyl[kForceBodies32];
     float frsm[kForceBodies32];

@@ -1778,9 +1778,6 @@ __global__ void __launch_bounds__(256, PAIR ? 4 : 3) k_derived_cfl(Geo g, Tables
         vm0 = block_sum(p0, red) / (double)nz;
         vm1 = block_sum(p1, red) / (double)nz;
     }
-    const double dxR = t.Rsup[i] - t.Rinf[i];
-    const double dxA = t.Rmed[i] * g.dphi;
-    const double cell = dxR < dxA ? dxR : dxA;
     double local = 1.0e300;
     if (do_cfl && i == 0) {
         const double denom = fabs(vm0 * t.InvRmed[0] - vm1 * t.InvRmed[1]) + 1.0e-100;
