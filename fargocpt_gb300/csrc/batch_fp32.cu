@@ -671,7 +671,7 @@ struct fgpu_batch {
 
     // FGPU_BATCH_PERSISTENT: the two substep sequences as cooperative
     // launches of seq_threads threads (measured on the 64-disk sweep: 4.26 ms
-    // per step with 128, against 2.32 with one launch per substep; with one cell
+    // per step with 128, against 2.23 with one launch per substep; with one cell
     // per thread 5.86, with 256 threads 6.26, with 512 8.79); their tile tables
     // and grids
     int mode = FGPU_BATCH_LAUNCHES;
