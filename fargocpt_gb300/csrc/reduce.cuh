@@ -169,10 +169,16 @@ __device__ __forceinline__ void block_compensated_rows(const double *__restrict_
         sums[1][warp] = c;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < kReduceThreads / 32; ++k)
-            add_compensated(s, c, sums[0][k], sums[1][k]);
-        out[w] = s - c;
+    if (warp == 0) {
+        constexpr int warps = kReduceThreads / 32;
+        s = lane < warps ? sums[0][lane] : 0.0;
+        c = lane < warps ? sums[1][lane] : 0.0;
+        for (int o = warps / 2; o > 0; o >>= 1) {
+            const double s2 = __shfl_down_sync(0xffffffffu, s, o);
+            const double c2 = __shfl_down_sync(0xffffffffu, c, o);
+            add_compensated(s, c, s2, c2);
+        }
+        if (lane == 0) out[w] = s - c;
     }
 }
 
