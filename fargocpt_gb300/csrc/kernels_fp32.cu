@@ -323,6 +323,12 @@ __global__ void __launch_bounds__(kForceThreads32, 8)
         if (EVEN) return *reinterpret_cast<const float2 *>(p + j);
         return make_float2(p[j], j + 1 < nz ? p[j + 1] : rest);
     };
+    // the same, the ring's last cell again past its end: a place and a smoothing
+    // of a real cell, whose distance to a body is not zero
+    auto load_place = [&](const float *p, int j) {
+        if (EVEN) return *reinterpret_cast<const float2 *>(p + j);
+        return make_float2(p[j], p[min(j + 1, nz - 1)]);
+    };
     // sum += x, compensated (TwoSum, Knuth 1969)
     auto add = [](fgpu::f2x2 &sum, float2 x) {
         const fgpu::f2x2 s = fgpu::two_sum(sum.h, x);
@@ -364,11 +370,11 @@ __global__ void __launch_bounds__(kForceThreads32, 8)
     const float2 eps = both(ph.eps_smooth);
 #pragma unroll 2
     for (int j = 2 * threadIdx.x; j < nz; j += 2 * kForceThreads32) {
-        const float2 ch = load(t.cosHi, j, 0.f), cl = load(t.cosLo, j, 0.f);
-        const float2 sh = load(t.sinHi, j, 0.f), sl = load(t.sinLo, j, 0.f);
+        const float2 ch = load_place(t.cosHi, j), cl = load_place(t.cosLo, j);
+        const float2 sh = load_place(t.sinHi, j), sl = load_place(t.sinLo, j);
         // (the cell past the ring's end: sigma at the mean, its terms zero)
         const float2 sg = load(S + row, j, m.x), sg_lo = load(S_lo + row, j, m.y);
-        const float2 sm = vmul(eps, load(H + row, j, 1.f));
+        const float2 sm = vmul(eps, load_place(H + row, j));
         const float2 sm2 = vmul(sm, sm);
         const float2 xh = vmul(rh, ch), yh = vmul(rh, sh);
         const float2 xl = vadd(vfma(rh, ch, fgpu::vneg(xh)), vfma(rh, cl, vmul(rl, ch)));

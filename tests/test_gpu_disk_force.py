@@ -44,3 +44,36 @@ def test_force_at_block_edges(nrad, naz, nbodies, mean):
         got = np.array(g.disk_on_nbody_accel(nbodies)).reshape(want.shape)
         err = np.hypot(*(got - want).T) / size
         assert np.all(err <= bar), (precision, err)
+
+
+@pytest.mark.parametrize("naz", [8, 59, 257])
+@pytest.mark.parametrize("mean", [0, 1])
+def test_force_without_smoothing(naz, mean):
+    """ThicknessSmoothing 0: the force on the central object, at the origin, where
+    only a cell's own distance keeps the inverse cube finite, also in the lane of
+    an odd ring that lacks its second cell.  Bars, of the sum of the terms'
+    magnitudes (a smooth disk's cancel to a thousandth of it): 1e-12 and 1e-6,
+    some ten roundings of a pair (2^-46) and of a float (2^-24)."""
+    from fargocpt_gb300.abi import params_from_dict
+    from fargocpt_gb300.engine import Engine, grid_radii
+    from oracle.oracle_py import OracleState
+
+    params, d = make_params(9, naz, adiabatic=True, thickness_smoothing=0.0,
+                            correct_disk_selfgravity=mean)
+    radii = np.asarray(grid_radii(d["radial_spacing"], d["rmin"], d["rmax"], d["nrad"]))
+    st = initial_state(d, radii, seed=5, noise=0.2)
+    bodies = [STAR, (0.1, 0.05, 1e-3, 0.0, math.hypot(0.1, 0.05))]
+    o = OracleState(params, radii)
+    load(o, st, bodies)
+    want = np.array([o.disk_on_planet_accel(k) for k in range(2)])
+    lo, hi = radii[:9, None], radii[1:10, None]
+    mid, phi = 2 / 3 * (hi ** 3 - lo ** 3) / (hi ** 2 - lo ** 2), 2 * np.pi * np.arange(naz) / naz
+    term = (np.pi / naz * (hi ** 2 - lo ** 2) * st["SIGMA"])[1:-1]
+    size = np.array([(term / np.abs(mid * np.exp(1j * phi) - complex(x, y))[1:-1] ** 2).sum()
+                     for x, y, *_ in bodies])
+    for precision, bar in ((0, 1e-12), (1, 1e-6)):
+        g = Engine(params_from_dict(dict(d, precision=precision)), radii)
+        load(g, st, bodies)
+        got = np.array(g.disk_on_nbody_accel(2)).reshape(want.shape)
+        err = np.hypot(*(got - want).T) / size
+        assert np.all(err <= bar), (precision, err)
