@@ -1975,14 +1975,14 @@ __device__ __forceinline__ void finish_cells(
     if (ph.adiabatic) q.store(E_out, row, e);
 }
 
-// damping zones (damping.cpp:311-776); block-wide over ring i
+// damping zones (damping.cpp:311-776); block-wide over ring i, part of parts
+// blocks that share its columns (the mean kind: one block)
 // red: 33 floats, redl: 33 long longs (shared memory)
 __device__ __forceinline__ void damp_ring_f(float *X, float *X0, const DampQF &d, int i, int nz,
                                             int outer, float dt, float *red, float *Xlo,
                                             long long *redl, int part, int parts)
 {
     const int kind = outer ? d.kind_out : d.kind_in;
-    if (kind == 3 && part > 0) return;  // the whole block
     const size_t row = (size_t)i * nz;
     float x0c = 0.f;
     if (kind == 3) {
@@ -1995,11 +1995,9 @@ __device__ __forceinline__ void damp_ring_f(float *X, float *X0, const DampQF &d
     const float factor = outer ? d.fac_out[i] : d.fac_in[i];
     const float tau = outer ? d.tau_out : d.tau_in;
     const float ef = __expf(-dt * factor / tau);
-    // a ring's blocks share its columns (the mean kind's one block takes them
-    // all), four loads of each thread in flight
-    const int step = kind == 3 ? blockDim.x : blockDim.x * parts;
-    const int first = kind == 3 ? threadIdx.x : part * blockDim.x + threadIdx.x;
-    for (int j = first; j < nz; j += 4 * step) {
+    // four loads of each thread in flight
+    const int step = blockDim.x * parts;
+    for (int j = part * blockDim.x + threadIdx.x; j < nz; j += 4 * step) {
         float x[4], x0[4], lo[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -2032,10 +2030,17 @@ __device__ __forceinline__ void damping_ring(const GeoF &g, const DampingF &dm, 
         const DampQF &d = dm.q[q];
         const int size = d.vector ? nr + 1 : nr;
         float *lo = q == 2 ? s.sigma_lo : nullptr;
-        if (d.kind_in != 0 && d.active_in && i <= d.limit_in)
-            damp_ring_f(X[q], X0[q], d, i, nz, 0, dt, red, lo, redl, part, parts);
-        if (d.kind_out != 0 && d.active_out && i >= d.limit_out && i < size)
-            damp_ring_f(X[q], X0[q], d, i, nz, 1, dt, red, lo, redl, part, parts);
+        const bool in = d.kind_in != 0 && d.active_in && i <= d.limit_in;
+        const bool out = d.kind_out != 0 && d.active_out && i >= d.limit_out && i < size;
+        // a ring mean, the ring's other damping (on a narrow disk the zones
+        // overlap) before or after it: one block, or one would read what another
+        // writes.  The other kinds leave each column to one thread, inner edge
+        // first.
+        const bool alone = (in && d.kind_in == 3) || (out && d.kind_out == 3);
+        if (alone && part > 0) continue;
+        const int p = alone ? 0 : part, of = alone ? 1 : parts;
+        if (in) damp_ring_f(X[q], X0[q], d, i, nz, 0, dt, red, lo, redl, p, of);
+        if (out) damp_ring_f(X[q], X0[q], d, i, nz, 1, dt, red, lo, redl, p, of);
     }
 }
 

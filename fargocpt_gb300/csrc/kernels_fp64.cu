@@ -1520,17 +1520,17 @@ __global__ void k_finish(Geo g, Tables t, Phys ph, double omf, const double *__r
 // ring of the damping zones; the "mean" kind writes X0(ring, 0) like the
 // reference does.
 // ---------------------------------------------------------------------------
+// part of parts blocks share the ring's columns (the mean kind: one block)
 __device__ void damp_ring(double *X, double *X0, const DampQ &d, int i, int nz, int outer,
-                          double dt, double *red)
+                          double dt, double *red, int part, int parts)
 {
     const int kind = outer ? d.kind_out : d.kind_in;
-    if (kind == 3 && blockIdx.z > 0) return;  // the whole block
     const size_t row = (size_t)i * nz;
     double x0c = 0.0;
     if (kind == 3) {
-        double part = 0.0;
-        for (int j = threadIdx.x; j < nz; j += blockDim.x) part += X[row + j];
-        const double mean = block_sum(part, red) / nz;
+        double sum = 0.0;
+        for (int j = threadIdx.x; j < nz; j += blockDim.x) sum += X[row + j];
+        const double mean = block_sum(sum, red) / nz;
         if (threadIdx.x == 0) X0[row] = mean;
         x0c = mean;
     } else if (kind == 2) {
@@ -1543,11 +1543,9 @@ __device__ void damp_ring(double *X, double *X0, const DampQ &d, int i, int nz, 
     if (threadIdx.x == 0) red[0] = exp(-dt * factor / tau);
     __syncthreads();
     const double ef = red[0];
-    // the blocks of a ring share its columns (the mean kind's one block takes
-    // them all), four loads of each thread in flight
-    const int step = kind == 3 ? blockDim.x : blockDim.x * gridDim.z;
-    const int first = kind == 3 ? threadIdx.x : blockIdx.z * blockDim.x + threadIdx.x;
-    for (int j = first; j < nz; j += 4 * step) {
+    // four loads of each thread in flight
+    const int step = blockDim.x * parts;
+    for (int j = part * blockDim.x + threadIdx.x; j < nz; j += 4 * step) {
         double x[4], x0[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -1575,12 +1573,16 @@ __global__ void k_damping(Geo g, Damping dm, double dt, const int *__restrict__ 
     double *X0[4] = {s.vr0, s.vaz0, s.sigma0, s.energy0};
     const DampQ &d = dm.q[q];
     const int size = d.vector ? nr + 1 : nr;
-    if (d.kind_in != 0 && d.active_in && i <= d.limit_in) {
-        damp_ring(X[q], X0[q], d, i, nz, 0, dt, red);
-    }
-    if (d.kind_out != 0 && d.active_out && i >= d.limit_out && i < size) {
-        damp_ring(X[q], X0[q], d, i, nz, 1, dt, red);
-    }
+    const bool in = d.kind_in != 0 && d.active_in && i <= d.limit_in;
+    const bool out = d.kind_out != 0 && d.active_out && i >= d.limit_out && i < size;
+    // a ring mean, the ring's other damping (on a narrow disk the zones overlap)
+    // before or after it: one block, or one would read what another writes.  The
+    // other kinds leave each column to one thread, inner edge first.
+    const bool alone = (in && d.kind_in == 3) || (out && d.kind_out == 3);
+    if (alone && blockIdx.z > 0) return;
+    const int part = alone ? 0 : blockIdx.z, parts = alone ? 1 : gridDim.z;
+    if (in) damp_ring(X[q], X0[q], d, i, nz, 0, dt, red, part, parts);
+    if (out) damp_ring(X[q], X0[q], d, i, nz, 1, dt, red, part, parts);
 }
 
 // ---------------------------------------------------------------------------
