@@ -37,16 +37,19 @@ struct fgpu_engine {
 
     double *field[FGPU_FIELD_COUNT] = {};
     double *sigma_alt = nullptr, *vr_alt = nullptr, *vaz_alt = nullptr, *energy_alt = nullptr;
-    char *mom_mem = nullptr;  // the momenta and ring phases below
+    char *mom_mem = nullptr;  // the buffers between the passes, and the ring values below
+    // the radial pass's momenta; in the pair form, whose azimuthal pass works out of
+    // place, the alternate velocities stand in for the first two, and its own
+    // momenta, sigma and energy are the others (the isothermal disk's sigma: the
+    // alternate energy).  A step thus ends on the buffers it began with.
     double *mom[4] = {};
-    double *mom_t[4] = {};  // pair form: the azimuthal pass's momenta (mom: the radial pass's)
+    double *mom_t[4] = {}, *sigma_t = nullptr, *energy_t = nullptr;
     double *ring_ws = nullptr;
     RingPhase *ring_phase = nullptr;  // pair form: the azimuthal pass's constants per ring
     size_t az_smem = 0;
     int az_block = 256;
     double *ring_mean = nullptr;    // pair form: mean v_phi per ring, for the CFL kernel
     unsigned *cfl_done = nullptr;   // blocks of the CFL kernel that have finished
-    bool dt_arrived = false;        // the last CFL step has reached h_pinned[kHostDt]
     bool pair_arith = true;  // the kernels' arithmetic in float pairs (else FP64)
     // div v and the stress tensor hold the stress kernel's float pairs
     // (stress_as_pairs), the artificial pressures those of the float-pair
@@ -1018,22 +1021,28 @@ static int create_engine(const fgpu_params *params, const double *radii, cudaStr
     // fewer rings, shorter ones give more blocks
     eng->radial_chunk = radial_chunk_for(eng->pair_arith, eng->ph.adiabatic, eng->nr, eng->nz);
     {
-        // the transported momenta (a second set in the pair form, whose
-        // azimuthal pass works out of place) and the ring phases, as parts of
-        // one allocation, each from a 256-byte boundary
-        const int sets = eng->pair_arith ? 2 : 1;
-        const size_t part = (eng->cells * sizeof(double) + 255) / 256 * 256;
+        // the buffers between the transport's passes, of v_r's size (the gas kick
+        // passes velocities through two of them), and the ring values, as parts
+        // of one allocation, each from a 256-byte boundary
+        const int parts = !eng->pair_arith ? 4 : eng->ph.adiabatic ? 8 : 6;
+        const size_t part = (eng->vcells * sizeof(double) + 255) / 256 * 256;
         const size_t per_ring = sizeof(RingPhase) + sizeof(double);
-        if (cudaMalloc(&eng->mom_mem, 4 * sets * part + per_ring * (size_t)eng->nr) !=
+        if (cudaMalloc(&eng->mom_mem, parts * part + per_ring * (size_t)eng->nr) !=
             cudaSuccess) {
             eng->err = "out of device memory (momenta)";
             return fail(FGPU_ERR_OOM);
         }
-        for (int k = 0; k < 4; ++k) {
-            eng->mom[k] = reinterpret_cast<double *>(eng->mom_mem + k * part);
-            if (sets == 2) eng->mom_t[k] = reinterpret_cast<double *>(eng->mom_mem + (4 + k) * part);
+        auto at = [&](int k) { return reinterpret_cast<double *>(eng->mom_mem + k * part); };
+        if (eng->pair_arith) {
+            eng->mom[2] = at(0);
+            eng->mom[3] = at(1);
+            for (int k = 0; k < 4; ++k) eng->mom_t[k] = at(2 + k);
+            eng->sigma_t = eng->ph.adiabatic ? at(6) : eng->energy_alt;
+            eng->energy_t = eng->ph.adiabatic ? at(7) : nullptr;
+        } else {
+            for (int k = 0; k < 4; ++k) eng->mom[k] = at(k);
         }
-        eng->ring_phase = reinterpret_cast<RingPhase *>(eng->mom_mem + 4 * sets * part);
+        eng->ring_phase = reinterpret_cast<RingPhase *>(eng->mom_mem + parts * part);
         eng->ring_mean = reinterpret_cast<double *>(eng->ring_phase + eng->nr);
     }
     if (!eng->pair_arith) {
@@ -1402,12 +1411,8 @@ extern "C" int fgpu_condition_cfl(fgpu_engine *eng, double *dt_out)
         if (rc) return rc;
         eng->cfl_valid = true;
     }
-    // the step is written to the host by the kernel that formed it; a call that
-    // waited for the stream since then has already brought it
-    if (!eng->dt_arrived) {
-        CK(cudaStreamSynchronize(eng->stream));
-        eng->dt_arrived = true;
-    }
+    // the step is written to the host by the kernel that formed it
+    CK(cudaStreamSynchronize(eng->stream));
     *dt_out = eng->h_pinned[kHostDt];
     return FGPU_OK;
 }
@@ -1446,7 +1451,6 @@ static void derived_cfl(fgpu_engine *eng, const Launch &L, int mode)
             cudaMemcpyAsync(eng->h_pinned + kHostDt, eng->d_dtmin, sizeof(double),
                             cudaMemcpyDeviceToHost, eng->stream);
     }
-    if (cfl) eng->dt_arrived = false;
 }
 
 // The centre-of-mass composite: its damping runs after the regular damping
@@ -1655,32 +1659,46 @@ static void gas_kick(fgpu_engine *eng, double dt, double t)
     const double omf = eng->bodies.omega_frame;
     double **f = eng->field;
     const bool adi = eng->ph.adiabatic;
+    const bool art = adi || eng->ph.art_visc_sn || eng->ph.art_visc_tw;
+    State s = state_of(eng);
+    // passes that write the velocities out of place: the last of them into the
+    // alternate buffers, so that a step (whose transport writes them back) ends
+    // where it began; passes before it go through those buffers or, where that
+    // would not come out, through two of the transport's
+    int passes = 1 + (L.pair && art) + stress_as_pairs(L);
+    double *vr_out = nullptr, *vaz_out = nullptr;
+    auto next_velocities = [&] {
+        const bool alt = --passes % 2 == 0, home = s.vr != f[FGPU_V_RADIAL];
+        vr_out = alt ? eng->vr_alt : home ? f[FGPU_V_RADIAL] : eng->mom_t[0];
+        vaz_out = alt ? eng->vaz_alt : home ? f[FGPU_V_AZIMUTHAL] : eng->mom_t[1];
+    };
+    auto take_velocities = [&] {
+        s.vr = vr_out;
+        s.vaz = vaz_out;
+    };
+    next_velocities();
     // CalculateNbodyPotential (simulation.cpp:170-174) and
     // update_with_sourceterms (:190), momentum updates
     if (L.pair && eng->bodies.star_plain) {
         // one kernel for both, timed as the source phase
         mark(eng, 0);
-        launch_source_window(L, dt, omf, eng->bodies, state_of(eng), eng->vr_alt, eng->vaz_alt);
+        launch_source_window(L, dt, omf, eng->bodies, s, vr_out, vaz_out);
     } else {
-        launch_potential(L, eng->bodies, f[FGPU_SCALE_HEIGHT], f[FGPU_POTENTIAL]);
+        launch_potential(L, eng->bodies, s.H, s.pot);
         mark(eng, 0);
-        launch_source(L, dt, omf, f[FGPU_SIGMA], f[FGPU_PRESSURE], f[FGPU_POTENTIAL],
-                      f[FGPU_V_RADIAL], f[FGPU_V_AZIMUTHAL], eng->vr_alt, eng->vaz_alt);
+        launch_source(L, dt, omf, s.sigma, s.P, s.pot, s.vr, s.vaz, vr_out, vaz_out);
     }
-    std::swap(f[FGPU_V_RADIAL], eng->vr_alt);
-    std::swap(f[FGPU_V_AZIMUTHAL], eng->vaz_alt);
+    take_velocities();
     mark(eng, 1);
-    State s = state_of(eng);
     // compression heating + artificial viscosity (simulation.cpp:190-194)
-    if (adi || eng->ph.art_visc_sn || eng->ph.art_visc_tw) {
+    if (art) {
         if (L.pair) {
             // one kernel for both, timed as the second
             if (eng->ph.art_visc_sn || eng->ph.art_visc_tw) eng->q_pairs = true;
             mark(eng, 2);
-            launch_artvisc_pair(L, dt, s, eng->vr_alt, eng->vaz_alt);
-            std::swap(f[FGPU_V_RADIAL], eng->vr_alt);
-            std::swap(f[FGPU_V_AZIMUTHAL], eng->vaz_alt);
-            s = state_of(eng);
+            next_velocities();
+            launch_artvisc_pair(L, dt, s, vr_out, vaz_out);
+            take_velocities();
         } else {
             launch_artvisc_q(L, dt, s.sigma, s.vr, s.vaz, s.energy, s.qr, s.qphi);
             mark(eng, 2);
@@ -1698,15 +1716,15 @@ static void gas_kick(fgpu_engine *eng, double dt, double t)
     if (eng->stress_pairs) {
         // one kernel for both, timed as the viscous phase
         mark(eng, 4);
-        launch_viscous_pair(L, dt, beta_inv_at(eng->p, t), adi ? 7 : 1, s, eng->vr_alt,
-                            eng->vaz_alt);
-        std::swap(f[FGPU_V_RADIAL], eng->vr_alt);
-        std::swap(f[FGPU_V_AZIMUTHAL], eng->vaz_alt);
+        next_velocities();
+        launch_viscous_pair(L, dt, beta_inv_at(eng->p, t), adi ? 7 : 1, s, vr_out, vaz_out);
     } else {
         launch_stress(L, s.sigma, s.vr, s.vaz, s.nu, s.divv, s.trr, s.tpp, s.trp);
         mark(eng, 4);
         launch_viscous(L, dt, beta_inv_at(eng->p, t), adi ? 7 : 1, s);
     }
+    std::swap(f[FGPU_V_RADIAL], eng->vr_alt);
+    std::swap(f[FGPU_V_AZIMUTHAL], eng->vaz_alt);
     mark(eng, 5);
 }
 
@@ -1717,20 +1735,20 @@ static void transport(fgpu_engine *eng, double dt)
     const double omf = eng->bodies.omega_frame;
     double **f = eng->field;
     State s = state_of(eng);
+    if (L.pair) {
+        // the alternate velocities, which the rebuild writes last
+        eng->mom[0] = eng->vr_alt;
+        eng->mom[1] = eng->vaz_alt;
+    }
     launch_transport_radial(L, dt, omf, eng->radial_chunk, s.sigma, s.vr, s.vaz, s.energy,
                             eng->mom, eng->energy_alt, eng->sigma_alt, eng->ring_phase);
     mark(eng, 7);
     if (L.pair) {
-        // out of place: into the state's sigma and energy, which the radial
-        // pass was the last to read; the rebuild writes back to the others
         launch_transport_azimuthal_pair(L, eng->mom, eng->energy_alt, eng->sigma_alt, s.vaz,
-                                        eng->mom_t, s.energy, s.sigma, eng->ring_phase);
+                                        eng->mom_t, eng->energy_t, eng->sigma_t, eng->ring_phase);
         mark(eng, 8);
-        launch_finish(L, omf, eng->mom_t, s.sigma, s.energy, s.vr, eng->vr_alt, eng->vaz_alt,
-                      eng->sigma_alt, eng->energy_alt, eng->ring_phase);
-        std::swap(f[FGPU_SIGMA], eng->sigma_alt);
-        // the isothermal step leaves the energy field alone
-        if (eng->ph.adiabatic) std::swap(f[FGPU_ENERGY], eng->energy_alt);
+        launch_finish(L, omf, eng->mom_t, eng->sigma_t, eng->energy_t, s.vr, eng->vr_alt,
+                      eng->vaz_alt, s.sigma, s.energy, eng->ring_phase);
     } else {
         launch_transport_azimuthal(L, dt, eng->az_block, eng->mom, eng->energy_alt,
                                    eng->sigma_alt, s.vaz, eng->ring_ws, eng->az_smem);
@@ -1831,7 +1849,6 @@ extern "C" int fgpu_disk_on_planet_accel(fgpu_engine *eng, int k, double accel[2
     int rc = check_launch(eng);
     if (rc) return rc;
     CK(cudaStreamSynchronize(eng->stream));
-    eng->dt_arrived = true;
     accel[0] = eng->h_pinned[0] + eng->h_pinned[2];
     accel[1] = eng->h_pinned[1] + eng->h_pinned[3];
     return FGPU_OK;
@@ -1861,7 +1878,6 @@ extern "C" int fgpu_disk_on_nbody_accel(fgpu_engine *eng, double *accel)
         int rc = check_launch(eng);
         if (rc) return rc;
         CK(cudaStreamSynchronize(eng->stream));
-        eng->dt_arrived = true;
         std::copy(eng->h_pinned + 16, eng->h_pinned + 16 + 5 * n, sums);
     }
     for (int k = 0; k < n; ++k) {

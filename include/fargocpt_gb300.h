@@ -245,7 +245,9 @@ int fgpu_create(const fgpu_params *params, const double *radii,
 		fgpu_engine **out);
 int fgpu_destroy(fgpu_engine *eng);
 const char *fgpu_last_error(const fgpu_engine *eng);
-/* CUDA stream (cudaStream_t) that orders all work of the handle. */
+/* CUDA stream (cudaStream_t) that orders all work of the handle.  A
+ * fgpu_step_euler captured from it into a CUDA graph may be launched again: a
+ * step uses the same buffers every time. */
 int fgpu_get_stream(const fgpu_engine *eng, void **stream);
 
 /* Host <-> device copies of whole fields; rows must be the field's row count
