@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kForceThreads32, 8)
         add(sum, load(S + row, j, 0.f));
         sum.l = vadd(sum.l, load(S_lo + row, j, 0.f));
     }
-    const double ring_sum = block_pair_sum(fgpu::pair_halves(sum), part);
+    const double ring_sum = block_pair_sum(sum, part);
     if (threadIdx.x == 0) {
         const double sigma1d = ph.correct_sg ? ring_sum / nz : 0.0;
         const float h = (float)sigma1d;

@@ -156,3 +156,23 @@ def test_disk_on_nbody_accel_matches_per_body_calls(precision):
     assert len(all_at_once) == len(bodies)
     for k in range(len(bodies)):
         assert all_at_once[k] == e.disk_on_planet_accel(k)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("naz", [60, 255, 256])
+def test_total_mass_keeps_small_cells_beside_a_large_one(precision, naz):
+    """Rings of one cell 1 + 2^-25 and others of 1.5 2^-50: added across a block
+    as float pairs, the low part of the large cell would swallow the others (2e-15 to
+    4e-15 of the mass).  Bar: 1e-15, a few FP64 roundings."""
+    from fargocpt_gb300.abi import params_from_dict
+    from fargocpt_gb300.engine import Engine, grid_radii
+
+    _, d = make_params(9, naz)
+    radii = np.asarray(grid_radii(d["radial_spacing"], d["rmin"], d["rmax"], d["nrad"]))
+    sigma = np.full((9, naz), 1.5 * 2.0 ** -50)
+    sigma[:, 0] = 1.0 + 2.0 ** -25
+    g = Engine(params_from_dict(dict(d, precision=precision)), radii)
+    g.set_field("SIGMA", sigma)
+    area = np.pi * (radii[1:10] ** 2 - radii[:9] ** 2) / naz
+    want = math.fsum(a * math.fsum(row) for a, row in zip(area[1:-1], sigma[1:-1]))
+    assert g.total_mass() == pytest.approx(want, rel=1e-15, abs=0.0)
