@@ -96,3 +96,26 @@ def sheared(st):
 def test_step_of_other_limits(change, naz, art):
     o, g = pair(24, naz, change, adiabatic=True, art_visc=art)
     check(o, g, True)
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -46, 2.0 ** 100])
+@pytest.mark.parametrize("art", [1, 2])
+def test_step_near_the_ends_of_the_pairs_range(scale, art):
+    """Sigma and energy near the smallest and the largest values a float pair holds
+    (2^-74, 2^126), the limit in one cell's heating: the bound in front of the pairs,
+    formed from truncated values, lets that cell through."""
+    def scaled(st):
+        for f in ("SIGMA", "ENERGY"):
+            st[f] *= scale
+
+    o, g = pair(24, 90, scaled, adiabatic=True, art_visc=art)
+    heat = np.zeros((24, 90))
+    cool = 0.125 * o.get_field("ENERGY")
+    heat[9, 31] = 4.0e4 * cool[9, 31]
+    for b in (o, g):
+        b.set_field("QPLUS", heat)
+        b.set_field("QMINUS", cool)
+    dt = check(o, g, True)
+    heat[9, 31] = 0.0
+    o.set_field("QPLUS", heat)
+    assert o.condition_cfl() > 1.5 * dt  # (the cell does limit)
