@@ -309,6 +309,45 @@ __global__ void __launch_bounds__(PER <= 4 ? 384 : 512, PER <= 4 ? 2 : 1)
     }
 }
 
+// the register-blocked ring transport (azimuthal_ring_rb, with
+// FARGO_GB300_AZIMUTHAL=blocked<PER>) over the rings of one group of disks with
+// the same ring length nz = PER x blockDim.x and quantity count; start holds only
+// the group's disks' rings
+template <int PER, int NQ>
+__global__ void __launch_bounds__(rb_max_threads(PER))
+    b_transport_azimuthal_rb(const DiskF *__restrict__ D, const StepF *__restrict__ S,
+                             const int *__restrict__ start, int nd)
+{
+    extern __shared__ __align__(16) float smf[];
+    __shared__ float redf[33];
+    __shared__ long long redl[33];
+    const int total = __ldg(start + nd);
+    for (int item = blockIdx.x; item < total; item += gridDim.x) {
+        const int d = disk_of(start, nd, item);
+        if (!S[d].run) continue;
+        const DiskF &k = D[d];
+        const int i = item - __ldg(start + d);
+        azimuthal_ring_rb<PER, NQ>(k.g, k.t, S[d].dt, k.ph.limiter_mc, k.ph.fast_transport,
+                                   k.dv_b, k.mom[0], k.mom[1], k.mom[2], k.mom[3], k.energy_t,
+                                   k.sigma_t, k.sigma_lo_t, i, smf, redf, redl,
+                                   k.ring_shift);
+    }
+}
+
+typedef void (*AzRbFn)(const DiskF *, const StepF *, const int *, int);
+template <int NQ>
+static AzRbFn az_rb_fn_nq(int per)
+{
+    switch (per) {
+    case 4: return b_transport_azimuthal_rb<4, NQ>;
+    case 8: return b_transport_azimuthal_rb<8, NQ>;
+    case 12: return b_transport_azimuthal_rb<12, NQ>;
+    case 16: return b_transport_azimuthal_rb<16, NQ>;
+    default: return nullptr;
+    }
+}
+static AzRbFn az_rb_fn(int per, int nq) { return nq == 5 ? az_rb_fn_nq<5>(per) : az_rb_fn_nq<4>(per); }
+
 // the window azimuthal pass (azimuthal_window): one window per warp, windows
 // of all disks' rings in one grid-stride sequence
 template <int NQ>
@@ -662,9 +701,16 @@ struct fgpu_batch {
     int grid[FGPU_BK_COUNT] = {};
     int az_per = 0;
     size_t az_smem = 0;
-    // the window pass, or with FARGO_GB300_AZIMUTHAL=strided the strided ring
-    // pass
+    // the window pass, or the ring pass that FARGO_GB300_AZIMUTHAL asked for: with
+    // blocked<PER> the disks grouped by ring length and quantity count (one launch
+    // per group), else the strided pass
     bool windows = true;
+    struct RbGroup {
+        int nz, nq, per, grid;
+        size_t smem;
+    };
+    std::vector<RbGroup> rb;
+    int *d_rb_tables = nullptr;  // rb.size() tables of nd + 1 tile starts
 
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
@@ -886,6 +932,12 @@ static void launch_kernel(fgpu_batch *b, int k, int ghost_b = 0)
         if (b->windows) {
             if (b->any_iso) fgpu::launch(b_transport_azimuthal_w<4>, g, th, 0, s, D, S, b->table(k), nd);
             if (b->any_adi) fgpu::launch(b_transport_azimuthal_w<5>, g, th, 0, s, D, S, b->table(k), nd);
+        } else if (!b->rb.empty()) {
+            for (size_t q = 0; q < b->rb.size(); ++q) {
+                const fgpu_batch::RbGroup &grp = b->rb[q];
+                az_rb_fn(grp.per, grp.nq)<<<grp.grid, grp.nz / grp.per, grp.smem, s>>>(
+                    D, S, b->d_rb_tables + q * (size_t)(nd + 1), nd);
+            }
         } else {
             if (b->any_iso) az_fn(b->az_per, 4)<<<g, th, b->az_smem, s>>>(D, S, b->table(k), nd);
             if (b->any_adi) az_fn(b->az_per, 5)<<<g, th, b->az_smem, s>>>(D, S, b->table(k), nd);
@@ -975,6 +1027,7 @@ static void release(fgpu_batch *b)
     cudaFree(b->d_seq_tables);
     cudaFree(b->d_seq_err);
     cudaFree(b->d_damp_items);
+    cudaFree(b->d_rb_tables);
     if (b->h_steps) cudaFreeHost(b->h_steps);
     if (b->h_clocks) cudaFreeHost(b->h_clocks);
     if (b->h_active) cudaFreeHost(b->h_active);
@@ -1094,6 +1147,41 @@ extern "C" int fgpu_batch_create(int n, const fgpu_params *params, const double 
     if (!damp.empty()) {
         CKC(cudaMalloc(&b->d_damp_items, sizeof(int2) * damp.size()));
         CKC(cudaMemcpy(b->d_damp_items, damp.data(), sizeof(int2) * damp.size(),
+                       cudaMemcpyHostToDevice));
+    }
+    // (every disk read the same request)
+    if (b->disks[0]->blocked_pass()) {
+        const int per = b->disks[0]->blocked_pass();
+        for (int d = 0; d < n; ++d) {
+            bool found = false;
+            for (auto &g : b->rb) found = found || (g.nz == b->nz[d] && g.nq == desc[d].nq);
+            if (!found)
+                b->rb.push_back({b->nz[d], desc[d].nq, per, 1,
+                                 rb_smem_floats(b->nz[d], desc[d].nq, b->nz[d] / per) *
+                                     sizeof(float)});
+        }
+        std::vector<int> h(b->rb.size() * (size_t)(n + 1), 0);
+        for (size_t q = 0; q < b->rb.size(); ++q) {
+            fgpu_batch::RbGroup &g = b->rb[q];
+            int *st = h.data() + q * (size_t)(n + 1);
+            long long acc = 0;
+            for (int d = 0; d < n; ++d) {
+                st[d] = (int)acc;
+                if (b->nz[d] == g.nz && desc[d].nq == g.nq) acc += b->nr[d];
+            }
+            st[n] = (int)acc;
+            const void *fn = (const void *)az_rb_fn(per, g.nq);
+            CKC(raise_smem_limit(fn, g.smem));
+            int per_sm = 0;
+            CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, g.nz / per, g.smem));
+            if (per_sm < 1) {
+                b->err = "the register-blocked ring pass cannot run on this device";
+                return fail(FGPU_ERR_UNSUPPORTED);
+            }
+            g.grid = (int)std::max(1LL, std::min((long long)per_sm * b->nsm, acc));
+        }
+        CKC(cudaMalloc(&b->d_rb_tables, sizeof(int) * h.size()));
+        CKC(cudaMemcpy(b->d_rb_tables, h.data(), sizeof(int) * h.size(),
                        cudaMemcpyHostToDevice));
     }
 #undef CKC

@@ -235,6 +235,8 @@ class Engine32 {
     int rings() const { return nr; }
     int azimuthal() const { return nz; }
     bool window_pass() const { return windows; }
+    // cells per thread of the register-blocked ring pass, if it was asked for (else 0)
+    int blocked_pass() const { return rb_per; }
     const int *damping_rings(int *n) const
     {
         *n = (p.damping && n_rings) ? n_rings : 0;

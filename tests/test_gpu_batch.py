@@ -347,3 +347,48 @@ def test_persistent_substep_sequences_give_the_same_bits():
         for k in range(len(out[0])):
             for f in EVOLVED:
                 assert np.array_equal(out[0][k][f], out[1][k][f]), (k, f)
+
+
+@pytest.mark.parametrize("per", [4, 12])
+def test_blocked_ring_pass_in_a_batch(monkeypatch, per):
+    """FARGO_GB300_AZIMUTHAL=blocked<PER> in a batch (the register-blocked ring pass
+    over groups of disks of one ring length and equation of state): the window
+    pass's bits, by the host's clock and by the device's in graphs; a ring it does
+    not fit refuses the batch."""
+    from fargocpt_gb300.batch import Batch, start_disks
+    from fargocpt_gb300.engine import EngineError
+    from fargocpt_gb300 import setups
+
+    disks = []
+    for n, (nr, nz, adiabatic) in enumerate([(20, 384, True), (13, 768, False),
+                                             (16, 384, False)]):
+        p, d = make_params(nr, nz, adiabatic, precision=1)
+        radii = setups.log_radii(nr, 0.4, 2.5)
+        disks.append((p, radii, initial_state(d, radii, seed=n)))
+    study = setups.sweep(n_disks=3, seed=13, nr_choices=(128, 256))
+    out = []
+    for variant in (f"blocked{per}", None):
+        if variant:
+            monkeypatch.setenv("FARGO_GB300_AZIMUTHAL", variant)
+        else:
+            monkeypatch.delenv("FARGO_GB300_AZIMUTHAL", raising=False)
+        b = Batch([p for p, *_ in disks], [r for _, r, _ in disks])
+        for be, (_, _, st) in zip(b.disks, disks):
+            _load(be, st, _bodies(0.0))
+        dts = np.array([0.2 * be.condition_cfl() for be in b.disks])
+        for _ in range(3):
+            b.step(dts, np.zeros(len(disks)))
+        fields = [{f: e.get_field(f) for f in EVOLVED} for e in b.disks]
+        b.close()
+        b = Batch([x[0] for x in study], [x[2] for x in study])
+        start_disks(b, study, t_end=1.0, monitor_dt=0.1)
+        b.run(6, steps_per_graph=3)
+        out.append(fields + [{f: e.get_field(f) for f in EVOLVED} for e in b.disks])
+        b.close()
+    for k, (a, c) in enumerate(zip(*out)):
+        for f in EVOLVED:
+            assert np.array_equal(a[f], c[f]), (k, f)
+    monkeypatch.setenv("FARGO_GB300_AZIMUTHAL", f"blocked{per}")
+    p, _ = make_params(16, 386, precision=1)
+    with pytest.raises(EngineError, match="UNSUPPORTED"):
+        Batch([disks[0][0], p], [disks[0][1], setups.log_radii(16, 0.4, 2.5)])
