@@ -9,10 +9,10 @@
 // Fast2Sum (Dekker 1971) and TwoProduct by fused multiply-add, combined as in
 // Joldes, Muller and Popescu, "Tight and rigorous error bounds for basic
 // building blocks of double-word arithmetic" (ACM TOMS 44, 2017): the sum of
-// two pairs (their algorithm 6, relative error below 3 u^2, u = 2^-24), the
-// product of two pairs (algorithm 12, below 5 u^2) and of a pair and a float
-// (algorithm 9).  Every operation is spelled with the round-to-nearest
-// intrinsics so that the compiler neither contracts nor reorders them.
+// two pairs (their algorithm 6, relative error below 3 u^2, u = 2^-24) and the
+// product of two pairs (algorithm 12, below 5 u^2).  Every operation is spelled
+// with the round-to-nearest intrinsics so that the compiler neither contracts nor
+// reorders them.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -59,12 +59,6 @@ __device__ __forceinline__ f2 f2_mul(f2 x, f2 y)
     const float t = __fmaf_rn(x.h, y.l, __fmul_rn(x.l, y.l));
     return fast_two_sum(c.h, __fadd_rn(c.l, __fmaf_rn(x.l, y.h, t)));
 }
-__device__ __forceinline__ f2 f2_mul_f(f2 x, float y)
-{
-    const f2 c = two_prod(x.h, y);
-    return fast_two_sum(c.h, __fmaf_rn(x.l, y, c.l));
-}
-
 // 1 / sqrt(d) for d > 0: the hardware estimate, one FP32 Newton step, then
 // one Newton step whose residual 1 - d r^2 is formed in pair arithmetic; the
 // result is within a few units of 2^-46 of the exact value
@@ -149,7 +143,7 @@ __device__ __forceinline__ double f2_to_double(f2 a)
 // to the operands' magnitudes (the pair representation itself carries 2^-48
 // of each value): the sloppy sum (Joldes, Muller and Popescu, algorithm 5),
 // absolute error within a few 2^-48 (|x| + |y|); the product without the
-// low-by-low term; quotient and reciprocal from the hardware reciprocal
+// low-by-low term; the quotient from the hardware reciprocal
 // estimate (rcp.approx, within 2^-22) with one correction in pair
 // arithmetic, relative error within a few 2^-46.
 // ---------------------------------------------------------------------------
@@ -187,15 +181,6 @@ __device__ __forceinline__ float rsqrt_approx(float x)
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
-}
-
-// 1 / d for a normal d: r = rcp(d.h), then r + r (1 - d r)
-__device__ __forceinline__ f2 f2_rcp(f2 d)
-{
-    const float r = rcp_approx(d.h);
-    const f2 p = f2_mul_f(d, r);  // about 1
-    const float e = __fsub_rn(__fsub_rn(1.0f, p.h), p.l);
-    return fast_two_sum(r, __fmul_rn(r, e));
 }
 
 // sqrt(x) for x > 0: x rsqrt(x)

@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kForceThreads32, 8)
     }
 }
 
-// the rows' components, one block (one warp) per component
+// the rows' components, one block per component
 __global__ void f_reduce_cols(const double *__restrict__ partial, int rows, int width,
                               double *__restrict__ out)
 {
@@ -429,11 +429,6 @@ __global__ void f_reduce_cols(const double *__restrict__ partial, int rows, int 
 }
 
 // one warp per component
-__global__ void f_reduce_rows(const double *__restrict__ partial, int rows, double *__restrict__ out)
-{
-    const int w = threadIdx.x >> 5;
-    if (w < 5) warp_compensated_rows(partial, rows, 5, w, out);
-}
 __global__ void f_reduce_rows2(const double *__restrict__ partial, int rows, double *__restrict__ out)
 {
     const int w = threadIdx.x >> 5;
@@ -926,7 +921,7 @@ int Engine32::create(const fgpu_params &prm, const double *radii, cudaStream_t s
         if (want.rfind("blocked", 0) == 0) {
             const int pc = atoi(want.c_str() + 7);
             if ((pc == 4 || pc == 8 || pc == 12 || pc == 16) &&
-                rb_fits(nz, nq, pc, 1, kMaxRingSmem)) {
+                rb_fits(nz, nq, pc, kMaxRingSmem)) {
                 rb_per = pc;
                 windows = false;
             } else {
