@@ -50,6 +50,8 @@ struct fgpu_engine {
     int az_block = 256;
     double *ring_mean = nullptr;    // pair form: mean v_phi per ring, for the CFL kernel
     unsigned *cfl_done = nullptr;   // blocks of the CFL kernel that have finished
+    bool dt_arrived = false;        // the last CFL step has reached h_pinned[kHostDt]
+    bool captured = false;          // a graph may launch the CFL kernel without a call here
     bool pair_arith = true;  // the kernels' arithmetic in float pairs (else FP64)
     // div v and the stress tensor hold the stress kernel's float pairs
     // (stress_as_pairs), the artificial pressures those of the float-pair
@@ -1411,8 +1413,14 @@ extern "C" int fgpu_condition_cfl(fgpu_engine *eng, double *dt_out)
         if (rc) return rc;
         eng->cfl_valid = true;
     }
-    // the step is written to the host by the kernel that formed it
-    CK(cudaStreamSynchronize(eng->stream));
+    // the step is written to the host by the kernel that formed it; a call that
+    // waited for the stream since then has already brought it, unless a graph
+    // formed another (a wait for the idle stream takes 1.5 us, of 100 a small
+    // disk's step takes)
+    if (!eng->dt_arrived || eng->captured) {
+        CK(cudaStreamSynchronize(eng->stream));
+        eng->dt_arrived = true;
+    }
     *dt_out = eng->h_pinned[kHostDt];
     return FGPU_OK;
 }
@@ -1450,6 +1458,14 @@ static void derived_cfl(fgpu_engine *eng, const Launch &L, int mode)
         if (cfl)
             cudaMemcpyAsync(eng->h_pinned + kHostDt, eng->d_dtmin, sizeof(double),
                             cudaMemcpyDeviceToHost, eng->stream);
+    }
+    if (cfl) {
+        eng->dt_arrived = false;
+        if (!eng->captured) {
+            cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+            eng->captured = cudaStreamIsCapturing(eng->stream, &status) != cudaSuccess ||
+                            status != cudaStreamCaptureStatusNone;
+        }
     }
 }
 
@@ -1849,6 +1865,7 @@ extern "C" int fgpu_disk_on_planet_accel(fgpu_engine *eng, int k, double accel[2
     int rc = check_launch(eng);
     if (rc) return rc;
     CK(cudaStreamSynchronize(eng->stream));
+    eng->dt_arrived = true;
     accel[0] = eng->h_pinned[0] + eng->h_pinned[2];
     accel[1] = eng->h_pinned[1] + eng->h_pinned[3];
     return FGPU_OK;
@@ -1878,6 +1895,7 @@ extern "C" int fgpu_disk_on_nbody_accel(fgpu_engine *eng, double *accel)
         int rc = check_launch(eng);
         if (rc) return rc;
         CK(cudaStreamSynchronize(eng->stream));
+        eng->dt_arrived = true;
         std::copy(eng->h_pinned + 16, eng->h_pinned + 16 + 5 * n, sums);
     }
     for (int k = 0; k < n; ++k) {
