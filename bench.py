@@ -49,9 +49,9 @@ KERNEL_BYTES_PER_CELL = {
 }
 # the float-pair FP64 form's fused kernels: the potential with the source terms,
 # the artificial pressures with their velocity update, the stress tensor with the
-# viscous update; the window azimuthal pass does not read v_phi
+# viscous update
 KERNEL_BYTES_PER_CELL_FP64 = dict(KERNEL_BYTES_PER_CELL, potential=0, source=64, artvisc_q=0,
-                                  artvisc_v=96, stress=0, transport_azimuthal=96)
+                                  artvisc_v=96, stress=0)
 STEP_BYTES_PER_CELL = {"adiabatic": 64, "isothermal": 48}   # one read + write of the state
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant
 # kernels from one-kernel ncu captures (profiles/ names the capture of each)

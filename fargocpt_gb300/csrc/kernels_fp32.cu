@@ -14,8 +14,9 @@
 // tau_r_phi (viscosity.cpp:201-207), the Keplerian angular momentum carried
 // by the radial mass flux (TransportEuler.cpp:545-591) -- become per-ring
 // constants computed once in FP64 on the host.  FP64 remains for the FARGO
-// shift phase of every ring, the cell-to-body separations (potential and disk
-// force), and the accumulation of the force and mass reductions.
+// shift phase of every ring, a central object off the origin, and the force and
+// mass sums beyond a warp; separations from bodies and the sums within a warp are
+// float pairs.
 //
 // The step has the same phases and order as the FP64 form (kernels_fp64.cu)
 // and FargoCPT's step_Euler (simulation.cpp:148-267).  The per-cell, per-column
@@ -165,9 +166,9 @@ __global__ void __launch_bounds__(64, 16) f_transport_radial(GeoF g, TablesF t, 
     fgpu::follow_predecessor();
     // the first rows of blocks form the ring phases of the window azimuthal
     // pass, a warp per ring: latency-bound sums that the sweep's blocks behind
-    // them overlap (2048 x 6144: 0.300 ms, the sweep alone 0.295; as a launch
-    // of their own 0.335; with block reductions, whose shared memory comes off
-    // the sweep's L1, 0.345)
+    // them overlap (2048 x 6144, with a sweep that took 0.295 ms alone: 0.300; as
+    // a launch of their own 0.335; with block reductions, whose shared memory comes
+    // off the sweep's L1, 0.345.  Now, the sweep asking L2 ahead, 0.277 together)
     if ((int)blockIdx.y < phase_rows) {
         const int i = (blockIdx.y * gridDim.x + blockIdx.x) * 2 + (threadIdx.x >> 5);
         if (i < g.nr) ring_phase_f(g, t, dt_d, dv, i, phase, ring_shift);

@@ -3,7 +3,7 @@
 // device once every block of its predecessor has started, and its blocks wait
 // in follow_predecessor() until the predecessor has completed and its writes are
 // visible.  What is hidden is the launch itself, about 2 us, which a small disk
-// pays for each of its thirteen kernels.  Every kernel launched this way must
+// pays for each of its ten kernels and the disk force's two.  Every kernel launched this way must
 // call follow_predecessor() before anything else, so that completion stays
 // transitive along the stream.
 #pragma once

@@ -412,7 +412,11 @@ int fgpu_synchronize(fgpu_engine *eng);
  * stream.  fgpu_phase_times waits for the recorded steps, writes the summed
  * milliseconds of each phase into ms[0 .. count-1] (count = number of
  * phases, at most capacity), the number of steps into *steps, and clears the
- * record.  fgpu_phase_name(k) names phase k. */
+ * record.  fgpu_phase_name(k) names phase k.  In the FP64 form with float-pair
+ * arithmetic one kernel may serve two phases; its time is then the second one's
+ * and the first reads about zero: "source" includes "potential" (a central object
+ * at the origin without smoothing), "artvisc_v" includes "artvisc_q", and
+ * "viscous_substep3" includes "stress" (but with StabilizeViscosity 1). */
 int fgpu_set_phase_timing(fgpu_engine *eng, int enable);
 int fgpu_phase_times(fgpu_engine *eng, double *ms, int capacity, int *count,
 		     int *steps);
